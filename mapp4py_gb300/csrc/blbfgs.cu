@@ -21,7 +21,7 @@
 #include <algorithm>
 #include <vector>
 
-#include "system.h"
+#include "eam_common.cuh"
 
 namespace mappg {
 
@@ -80,22 +80,26 @@ __device__ __forceinline__ int slot_of(const BlCell& c, int i, int m) { return (
 // block sums (K <= 4) of one chunk into part[ch][0..K-1]; op 1 = max
 template <int K>
 __device__ __forceinline__ void bl_store(const double (&v)[K], const int (&op)[K], double* out) {
-    __shared__ double red[8][4];
+    __shared__ unsigned long long redm[8][K];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    // maxima of non-negative values as integers, sums together
+    double u[K];
 #pragma unroll
     for (int k = 0; k < K; k++) {
-        double t = v[k];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const double u = __shfl_xor_sync(0xffffffffu, t, o);
-            t = op[k] ? fmax(t, u) : t + u;
+        u[k] = op[k] ? 0.0 : v[k];
+        if (op[k]) {
+            unsigned long long m[1] = {(unsigned long long)__double_as_longlong(v[k])};
+            const unsigned long long t = warp_reduce(m, RedMaxBits());
+            if (lane == 0) redm[w][k] = t;
         }
-        if (lane == 0) red[w][k] = t;
     }
-    __syncthreads();
+    double t = block_sums<K>(u);
     if (threadIdx.x < K) {
-        double t = 0.0;
-        for (int q = 0; q < nw; q++) t = op[threadIdx.x] ? fmax(t, red[q][threadIdx.x]) : t + red[q][threadIdx.x];
+        if (op[threadIdx.x]) {
+            unsigned long long m = 0;
+            for (int q = 0; q < nw; q++) m = RedMaxBits()(m, redm[q][threadIdx.x]);
+            t = __longlong_as_double((long long)m);
+        }
         out[threadIdx.x] = t;
     }
     __syncthreads();

@@ -234,8 +234,15 @@ __global__ void __launch_bounds__(256) k_density64(EamArgs a) {
             eacc += Fv;
         }
     }
-    double v[1] = {eacc};
-    if (block_partials<1>(v, a.partials, 15, &a.sc->counter[1]) && threadIdx.x == 0) a.sc->counter[1] = 0;
+    const double v[1] = {eacc};
+    __shared__ double tot[1];
+    if (block_partials<1>(v, a.partials, 0, &a.sc->counter[1])) {
+        final_sums<1>(a.partials, gridDim.x, tot);
+        if (threadIdx.x == 0) {
+            a.sc->e_embed = tot[0];
+            a.sc->counter[1] = 0;
+        }
+    }
 }
 
 // batch: FP64 density per chunk, embedding energy into chunk slot 13
@@ -270,7 +277,8 @@ __global__ void __launch_bounds__(256) k_density64b(EamArgs a, const int* __rest
                 eacc += Fv;
             }
         }
-        chunk_store<1>([&](int) { return eacc; }, a.chunk_part + (size_t)ch * kChunkSlots + 13);
+        const double v[1] = {eacc};
+        chunk_store<1>(v, a.chunk_part + (size_t)ch * kChunkSlots + 13);
     }
 }
 
@@ -306,15 +314,15 @@ __global__ void __launch_bounds__(256) k_force64(EamArgs a) {
             a.f[2 * a.n + i] = fz;
         }
     }
-    double v[7] = {0.5 * ep, 0.5 * w[0], 0.5 * w[1], 0.5 * w[2], 0.5 * w[3], 0.5 * w[4], 0.5 * w[5]};
-    if (block_partials<7>(v, a.partials, 0, &a.sc->counter[0]) && threadIdx.x < 32) {
-        // totals over blocks in a fixed order; slot 15 holds the embedding
-        // energy written by the density kernel on the same grid
-        double tot[16];
-        final_sums<16>(a.partials, gridDim.x, tot);
+    const double v[7] = {ep, w[0], w[1], w[2], w[3], w[4], w[5]};
+    __shared__ double tot[7];
+    if (block_partials<7>(v, a.partials, 0, &a.sc->counter[0])) {
+        // totals over blocks in a fixed order, and the density pass's
+        // embedding energy
+        final_sums<7>(a.partials, gridDim.x, tot);
         if (threadIdx.x == 0) {
-            a.sc->energy = tot[0] + tot[15];
-            for (int k = 0; k < 6; k++) a.sc->virial[k] = tot[k + 1];
+            a.sc->energy = 0.5 * tot[0] + a.sc->e_embed;
+            for (int k = 0; k < 6; k++) a.sc->virial[k] = 0.5 * tot[k + 1];
             a.sc->counter[0] = 0;
         }
     }
@@ -354,7 +362,8 @@ __global__ void __launch_bounds__(256) k_force64b(EamArgs a, const int* __restri
                 a.f[2 * a.n + i] = fz;
             }
         }
-        chunk_store<7>([&](int k) { return 0.5 * (k == 0 ? ep : w[k - 1]); }, a.chunk_part + (size_t)ch * kChunkSlots);
+        const double v[7] = {0.5 * ep, 0.5 * w[0], 0.5 * w[1], 0.5 * w[2], 0.5 * w[3], 0.5 * w[4], 0.5 * w[5]};
+        chunk_store<7>(v, a.chunk_part + (size_t)ch * kChunkSlots);
     }
 }
 
@@ -480,9 +489,9 @@ __global__ void __launch_bounds__(256) k_energy64(EamArgs a) {
             eacc += Fv;
         }
     }
-    double v[1] = {eacc + 0.5 * ep};
-    if (block_partials<1>(v, a.partials, 0, &a.sc->counter[2]) && threadIdx.x < 32) {
-        double tot[1];
+    const double v[1] = {eacc + 0.5 * ep};
+    __shared__ double tot[1];
+    if (block_partials<1>(v, a.partials, 0, &a.sc->counter[2])) {
         final_sums<1>(a.partials, gridDim.x, tot);
         if (threadIdx.x == 0) {
             a.sc->energy = tot[0];
@@ -537,7 +546,8 @@ __global__ void __launch_bounds__(256) k_energy64b(EamArgs a, const int* __restr
                 eacc += Fv;
             }
         }
-        chunk_store<1>([&](int) { return eacc + 0.5 * ep; }, a.chunk_part + (size_t)ch * kChunkSlots);
+        const double v[1] = {eacc + 0.5 * ep};
+        chunk_store<1>(v, a.chunk_part + (size_t)ch * kChunkSlots);
     }
 }
 
@@ -556,6 +566,11 @@ static int grid64(mappg_sys* s) {
 
 void launch_cells_done(mappg_sys* s, const EamArgs& a, int what);  // eam32.cu
 
+// FP64 batch passes take a block per chunk: a chunk is 50-100 us of FP64
+// work, so the hardware's own assignment of blocks to free SMs beats a fixed
+// share of the chunks per block (10 relaxation steps of 64 cells with 128-atom
+// chunks: 48.5 -> 47.9 ms)
+
 void launch_density_only(mappg_sys* s) {
     EamArgs a = eam_args(s);
     if (s->precision == MAPPG_MIXED && !s->force64) {
@@ -563,7 +578,7 @@ void launch_density_only(mappg_sys* s) {
         return;
     }
     if (s->ncell > 1) {
-        k_density64b<8><<<std::min(s->nchunk, s->sm_count * 8), 256, 0, s->stream>>>(a, s->cell_of);
+        k_density64b<8><<<s->nchunk, 256, 0, s->stream>>>(a, s->cell_of);
     } else {
         MAPPG_TPA64(k_density64)
     }
@@ -600,7 +615,7 @@ void launch_force_only(mappg_sys* s) {
         return;
     }
     if (s->ncell > 1) {
-        k_force64b<8><<<std::min(s->nchunk, s->sm_count * 8), 256, 0, s->stream>>>(a, s->cell_of);
+        k_force64b<8><<<s->nchunk, 256, 0, s->stream>>>(a, s->cell_of);
         MAPPG_CUDA(cudaGetLastError());
         launch_cells_done(s, a, 0);
     } else {
@@ -654,7 +669,7 @@ void preload_force64() {
 void launch_energy64(mappg_sys* s) {
     EamArgs a = eam_args(s);
     if (s->ncell > 1) {
-        k_energy64b<8><<<std::min(s->nchunk, s->sm_count * 8), 256, 0, s->stream>>>(a, s->cell_of);
+        k_energy64b<8><<<s->nchunk, 256, 0, s->stream>>>(a, s->cell_of);
         MAPPG_CUDA(cudaGetLastError());
         launch_cells_done(s, a, 1);
         return;

@@ -43,11 +43,8 @@
 namespace mappg {
 
 struct Smem32 {
-    float4 off[27];
     float cut_sq[kMaxElem * kMaxElem];
     __device__ void fill(const EamArgs& a) {
-        for (int t = threadIdx.x; t < 27; t += blockDim.x)
-            off[t] = make_float4(a.fr.off[t][0], a.fr.off[t][1], a.fr.off[t][2], 0.f);
         for (int t = threadIdx.x; t < a.ne * a.ne; t += blockDim.x) cut_sq[t] = (float)a.cut_sq[t];
         __syncthreads();
     }
@@ -119,13 +116,6 @@ struct Consts32 {
         dri_lo = (float)(a.dr_inv - (double)dri);
     }
 };
-
-// s + e == a + b exactly (Knuth's two-sum)
-__device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
-    s = a + b;
-    const float bb = s - a;
-    e = (a - (s - bb)) + (b - bb);
-}
 
 // a lane's compensated partial (s, c), whose value is s - c, summed over the
 // TPA lanes of one atom: the rounding error of every addition goes into the
@@ -208,7 +198,9 @@ __device__ __forceinline__ void embed32f(const EamArgs& a, int ei, float s, floa
     Fv = cc.x + (__ldg(a.F32lo + k) + fr * fmaf(fmaf(cc.w, fr, cc.z), fr, cc.y));
 }
 
-// per-kernel persistent grid: as many blocks as fit on the GPU at once
+// per-kernel persistent grid: as many blocks as fit on the GPU at once (the
+// launches take no more than the atoms need: idle blocks of a small system
+// would still pay for the block sums)
 template <class Kern>
 static int occupancy_grid(mappg_sys* s, Kern k, int block) {
     int per_sm = 0;
@@ -218,6 +210,9 @@ static int occupancy_grid(mappg_sys* s, Kern k, int block) {
     if (g > kMaxBlocks) g = kMaxBlocks;
     return (int)g;
 }
+
+// blocks of 256 threads for TPA lanes an atom
+static int atom_blocks(const mappg_sys* s, int tpa) { return (int)(((long long)s->n * tpa + 255) / 256); }
 
 // frame of a batch cell (the G head/tail of CellGeo), read once per chunk
 struct CellFrame {
@@ -327,9 +322,9 @@ __global__ void __launch_bounds__(256) k_density32(EamArgs a) {
         if (!__any_sync(0xffffffffu, active)) break;
         density_atom<TPA, ORTHO, U>(a, S, K, a.fr, i, lane, active, es, ec);
     }
-    double v[1] = {(double)es - (double)ec};
-    if (block_partials<1>(v, a.partials, 0, &a.sc->counter[1]) && threadIdx.x < 32) {
-        double tot[1];
+    const Pair32 v[1] = {{es, -ec}};
+    __shared__ double tot[1];
+    if (block_partials<1>(v, a.partials, 0, &a.sc->counter[1])) {
         final_sums<1>(a.partials, gridDim.x, tot);
         if (threadIdx.x == 0) {
             a.sc->e_embed = tot[0];
@@ -364,9 +359,9 @@ __global__ void __launch_bounds__(1024, 1) k_density32s(EamArgs a) {
         if (!__any_sync(0xffffffffu, active)) break;
         density_atom<TPA, ORTHO, U, Frame, true>(a, S, K, a.fr, i, lane, active, es, ec, stab);
     }
-    double v[1] = {(double)es - (double)ec};
-    if (block_partials<1>(v, a.partials, 0, &a.sc->counter[1]) && threadIdx.x < 32) {
-        double tot[1];
+    const Pair32 v[1] = {{es, -ec}};
+    __shared__ double tot[1];
+    if (block_partials<1>(v, a.partials, 0, &a.sc->counter[1])) {
         final_sums<1>(a.partials, gridDim.x, tot);
         if (threadIdx.x == 0) {
             a.sc->e_embed = tot[0];
@@ -392,7 +387,8 @@ __global__ void __launch_bounds__(256) k_density32b(EamArgs a) {
             const int i = i0 + (int)threadIdx.x / TPA;
             density_atom<TPA, ORTHO, U>(a, S, K, fr, i, lane, i < hi, es, ec);
         }
-        chunk_store<1>([&](int) { return (double)es - (double)ec; }, a.chunk_part + (size_t)ch * kChunkSlots + 13);
+        const Pair32 v[1] = {{es, -ec}};
+        chunk_store<1>(v, a.chunk_part + (size_t)ch * kChunkSlots + 13);
     }
 }
 
@@ -548,16 +544,14 @@ __global__ void __launch_bounds__(256, 4) k_force32(EamArgs a) {
         if (!__any_sync(0xffffffffu, active)) break;
         force_atom<TPA, ORTHO, U>(a, S, K, a.fr, i, lane, active, es, ec, w);
     }
-    auto sum_k = [&](int k) -> double {
-        return k == 0 ? 0.5 * ((double)es - (double)ec) : 0.5 * (double)w[k - 1];
-    };
+    const Pair32 v[7] = {{es, -ec}, {w[0], 0.f}, {w[1], 0.f}, {w[2], 0.f}, {w[3], 0.f}, {w[4], 0.f}, {w[5], 0.f}};
     __shared__ double tot[7];
-    if (block_partials_fn<7>(sum_k, a.partials, 0, &a.sc->counter[0]) && threadIdx.x < 32) {
-        final_sums_smem<7>(a.partials, gridDim.x, tot);
+    if (block_partials<7>(v, a.partials, 0, &a.sc->counter[0])) {
+        final_sums<7>(a.partials, gridDim.x, tot);
         if (threadIdx.x == 0) {
             DevScalars* sc = a.sc;
-            sc->energy = tot[0] + sc->e_embed;
-            for (int k = 0; k < 6; k++) sc->virial[k] = tot[k + 1];
+            sc->energy = 0.5 * tot[0] + sc->e_embed;  // each pair stands in both rows
+            for (int k = 0; k < 6; k++) sc->virial[k] = 0.5 * tot[k + 1];
             sc->counter[0] = 0;
         }
     }
@@ -598,16 +592,14 @@ __global__ void __launch_bounds__(1024, 1) k_force32s(EamArgs a) {
             force_atom<TPA, ORTHO, U, Frame, true>(a, S, K, a.fr, i, lane, active, es, ec, w, ftab_s);
         }
     }
-    auto sum_k = [&](int k) -> double {
-        return k == 0 ? 0.5 * ((double)es - (double)ec) : 0.5 * (double)w[k - 1];
-    };
+    const Pair32 v[7] = {{es, -ec}, {w[0], 0.f}, {w[1], 0.f}, {w[2], 0.f}, {w[3], 0.f}, {w[4], 0.f}, {w[5], 0.f}};
     __shared__ double tot[7];
-    if (block_partials_fn<7>(sum_k, a.partials, 0, &a.sc->counter[0]) && threadIdx.x < 32) {
-        final_sums_smem<7>(a.partials, gridDim.x, tot);
+    if (block_partials<7>(v, a.partials, 0, &a.sc->counter[0])) {
+        final_sums<7>(a.partials, gridDim.x, tot);
         if (threadIdx.x == 0) {
             DevScalars* sc = a.sc;
-            sc->energy = tot[0] + sc->e_embed;
-            for (int k = 0; k < 6; k++) sc->virial[k] = tot[k + 1];
+            sc->energy = 0.5 * tot[0] + sc->e_embed;  // each pair stands in both rows
+            for (int k = 0; k < 6; k++) sc->virial[k] = 0.5 * tot[k + 1];
             sc->counter[0] = 0;
         }
     }
@@ -659,11 +651,10 @@ __global__ void __launch_bounds__(256, 4) k_force32b(EamArgs a) {
             const int i = i0 + (int)threadIdx.x / TPA;
             force_atom<TPA, ORTHO, U>(a, S, K, fr, i, lane, i < hi, es, ec, w);
         }
-        chunk_store<7>(
-            [&](int k) -> double {
-                return k == 0 ? 0.5 * ((double)es - (double)ec) : 0.5 * (double)w[k - 1];
-            },
-            a.chunk_part + (size_t)ch * kChunkSlots);
+        // halves, as each pair stands in both rows (exact)
+        const Pair32 v[7] = {{0.5f * es, -0.5f * ec}, {0.5f * w[0], 0.f}, {0.5f * w[1], 0.f}, {0.5f * w[2], 0.f},
+                             {0.5f * w[3], 0.f},      {0.5f * w[4], 0.f}, {0.5f * w[5], 0.f}};
+        chunk_store<7>(v, a.chunk_part + (size_t)ch * kChunkSlots);
     }
 }
 
@@ -730,9 +721,9 @@ __global__ void __launch_bounds__(256) k_energy32(EamArgs a) {
         if (!__any_sync(0xffffffffu, active)) break;
         energy_atom<TPA, ORTHO>(a, S, K, a.fr, i, lane, active, es, ec);
     }
-    double v[1] = {(double)es - (double)ec};
-    if (block_partials<1>(v, a.partials, 0, &a.sc->counter[2]) && threadIdx.x < 32) {
-        double tot[1];
+    const Pair32 v[1] = {{es, -ec}};
+    __shared__ double tot[1];
+    if (block_partials<1>(v, a.partials, 0, &a.sc->counter[2])) {
         final_sums<1>(a.partials, gridDim.x, tot);
         if (threadIdx.x == 0) {
             a.sc->energy = tot[0];
@@ -758,7 +749,8 @@ __global__ void __launch_bounds__(256) k_energy32b(EamArgs a) {
             const int i = i0 + (int)threadIdx.x / TPA;
             energy_atom<TPA, ORTHO>(a, S, K, fr, i, lane, i < hi, es, ec);
         }
-        chunk_store<1>([&](int) { return (double)es - (double)ec; }, a.chunk_part + (size_t)ch * kChunkSlots);
+        const Pair32 v[1] = {{es, -ec}};
+        chunk_store<1>(v, a.chunk_part + (size_t)ch * kChunkSlots);
     }
 }
 
@@ -928,9 +920,9 @@ __global__ void __launch_bounds__(256) k_de32(EamArgs a) {
         if (!__any_sync(0xffffffffu, active)) break;
         de_atom<TPA, ORTHO>(a, S, K, a.fr, i, lane, active, alpha, es, ec);
     }
-    double v[1] = {(double)es - (double)ec};
-    if (block_partials<1>(v, a.partials, 0, &a.sc->counter[6]) && threadIdx.x < 32) {
-        double tot[1];
+    const Pair32 v[1] = {{es, -ec}};
+    __shared__ double tot[1];
+    if (block_partials<1>(v, a.partials, 0, &a.sc->counter[6])) {
         final_sums<1>(a.partials, gridDim.x, tot);
         if (threadIdx.x == 0) {
             a.sc->de = tot[0];
@@ -959,7 +951,8 @@ __global__ void __launch_bounds__(256) k_de32b(EamArgs a) {
             const int i = i0 + (int)threadIdx.x / TPA;
             de_atom<TPA, ORTHO>(a, S, K, fr, i, lane, i < hi, alpha, es, ec);
         }
-        chunk_store<1>([&](int) { return (double)es - (double)ec; }, a.chunk_part + (size_t)ch * kChunkSlots);
+        const Pair32 v[1] = {{es, -ec}};
+        chunk_store<1>(v, a.chunk_part + (size_t)ch * kChunkSlots);
     }
 }
 
@@ -1017,6 +1010,12 @@ __global__ void k_cells_done(EamArgs a, const int* __restrict__ cell_chunk, Cell
 // loop step U); TPA and U come from the system (mappg_sys_autotune)
 template <int TPA, bool ORTHO, int U>
 static void density_t(mappg_sys* s, const EamArgs& a) {
+    if (s->n <= kDensSmallAtoms) {
+        static int grid = 0;
+        if (!grid) grid = occupancy_grid(s, k_density32<TPA, ORTHO, U>, 256);
+        k_density32<TPA, ORTHO, U><<<std::min(grid, atom_blocks(s, TPA)), 256, 0, s->stream>>>(a);
+        return;
+    }
     static bool attr = false;
     if (!attr) {
         MAPPG_CUDA(cudaFuncSetAttribute(k_density32s<TPA, ORTHO, U>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1042,21 +1041,21 @@ static void force_t(mappg_sys* s, const EamArgs& a) {
     }
     static int grid = 0;
     if (!grid) grid = occupancy_grid(s, k_force32<TPA, ORTHO, U>, 256);
-    k_force32<TPA, ORTHO, U><<<grid, 256, 0, s->stream>>>(a);
+    k_force32<TPA, ORTHO, U><<<std::min(grid, atom_blocks(s, TPA)), 256, 0, s->stream>>>(a);
 }
 
 template <int TPA, bool ORTHO, int U>
 static void energy_t(mappg_sys* s, const EamArgs& a) {
     static int grid = 0;
     if (!grid) grid = occupancy_grid(s, k_energy32<TPA, ORTHO>, 256);
-    k_energy32<TPA, ORTHO><<<grid, 256, 0, s->stream>>>(a);
+    k_energy32<TPA, ORTHO><<<std::min(grid, atom_blocks(s, TPA)), 256, 0, s->stream>>>(a);
 }
 
 template <int TPA, bool ORTHO, int U>
 static void de_t(mappg_sys* s, const EamArgs& a) {
     static int grid = 0;
     if (!grid) grid = occupancy_grid(s, k_de32<TPA, ORTHO>, 256);
-    k_de32<TPA, ORTHO><<<grid, 256, 0, s->stream>>>(a);
+    k_de32<TPA, ORTHO><<<std::min(grid, atom_blocks(s, TPA)), 256, 0, s->stream>>>(a);
 }
 
 template <int TPA, bool ORTHO, int U>

@@ -20,8 +20,8 @@
 #include <algorithm>
 #include <vector>
 
+#include "eam_common.cuh"
 #include "linesearch.h"
-#include "system.h"
 
 namespace mappg {
 
@@ -40,54 +40,7 @@ struct LbScal {
     unsigned long long dxbits;  // the same by k_lb_dxmax (bits of a non-negative double)
 };
 
-__device__ __forceinline__ void warp_sum(double& t) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-}
-
-template <int K>
-__device__ bool lb_block(double (&v)[K], double* partials, unsigned* counter, bool is_max = false) {
-    __shared__ double red[32][K];
-    __shared__ bool last;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-        double t = v[k];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            double u = __shfl_xor_sync(0xffffffffu, t, o);
-            t = is_max ? fmax(t, u) : t + u;
-        }
-        if (lane == 0) red[w][k] = t;
-    }
-    __syncthreads();
-    if (threadIdx.x < K) {
-        double t = is_max ? 0.0 : 0.0;
-        for (int q = 0; q < nw; q++) t = is_max ? fmax(t, red[q][threadIdx.x]) : t + red[q][threadIdx.x];
-        partials[blockIdx.x * kRedSlots + threadIdx.x] = t;
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
-    __syncthreads();
-    return last;
-}
-
-template <int K>
-__device__ void lb_final(const double* partials, int nblk, double (&tot)[K], bool is_max = false) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-        double t = 0.0;
-        for (int b = lane; b < nblk; b += 32) t = is_max ? fmax(t, partials[b * kRedSlots + k]) : t + partials[b * kRedSlots + k];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            double u = __shfl_xor_sync(0xffffffffu, t, o);
-            t = is_max ? fmax(t, u) : t + u;
-        }
-        tot[k] = t;
-    }
-}
+constexpr int kLbU = 4;  // components a thread of the vector kernels loads at a time
 
 // h <- h + coef*y, then dot = s.h (s may be null: no dot).  coef is read
 // from the device: mode 0: coef = 0 (plain dot); mode 1: alpha_i =
@@ -107,23 +60,41 @@ __global__ void __launch_bounds__(256) k_lb_axpy_dot(int N, double* __restrict__
     } else if (mode == 3) {
         coef = L->gamma;
     }
+    const double tau = mode == 4 ? L->tau : 0.0;
     double acc = 0.0;
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < N; q += gridDim.x * blockDim.x) {
-        double hv = h[q];
-        if (mode == 1 || mode == 2)
-            hv = hv + coef * y[q];
-        else if (mode == 3)
-            hv = hv * coef;
-        else if (mode == 4)
-            hv = hv * (L->tau * y[q]);
-        if (mode) h[q] = hv;
-        if (s) acc += s[q] * hv;
+    // kLbU components in flight per thread: their loads are issued together
+    // (a thread has ~10 components in all, so the pass is load latency);
+    // the products are added in component order
+    const int stride = gridDim.x * blockDim.x;
+    for (int q0 = blockIdx.x * blockDim.x + threadIdx.x; q0 < N; q0 += kLbU * stride) {
+        double hv[kLbU], yv[kLbU], sv[kLbU];
+#pragma unroll
+        for (int u = 0; u < kLbU; u++) {
+            const int q = q0 + u * stride;
+            const bool in = q < N;
+            hv[u] = in ? h[q] : 0.0;
+            yv[u] = in && y ? y[q] : 0.0;
+            sv[u] = in && s ? s[q] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < kLbU; u++) {
+            const int q = q0 + u * stride;
+            if (q >= N) break;
+            if (mode == 1 || mode == 2)
+                hv[u] = hv[u] + coef * yv[u];
+            else if (mode == 3)
+                hv[u] = hv[u] * coef;
+            else if (mode == 4)
+                hv[u] = hv[u] * (tau * yv[u]);
+            if (mode) h[q] = hv[u];
+            if (s) acc += sv[u] * hv[u];
+        }
     }
     if (!s) return;
     double v[1] = {acc};
-    if (lb_block<1>(v, partials, counter) && threadIdx.x < 32) {
-        double t[1];
-        lb_final<1>(partials, gridDim.x, t);
+    __shared__ double t[1];
+    if (block_partials<1>(v, partials, 0, counter)) {
+        final_sums<1>(partials, gridDim.x, t);
         if (threadIdx.x == 0) {
             L->dot[dot_out] = t[0];
             *counter = 0;
@@ -138,58 +109,59 @@ __global__ void __launch_bounds__(256) k_lb_prep(int N, const double* __restrict
                                                  const double* __restrict__ x, const double* __restrict__ xb,
                                                  LbScal* L, double* partials, unsigned* counter) {
     double v[2] = {0.0, 0.0};
-    double mx[3] = {0.0, 0.0, 0.0};
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < N; q += gridDim.x * blockDim.x) {
-        double hv = h[q], fv = f[q];
-        v[0] += fv * hv;
-        v[1] += hv * hv;
-        mx[0] = fmax(mx[0], fabs(hv));
-        mx[1] = fmax(mx[1], fabs(fv));
-        if (x) mx[2] = fmax(mx[2], fabs(x[q] - xb[q]));
+    unsigned long long mx[4] = {0, 0, 0, 0};  // bits of the maxima (integer compares; FP64 ones are slow here)
+    const int stride = gridDim.x * blockDim.x;
+    for (int q0 = blockIdx.x * blockDim.x + threadIdx.x; q0 < N; q0 += kLbU * stride) {
+        double hv[kLbU], fv[kLbU], dx[kLbU];
+#pragma unroll
+        for (int u = 0; u < kLbU; u++) {
+            const int q = q0 + u * stride;
+            const bool in = q < N;
+            hv[u] = in ? h[q] : 0.0;
+            fv[u] = in ? f[q] : 0.0;
+            dx[u] = in && x ? x[q] - xb[q] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < kLbU; u++) {
+            v[0] += fv[u] * hv[u];
+            v[1] += hv[u] * hv[u];
+            mx[0] = RedMaxBits()(mx[0], bits_of_abs(hv[u]));
+            mx[1] = RedMaxBits()(mx[1], bits_of_abs(fv[u]));
+            mx[2] = RedMaxBits()(mx[2], bits_of_abs(dx[u]));
+        }
     }
-    // sums into slots 0,1 and maxima into slots 2,3,4 of the same partial row
-    __shared__ double red[32][5];
-    __shared__ bool last;
+    // maxima into slots 2,3,4 of the partial row that takes the sums
+    __shared__ unsigned long long redm[32][4];
+    __shared__ double tot[2];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    double t[5] = {v[0], v[1], mx[0], mx[1], mx[2]};
-#pragma unroll
-    for (int k = 0; k < 5; k++) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            double u = __shfl_xor_sync(0xffffffffu, t[k], o);
-            t[k] = k < 2 ? t[k] + u : fmax(t[k], u);
-        }
-        if (lane == 0) red[w][k] = t[k];
+    const unsigned long long m = warp_reduce(mx, RedMaxBits());
+    if (lane % 8 == 0) redm[w][lane / 8] = m;
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        unsigned long long r = 0;
+        for (int q = 0; q < nw; q++) r = RedMaxBits()(r, redm[q][threadIdx.x]);
+        partials[blockIdx.x * kRedSlots + 2 + threadIdx.x] = __longlong_as_double((long long)r);
     }
-    __syncthreads();
-    if (threadIdx.x < 5) {
-        double r = 0.0;
-        for (int q = 0; q < nw; q++) r = threadIdx.x < 2 ? r + red[q][threadIdx.x] : fmax(r, red[q][threadIdx.x]);
-        partials[blockIdx.x * kRedSlots + threadIdx.x] = r;
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (last && threadIdx.x < 32) {
-        double s2[2], m3[3];
-        for (int k = 0; k < 2; k++) {
-            double a = 0.0;
-            for (int bb = lane; bb < (int)gridDim.x; bb += 32) a += partials[bb * kRedSlots + k];
+    if (block_partials<2>(v, partials, 0, counter)) {
+        final_sums<2>(partials, gridDim.x, tot);
+        unsigned long long b[4] = {0, 0, 0, 0};
+        for (int bb = threadIdx.x; bb < (int)gridDim.x; bb += blockDim.x)
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-            s2[k] = a;
-        }
-        for (int k = 0; k < 3; k++) {
-            double b = 0.0;
-            for (int bb = lane; bb < (int)gridDim.x; bb += 32) b = fmax(b, partials[bb * kRedSlots + 2 + k]);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) b = fmax(b, __shfl_xor_sync(0xffffffffu, b, o));
-            m3[k] = b;
-        }
+            for (int k = 0; k < 3; k++)
+                b[k] = RedMaxBits()(b[k], (unsigned long long)__double_as_longlong(
+                                              __ldcg(partials + bb * kRedSlots + 2 + k)));
+        const unsigned long long t = warp_reduce(b, RedMaxBits());
+        if (lane % 8 == 0) redm[w][lane / 8] = t;
+        __syncthreads();
         if (threadIdx.x == 0) {
-            L->fh = s2[0];
-            L->hh = s2[1];
+            double m3[3];
+            for (int k = 0; k < 3; k++) {
+                unsigned long long r = 0;
+                for (int q = 0; q < nw; q++) r = RedMaxBits()(r, redm[q][k]);
+                m3[k] = __longlong_as_double((long long)r);
+            }
+            L->fh = tot[0];
+            L->hh = tot[1];
             L->hmax = m3[0];
             L->fmax = m3[1];
             L->dxmax = m3[2];
@@ -242,9 +214,9 @@ __global__ void __launch_bounds__(256) k_lb_hist(int N, double* __restrict__ s0,
         v[1] += yv * yv;
         if (P) v[2] += yv * yv * P[q];
     }
-    if (lb_block<3>(v, partials, counter) && threadIdx.x < 32) {
-        double t[3];
-        lb_final<3>(partials, gridDim.x, t);
+    __shared__ double t[3];
+    if (block_partials<3>(v, partials, 0, counter)) {
+        final_sums<3>(partials, gridDim.x, t);
         if (threadIdx.x == 0) {
             if (t[0] > 0.0 && t[1] > 0.0) {
                 L->gamma = t[0] / t[1];
@@ -673,9 +645,9 @@ __global__ void __launch_bounds__(256) k_cg_dots(int N, const double* __restrict
         v[0] += f[q] * f[q];
         v[1] += f[q] * f0[q];
     }
-    if (lb_block<2>(v, partials, counter) && threadIdx.x < 32) {
-        double t[2];
-        lb_final<2>(partials, gridDim.x, t);
+    __shared__ double t[2];
+    if (block_partials<2>(v, partials, 0, counter)) {
+        final_sums<2>(partials, gridDim.x, t);
         if (threadIdx.x == 0) {
             L->dot[0] = t[0];
             L->dot[1] = t[1];

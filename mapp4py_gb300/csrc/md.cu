@@ -94,11 +94,6 @@ __device__ __forceinline__ NhcParams cell_nhc(const NhcParams& P0, const CellMd*
     return P;
 }
 
-template <int K>
-__device__ bool md_block_partials(double (&v)[K], double* partials, unsigned* counter) {
-    return block_partials<K>(v, partials, 0, counter);
-}
-
 // pre_init (md_nvt.cpp:256-340): kinetic tensor and temperature of the
 // incoming velocities
 __global__ void k_mvv_init(MdArgs a) {
@@ -120,8 +115,8 @@ __global__ void k_mvv_init(MdArgs a) {
         d[4] += __dmul_rn(__dmul_rn(v1, v2), m);
         d[5] += __dmul_rn(__dmul_rn(v2, v2), m);
     }
-    if (md_block_partials<6>(d, a.partials, &a.sc->counter[3]) && threadIdx.x < 32) {
-        double t[6];
+    __shared__ double t[6];
+    if (block_partials<6>(d, a.partials, 0, &a.sc->counter[3])) {
         final_sums<6>(a.partials, gridDim.x, t);
         if (threadIdx.x == 0) {
             for (int k = 0; k < 6; k++) a.sc->mvv[k] = t[k];
@@ -162,8 +157,8 @@ __global__ void __launch_bounds__(256) k_kick_drift64(MdArgs a) {
             a.x[c * n + i] = xx;
         }
     }
-    if (md_block_partials<3>(dsum, a.partials, &a.sc->counter[4]) && threadIdx.x < 32) {
-        double t[3];
+    __shared__ double t[3];
+    if (block_partials<3>(dsum, a.partials, 0, &a.sc->counter[4])) {
         final_sums<3>(a.partials, gridDim.x, t);
         if (threadIdx.x == 0) {
             double natms = (double)n;
@@ -218,8 +213,8 @@ __global__ void __launch_bounds__(256) k_kick2_64(MdArgs a) {
         d[4] += __dmul_rn(__dmul_rn(vv[1], vv[2]), m);
         d[5] += __dmul_rn(__dmul_rn(vv[2], vv[2]), m);
     }
-    if (md_block_partials<6>(d, a.partials, &a.sc->counter[5]) && threadIdx.x < 32) {
-        double t[6];
+    __shared__ double t[6];
+    if (block_partials<6>(d, a.partials, 0, &a.sc->counter[5])) {
         final_sums<6>(a.partials, gridDim.x, t);
         if (threadIdx.x == 0) {
             DevScalars* sc = a.sc;
@@ -312,8 +307,8 @@ __global__ void __launch_bounds__(256) k_integrate32(MdArgs a) {
     }
     if (__syncthreads_or(moved) && threadIdx.x == 0) a.sc->rebuild = 1;
     const float dv[3] = {dsum0, dsum1, dsum2};
-    if (block_partials_f32<3>(dv, a.partials, 0, &a.sc->counter[4]) && threadIdx.x < 32) {
-        double t[3];
+    __shared__ double t[3];
+    if (block_partials<3>(dv, a.partials, 0, &a.sc->counter[4])) {
         final_sums<3>(a.partials, gridDim.x, t);
         if (threadIdx.x == 0) {
             const double natms = (double)n;
@@ -355,8 +350,8 @@ __global__ void __launch_bounds__(256) k_close32(MdArgs a) {
         k5 = fmaf(mz, vz, k5);
     }
     const float d[6] = {k0, k1, k2, k3, k4, k5};
-    if (block_partials_f32<6>(d, a.partials, 0, &a.sc->counter[5]) && threadIdx.x < 32) {
-        double t[6];
+    __shared__ double t[6];
+    if (block_partials<6>(d, a.partials, 0, &a.sc->counter[5])) {
         final_sums<6>(a.partials, gridDim.x, t);
         if (threadIdx.x == 0) {
             DevScalars* sc = a.sc;
@@ -393,7 +388,7 @@ __global__ void __launch_bounds__(256) k_ke32b(MdArgs a) {
             k[4] = fmaf(my, vz, k[4]);
             k[5] = fmaf(mz, vz, k[5]);
         }
-        chunk_store_f32<6>(k, a.chunk_part + (size_t)ch * kChunkSlots + 7);
+        chunk_store<6>(k, a.chunk_part + (size_t)ch * kChunkSlots + 7);
     }
 }
 
@@ -450,7 +445,7 @@ __global__ void __launch_bounds__(256) k_mvv_init_b(MdArgs a) {
             d[4] += __dmul_rn(__dmul_rn(v1, v2), m);
             d[5] += __dmul_rn(__dmul_rn(v2, v2), m);
         }
-        chunk_store<6>([&](int k) { return d[k]; }, a.chunk_part + (size_t)ch * kChunkSlots + 7);
+        chunk_store<6>(d, a.chunk_part + (size_t)ch * kChunkSlots + 7);
     }
 }
 
@@ -546,7 +541,7 @@ __global__ void __launch_bounds__(256) k_integrate32b(MdArgs a) {
             if (threadIdx.x == 0) a.cell_reb[c] = 1;
         }
         const float ds[3] = {dsum0, dsum1, dsum2};
-        chunk_store_f32<3>(ds, a.chunk_disp + (size_t)ch * 4);
+        chunk_store<3>(ds, a.chunk_disp + (size_t)ch * 4);
     }
     if (__syncthreads_or(moved) && threadIdx.x == 0) a.sc->rebuild = 1;
 }

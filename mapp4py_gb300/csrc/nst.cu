@@ -62,15 +62,11 @@ __host__ __device__ __forceinline__ void vmlt(const double* v, const double (&M)
 
 template <int K>
 __device__ void nst_reduce(const NstAtoms& a, double (&v)[K]) {
+    __shared__ double tot[K];
     if (block_partials<K>(v, a.part, 0, a.counter)) {
-        if (threadIdx.x < 32) {
-            double tot[K];
-            final_sums<K>(a.part, gridDim.x, tot);
-            if (threadIdx.x == 0) {
-                for (int k = 0; k < K; k++) a.out[k] = tot[k];
-                *a.counter = 0;
-            }
-        }
+        final_sums<K>(a.part, gridDim.x, tot);
+        if (threadIdx.x < K) a.out[threadIdx.x] = tot[threadIdx.x];
+        if (threadIdx.x == 0) *a.counter = 0;
     }
 }
 

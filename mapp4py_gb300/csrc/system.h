@@ -136,7 +136,12 @@ constexpr int kMaxCells = 1 << 16;
 // shared memory given to the density tables of k_density32s: the rest of
 // the SM's 256 KB stays L1 for the neighbour-position gathers
 constexpr size_t kDensSmemBytes = 94 * 1024;
-// static shared memory of k_force32s (frame offsets, cutoffs, block sums),
+// systems up to this size read the density tables through L1 (k_density32):
+// the copy into every SM's shared memory does not pay for itself there
+// (through L1 / copied: 14.4 / 18.5 us at 4,000 atoms, 47.1 / 51.3 at 131,000,
+// 82.2 / 86.2 at 256,000, 148.4 / 148.2 at 500,000)
+constexpr int kDensSmallAtoms = 300000;
+// static shared memory of k_force32s (cutoffs, block sums),
 // kept out of its dynamic table budget
 constexpr size_t kForceSmemReserve = 4 * 1024;
 
