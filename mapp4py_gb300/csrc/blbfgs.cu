@@ -555,7 +555,7 @@ __global__ void k_bl_count(BlArgs a, int st) {
 // k_bl_refresh), the frame positions, and the capacity check of lb_update
 static void bl_rebuild_flagged(mappg_sys* s) {
     launch_rebuild_chain(s);
-    launch_shadow(s, false);
+    launch_shadow(s);
     int ov = 0;
     MAPPG_CUDA(cudaMemcpyAsync(&ov, &s->sc->overflow, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
     MAPPG_CUDA(cudaStreamSynchronize(s->stream));

@@ -268,7 +268,7 @@ void lb_update(mappg_sys* s) {
     launch_skin_test(s);
     launch_rebuild_chain(s);
     // positions moved without a rebuild: refresh the mixed kernels' frame
-    if (s->precision == MAPPG_MIXED) launch_shadow(s, false);
+    if (s->precision == MAPPG_MIXED) launch_shadow(s);
     MAPPG_CUDA(cudaGetLastError());
     // a relaxation can crowd atoms beyond the rows' capacity: a rebuild that
     // ran out of room is redone with wider rows

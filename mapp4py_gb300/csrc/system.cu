@@ -74,17 +74,14 @@ void sys_set_box(mappg_sys* s, const double* H) {
             fr.G[d][k] = (float)g;
             fr.Glo[d][k] = (float)(g - (double)fr.G[d][k]);
         }
-    // neighbour code c = (d0+1)+3(d1+1)+9(d2+1): the image's bin is atom i's
-    // bin + d; its frame offset is exactly -8 d
+    // image shifts n H, indexed by image code (n0+1) + 3(n1+1) + 9(n2+1)
     for (int c = 0; c < 27; c++) {
         int d[3] = {c % 3 - 1, (c / 3) % 3 - 1, c / 9 - 1};
         for (int k = 0; k < 3; k++) {
             double sh = 0.0;
             for (int q = 0; q < 3; q++) sh += d[q] * s->box.H[q][k];
-            fr.off[c][k] = -kBinW * d[k];
-            s->shift[c][k] = sh;  // indexed by image code n instead of d
+            s->shift[c][k] = sh;
         }
-        fr.off[c][3] = 0.f;
     }
     double pmax = s->skin;
     for (int q = 0; q < 3; q++) {
@@ -250,9 +247,26 @@ __device__ __forceinline__ void s2x(const double* h, double s0, double s1, doubl
     x2 = dmul(s2, h[5]);
 }
 
-// rebuild step 1: wrap x into the cell (x2s_lcl then s2x_all), bin, count
-__global__ void k_wrap_bin(int n, double* __restrict__ x, double* __restrict__ s, Geo g, int* __restrict__ binc,
-                           int* __restrict__ binid, int* __restrict__ bin_count, DevScalars* sc) {
+// FP32 positions in the scaled bin frame, relative to the atom's bin corner:
+// p'_d = (x B)_d * 8 nb_d - 8 b_d (x not wrapped between builds, so p' may
+// leave [0,8) by the drift since the build)
+__device__ __forceinline__ float4 frame_pos(const double* bs, double x0, double x1, double x2, int bc) {
+    double u0 = bs[0] * x0 + (bs[1] * x1 + bs[2] * x2);
+    double u1 = bs[3] * x1 + bs[4] * x2;
+    double u2 = bs[5] * x2;
+    float4 p;
+    p.x = (float)(u0 - (double)(8 * (bc & 1023)));
+    p.y = (float)(u1 - (double)(8 * ((bc >> 10) & 1023)));
+    p.z = (float)(u2 - (double)(8 * ((bc >> 20) & 1023)));
+    p.w = 0.f;
+    return p;
+}
+
+// rebuild step 1: wrap x into the cell (x2s_lcl then s2x_all), bin, count;
+// the build positions (x0, and p0 in the frame) are the wrapped ones
+__global__ void k_wrap_bin(int n, double* __restrict__ x, double* __restrict__ s, double* __restrict__ xb, Geo g,
+                           int* __restrict__ binc, int* __restrict__ binid, int* __restrict__ bin_count,
+                           float4* __restrict__ p32, float4* __restrict__ p0, DevScalars* sc) {
     if (!sc->rebuild) return;
     int bad = 0;
     const double drift0 = sc->drift[0], drift1 = sc->drift[1], drift2 = sc->drift[2];
@@ -266,16 +280,18 @@ __global__ void k_wrap_bin(int n, double* __restrict__ x, double* __restrict__ s
         double s2 = dmul(x2, g.b6[5]);
         s2 = wrap01(s2, &bad);
         s2x(g.h6, s0, s1, s2, x0, x1, x2);
-        x[i] = x0;
-        x[n + i] = x1;
-        x[2 * n + i] = x2;
+        x[i] = xb[i] = x0;
+        x[n + i] = xb[n + i] = x1;
+        x[2 * n + i] = xb[2 * n + i] = x2;
         s[i] = s0;
         s[n + i] = s1;
         s[2 * n + i] = s2;
         int b0 = min((int)(s0 * g.nb[0]), g.nb[0] - 1);
         int b1 = min((int)(s1 * g.nb[1]), g.nb[1] - 1);
         int b2 = min((int)(s2 * g.nb[2]), g.nb[2] - 1);
-        binc[i] = b0 | (b1 << 10) | (b2 << 20);
+        const int bc = b0 | (b1 << 10) | (b2 << 20);
+        binc[i] = bc;
+        p32[i] = p0[i] = frame_pos(g.bs, x0, x1, x2, bc);
         int b = b0 + g.nb[0] * (b1 + g.nb[1] * b2);
         binid[i] = b;
         atomicAdd(&bin_count[b], 1);
@@ -285,10 +301,11 @@ __global__ void k_wrap_bin(int n, double* __restrict__ x, double* __restrict__ s
 
 // batch variant of step 1: each atom uses its cell's box, bins and drift
 // (cells without their rebuild flag keep their wrap, bins and rows)
-__global__ void k_wrap_bin_b(int n, double* __restrict__ x, double* __restrict__ s, const CellGeo* __restrict__ cells,
-                             const int* __restrict__ cell_of, const CellMd* __restrict__ cmd, int* __restrict__ binc,
-                             int* __restrict__ binid, int* __restrict__ bin_count, const uint8_t* __restrict__ cell_reb,
-                             DevScalars* sc) {
+__global__ void k_wrap_bin_b(int n, double* __restrict__ x, double* __restrict__ s, double* __restrict__ xb,
+                             const CellGeo* __restrict__ cells, const int* __restrict__ cell_of,
+                             const CellMd* __restrict__ cmd, int* __restrict__ binc, int* __restrict__ binid,
+                             int* __restrict__ bin_count, const uint8_t* __restrict__ cell_reb,
+                             float4* __restrict__ p32, float4* __restrict__ p0, DevScalars* sc) {
     if (!sc->rebuild) return;
     int bad = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -304,21 +321,31 @@ __global__ void k_wrap_bin_b(int n, double* __restrict__ x, double* __restrict__
         double s2 = dmul(x2, g.b6[5]);
         s2 = wrap01(s2, &bad);
         s2x(g.h6, s0, s1, s2, x0, x1, x2);
-        x[i] = x0;
-        x[n + i] = x1;
-        x[2 * n + i] = x2;
+        x[i] = xb[i] = x0;
+        x[n + i] = xb[n + i] = x1;
+        x[2 * n + i] = xb[2 * n + i] = x2;
         s[i] = s0;
         s[n + i] = s1;
         s[2 * n + i] = s2;
         int b0 = min((int)(s0 * g.nb[0]), g.nb[0] - 1);
         int b1 = min((int)(s1 * g.nb[1]), g.nb[1] - 1);
         int b2 = min((int)(s2 * g.nb[2]), g.nb[2] - 1);
-        binc[i] = b0 | (b1 << 10) | (b2 << 20);
+        const int bc = b0 | (b1 << 10) | (b2 << 20);
+        binc[i] = bc;
+        p32[i] = p0[i] = frame_pos(g.bs, x0, x1, x2, bc);
         int b = g.bin_base + b0 + g.nb[0] * (b1 + g.nb[1] * b2);
         binid[i] = b;
         atomicAdd(&bin_count[b], 1);
     }
     if (bad) sc->bad = 1;
+}
+
+// what a rebuild resets once step 1 has taken the mean displacement out of x
+__device__ __forceinline__ void rebuild_reset(DevScalars* sc) {
+    sc->maxrow = 0;
+    sc->sumrow = 0;
+    sc->drift[0] = sc->drift[1] = sc->drift[2] = 0.0;
+    sc->nrebuild++;
 }
 
 // rebuild step 2: exclusive scan of bin counts (one block), counts zeroed
@@ -346,10 +373,7 @@ __global__ void k_scan_bins(int nbins, int* __restrict__ bin_count, int* __restr
         bin_count[b] = 0;
     }
     if (t == T - 1) bin_start[nbins] = part[T - 1];
-    if (t == 0) {
-        sc->maxrow = 0;
-        sc->sumrow = 0;
-    }
+    if (t == 0) rebuild_reset(sc);
 }
 
 // batch variant of step 2: one warp per flagged cell scans its own bins,
@@ -357,20 +381,20 @@ __global__ void k_scan_bins(int nbins, int* __restrict__ bin_count, int* __restr
 // other cells' bin starts stay valid)
 __global__ void k_scan_bins_b(int ncell, int n, int nbins, const CellGeo* __restrict__ cells,
                               const uint8_t* __restrict__ cell_reb, int* __restrict__ bin_count,
-                              int* __restrict__ bin_start, DevScalars* sc) {
+                              int* __restrict__ bin_start, CellMd* __restrict__ cmd, DevScalars* sc) {
     if (!sc->rebuild) return;
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         bin_start[nbins] = n;
-        sc->maxrow = 0;
-        sc->sumrow = 0;
+        rebuild_reset(sc);
     }
     for (int c = warp; c < ncell; c += nw) {
         if (!cell_reb[c]) continue;
         const CellGeo& g = cells[c];
         const int nb = g.nb[0] * g.nb[1] * g.nb[2], base = g.bin_base;
         int run = g.begin;
+        if (lane < 3) cmd[c].drift[lane] = 0.0;
         for (int k0 = 0; k0 < nb; k0 += 32) {
             const int k = k0 + lane;
             const int v = k < nb ? bin_count[base + k] : 0;
@@ -404,9 +428,12 @@ __global__ void k_scatter_bins(int n, const int* __restrict__ binid, const int* 
 }
 
 // rebuild step 4: one warp per bin ranks its atoms by index (deterministic
-// order), counts zeroed for the next rebuild
+// order) and writes their frame positions with the entry bits of atom and
+// element in w, bin by bin: what the builder stages of a candidate in one
+// coalesced load; counts zeroed for the next rebuild
 __global__ void k_sort_bins(int nbins, const int* __restrict__ bin_start, const int* __restrict__ bin_tmp,
-                            int* __restrict__ bin_atoms, int* __restrict__ bin_count, const int* __restrict__ cell_of,
+                            const float4* __restrict__ p32, const uint8_t* __restrict__ elem,
+                            float4* __restrict__ bin_pos, int* __restrict__ bin_count, const int* __restrict__ cell_of,
                             const uint8_t* __restrict__ cell_reb, DevScalars* sc) {
     if (!sc->rebuild) return;
     int lane = threadIdx.x & 31;
@@ -421,66 +448,38 @@ __global__ void k_sort_bins(int nbins, const int* __restrict__ bin_start, const 
             int a = bin_tmp[k];
             int r = 0;
             for (int q = lo; q < hi; q++) r += bin_tmp[q] < a;
-            bin_atoms[lo + r] = a;
+            float4 p = p32[a];
+            p.w = __int_as_float(make_entry(a, elem[a], 0));
+            bin_pos[lo + r] = p;
         }
         if (lane == 0) bin_count[b] = 0;
     }
 }
 
-// FP32 positions in the scaled bin frame, relative to the atom's bin corner:
-// p'_d = (x B)_d * 8 nb_d - 8 b_d (x not wrapped between builds, so p' may
-// leave [0,8) by the drift since the build); gated == true only in a rebuild
-__device__ __forceinline__ float4 frame_pos(const Geo& g, double x0, double x1, double x2, int bc) {
-    double u0 = g.bs[0] * x0 + (g.bs[1] * x1 + g.bs[2] * x2);
-    double u1 = g.bs[3] * x1 + g.bs[4] * x2;
-    double u2 = g.bs[5] * x2;
-    float4 p;
-    p.x = (float)(u0 - (double)(8 * (bc & 1023)));
-    p.y = (float)(u1 - (double)(8 * ((bc >> 10) & 1023)));
-    p.z = (float)(u2 - (double)(8 * ((bc >> 20) & 1023)));
-    p.w = 0.f;
-    return p;
-}
-
+// frame positions of atoms that moved without a rebuild
 __global__ void k_shadow(int n, const double* __restrict__ x, const int* __restrict__ binc, float4* __restrict__ p32,
-                         float4* __restrict__ p0, Geo g, int gated, DevScalars* sc) {
-    if (gated && !sc->rebuild) return;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float4 p = frame_pos(g, x[i], x[n + i], x[2 * n + i], binc[i]);
-        p32[i] = p;
-        if (gated) p0[i] = p;
-    }
+                         Geo g) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        p32[i] = frame_pos(g.bs, x[i], x[n + i], x[2 * n + i], binc[i]);
 }
 
 __global__ void k_shadow_b(int n, const double* __restrict__ x, const int* __restrict__ binc,
                            const CellGeo* __restrict__ cells, const int* __restrict__ cell_of,
-                           float4* __restrict__ p32, float4* __restrict__ p0, int gated,
-                           const uint8_t* __restrict__ cell_reb, DevScalars* sc) {
-    if (gated && !sc->rebuild) return;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        if (gated && !cell_reb[cell_of[i]]) continue;
-        const CellGeo& cg = cells[cell_of[i]];
-        Geo g;
-        for (int k = 0; k < 6; k++) g.bs[k] = cg.bs[k];
-        float4 p = frame_pos(g, x[i], x[n + i], x[2 * n + i], binc[i]);
-        p32[i] = p;
-        if (gated) p0[i] = p;
-    }
+                           float4* __restrict__ p32) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        p32[i] = frame_pos(cells[cell_of[i]].bs, x[i], x[n + i], x[2 * n + i], binc[i]);
 }
 
 struct BuildArgs {
     int n, maxnbr, ne;
     const double* x;
     const double* s;
-    const float4* p32;
-    const uint8_t* elem;
+    const float4* bin_pos;
     const int* bin_start;
-    const int* bin_atoms;
     int* nbr;
     int* nnbr;
-    double* x0;
     Geo g;
-    Frame fr;
+    float G[3][3];  // frame to Cartesian
     float lo2[kMaxElem * kMaxElem], hi2[kMaxElem * kMaxElem];
     float in2[kMaxElem * kMaxElem];  // pair cutoff squared: entries below it lead their row
     double cut_sk_sq[kMaxElem * kMaxElem];
@@ -489,243 +488,265 @@ struct BuildArgs {
     const uint8_t* cell_reb;  // batch: the cells to rebuild
 };
 
-// frame displacement to Cartesian: dx' G with G as head + tail
-template <class FR>
-__device__ __forceinline__ void frame_to_cart(const FR& fr, float a, float b, float c, float& x, float& y,
-                                              float& z) {
-    if (fr.ortho) {
-        x = fmaf(a, fr.G[0][0], a * fr.Glo[0][0]);
-        y = fmaf(b, fr.G[1][1], b * fr.Glo[1][1]);
-        z = fmaf(c, fr.G[2][2], c * fr.Glo[2][2]);
-    } else {
-        x = fmaf(a, fr.G[0][0], fmaf(b, fr.G[1][0], fmaf(c, fr.G[2][0], a * fr.Glo[0][0] + b * fr.Glo[1][0] +
-                                                                        c * fr.Glo[2][0])));
-        y = fmaf(b, fr.G[1][1], fmaf(c, fr.G[2][1], b * fr.Glo[1][1] + c * fr.Glo[2][1]));
-        z = fmaf(c, fr.G[2][2], c * fr.Glo[2][2]);
-    }
-}
-
 // the reference's predicate for a pair inside the FP32 band: x_j' =
-// S2X(s_j + n) in FP64 without fused multiply-adds, RSQ < (cut + skin)^2
-__device__ __forceinline__ bool exact_keep(const BuildArgs& a, const double* h6, double xi0, double xi1, double xi2,
-                                           int j, int im, int pe) {
-    const int n = a.n;
-    const int n0 = (im & 3) - 1, n1 = ((im >> 2) & 3) - 1, n2 = ((im >> 4) & 3) - 1;
+// S2X(s_j + n) in FP64 without fused multiply-adds, RSQ < (cut + skin)^2;
+// n: the image that the bin step of entry ent reaches from bin geo[0..2]
+// of geo[3..5]
+__device__ __noinline__ bool exact_keep(const BuildArgs& a, const double* h6, const int* geo, int i, int ent, int pe) {
+    const int n = a.n, j = entry_j(ent);
+    const int u0 = geo[0] + entry_step(ent, 0), u1 = geo[1] + entry_step(ent, 1), u2 = geo[2] + entry_step(ent, 2);
     double s0 = a.s[j], s1 = a.s[n + j], s2 = a.s[2 * n + j];
-    if (n0 > 0) s0 = dadd(s0, 1.0);
-    if (n0 < 0) s0 = dsub(s0, 1.0);
-    if (n1 > 0) s1 = dadd(s1, 1.0);
-    if (n1 < 0) s1 = dsub(s1, 1.0);
-    if (n2 > 0) s2 = dadd(s2, 1.0);
-    if (n2 < 0) s2 = dsub(s2, 1.0);
+    if (u0 >= geo[3]) s0 = dadd(s0, 1.0);
+    if (u0 < 0) s0 = dsub(s0, 1.0);
+    if (u1 >= geo[4]) s1 = dadd(s1, 1.0);
+    if (u1 < 0) s1 = dsub(s1, 1.0);
+    if (u2 >= geo[5]) s2 = dadd(s2, 1.0);
+    if (u2 < 0) s2 = dsub(s2, 1.0);
     double xj0, xj1, xj2;
     s2x(h6, s0, s1, s2, xj0, xj1, xj2);
-    double e0 = dsub(xi0, xj0), e1 = dsub(xi1, xj1), e2 = dsub(xi2, xj2);
+    double e0 = dsub(a.x[i], xj0), e1 = dsub(a.x[n + i], xj1), e2 = dsub(a.x[2 * n + i], xj2);
     double rsq = dadd(dmul(e0, e0), dadd(dmul(e1, e1), dmul(e2, e2)));
     return rsq < a.cut_sk_sq[pe];
 }
 
-// rebuild step 5: one warp per bin.  The candidates of the bin's 27-bin
-// stencil are read 32 at a time, once for all atoms of the bin, and every
-// atom of the bin tests them in turn, so a candidate's gathers and its place
-// in the bin sequence are paid once per bin instead of once per atom.  A
-// row holds first its atom's neighbours inside the pair cutoff at build time,
-// in (bin step, bin order) order, bin steps c = (d0+1) + 3(d1+1) + 9(d2+1),
-// then those of the skin shell, in the reverse of that order: the shell's
-// entries are written backwards from the row's end and moved behind the
-// inner ones once the bin's candidates are done.  Lanes test candidates and
-// ballots keep their order.  With the inner entries in front, the lanes of
-// an atom (slots lane, lane + TPA, ...) get equal shares of the pairs inside
-// the cutoff, and the density pass's lanes reach the shell together.  A
-// batch finds the bin's cell through its first atom (the bins of a cell hold
-// only that cell's atoms).
+constexpr int kBuildWarps = 4;    // warps of a builder block
+constexpr int kBuildTile = 768;   // candidates staged at a time (12 KB)
+constexpr int kBuildHome = 32;    // atoms of the bin worked on at a time
+constexpr int kBuildRow = 256;    // longest row put together on chip
+
+// list thresholds of a pair: kept below lo2, decided in FP64 up to hi2, leading its row below in2
+template <bool UNI>
+struct BuildCut {
+    float lo2, hi2, in2;  // UNI: the same for every pair
+    const float* tab;     // else lo2, hi2, in2 of pair e at tab[e], tab[64 + e], tab[128 + e]
+    __device__ __forceinline__ float lo(int e) const { return UNI ? lo2 : tab[e]; }
+    __device__ __forceinline__ float hi(int e) const { return UNI ? hi2 : tab[kMaxElem * kMaxElem + e]; }
+    __device__ __forceinline__ float in(int e) const { return UNI ? in2 : tab[2 * kMaxElem * kMaxElem + e]; }
+};
+
+// the staged candidates (nt of them, the rest of the last 32 far away)
+// against atom h: its inner entries go to dst[0], dst[1], ..., its shell
+// entries to dst[cap - 1], dst[cap - 2], ...; entries that would leave the
+// row or meet are dropped (the caller sees it from the counts)
+template <bool UNI>
+__device__ __forceinline__ void build_scan(const BuildArgs& a, const BuildCut<UNI>& cut, const float4* cand, int nt,
+                                           const float4& h, int self, const int* geo, const double* h6, int* dst,
+                                           int cap, int& cin, int& cout) {
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const int pe0 = entry_elem(self) * a.ne;
+#pragma unroll 2
+    for (int k0 = 0; k0 < nt; k0 += 32) {
+        const float4 p = cand[k0 + lane];
+        const int ent = __float_as_int(p.w);
+        const float dx = h.x - p.x, dy = h.y - p.y, dz = h.z - p.z;
+        const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+        const bool other = ent != self;
+        const int pe = UNI ? 0 : pe0 + entry_elem(ent);
+        const unsigned mh = __ballot_sync(0xffffffffu, other && r2 <= cut.hi(pe));
+        if (mh == 0u) continue;
+        unsigned m = __ballot_sync(0xffffffffu, other && r2 < cut.lo(pe));
+        if (m != mh) {
+            // pairs within the FP32 rounding of the list cutoff
+            bool keep = (m >> lane) & 1u;
+            if (!keep && ((mh >> lane) & 1u))
+                keep = exact_keep(a, h6, geo, entry_j(self), ent, pe0 + entry_elem(ent));
+            m = __ballot_sync(0xffffffffu, keep);
+        }
+        const bool inner = r2 < cut.in(pe);
+        const unsigned mi = __ballot_sync(0xffffffffu, inner) & m, mo = m & ~mi;
+        const int at = __popc((inner ? mi : mo) & below);
+        const int pos = inner ? cin + at : cap - 1 - cout - at;
+        if (((m >> lane) & 1u) && (unsigned)pos < (unsigned)cap) dst[pos] = ent;
+        cin += __popc(mi);
+        cout += __popc(mo);
+    }
+}
+
+// rebuild step 5: one block per bin.  The candidates of the bin's 27-bin
+// stencil are staged in shared memory as Cartesian positions beside the bin
+// (bin_pos: one coalesced load a candidate), and the block's warps take the
+// bin's atoms in turn, 32 candidates against one atom at a time.  A row
+// holds first its atom's neighbours inside the pair cutoff at build time, in
+// (bin step, bin order) order, bin steps c = (d0+1) + 3(d1+1) + 9(d2+1), then
+// those of the skin shell in the reverse of that order: it is put together
+// in shared memory, inner entries from the front and shell entries from the
+// end, and written out in one piece.  Rows longer than kBuildRow, and those
+// of bins whose candidates need several tiles, are put together in place.
+// With the inner entries in front, the lanes of an atom (slots lane,
+// lane + TPA, ...) get equal shares of the pairs inside the cutoff, and the
+// density pass's lanes reach the shell together.  A batch finds the bin's
+// cell through its first atom (the bins of a cell hold only that cell's
+// atoms).
+//
+// Bound by instruction issue.  The atom's two counters are uniform in its
+// warp, so 32 tests are the distance, three ballots and a store, and a step
+// without any neighbour (a quarter of them) ends at the first ballot.  With
+// the warp walking candidates in the outer loop (one warp per bin, as this
+// kernel was built before) the counters went through shuffles, an iteration
+// waited ~800 clocks on its chain, and the bins of a 500-atom cell had 27
+// warps in all.
+// Whole rebuild (all its kernels) before and now: 4,000 atoms 129 -> 45 us,
+// 32,000 164 -> 68, 256,000 509 -> 318, 500,000 905 -> 599.
 // ORTHO: every cell orthorhombic (one product per axis to Cartesian).
 // UNI: every pair type has the same list cutoff (thresholds in registers).
 template <bool BATCH, bool ORTHO, bool UNI>
-__global__ void __launch_bounds__(256) k_build_bins(BuildArgs a, int nbins, DevScalars* sc) {
+__global__ void __launch_bounds__(32 * kBuildWarps) k_build_bins(const __grid_constant__ BuildArgs a, int nbins,
+                                                                 DevScalars* sc) {
     if (!sc->rebuild) return;
-    __shared__ float4 off[27];
-    __shared__ int s_pre[8][32], s_lo[8][32], s_img[8][32];  // per warp: the bin's 27 stencil bins
-    __shared__ float4 s_at[8][32];  // per warp: the bin's atoms (frame position, w = index << 3 | element)
-    __shared__ float s_lo2[kMaxElem * kMaxElem], s_hi2[kMaxElem * kMaxElem], s_in2[kMaxElem * kMaxElem];
-    if (threadIdx.x < 27)
-        off[threadIdx.x] = make_float4(a.fr.off[threadIdx.x][0], a.fr.off[threadIdx.x][1], a.fr.off[threadIdx.x][2], 0.f);
-    if (threadIdx.x < a.ne * a.ne) {
-        s_lo2[threadIdx.x] = a.lo2[threadIdx.x];
-        s_hi2[threadIdx.x] = a.hi2[threadIdx.x];
-        s_in2[threadIdx.x] = a.in2[threadIdx.x];
-    }
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    const int n = a.n;
-    const float lo2u = a.lo2[0], hi2u = a.hi2[0], in2u = a.in2[0];
+    __shared__ float4 cand[kBuildTile], home[kBuildHome];
+    __shared__ int s_pre[33], s_lo[32], s_cin[kBuildHome], s_cout[kBuildHome], s_geo[6];
+    __shared__ int s_row[kBuildWarps][kBuildRow];
+    __shared__ float s_cut[UNI ? 1 : 3 * kMaxElem * kMaxElem];
+    if (!UNI)
+        for (int t = threadIdx.x; t < a.ne * a.ne; t += 32 * kBuildWarps) {
+            s_cut[t] = a.lo2[t];
+            s_cut[kMaxElem * kMaxElem + t] = a.hi2[t];
+            s_cut[2 * kMaxElem * kMaxElem + t] = a.in2[t];
+        }
+    const BuildCut<UNI> cut{a.lo2[0], a.hi2[0], a.in2[0], s_cut};
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int maxrow = 0, overflow = 0;
     long long sumrow = 0;
-    for (int b = warp; b < nbins; b += nw) {
+    for (int b = blockIdx.x; b < nbins; b += gridDim.x) {
         const int a0 = a.bin_start[b];
         const int na = a.bin_start[b + 1] - a0;
         if (na == 0) continue;
         const int cell = BATCH ? a.cell_of[a0] : 0;  // a batch bin's slots lie in its cell's atom range
         if (BATCH && !a.cell_reb[cell]) continue;
         const CellGeo* cg = BATCH ? a.cells + cell : nullptr;
-        const int nbx = BATCH ? cg->nb[0] : a.g.nb[0], nby = BATCH ? cg->nb[1] : a.g.nb[1],
-                  nbz = BATCH ? cg->nb[2] : a.g.nb[2];
+        const int* nb = BATCH ? cg->nb : a.g.nb;
+        const double* h6 = BATCH ? cg->h6 : a.g.h6;
+        const float(*G)[3] = BATCH ? cg->G : a.G;
         const int bin_base = BATCH ? cg->bin_base : 0;
-        const float G0 = BATCH ? cg->G[0][0] : a.fr.G[0][0], G1 = BATCH ? cg->G[1][1] : a.fr.G[1][1],
-                    G2 = BATCH ? cg->G[2][2] : a.fr.G[2][2];
-        double h6[6];
-#pragma unroll
-        for (int k = 0; k < 6; k++) h6[k] = BATCH ? cg->h6[k] : a.g.h6[k];
         const int bl = b - bin_base;
-        const int b0 = bl % nbx, b1 = (bl / nbx) % nby, b2 = bl / (nbx * nby);
-        int lo = 0, ncand = 0, img = 0;
-        if (lane < 27) {
-            const int c = lane;
-            int u0 = b0 + c % 3 - 1, u1 = b1 + (c / 3) % 3 - 1, u2 = b2 + c / 9 - 1;
-            int n0 = u0 < 0 ? -1 : (u0 >= nbx ? 1 : 0);
-            int n1 = u1 < 0 ? -1 : (u1 >= nby ? 1 : 0);
-            int n2 = u2 < 0 ? -1 : (u2 >= nbz ? 1 : 0);
-            int w = bin_base + (u0 - n0 * nbx) + nbx * ((u1 - n1 * nby) + nby * (u2 - n2 * nbz));
-            lo = a.bin_start[w];
-            ncand = a.bin_start[w + 1] - lo;
-            img = (n0 + 1) | ((n1 + 1) << 2) | ((n2 + 1) << 4);
-        }
-        int incl = ncand;
+        const int b0 = bl % nb[0], b1 = (bl / nb[0]) % nb[1], b2 = bl / (nb[0] * nb[1]);
+        auto cart = [&](float4& p) {
+            if (ORTHO) {
+                p.x *= G[0][0];
+                p.y *= G[1][1];
+                p.z *= G[2][2];
+            } else {
+                p.x = fmaf(p.x, G[0][0], fmaf(p.y, G[1][0], p.z * G[2][0]));
+                p.y = fmaf(p.y, G[1][1], p.z * G[2][1]);
+                p.z *= G[2][2];
+            }
+        };
+        __syncthreads();  // the previous bin's tables are no longer read
+        if (w == 0) {
+            int lo = 0, ncand = 0;
+            if (lane < 27) {
+                int u0 = b0 + lane % 3 - 1, u1 = b1 + (lane / 3) % 3 - 1, u2 = b2 + lane / 9 - 1;
+                if (u0 < 0) u0 += nb[0];
+                if (u0 >= nb[0]) u0 -= nb[0];
+                if (u1 < 0) u1 += nb[1];
+                if (u1 >= nb[1]) u1 -= nb[1];
+                if (u2 < 0) u2 += nb[2];
+                if (u2 >= nb[2]) u2 -= nb[2];
+                const int v = bin_base + u0 + nb[0] * (u1 + nb[1] * u2);
+                lo = a.bin_start[v];
+                ncand = a.bin_start[v + 1] - lo;
+            }
+            int incl = ncand;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        s_pre[wib][lane] = incl - ncand;
-        s_lo[wib][lane] = lo;
-        s_img[wib][lane] = img;
-        for (int g0 = 0; g0 < na; g0 += 32) {
-            const int ng = min(32, na - g0);
-            __syncwarp();  // the previous group's atoms are no longer read
-            if (lane < ng) {
-                const int i = a.bin_atoms[a0 + g0 + lane];
-                float4 p = a.p32[i];
-                p.w = __int_as_float((i << 3) | a.elem[i]);
-                s_at[wib][lane] = p;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
             }
-            __syncwarp();
-            int mycnt = 0;  // lane q: inner entries so far of the group's atom q (row front)
-            int myout = 0;  // lane q: shell entries so far (row end, backwards)
-            int c = 0, cpre = 0, cnext = s_pre[wib][1], clo = s_lo[wib][0], cimg = s_img[wib][0];
-            for (int t0 = 0; t0 < total; t0 += 32) {
-                const int t = t0 + lane;
-                const bool valid = t < total;
-                int j = -1, ej = 0, im = 21;
-                int selfq = -1;  // the group atom this candidate is (its own bin, no image shift)
-                float qx = 0.f, qy = 0.f, qz = 0.f;  // candidate minus its bin-step offset
-                if (valid) {
-                    while (t >= cnext) {
-                        c++;
-                        cpre = cnext;
-                        cnext = c < 26 ? s_pre[wib][c + 1] : total;
-                        clo = s_lo[wib][c];
-                        cimg = s_img[wib][c];
-                    }
-                    j = a.bin_atoms[clo + (t - cpre)];
-                    const float4 pj = a.p32[j];
-                    const float4 o = off[c];
-                    ej = a.elem[j];
-                    im = cimg;
-                    // the bin's own atoms appear once unshifted, as bin step 13
-                    if (c == 13 && im == 21) selfq = (t - cpre) - g0;
-                    qx = pj.x - o.x;
-                    qy = pj.y - o.y;
-                    qz = pj.z - o.z;
-                }
-                const int ent = valid ? make_entry(j, ej, c) : 0;
-                for (int q = 0; q < ng; q++) {
-                    const float4 pq = s_at[wib][q];
-                    const int iw = __float_as_int(pq.w);
-                    const int i = iw >> 3;
-                    bool keep = false, inner = false;
-                    if (valid && q != selfq) {
-                        float dx, dy, dz;
-                        if (ORTHO) {
-                            dx = (pq.x - qx) * G0;
-                            dy = (pq.y - qy) * G1;
-                            dz = (pq.z - qz) * G2;
-                        } else if (BATCH) {
-                            frame_to_cart(*cg, pq.x - qx, pq.y - qy, pq.z - qz, dx, dy, dz);
-                        } else {
-                            frame_to_cart(a.fr, pq.x - qx, pq.y - qy, pq.z - qz, dx, dy, dz);
-                        }
-                        const float r2 = dx * dx + (dy * dy + dz * dz);
-                        const int pe = UNI ? 0 : (iw & 7) * a.ne + ej;
-                        if (r2 < (UNI ? lo2u : s_lo2[pe]))
-                            keep = true;
-                        else if (r2 <= (UNI ? hi2u : s_hi2[pe]))
-                            keep = exact_keep(a, h6, a.x[i], a.x[n + i], a.x[2 * n + i], j, im,
-                                              UNI ? (iw & 7) * a.ne + ej : pe);
-                        inner = keep && r2 < (UNI ? in2u : s_in2[pe]);
-                    }
-                    const unsigned m = __ballot_sync(0xffffffffu, keep);
-                    if (m) {
-                        const unsigned mi = __ballot_sync(0xffffffffu, inner);
-                        const unsigned mo = m & ~mi;
-                        const unsigned below = (1u << lane) - 1u;
-                        const int cin = __shfl_sync(0xffffffffu, mycnt, q);
-                        const int cout = __shfl_sync(0xffffffffu, myout, q);
-                        if (keep) {
-                            // both streams stay inside the row; where they
-                            // meet the row has overflowed and is built again
-                            // with a larger capacity
-                            const int pos = inner ? cin + __popc(mi & below)
-                                                  : a.maxnbr - 1 - (cout + __popc(mo & below));
-                            if (pos >= 0 && pos < a.maxnbr) a.nbr[(size_t)i * a.maxnbr + pos] = ent;
-                        }
-                        if (lane == q) {
-                            mycnt = cin + __popc(mi);
-                            myout = cout + __popc(mo);
-                        }
-                    }
-                }
-            }
-            // each row's shell entries move from the row's end to follow its
-            // inner ones: a move to lower slots, 32 entries at a time, each
-            // batch read before it is written (the gap is never negative)
-            __syncwarp();
-            for (int q = 0; q < ng; q++) {
-                const int cin = __shfl_sync(0xffffffffu, mycnt, q);
-                const int cout = __shfl_sync(0xffffffffu, myout, q);
-                if (cout == 0 || cin + cout > a.maxnbr) continue;
-                int* row = a.nbr + (size_t)(__float_as_int(s_at[wib][q].w) >> 3) * a.maxnbr;
-                const int src = a.maxnbr - cout;
-                for (int k0 = 0; k0 < cout; k0 += 32) {
-                    const int k = k0 + lane;
-                    const int v = k < cout ? row[src + k] : 0;
-                    __syncwarp();
-                    if (k < cout) row[cin + k] = v;
-                    __syncwarp();
-                }
-            }
-            if (lane < ng) {
-                const int i = __float_as_int(s_at[wib][lane].w) >> 3;
-                const int tot = mycnt + myout;
-                a.nnbr[i] = min(tot, a.maxnbr);
-                if (tot > a.maxnbr) overflow = 1;
-                maxrow = max(maxrow, tot);
-                sumrow += tot;
-                a.x0[i] = a.x[i];
-                a.x0[n + i] = a.x[n + i];
-                a.x0[2 * n + i] = a.x[2 * n + i];
+            s_pre[lane + 1] = incl;
+            if (lane == 0) s_pre[0] = 0;
+            s_lo[lane] = lo;
+            // bin coordinates and counts, for the images of exact_keep
+            if (lane < 3) {
+                s_geo[lane] = lane == 0 ? b0 : lane == 1 ? b1 : b2;
+                s_geo[3 + lane] = nb[lane];
             }
         }
-        __syncwarp();  // the stencil table is rewritten for the next bin
-    }
+        __syncthreads();
+        const int total = s_pre[32];
+        const bool one_tile = total <= kBuildTile;
+        for (int g0 = 0; g0 < na; g0 += kBuildHome) {
+            const int ng = min(kBuildHome, na - g0);
+            if (g0) __syncthreads();  // the previous group's atoms are no longer read
+            if (threadIdx.x < ng) {
+                float4 p = a.bin_pos[a0 + g0 + threadIdx.x];
+                cart(p);
+                home[threadIdx.x] = p;
+                s_cin[threadIdx.x] = s_cout[threadIdx.x] = 0;
+            }
+            for (int t0 = 0; t0 < total; t0 += kBuildTile) {
+                const int nt = min(kBuildTile, total - t0);
+                const bool last = t0 + kBuildTile >= total;
+                if (t0) __syncthreads();  // the previous tile is no longer read
+                if (!one_tile || g0 == 0)
+                    for (int k = threadIdx.x; k < ((nt + 31) & ~31); k += 32 * kBuildWarps) {
+                        float4 p = make_float4(1e18f, 0.f, 0.f, 0.f);
+                        if (k < nt) {
+                            const int t = t0 + k;
+                            int c = 0;  // the stencil bin of candidate t: s_pre[c] <= t < s_pre[c + 1]
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        maxrow = max(maxrow, __shfl_xor_sync(0xffffffffu, maxrow, o));
-        overflow |= __shfl_xor_sync(0xffffffffu, overflow, o);
-        sumrow += __shfl_xor_sync(0xffffffffu, sumrow, o);
+                            for (int o = 16; o > 0; o >>= 1)
+                                if (s_pre[c + o] <= t) c += o;
+                            p = a.bin_pos[s_lo[c] + (t - s_pre[c])];
+                            p.x += kBinW * (float)(c % 3 - 1);
+                            p.y += kBinW * (float)((c / 3) % 3 - 1);
+                            p.z += kBinW * (float)(c / 9 - 1);
+                            cart(p);
+                            p.w = __int_as_float(__float_as_int(p.w) | make_entry(0, 0, c));
+                        }
+                        cand[k] = p;
+                    }
+                __syncthreads();
+                for (int q = w; q < ng; q += kBuildWarps) {
+                    const float4 h = home[q];
+                    const int self = __float_as_int(h.w) | make_entry(0, 0, 13);  // the atom itself, unshifted
+                    const int i = entry_j(self);
+                    int* row = a.nbr + (size_t)i * a.maxnbr;
+                    int cin = 0, cout = 0, tot = kBuildRow + 1;
+                    if (one_tile) {
+                        build_scan<UNI>(a, cut, cand, nt, h, self, s_geo, h6, s_row[w], kBuildRow, cin, cout);
+                        tot = cin + cout;
+                        __syncwarp();
+                        if (tot <= min(kBuildRow, a.maxnbr))
+                            for (int k = lane; k < tot; k += 32) row[k] = s_row[w][k < cin ? k : kBuildRow - tot + k];
+                        __syncwarp();  // s_row is refilled for the warp's next atom
+                    }
+                    if (tot > kBuildRow) {
+                        if (one_tile)
+                            cin = cout = 0;
+                        else
+                            cin = s_cin[q], cout = s_cout[q];
+                        build_scan<UNI>(a, cut, cand, nt, h, self, s_geo, h6, row, a.maxnbr, cin, cout);
+                        tot = cin + cout;
+                        if (!last) {
+                            if (lane == 0) {
+                                s_cin[q] = cin;
+                                s_cout[q] = cout;
+                            }
+                            continue;
+                        }
+                        // the shell entries at the row's end move behind the
+                        // inner ones, 32 at a time, each batch read before
+                        // it is written (to lower slots: the gap is never
+                        // negative)
+                        __syncwarp();
+                        for (int k0 = 0; tot <= a.maxnbr && k0 < cout; k0 += 32) {
+                            const int k = k0 + lane;
+                            const int v = k < cout ? row[a.maxnbr - cout + k] : 0;
+                            __syncwarp();
+                            if (k < cout) row[cin + k] = v;
+                            __syncwarp();
+                        }
+                    }
+                    // a row that does not fit is built again with a larger
+                    // capacity
+                    if (lane == 0) a.nnbr[i] = min(tot, a.maxnbr);
+                    overflow |= tot > a.maxnbr;
+                    maxrow = max(maxrow, tot);
+                    sumrow += tot;
+                }
+            }
+        }
     }
     if (lane == 0) {
         if (overflow) sc->overflow = 1;
@@ -734,23 +755,10 @@ __global__ void __launch_bounds__(256) k_build_bins(BuildArgs a, int nbins, DevS
     }
 }
 
-__global__ void k_rebuild_done(DevScalars* sc) {
+// batch: the rebuilt cells' flags
+__global__ void k_rebuild_done_b(DevScalars* sc, uint8_t* cell_reb, int ncell) {
     if (!sc->rebuild) return;
-    sc->nrebuild++;
-    sc->drift[0] = sc->drift[1] = sc->drift[2] = 0.0;
-}
-
-__global__ void k_rebuild_done_b(DevScalars* sc, CellMd* cmd, uint8_t* cell_reb, int ncell) {
-    if (!sc->rebuild) return;
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell; c += gridDim.x * blockDim.x) {
-        if (!cell_reb[c]) continue;
-        cmd[c].drift[0] = cmd[c].drift[1] = cmd[c].drift[2] = 0.0;
-        cell_reb[c] = 0;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        sc->nrebuild++;
-        sc->drift[0] = sc->drift[1] = sc->drift[2] = 0.0;
-    }
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell; c += gridDim.x * blockDim.x) cell_reb[c] = 0;
 }
 
 // skin test of DynamicMD::decide (dynamic_md.cpp:90-105): rebuild when any
@@ -824,16 +832,12 @@ void request_rebuild(mappg_sys* s) {
     if (s->cell_reb) MAPPG_CUDA(cudaMemsetAsync(s->cell_reb, 1, s->ncell, s->stream));
 }
 
-void launch_shadow(mappg_sys* s, bool gated) {
-    if (s->ncell > 1) {
-        k_shadow_b<<<grid_for(s, s->n, 256), 256, 0, s->stream>>>(s->n, s->x, s->binc, s->cells_dev, s->cell_of,
-                                                                   s->p32, s->p0, gated ? 1 : 0, s->cell_reb, s->sc);
-        MAPPG_CUDA(cudaGetLastError());
-        return;
-    }
-    Geo g = make_geo(s);
-    k_shadow<<<grid_for(s, s->n, 256), 256, 0, s->stream>>>(s->n, s->x, s->binc, s->p32, s->p0, g, gated ? 1 : 0,
-                                                            s->sc);
+void launch_shadow(mappg_sys* s) {
+    const int gb = grid_for(s, s->n, 256);
+    if (s->ncell > 1)
+        k_shadow_b<<<gb, 256, 0, s->stream>>>(s->n, s->x, s->binc, s->cells_dev, s->cell_of, s->p32);
+    else
+        k_shadow<<<gb, 256, 0, s->stream>>>(s->n, s->x, s->binc, s->p32, make_geo(s));
     MAPPG_CUDA(cudaGetLastError());
 }
 
@@ -846,38 +850,30 @@ void launch_rebuild_chain(mappg_sys* s) {
     // all of its atoms
     const uint8_t* reb = batch ? s->cell_reb : nullptr;
     if (batch) {
-        k_wrap_bin_b<<<gb, B, 0, s->stream>>>(s->n, s->x, s->s, s->cells_dev, s->cell_of, s->cmd, s->binc, s->binid,
-                                              s->bin_count, s->cell_reb, s->sc);
+        k_wrap_bin_b<<<gb, B, 0, s->stream>>>(s->n, s->x, s->s, s->x0, s->cells_dev, s->cell_of, s->cmd, s->binc,
+                                              s->binid, s->bin_count, s->cell_reb, s->p32, s->p0, s->sc);
         k_scan_bins_b<<<(s->ncell * 32 + B - 1) / B, B, 0, s->stream>>>(s->ncell, s->n, s->nbins, s->cells_dev,
                                                                          s->cell_reb, s->bin_count, s->bin_start,
-                                                                         s->sc);
+                                                                         s->cmd, s->sc);
     } else {
-        k_wrap_bin<<<gb, B, 0, s->stream>>>(s->n, s->x, s->s, g, s->binc, s->binid, s->bin_count, s->sc);
+        k_wrap_bin<<<gb, B, 0, s->stream>>>(s->n, s->x, s->s, s->x0, g, s->binc, s->binid, s->bin_count, s->p32, s->p0,
+                                            s->sc);
         k_scan_bins<<<1, 1024, 0, s->stream>>>(s->nbins, s->bin_count, s->bin_start, s->sc);
     }
-    int* bin_tmp = s->bin_atoms + s->n;
-    k_scatter_bins<<<gb, B, 0, s->stream>>>(s->n, s->binid, s->bin_start, s->bin_count, bin_tmp, s->cell_of, reb,
+    k_scatter_bins<<<gb, B, 0, s->stream>>>(s->n, s->binid, s->bin_start, s->bin_count, s->bin_tmp, s->cell_of, reb,
                                             s->sc);
     k_sort_bins<<<grid_for(s, (long long)s->nbins * 32, B), B, 0, s->stream>>>(
-        s->nbins, s->bin_start, bin_tmp, s->bin_atoms, s->bin_count, s->cell_of, reb, s->sc);
-    if (batch)
-        k_shadow_b<<<gb, B, 0, s->stream>>>(s->n, s->x, s->binc, s->cells_dev, s->cell_of, s->p32, s->p0, 1,
-                                            s->cell_reb, s->sc);
-    else
-        k_shadow<<<gb, B, 0, s->stream>>>(s->n, s->x, s->binc, s->p32, s->p0, g, 1, s->sc);
+        s->nbins, s->bin_start, s->bin_tmp, s->p32, s->elem, s->bin_pos, s->bin_count, s->cell_of, reb, s->sc);
     BuildArgs a;
     a.n = s->n;
     a.maxnbr = s->maxnbr;
     a.ne = s->ne;
     a.x = s->x;
     a.s = s->s;
-    a.p32 = s->p32;
-    a.elem = s->elem;
+    a.bin_pos = s->bin_pos;
     a.bin_start = s->bin_start;
-    a.bin_atoms = s->bin_atoms;
     a.nbr = s->nbr;
     a.nnbr = s->nnbr;
-    a.x0 = s->x0;
     a.g = g;
     for (int p = 0; p < s->ne * s->ne; p++) {
         a.cut_sk_sq[p] = s->cut_sk_sq[p];
@@ -885,16 +881,20 @@ void launch_rebuild_chain(mappg_sys* s) {
         a.hi2[p] = (float)(s->cut_sk_sq[p] + s->band);
         a.in2[p] = (float)s->cut_sq[p];
     }
-    a.fr = s->frame;
+    memcpy(a.G, s->frame.G, sizeof(a.G));
     a.cells = s->cells_dev;
     a.cell_of = s->cell_of;
     a.cell_reb = reb;
-    const int gbins = grid_for(s, (long long)s->nbins * 32, B);
     bool uni = true;
     for (int p = 1; p < s->ne * s->ne; p++) uni = uni && a.lo2[p] == a.lo2[0] && a.hi2[p] == a.hi2[0];
     auto launch = [&](auto BT, auto OT, auto UT) {
-        k_build_bins<decltype(BT)::value, decltype(OT)::value, decltype(UT)::value>
-            <<<gbins, B, 0, s->stream>>>(a, s->nbins, s->sc);
+        constexpr auto kern = k_build_bins<decltype(BT)::value, decltype(OT)::value, decltype(UT)::value>;
+        static int per_sm = 0;
+        if (!per_sm) {
+            MAPPG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kBuildWarps, 0));
+            per_sm = std::max(per_sm, 1);
+        }
+        kern<<<std::min(s->nbins, per_sm * s->sm_count), 32 * kBuildWarps, 0, s->stream>>>(a, s->nbins, s->sc);
     };
     auto by_uni = [&](auto BT, auto OT) {
         if (uni)
@@ -907,13 +907,12 @@ void launch_rebuild_chain(mappg_sys* s) {
             by_uni(std::true_type(), std::true_type());
         else
             by_uni(std::true_type(), std::false_type());
-        k_rebuild_done_b<<<(s->ncell + 255) / 256, 256, 0, s->stream>>>(s->sc, s->cmd, s->cell_reb, s->ncell);
+        k_rebuild_done_b<<<(s->ncell + 255) / 256, 256, 0, s->stream>>>(s->sc, s->cell_reb, s->ncell);
     } else {
         if (s->frame.ortho)
             by_uni(std::false_type(), std::true_type());
         else
             by_uni(std::false_type(), std::false_type());
-        k_rebuild_done<<<1, 1, 0, s->stream>>>(s->sc);
     }
     MAPPG_CUDA(cudaGetLastError());
 }
@@ -1021,7 +1020,7 @@ static void dev_alloc(void** p, size_t bytes) { MAPPG_CUDA(cudaMalloc(p, bytes >
 
 void sys_free(mappg_sys* s) {
     void* ptrs[] = {s->x, s->v, s->f, s->x0, s->s, s->elem, s->id, s->inv, s->p32, s->q32, s->p0, s->f32, s->v32,
-                    s->rho32, s->binc, s->binid, s->bin_count, s->bin_start, s->bin_atoms, s->nbr, s->nnbr,
+                    s->rho32, s->binc, s->binid, s->bin_count, s->bin_start, s->bin_tmp, s->bin_pos, s->nbr, s->nnbr,
                     s->rho, s->dF, s->partials, s->sc, s->stage, s->thermo_dev, s->cells_dev, s->cell_of,
                     s->chunk_begin, s->chunk_cell, s->cell_chunk, s->chunk_part, s->chunk_disp, s->cmd,
                     s->cell_out, s->dof, s->stage2, s->cutmask, s->fs_tab, s->grp_atoms, s->cell_reb};
@@ -1095,7 +1094,8 @@ void sys_alloc(mappg_sys* s, const double* x_host) {
     if (s->precision == MAPPG_MIXED) dev_alloc((void**)&s->cutmask, sizeof(unsigned) * 32 * (size_t)n);
     dev_alloc((void**)&s->binc, sizeof(int) * n);
     dev_alloc((void**)&s->binid, sizeof(int) * n);
-    dev_alloc((void**)&s->bin_atoms, sizeof(int) * 2 * (size_t)n);
+    dev_alloc((void**)&s->bin_tmp, sizeof(int) * (size_t)n);
+    dev_alloc((void**)&s->bin_pos, sizeof(float4) * (size_t)n);
     dev_alloc((void**)&s->nnbr, sizeof(int) * n);
     dev_alloc((void**)&s->rho, sizeof(double) * n);
     dev_alloc((void**)&s->dF, sizeof(double) * n);

@@ -94,7 +94,6 @@ struct NhcParams {
 struct Frame {
     float G[3][3];     // Cartesian = dx' G (row vector), head
     float Glo[3][3];   // tail
-    float off[27][4];  // -8 d for code c (exact)
     int ortho;         // H has no off-diagonal terms
 };
 
@@ -272,7 +271,8 @@ struct mappg_sys {
     int* binid = nullptr;
     int* bin_count = nullptr;
     int* bin_start = nullptr;
-    int* bin_atoms = nullptr;
+    int* bin_tmp = nullptr;      // atoms by bin, any order
+    float4* bin_pos = nullptr;   // by bin in index order: frame position, w = the entry bits of atom and element
     int maxnbr = 0;
     int* nbr = nullptr;
     int* nnbr = nullptr;
@@ -348,7 +348,7 @@ void sys_set_cells(mappg_sys* s, int ncell, const int* natoms, const double* H);
 void sys_rechunk(mappg_sys* s, int chunk_atoms);  // a batch's chunks of at most chunk_atoms atoms
 void launch_rebuild_chain(mappg_sys* s);   // kernels gated by sc->rebuild
 void request_rebuild(mappg_sys* s);        // host sets the gate
-void launch_shadow(mappg_sys* s, bool gated);
+void launch_shadow(mappg_sys* s);          // frame positions of moved atoms
 void check_build(mappg_sys* s);            // host: overflow / capacity
 void launch_skin_test(mappg_sys* s);       // sets sc->rebuild if needed
 void sync_forces64(mappg_sys* s);          // f (FP64) from f32 when needed

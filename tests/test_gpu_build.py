@@ -1,0 +1,61 @@
+"""Neighbour sets of the list builder where its staging changes shape: rows
+and candidates beyond what a block holds on chip, bins of more atoms than a
+block takes at a time, empty bins, single atoms, tilted boxes.  The sets equal
+the oracle's exactly."""
+import numpy as np
+import pytest
+
+import oracle as O
+from mapp4py_gb300 import _lib, synth
+from test_gpu_parity import keys
+
+pytestmark = pytest.mark.gpu
+
+
+def _cell(kind):
+    rng = np.random.default_rng(17)
+    if kind == "wide":  # a reach of 10.5 A: ~400 entries a row, several tiles of candidates
+        c = synth.alloy((7, 6, 8), xB=0.5, sigma=0.1, seed=3)
+        return c.H, c.x, c.elem, 5.0
+    if kind == "wide_tilted":
+        H = np.array([[26.0, 0, 0], [3.0, 25.0, 0], [-2.0, 4.0, 27.0]])
+        return H, synth.wrap(H, rng.random((1400, 3)) @ H), (rng.random(1400) < 0.5).astype(np.uint8), 5.0
+    if kind == "cluster":  # one bin holds 300 atoms, all of them neighbours: rows of 299
+        x = 20.0 + rng.uniform(-1.4, 1.4, (300, 3))
+        return np.diag([43.0, 41.0, 40.0]), x, (rng.random(300) < 0.5).astype(np.uint8), 0.5
+    if kind == "gas":  # mostly empty bins, rows of 0 to a few entries
+        H = np.array([[61.0, 0, 0], [5.0, 55.0, 0], [0.0, -7.0, 50.0]])
+        return H, rng.random((257, 3)) @ H, (rng.random(257) < 0.5).astype(np.uint8), 0.5
+    if kind == "one":  # an atom and its own images
+        return np.diag([6.6, 7.0, 9.0]), np.array([[6.5, 0.1, 4.0]]), np.zeros(1, np.uint8), 0.9
+    raise KeyError(kind)
+
+
+@pytest.mark.parametrize("precision", [_lib.FP64, _lib.MIXED])
+@pytest.mark.parametrize("kind", ["wide", "wide_tilted", "cluster", "gas", "one"])
+def test_neighbor_sets_at_the_builders_edges(potentials, kind, precision):
+    path, _ = potentials[("A", "B")]
+    H, x, elem, skin = _cell(kind)
+    masses = [synth.MASS, synth.MASS]
+    o = O.System(O.Eam.setfl(path), H, x, elem, masses, skin=skin, pair_wise=False)
+    o.init_dynamic()
+    s = _lib.System(_lib.ForceField.setfl(path), H, x, elem, masses, skin=skin, precision=precision)
+    s.build()
+    assert np.array_equal(keys(*s.neighbors()), keys(*o.neighbors()))
+
+
+def test_batch_rows_equal_single_cells_at_the_builders_edges(potentials):
+    path, _ = potentials[("A", "B")]
+    ff = _lib.ForceField.setfl(path)
+    masses = [synth.MASS, synth.MASS]
+    cells = [_cell(k)[:3] for k in ("wide", "cluster", "gas", "wide_tilted")]
+    b = _lib.Batch(ff, cells, masses, skin=5.0)
+    b.build()
+    cnt, ent = b.neighbors()
+    at = np.concatenate([[0], np.cumsum(cnt)])
+    for k, (H, x, elem) in enumerate(cells):
+        lo, hi = b.offsets[k], b.offsets[k + 1]
+        e = ent[at[lo]:at[hi]].copy()
+        e[:, 0] -= lo
+        s = _lib.System(ff, H, x, elem, masses, skin=5.0, precision=_lib.MIXED)
+        assert np.array_equal(keys(cnt[lo:hi], e), keys(*s.neighbors()))
