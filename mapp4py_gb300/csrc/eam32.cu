@@ -989,6 +989,7 @@ __global__ void k_cells_done(EamArgs a, const int* __restrict__ cell_chunk, Cell
     if (what == 2) {
         NhcParams P = a.nhc;
         P.T = m->T;
+        P.T_inv = 1.0 / m->T;
         P.ndof = (int)m->ndof;
         P.ndof_kB = m->ndof_kB;
         for (int k = 0; k < 6; k++) m->mvv[k] = t[7 + k];

@@ -119,43 +119,59 @@ __device__ __forceinline__ T warp_reduce(T (&v)[P], Op op) {
     return t;
 }
 
-// one row of up to eight doubles per warp, shared by the sums of a kernel
-__device__ __forceinline__ double (*red_rows())[8] {
-    __shared__ double red[32][8];
+// one row of P doubles (room for 8 or 16) per warp, shared by the sums of a
+// kernel
+constexpr int red_width(int p) { return p <= 8 ? 8 : 16; }
+template <int W>
+__device__ __forceinline__ double (*red_rows())[W] {
+    __shared__ double red[32][W];
     return red;
 }
 
-// block totals of K values of type T: the warps' totals go to red_rows, and
-// thread k < K gets value k as a double
+// the sum of the block's rows of P values in red_rows, by the first warp:
+// lane k < P returns value k (a dependent FP64 add takes 65 clocks here, so
+// the lanes share the rows and add up pairwise)
+template <int P>
+__device__ __forceinline__ double rows_sum() {
+    double(*red)[red_width(P)] = red_rows<red_width(P)>();
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    double t = 0.0;
+    for (int q = lane / P; q < nw; q += 32 / P) t += red[q][lane % P];
+#pragma unroll
+    for (int o = P; o < 32; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
+}
+
+// block totals of K values of type T, as doubles: value k in lane k of the
+// first warp
 template <int K, class T>
 __device__ __forceinline__ double block_sums(const T (&v)[K]) {
     constexpr int P = red_pow2(K);
-    static_assert(P <= 8, "red_rows holds eight values");
-    double(*red)[8] = red_rows();
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    static_assert(P <= 16, "a row holds 16 values");
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     T u[P];
 #pragma unroll
     for (int k = 0; k < P; k++) u[k] = k < K ? v[k < K ? k : 0] : red_zero<T>();
     const T t = warp_reduce(u, RedAdd());
-    if (lane % (32 / P) == 0) red[w][lane / (32 / P)] = red_double(t);
+    if (lane % (32 / P) == 0) red_rows<red_width(P)>()[w][lane / (32 / P)] = red_double(t);
     __syncthreads();
-    double r = 0.0;
-    if (threadIdx.x < K)
-        for (int q = 0; q < nw; q++) r += red[q][threadIdx.x];
-    return r;
+    return w == 0 ? rows_sum<P>() : 0.0;
 }
 
-// thread 0 of the first warp, whose threads stored the block's partials,
-// counts the block in; true in every thread of the block that came last
+// the first warp, whose lanes stored the block's partials, counts the block
+// in; true in every thread of the block that came last, which then sees all
+// blocks' partials
 __device__ __forceinline__ bool last_block(unsigned* counter) {
     __shared__ bool last;
     if (threadIdx.x < 32) {
         __threadfence();
         __syncwarp();
-        if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
+        if (threadIdx.x == 0) {
+            last = atomicAdd(counter, 1u) == gridDim.x - 1;
+            if (last) __threadfence();
+        }
     }
     __syncthreads();
-    if (last) __threadfence();
     return last;
 }
 
@@ -173,26 +189,43 @@ __device__ bool block_partials(const T (&v)[K], double* partials, int slot0, uns
 
 // sums of the first K partial slots over nblk blocks by the whole block, in
 // a fixed order, into tot[0..K-1] (shared memory, ready for every thread on
-// return)
+// return); four rows per thread are loaded at a time.  nblk8: the rows of
+// slots 8 and up, where another kernel's blocks left them (-1: nblk)
 template <int K>
-__device__ void final_sums(const double* partials, int nblk, double* tot) {
+__device__ void final_sums(const double* partials, int nblk, double* tot, int nblk8 = -1) {
     constexpr int P = red_pow2(K);
-    double(*red)[8] = red_rows();
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    if (K > 8 && nblk8 >= 0 && threadIdx.x % P >= 8) nblk = nblk8;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int k = threadIdx.x % P, rows = blockDim.x / P;
     double t = 0.0;
-    if (k < K)
-        for (int b = threadIdx.x / P; b < nblk; b += rows) t += __ldcg(partials + b * kRedSlots + k);
+    for (int b0 = threadIdx.x / P; b0 < nblk; b0 += 4 * rows) {
+        double u[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int b = b0 + q * rows;
+            u[q] = k < K && b < nblk ? __ldcg(partials + b * kRedSlots + k) : 0.0;
+        }
+        t += (u[0] + u[1]) + (u[2] + u[3]);
+    }
 #pragma unroll
     for (int o = P; o < 32; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (lane < P) red[w][lane] = t;
+    if (lane < P) red_rows<red_width(P)>()[w][lane] = t;
     __syncthreads();
-    if (threadIdx.x < K) {
-        double r = 0.0;
-        for (int q = 0; q < nw; q++) r += red[q][threadIdx.x];
-        tot[threadIdx.x] = r;
+    if (w == 0) {
+        const double r = rows_sum<P>();
+        if (lane < K) tot[lane] = r;
     }
     __syncthreads();
+}
+
+// mixed MD: the mean displacement not yet removed from x, in every thread of
+// the block: what earlier steps left in sc->drift, and the running step's
+// per-block sums in slots 8-10 of the first `rows` partial rows (0: none)
+__device__ inline void drift_now(const DevScalars* sc, const double* partials, int rows, double n_inv,
+                                 double (&d)[3]) {
+    __shared__ double tot[3];
+    if (rows) final_sums<3>(partials + 8, rows, tot);
+    for (int c = 0; c < 3; c++) d[c] = sc->drift[c] + (rows ? tot[c] * n_inv : 0.0);
 }
 
 // block sums of K values (as block_partials) into out[0..K-1], one batch chunk

@@ -3,31 +3,34 @@
 // One step of MDNVT::run (md_nvt.cpp:409-438) is a fixed kernel sequence,
 // captured once into a CUDA graph and replayed.
 //
-// FP64 path (the reference's operation order, f*dt2/m with a division and no
-// fused multiply-adds, so the trajectory follows the oracle to rounding):
-//   k_step_open      fac_x_d *= chain(T/T0), the opening thermostat half
+// FP64 path (the reference's operation order without fused multiply-adds,
+// f*(dt2/m) for its f*dt2/m, so the trajectory follows the oracle to rounding;
+// three FP64 divisions an atom cost more than the rest of a kick):
 //   k_kick_drift64   v = v*fac_x_d + f*dt2/m; x += v*dt; sum of v*dt
-//                    (update_x_d__x, md_nvt.cpp:70-102)
+//                    (update_x_d__x, md_nvt.cpp:70-102); fac_x_d holds the
+//                    opening thermostat half, chain(T/T0)
 //   k_com_skin64     x -= mean displacement; skin test (DynamicMD::decide,
 //                    dynamic_md.cpp:90-105) opens the rebuild gate
 //   rebuild chain    (system.cu) only when the gate is open
 //   density, force   (eam.cu)
 //   k_kick2_64       v += f*dt2/m, kinetic tensor (update_x_d,
-//                    md_nvt.cpp:106-128), closing thermostat half, thermo row
+//                    md_nvt.cpp:106-128), closing thermostat half, thermo
+//                    row, and the next step's opening half
 //
 // Mixed path (FP64 state, fewer FP64 instructions; GB300 runs FP64 at a
 // small fraction of FP32):
-//   k_step_open32    opening half; the pending closing kick of the previous
-//                    step and this step's kick fold into v <- A v + B f dt/2m
-//                    (A = fc*fo, B = 1 + fc*fo; A = fo, B = 1 on the first)
-//   k_integrate32    that kick, x += v dt (FP64), v32 = (float)v, the frame
+//   k_integrate32    the pending closing kick of the previous step and this
+//                    step's kick as one, v <- A v + B f dt/2m (A = fc*fo,
+//                    B = 1 + fc*fo; A = fo, B = 1 on the first), fo the
+//                    opening half; x += v dt (FP64), v32 = (float)v, the frame
 //                    position p32 from x, the FP32 skin test and the
-//                    displacement sum; the mean displacement is accumulated
-//                    in sc->drift and removed from x at the next rebuild and
+//                    displacement sums; the mean displacement is accumulated
+//                    in sc->drift (k_close32) and removed from x at the next rebuild and
 //                    at the end of the run (a uniform shift leaves forces and
 //                    energies unchanged)
-//   rebuild chain, k_density32, k_force32 with the MD tail (kinetic tensor of
-//   v + f dt/2m, closing half, thermo row)
+//   rebuild chain, k_density32, k_force32
+//   k_close32        kinetic tensor of v + f dt/2m, closing half, thermo row,
+//                    the next step's opening half
 // Velocity scaling stays lazy as in the reference: the chain's factor is
 // folded into the next kick and applied at the end of the run
 // (update_x_d_final, md_nvt.cpp:51-56).
@@ -63,7 +66,8 @@ struct MdArgs {
     double dtm[kMaxElem];  // dt2/m
     float dtm32[kMaxElem];
     float m32[kMaxElem];   // masses as floats (the kinetic tensors' FP32 products)
-    double dt, dt2, skin_sq;
+    double dt, dt2, n_inv, skin_sq;
+    int drift_rows;        // mixed: blocks of k_integrate32
     float dt32, skin_sq32;
     double bs[6];          // x -> scaled frame
     Frame fr;
@@ -89,6 +93,7 @@ struct MdArgs {
 __device__ __forceinline__ NhcParams cell_nhc(const NhcParams& P0, const CellMd* m) {
     NhcParams P = P0;
     P.T = m->T;
+    P.T_inv = 1.0 / m->T;
     P.ndof = (int)m->ndof;
     P.ndof_kB = m->ndof_kB;
     return P;
@@ -120,26 +125,115 @@ __global__ void k_mvv_init(MdArgs a) {
         final_sums<6>(a.partials, gridDim.x, t);
         if (threadIdx.x == 0) {
             for (int k = 0; k < 6; k++) a.sc->mvv[k] = t[k];
-            a.sc->T_part = (t[0] + (t[3] + t[5])) / a.nhc.ndof_kB;
+            a.sc->T_part = (t[0] + (t[3] + t[5])) * a.nhc.ndof_kB_inv;
             a.sc->counter[3] = 0;
             a.sc->step = 0;
         }
     }
 }
 
-// run start: thermo row 0, no pending velocity scale or kick
+// What the last block of a step's closing kernel does with the kinetic
+// tensor mvv of the step (MDNVT::run, md_nvt.cpp:427-432, then 409-412 of the
+// next step): the closing half of the thermostat, the thermo row, and the
+// next step's opening half, taken ahead by the thread that has just closed
+// this one.  The chain state before that opening half stays in sc->eta (the
+// run may end here, and exports read it), the one after it in sc->eta_next.
+// The device scalars it needs are read at the start of the kernel (load),
+// and a thread that waits for the block to be counted in forms what the chain
+// can without the temperature (pre): the serial part is the chain's latency.
+struct CloseStep {
+    double eta[kMaxChain], ev[7], T, fac;
+    long long step;
+    Chain3 c;
+    __device__ __forceinline__ static bool three(const MdArgs& a) { return a.nhc.L == 3 && a.nhc.niters == 1; }
+    __device__ __forceinline__ void load(const DevScalars* sc) {
+        const int t = threadIdx.x;
+        if (t < kMaxChain) eta[t] = sc->eta_next[t];
+        if (t >= kMaxChain && t < kMaxChain + 7) ev[t - kMaxChain] = t == kMaxChain ? sc->energy : sc->virial[t - kMaxChain - 1];
+        if (t == 31) step = sc->step;
+    }
+    __device__ __forceinline__ void pre(const MdArgs& a) {
+        if (three(a)) c.pre(a.nhc, eta);
+    }
+    // one half on eta (one thread); c.pre is done
+    __device__ __forceinline__ double half(const MdArgs& a, double T_r) {
+        if (three(a)) {
+            const double f = c.post(a.nhc, T_r);
+            if (c.in_range) {
+                eta[0] = c.e0;
+                eta[1] = c.e1;
+                eta[2] = c.e2;
+                return f;
+            }
+        }
+        return nhc_any(a.nhc, eta, T_r);
+    }
+    // first warp of the block; returns the closing factor
+    __device__ __forceinline__ double close(const MdArgs& a, const double* mvv) {
+        const int lane = threadIdx.x;
+        DevScalars* sc = a.sc;
+        if (lane == 0) {
+            T = (mvv[0] + (mvv[3] + mvv[5])) * a.nhc.ndof_kB_inv;
+            fac = half(a, T * a.nhc.T_inv);
+            T *= fac * fac;
+        }
+        __syncwarp();
+        const double f2 = fac * fac;
+        const long long st = step + 1;
+        if (lane < kMaxChain) sc->eta[lane] = eta[lane];
+        if (a.thermo && st <= a.nsteps && lane < 14)
+            a.thermo[14 * st + lane] = lane == 0   ? ev[0]
+                                       : lane == 1 ? T
+                                       : lane < 8  ? mvv[lane - 2] * f2
+                                                   : ev[lane - 7];
+        if (lane == 0) {
+            sc->step = st;
+            if (!(isfinite(ev[0]) && isfinite(T))) sc->bad = 1;
+        }
+        __syncwarp();
+        return fac;
+    }
+    // lane 0: the opening factor of the next step, whose list check starts anew
+    __device__ __forceinline__ double open(const MdArgs& a) {
+        pre(a);
+        const double fo = half(a, T * a.nhc.T_inv);
+        for (int k = 0; k < a.nhc.L; k++) a.sc->eta_next[k] = eta[k];
+        a.sc->rebuild = 0;
+        return fo;
+    }
+};
+
+// block_partials of a kernel that ends a step: a thread of the second warp
+// does S.pre while the first counts the block in
+template <int K, class T>
+__device__ __forceinline__ bool close_partials(const T (&v)[K], const MdArgs& a, unsigned* counter, CloseStep& S) {
+    const double t = block_sums<K>(v);
+    if (threadIdx.x < K) a.partials[blockIdx.x * kRedSlots + threadIdx.x] = t;
+    if (threadIdx.x == 32) S.pre(a);
+    return last_block(counter);
+}
+
+// run start: thermo row 0, no pending velocity scale or kick, the first
+// step's opening half
 __global__ void k_run_begin(MdArgs a) {
-    write_thermo_row(a.thermo, a.sc, 0);
-    a.sc->fac_x_d = 1.0;
-    a.sc->pending_kick = 0;
+    DevScalars* sc = a.sc;
+    write_thermo_row(a.thermo, sc, 0);
+    double eta[kMaxChain];
+    for (int k = 0; k < a.nhc.L; k++) eta[k] = sc->eta[k];
+    const double fo = nhc_step(a.nhc, eta, sc->T_part * a.nhc.T_inv);
+    for (int k = 0; k < a.nhc.L; k++) sc->eta_next[k] = eta[k];
+    sc->fac_x_d = 1.0;
+    sc->fac_next = fo;
+    sc->pending_kick = 0;
+    sc->kickA = fo;
+    sc->kickB = 1.0;
+    sc->rebuild = 0;
 }
 
 // ------------------------------------------------------------------ FP64 path
-__global__ void k_step_open(MdArgs a) { a.sc->fac_x_d *= thermo_half(a.nhc, a.sc); }
-
 __global__ void __launch_bounds__(256) k_kick_drift64(MdArgs a) {
     const int n = a.n;
-    const double fac = a.sc->fac_x_d;
+    const double fac = a.sc->fac_next;
     double dsum[3] = {0, 0, 0};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int e = a.elem[i];
@@ -149,7 +243,7 @@ __global__ void __launch_bounds__(256) k_kick_drift64(MdArgs a) {
             double vv = a.v[c * n + i], ff = a.f[c * n + i], xx = a.x[c * n + i];
             // a frozen component keeps its velocity and still drifts
             // (update_x_d__x_w_dof, md_nvt.cpp:144-180)
-            if ((b >> c) & 1u) vv = __dadd_rn(__dmul_rn(vv, fac), __ddiv_rn(__dmul_rn(ff, a.dt2), a.masses[e]));
+            if ((b >> c) & 1u) vv = __dadd_rn(__dmul_rn(vv, fac), __dmul_rn(ff, a.dtm[e]));
             double dx = __dmul_rn(vv, a.dt);
             dsum[c] = __dadd_rn(dsum[c], dx);
             xx = __dadd_rn(xx, dx);
@@ -161,9 +255,7 @@ __global__ void __launch_bounds__(256) k_kick_drift64(MdArgs a) {
     if (block_partials<3>(dsum, a.partials, 0, &a.sc->counter[4])) {
         final_sums<3>(a.partials, gridDim.x, t);
         if (threadIdx.x == 0) {
-            double natms = (double)n;
-            for (int c = 0; c < 3; c++) a.sc->com[c] = a.com_on[c] ? t[c] / natms : 0.0;
-            a.sc->rebuild = 0;
+            for (int c = 0; c < 3; c++) a.sc->com[c] = a.com_on[c] ? t[c] * a.n_inv : 0.0;
             a.sc->counter[4] = 0;
         }
     }
@@ -187,6 +279,8 @@ __global__ void __launch_bounds__(256) k_com_skin64(MdArgs a) {
 
 __global__ void __launch_bounds__(256) k_kick2_64(MdArgs a) {
     const int n = a.n;
+    __shared__ CloseStep S;
+    S.load(a.sc);
     double d[6] = {0, 0, 0, 0, 0, 0};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int e = a.elem[i];
@@ -199,7 +293,7 @@ __global__ void __launch_bounds__(256) k_kick2_64(MdArgs a) {
             // neither kicked nor counted in the kinetic tensor
             if ((b >> c) & 1u) {
                 double v0 = a.v[c * n + i], ff = a.f[c * n + i];
-                v0 = __dadd_rn(v0, __ddiv_rn(__dmul_rn(ff, a.dt2), m));
+                v0 = __dadd_rn(v0, __dmul_rn(ff, a.dtm[e]));
                 a.v[c * n + i] = v0;
                 vv[c] = v0;
             } else {
@@ -214,17 +308,15 @@ __global__ void __launch_bounds__(256) k_kick2_64(MdArgs a) {
         d[5] += __dmul_rn(__dmul_rn(vv[2], vv[2]), m);
     }
     __shared__ double t[6];
-    if (block_partials<6>(d, a.partials, 0, &a.sc->counter[5])) {
+    if (close_partials<6>(d, a, &a.sc->counter[5], S)) {
         final_sums<6>(a.partials, gridDim.x, t);
-        if (threadIdx.x == 0) {
-            DevScalars* sc = a.sc;
-            for (int k = 0; k < 6; k++) sc->mvv[k] = t[k];
-            sc->T_part = (t[0] + (t[3] + t[5])) / a.nhc.ndof_kB;
-            sc->fac_x_d = thermo_half(a.nhc, sc);
-            long long st = ++sc->step;
-            if (st <= a.nsteps) write_thermo_row(a.thermo, sc, st);
-            if (!(isfinite(sc->energy) && isfinite(sc->T_part))) sc->bad = 1;
-            sc->counter[5] = 0;
+        if (threadIdx.x < 32) {
+            const double fac = S.close(a, t);
+            if (threadIdx.x == 0) {
+                a.sc->fac_x_d = fac;
+                a.sc->fac_next = fac * S.open(a);
+                a.sc->counter[5] = 0;
+            }
         }
     }
 }
@@ -237,20 +329,6 @@ __global__ void k_run_end64(MdArgs a) {
 }
 
 // ------------------------------------------------------------------ mixed path
-__global__ void k_step_open32(MdArgs a) {
-    DevScalars* sc = a.sc;
-    const double fo = thermo_half(a.nhc, sc);
-    if (sc->pending_kick) {
-        const double F = sc->fac_close * fo;
-        sc->kickA = F;
-        sc->kickB = 1.0 + F;
-    } else {
-        sc->kickA = fo;
-        sc->kickB = 1.0;
-    }
-    sc->rebuild = 0;
-}
-
 template <bool ORTHO>
 __global__ void __launch_bounds__(256) k_integrate32(MdArgs a) {
     const int n = a.n;
@@ -306,28 +384,21 @@ __global__ void __launch_bounds__(256) k_integrate32(MdArgs a) {
         moved |= fmaf(cx, cx, fmaf(cy, cy, cz * cz)) > a.skin_sq32;
     }
     if (__syncthreads_or(moved) && threadIdx.x == 0) a.sc->rebuild = 1;
-    const float dv[3] = {dsum0, dsum1, dsum2};
-    __shared__ double t[3];
-    if (block_partials<3>(dv, a.partials, 0, &a.sc->counter[4])) {
-        final_sums<3>(a.partials, gridDim.x, t);
-        if (threadIdx.x == 0) {
-            const double natms = (double)n;
-            for (int c = 0; c < 3; c++) {
-                a.sc->com[c] = a.com_on[c] ? t[c] / natms : 0.0;
-                a.sc->drift[c] += a.sc->com[c];
-            }
-            a.sc->pending_kick = 0;
-            a.sc->counter[4] = 0;
-        }
-    }
+    // the block's displacement sum; k_close32 adds the blocks' up, and a
+    // rebuild or the run's last export before that (drift_now)
+    const float dv[3] = {a.com_on[0] ? dsum0 : 0.f, a.com_on[1] ? dsum1 : 0.f, a.com_on[2] ? dsum2 : 0.f};
+    const double t = block_sums<3>(dv);
+    if (threadIdx.x < 3) a.partials[blockIdx.x * kRedSlots + 8 + threadIdx.x] = t;
 }
 
 // update_x_d (md_nvt.cpp:106-128) and the closing half of the thermostat
 // (md_nvt.cpp:427-432) of a mixed step: kinetic tensor of the half-kicked
 // velocity v + f dt/2m (FP32 terms, FP64 sums), then in the last block the
-// chain, the pending kick and the thermo row
+// mean displacement of the step and what CloseStep does
 __global__ void __launch_bounds__(256) k_close32(MdArgs a) {
     const int n = a.n;
+    __shared__ CloseStep S;
+    S.load(a.sc);
     float k0 = 0.f, k1 = 0.f, k2 = 0.f, k3 = 0.f, k4 = 0.f, k5 = 0.f;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int e = a.elem[i];
@@ -350,19 +421,23 @@ __global__ void __launch_bounds__(256) k_close32(MdArgs a) {
         k5 = fmaf(mz, vz, k5);
     }
     const float d[6] = {k0, k1, k2, k3, k4, k5};
-    __shared__ double t[6];
-    if (block_partials<6>(d, a.partials, 0, &a.sc->counter[5])) {
-        final_sums<6>(a.partials, gridDim.x, t);
-        if (threadIdx.x == 0) {
-            DevScalars* sc = a.sc;
-            for (int k = 0; k < 6; k++) sc->mvv[k] = t[k];
-            sc->T_part = (t[0] + (t[3] + t[5])) / a.nhc.ndof_kB;
-            sc->fac_close = thermo_half(a.nhc, sc);
-            sc->pending_kick = 1;
-            long long st = ++sc->step;
-            if (st <= a.nsteps) write_thermo_row(a.thermo, sc, st);
-            if (!(isfinite(sc->energy) && isfinite(sc->T_part))) sc->bad = 1;
-            sc->counter[5] = 0;
+    __shared__ double t[11];
+    if (close_partials<6>(d, a, &a.sc->counter[5], S)) {
+        // the kinetic tensor in t[0..5], k_integrate32's displacement sums
+        // in t[8..10]
+        final_sums<11>(a.partials, gridDim.x, t, a.drift_rows);
+        for (int q = threadIdx.x; q < 3 * a.drift_rows; q += blockDim.x) a.partials[(q / 3) * kRedSlots + 8 + q % 3] = 0.0;
+        if (threadIdx.x < 32) {
+            const double fac = S.close(a, t);
+            if (threadIdx.x < 3) a.sc->drift[threadIdx.x] += t[8 + threadIdx.x] * a.n_inv;
+            if (threadIdx.x == 0) {
+                a.sc->fac_close = fac;
+                a.sc->pending_kick = 1;
+                const double F = fac * S.open(a);
+                a.sc->kickA = F;
+                a.sc->kickB = 1.0 + F;
+                a.sc->counter[5] = 0;
+            }
         }
     }
 }
@@ -468,7 +543,7 @@ __global__ void k_cells_begin(MdArgs a) {
     }
 }
 
-// opening half of every cell's chain and its kick factors (k_step_open32)
+// opening half of every cell's chain and its kick factors (open_ahead)
 __global__ void k_cells_open(MdArgs a) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c == 0) a.sc->rebuild = 0;
@@ -609,6 +684,7 @@ static MdArgs md_args(mappg_sys* s, double T, double dt, double kB, double t_rel
     a.p0 = s->p0;
     a.dt = dt;
     a.dt2 = dt / 2.0;
+    a.n_inv = 1.0 / (double)s->n;
     a.dt32 = (float)dt;
     for (int e = 0; e < s->ne; e++) {
         a.masses[e] = s->masses[e];
@@ -634,6 +710,7 @@ static MdArgs md_args(mappg_sys* s, double T, double dt, double kB, double t_rel
     // ThermostatNHC(dt/2, t_relax, L, niters)  md_nvt.cpp:19, thermostat.cpp:20-36
     const double tdt = dt / 2.0;
     a.nhc.T = T;
+    a.nhc.T_inv = 1.0 / T;
     a.nhc.ddt = tdt / (double)niters;
     a.nhc.ddt2 = 0.5 * tdt / (double)niters;
     a.nhc.freq_sq = 1.0 / (t_relax * t_relax);
@@ -645,6 +722,8 @@ static MdArgs md_args(mappg_sys* s, double T, double dt, double kB, double t_rel
     a.nhc.ndof = 3 * s->n - (s->dof_frozen[0] + s->dof_frozen[1] + s->dof_frozen[2]);
     for (int c = 0; c < 3; c++) a.com_on[c] = s->dof_frozen[c] == 0;
     a.nhc.ndof_kB = a.nhc.ndof * kB;
+    a.nhc.ndof_kB_inv = 1.0 / a.nhc.ndof_kB;
+    a.nhc.ndof_d = (double)a.nhc.ndof;
     a.nhc.L = L;
     a.nhc.niters = niters;
     a.sc = s->sc;
@@ -662,35 +741,53 @@ static MdArgs md_args(mappg_sys* s, double T, double dt, double kB, double t_rel
     return a;
 }
 
-// mark: record s->ev_main once the step's positions are final (after the
-// list check; the passes after it do not move the atoms)
-static void launch_step64(mappg_sys* s, const MdArgs& a, bool mark = false) {
-    int g = grid_for(s, s->n, 256);
-    k_step_open<<<1, 1, 0, s->stream>>>(a);
-    k_kick_drift64<<<g, 256, 0, s->stream>>>(a);
-    k_com_skin64<<<g, 256, 0, s->stream>>>(a);
-    launch_rebuild_chain(s);
-    if (mark) MAPPG_CUDA(cudaEventRecord(s->ev_main, s->stream));
-    launch_force(s);
-    k_kick2_64<<<g, 256, 0, s->stream>>>(a);
+// launch shapes of the streaming MD kernels.  FP64 work per atom (wide): a
+// small system is spread over all SMs, 64 threads a block and up, as the FP64
+// pipe of an SM is what its atoms wait for.  FP32 work and one reduction:
+// blocks of 256, few partials.  A large system takes four blocks of 256 per
+// SM, which keep loads in flight and the sum over the blocks' partials short.
+struct MdShape {
+    int grid, block;
+};
+static MdShape md_shape(const mappg_sys* s, bool wide) {
+    const int per = ((s->n + s->sm_count - 1) / s->sm_count + 31) / 32 * 32;
+    const int block = wide ? std::max(64, std::min(256, per)) : 256;
+    return {std::max(1, std::min((s->n + block - 1) / block, 4 * s->sm_count)), block};
 }
 
-static void launch_step32(mappg_sys* s, const MdArgs& a, bool mark = false) {
-    // streaming kernels with a last-block reduction: four blocks per SM keep
-    // loads in flight and the serial tail (the fixed-order sum over block
-    // partials) short
-    int g = std::min(grid_for(s, s->n, 256), 4 * s->sm_count);
-    k_step_open32<<<1, 1, 0, s->stream>>>(a);
-    if (a.fr.ortho)
-        k_integrate32<true><<<g, 256, 0, s->stream>>>(a);
-    else
-        k_integrate32<false><<<g, 256, 0, s->stream>>>(a);
+struct NoHook {
+    void operator()() const {}
+};
+
+// listed() is called once the step's positions are final (after the list
+// check; the passes after it do not move the atoms), closing() before the
+// kernel that closes the step
+template <class A = NoHook, class B = NoHook>
+static void launch_step64(mappg_sys* s, const MdArgs& a, A listed = A(), B closing = B()) {
+    const MdShape m = md_shape(s, true);
+    k_kick_drift64<<<m.grid, m.block, 0, s->stream>>>(a);
+    k_com_skin64<<<m.grid, m.block, 0, s->stream>>>(a);
     launch_rebuild_chain(s);
-    if (mark) MAPPG_CUDA(cudaEventRecord(s->ev_main, s->stream));
+    listed();
+    launch_force(s);
+    closing();
+    k_kick2_64<<<m.grid, m.block, 0, s->stream>>>(a);
+}
+
+template <class A = NoHook, class B = NoHook>
+static void launch_step32(mappg_sys* s, const MdArgs& a, A listed = A(), B closing = B()) {
+    const MdShape m = md_shape(s, true), c = md_shape(s, false);
+    if (a.fr.ortho)
+        k_integrate32<true><<<m.grid, m.block, 0, s->stream>>>(a);
+    else
+        k_integrate32<false><<<m.grid, m.block, 0, s->stream>>>(a);
+    launch_rebuild_chain(s);
+    listed();
     EamArgs e = eam_args(s);
     launch_density32(s, e);
     launch_force32(s, e);
-    k_close32<<<g, 256, 0, s->stream>>>(a);
+    closing();
+    k_close32<<<c.grid, c.block, 0, s->stream>>>(a);
 }
 
 static void launch_step32b(mappg_sys* s, const MdArgs& a) {
@@ -733,6 +830,7 @@ static void run_clear(mappg_sys* s) {
     if (r->graph_many) cudaGraphDestroy(r->graph_many);
     delete r;
     s->run = nullptr;
+    s->drift_rows = 0;
 }
 
 void nvt_free(mappg_sys* s) { run_clear(s); }
@@ -846,8 +944,9 @@ void nvt_begin(mappg_sys* s, double T, double dt, double kB, double t_relax, int
     // the list and the opening force do not read velocities: an upload of
     // them on the side stream (nvt_run_host) overlaps them and is joined here
     sys_join_side(s);
-    k_mvv_init<<<g, 256, 0, s->stream>>>(a);
+    k_mvv_init<<<md_shape(s, true).grid, md_shape(s, true).block, 0, s->stream>>>(a);
     k_run_begin<<<1, 1, 0, s->stream>>>(a);
+    if (s->precision == MAPPG_MIXED) s->drift_rows = a.drift_rows = md_shape(s, true).grid;
     MAPPG_CUDA(cudaGetLastError());
     if (nsteps < kGraphMinSteps) return;  // nvt_steps launches the kernels itself
     MAPPG_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
@@ -979,8 +1078,11 @@ void nvt_snapshot(mappg_sys* s, double* x, double* v) {
 // positions in the caller's order less the mean displacement not yet
 // removed (sc->drift; zero on the FP64 path): what the run's end leaves in x
 __global__ void k_scatter_x_final(int n, const int* __restrict__ id, const double* __restrict__ x,
-                                  const DevScalars* __restrict__ sc, double* __restrict__ out) {
-    const double d0 = sc->drift[0], d1 = sc->drift[1], d2 = sc->drift[2];
+                                  const DevScalars* __restrict__ sc, const double* __restrict__ partials, int rows,
+                                  double n_inv, double* __restrict__ out) {
+    double d[3];
+    drift_now(sc, partials, rows, n_inv, d);
+    const double d0 = d[0], d1 = d[1], d2 = d[2];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const size_t u = 3 * (size_t)id[i];
         out[u] = x[i] - d0;
@@ -1000,16 +1102,22 @@ void nvt_run_xout(mappg_sys* s, double T, double dt, double kB, double t_relax, 
     NvtRun* r = (NvtRun*)s->run;
     if (nsteps > 0) {
         nvt_steps(s, nsteps - 1);
+        auto gather = [&] {
+            MAPPG_CUDA(cudaEventRecord(s->ev_main, s->stream));
+            MAPPG_CUDA(cudaStreamWaitEvent(s->side, s->ev_main, 0));
+            k_scatter_x_final<<<grid_for(s, s->n, 256), 256, 0, s->side>>>(s->n, s->id, s->x, s->sc, s->partials,
+                                                                           s->drift_rows, r->a.n_inv, s->stage2);
+            MAPPG_CUDA(cudaGetLastError());
+            MAPPG_CUDA(cudaEventRecord(s->ev_side, s->side));
+        };
+        // the closing kernel moves the step's displacement into sc->drift,
+        // which the gather reads
+        auto gathered = [&] { MAPPG_CUDA(cudaStreamWaitEvent(s->stream, s->ev_side, 0)); };
         if (s->precision == MAPPG_MIXED)
-            launch_step32(s, r->a, true);
+            launch_step32(s, r->a, gather, gathered);
         else
-            launch_step64(s, r->a, true);
+            launch_step64(s, r->a, gather, gathered);
         r->done += 1;
-        MAPPG_CUDA(cudaStreamWaitEvent(s->side, s->ev_main, 0));
-        k_scatter_x_final<<<grid_for(s, s->n, 256), 256, 0, s->side>>>(s->n, s->id, s->x, s->sc, s->stage2);
-        MAPPG_CUDA(cudaGetLastError());
-        MAPPG_CUDA(cudaEventRecord(s->ev_side, s->side));
-        s->v_pending = true;
         MAPPG_CUDA(cudaMemcpyAsync(x_out, s->stage2, sizeof(double) * 3 * (size_t)s->n, cudaMemcpyDeviceToHost,
                                    s->side));
     }

@@ -20,7 +20,7 @@
 #include <type_traits>
 #include <vector>
 
-#include "system.h"
+#include "eam_common.cuh"
 
 namespace mappg {
 
@@ -266,10 +266,13 @@ __device__ __forceinline__ float4 frame_pos(const double* bs, double x0, double 
 // the build positions (x0, and p0 in the frame) are the wrapped ones
 __global__ void k_wrap_bin(int n, double* __restrict__ x, double* __restrict__ s, double* __restrict__ xb, Geo g,
                            int* __restrict__ binc, int* __restrict__ binid, int* __restrict__ bin_count,
-                           float4* __restrict__ p32, float4* __restrict__ p0, DevScalars* sc) {
+                           float4* __restrict__ p32, float4* __restrict__ p0, const double* __restrict__ partials,
+                           int drift_rows, DevScalars* sc) {
     if (!sc->rebuild) return;
     int bad = 0;
-    const double drift0 = sc->drift[0], drift1 = sc->drift[1], drift2 = sc->drift[2];
+    double drift[3];
+    drift_now(sc, partials, drift_rows, 1.0 / (double)n, drift);
+    const double drift0 = drift[0], drift1 = drift[1], drift2 = drift[2];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         // the mixed MD path defers its mean-displacement removal to here
         double x0 = dsub(x[i], drift0), x1 = dsub(x[n + i], drift1), x2 = dsub(x[2 * n + i], drift2);
@@ -349,8 +352,11 @@ __device__ __forceinline__ void rebuild_reset(DevScalars* sc) {
 }
 
 // rebuild step 2: exclusive scan of bin counts (one block), counts zeroed
-__global__ void k_scan_bins(int nbins, int* __restrict__ bin_count, int* __restrict__ bin_start, DevScalars* sc) {
+__global__ void k_scan_bins(int nbins, int* __restrict__ bin_count, int* __restrict__ bin_start,
+                            double* __restrict__ partials, int drift_rows, DevScalars* sc) {
     if (!sc->rebuild) return;
+    // the running step's displacement sums went into x with the drift
+    for (int q = threadIdx.x; q < 3 * drift_rows; q += blockDim.x) partials[(q / 3) * kRedSlots + 8 + q % 3] = 0.0;
     __shared__ int part[1024];
     int t = threadIdx.x, T = blockDim.x;
     int chunk = (nbins + T - 1) / T;
@@ -857,8 +863,9 @@ void launch_rebuild_chain(mappg_sys* s) {
                                                                          s->cmd, s->sc);
     } else {
         k_wrap_bin<<<gb, B, 0, s->stream>>>(s->n, s->x, s->s, s->x0, g, s->binc, s->binid, s->bin_count, s->p32, s->p0,
-                                            s->sc);
-        k_scan_bins<<<1, 1024, 0, s->stream>>>(s->nbins, s->bin_count, s->bin_start, s->sc);
+                                            s->partials, s->drift_rows, s->sc);
+        k_scan_bins<<<1, 1024, 0, s->stream>>>(s->nbins, s->bin_count, s->bin_start, s->partials, s->drift_rows,
+                                               s->sc);
     }
     k_scatter_bins<<<gb, B, 0, s->stream>>>(s->n, s->binid, s->bin_start, s->bin_count, s->bin_tmp, s->cell_of, reb,
                                             s->sc);

@@ -81,12 +81,14 @@ struct DevScalars {
     double kickA;      // mixed MD: v <- A v + B f dt/2m
     double kickB;
     double eta[kMaxChain];
+    double eta_next[kMaxChain];  // the chain after the next step's opening half
+    double fac_next;   // FP64 MD: the velocity scale of the next kick
     long long step;    // steps done in this run
     long long nrebuild;
 };
 
 struct NhcParams {
-    double T, ddt, ddt2, freq_sq, kB, ndof_kB;
+    double T, T_inv, ddt, ddt2, freq_sq, kB, ndof_kB, ndof_kB_inv, ndof_d;
     int L, niters, ndof;
 };
 
@@ -308,6 +310,9 @@ struct mappg_sys {
     double* cell_out = nullptr;          // ncell x 8 (pe, virial6, spare) staging
 
     void* run = nullptr;  // an NVT run in progress (md.cu)
+    // mixed MD run: partial rows that hold the running step's displacement
+    // sums in slots 8-10 (0 outside a run)
+    int drift_rows = 0;
     bool built = false;
     bool list_box = false;  // a neighbour list exists for the current box (skin test may reuse it)
     bool have_v = false;
