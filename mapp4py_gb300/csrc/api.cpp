@@ -327,6 +327,13 @@ int mappg_sys_create(const mappg_ff* ff, int natoms, const double* H, const doub
             MAPPG_CUDA(cudaGetDeviceProperties(&p, s->device));
             s->sm_count = p.multiProcessorCount;
             s->smem_optin = (int)p.sharedMemPerBlockOptin;
+            // a small mixed system walks four entries per step until it is
+            // tuned: its lanes wait for memory, not for each other, and one
+            // block of 256 threads per SM (32 atoms) leaves the registers for
+            // it.  Density + force with one / four: 500 atoms 25.7 / 20.6 us,
+            // 4,000 27.8 / 20.8; beyond the line 8,788 30.1 / 30.7, 32,000
+            // 49.0 / 77.7
+            if (precision == MAPPG_MIXED && natoms <= 32 * s->sm_count) s->unroll = 4;
             sys_set_box(s, H);
             sys_alloc(s, x);
             sys_alloc_bins(s);

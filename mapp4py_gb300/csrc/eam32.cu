@@ -274,7 +274,47 @@ __device__ __forceinline__ void density_atom(const EamArgs& a, const Smem32& S, 
         // bit t of `bits`: this lane's t-th entry (row slot lane + t TPA) is
         // inside the cutoff
         unsigned bits = 0u;
-        if (U == 1) {
+        if constexpr (U == 4) {
+            // a small system, where a lane's waits are the time: the row
+            // slots, positions and records of four entries are each loaded
+            // together; the additions keep the order of the one-entry loop
+            int t = 0;
+            for (int k = lane; k < nn; k += U * TPA, t += U) {
+                int e[U], m[U];
+                float4 q[U], c[U];
+                float p[U];
+                bool in[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) e[u] = __ldg(row + (u == 0 || k + u * TPA < nn ? k + u * TPA : k));
+#pragma unroll
+                for (int u = 0; u < U; u++) q[u] = __ldg(a.p32 + entry_j(e[u]));
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int ej = entry_elem(e[u]);
+                    float4 o;
+                    image_offset(e[u], o);
+                    float dx, dy, dz;
+                    cart<ORTHO>(fr, (pi.x - q[u].x) + o.x, (pi.y - q[u].y) + o.y, (pi.z - q[u].z) + o.z, dx, dy, dz);
+                    const float rsq = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                    in[u] = rsq < (a.cut_uniform ? cut0 : S.cut_sq[ei * a.ne + ej]) && (u == 0 || k + u * TPA < nn);
+                    if (in[u]) {
+                        const float r = rsq * inv_sqrt(rsq);
+                        m[u] = knot32(fmaf(r, K.dri, r * K.dri_lo), a.nr - 2, p[u]);
+                        const int ms = m[u] - a.rho_mlo;
+                        if (SM && ms >= 0)
+                            c[u] = stab[(a.rho_ei ? ej * a.ne + ei : ej) * a.rho_w + ms];
+                        else
+                            c[u] = __ldg(a.rho32 + (size_t)(ej * a.ne + ei * a.rho_ei) * a.nr + m[u]);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    if (in[u]) {
+                        kahan_add(acc, acc_c, fmaf(fmaf(fmaf(c[u].w, p[u], c[u].z), p[u], c[u].y), p[u], c[u].x));
+                        if (t + u < 32) bits |= 1u << (t + u);
+                    }
+            }
+        } else if (U == 1) {
             int t = 0;
             for (int k = lane; k < nn; k += TPA, t++) {
                 const int e = __ldg(row + k);
@@ -410,109 +450,212 @@ __device__ __forceinline__ void force_atom(const EamArgs& a, const Smem32& S, co
         const int nn = __ldg(a.nnbr + i);
         const int* row = a.nbr + (size_t)i * a.maxnbr;
         const float cut0 = S.cut_sq[0];
-        // inside: the entry is known to lie inside the cutoff (a set bit of the
-        // density pass's mask: the same positions and arithmetic give the same
-        // test), so the test is left out
-        auto pair = [&](int e, const float4& q, bool inside) {
-            const int ej = entry_elem(e);
-            const int t = ei * a.ne + ej;
-            float4 o;
-            image_offset(e, o);
-            float dx, dy, dz;
-            cart<ORTHO>(fr, (pi.x - q.x) + o.x, (pi.y - q.y) + o.y, (pi.z - q.z) + o.z, dx, dy, dz);
-            const float rsq = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-            if (inside || rsq < (a.cut_uniform ? cut0 : S.cut_sq[t])) {
-                const float rinv = inv_sqrt(rsq);
-                const float r = rsq * rinv;
-                float fr;
-                const int m = knot32(fmaf(r, K.dri, r * K.dri_lo), a.nr - 2, fr);
-                const size_t kt = (size_t)t * a.nr + m;
-                const int ms = m - a.fs_mlo;
-                const bool in_smem = SM && ms >= 0 && ms < a.fs_w;
-                float4 r0, r1;
-                if (in_smem) {
-                    const float4 z = stab[ej * a.fs_w + ms];
-                    const float4 d = stab[(a.ne + ej) * a.fs_w + ms];
-                    r0 = make_float4(d.x, d.y, d.z, z.w);
-                    r1 = make_float4(z.x, z.y, z.z, d.w);
-                } else {
-                    ldg8(a.ftab + 2 * kt, r0, r1);
-                }
-                const float der_i = fmaf(fmaf(r0.z, fr, r0.y), fr, r0.x);
-                float der_j = der_i;
-                if (ej != ei) {
-                    float4 r2;
-                    if (in_smem) {
-                        // rho'_{g->ej}: with one density function per source
-                        // element it is the group's own rho'_{g->g} record
-                        const int rj = a.rho_ei ? 2 * a.ne + (ej < ei ? ej : ej - 1) : a.ne + ei;
-                        r2 = stab[rj * a.fs_w + ms];
-                    } else {
-                        r2 = __ldg(a.fjtab + kt);
+        if constexpr (U == 4) {
+            // one step's entries e[0..cnt-1]: positions and records loaded
+            // together, forces added in order.  inside: the entries are known to
+            // lie inside the cutoff (set bits of the density pass's mask: the
+            // same positions and arithmetic give the same test), so the test is
+            // left out
+            auto step = [&](const int (&e)[U], int cnt, bool inside) {
+                float4 q[U], r0[U], r1[U], r2[U];
+                float dx[U], dy[U], dz[U], ri[U], p[U];
+                bool in[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) q[u] = __ldg(a.q32 + entry_j(e[u]));
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int ej = entry_elem(e[u]);
+                    const int t = ei * a.ne + ej;
+                    float4 o;
+                    image_offset(e[u], o);
+                    cart<ORTHO>(fr, (pi.x - q[u].x) + o.x, (pi.y - q[u].y) + o.y, (pi.z - q[u].z) + o.z, dx[u], dy[u],
+                                dz[u]);
+                    const float rsq = fmaf(dx[u], dx[u], fmaf(dy[u], dy[u], dz[u] * dz[u]));
+                    in[u] = (u == 0 || u < cnt) && (inside || rsq < (a.cut_uniform ? cut0 : S.cut_sq[t]));
+                    if (in[u]) {
+                        ri[u] = inv_sqrt(rsq);
+                        const float r = rsq * ri[u];
+                        const int m = knot32(fmaf(r, K.dri, r * K.dri_lo), a.nr - 2, p[u]);
+                        const size_t kt = (size_t)t * a.nr + m;
+                        const int ms = m - a.fs_mlo;
+                        const bool in_smem = SM && ms >= 0 && ms < a.fs_w;
+                        if (in_smem) {
+                            const float4 z = stab[ej * a.fs_w + ms];
+                            const float4 d = stab[(a.ne + ej) * a.fs_w + ms];
+                            r0[u] = make_float4(d.x, d.y, d.z, z.w);
+                            r1[u] = make_float4(z.x, z.y, z.z, d.w);
+                        } else {
+                            ldg8(a.ftab + 2 * kt, r0[u], r1[u]);
+                        }
+                        if (ej != ei) {
+                            if (in_smem) {
+                                // rho'_{g->ej}: with one density function per source
+                                // element it is the group's own rho'_{g->g} record
+                                const int rj = a.rho_ei ? 2 * a.ne + (ej < ei ? ej : ej - 1) : a.ne + ei;
+                                r2[u] = stab[rj * a.fs_w + ms];
+                            } else {
+                                r2[u] = __ldg(a.fjtab + kt);
+                            }
+                        }
                     }
-                    der_j = fmaf(fmaf(r2.z, fr, r2.y), fr, r2.x);
                 }
-                const float zpoly = fmaf(fmaf(r1.z, fr, r1.y), fr, r1.x);
-                const float z = r0.w + fmaf(fr, zpoly, r1.w);
-                const float zp = fmaf(fmaf(3.0f * r1.z, fr, 2.0f * r1.y), fr, r1.x) * K.dri;
-                const float phi = z * rinv;
-                const float dphi = (zp - phi) * rinv;
-                const float fp = -fmaf(dFi, der_i, fmaf(q.w, der_j, dphi)) * rinv;
-                const float fdx = fp * dx, fdy = fp * dy, fdz = fp * dz;
-                kahan_add(fx, fxc, fdx);
-                kahan_add(fy, fyc, fdy);
-                kahan_add(fz, fzc, fdz);
-                kahan_add(ep, epc, phi);
-                w[0] = fmaf(fdx, dx, w[0]);
-                w[1] = fmaf(fdx, dy, w[1]);
-                w[2] = fmaf(fdx, dz, w[2]);
-                w[3] = fmaf(fdy, dy, w[3]);
-                w[4] = fmaf(fdy, dz, w[4]);
-                w[5] = fmaf(fdz, dz, w[5]);
-            }
-        };
-        if (a.cutmask && nn <= 32 * TPA) {
-            // only the entries the density pass found inside the cutoff (the
-            // same positions), in the same order: the skin shell's entries
-            // cost no gather and no geometry here
-            unsigned bits = __ldg(a.cutmask + (size_t)i * TPA + lane);
-            if (U == 1) {
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    if (!in[u]) continue;
+                    const float der_i = fmaf(fmaf(r0[u].z, p[u], r0[u].y), p[u], r0[u].x);
+                    float der_j = der_i;
+                    if (entry_elem(e[u]) != ei) der_j = fmaf(fmaf(r2[u].z, p[u], r2[u].y), p[u], r2[u].x);
+                    const float zpoly = fmaf(fmaf(r1[u].z, p[u], r1[u].y), p[u], r1[u].x);
+                    const float z = r0[u].w + fmaf(p[u], zpoly, r1[u].w);
+                    const float zp = fmaf(fmaf(3.0f * r1[u].z, p[u], 2.0f * r1[u].y), p[u], r1[u].x) * K.dri;
+                    const float phi = z * ri[u];
+                    const float dphi = (zp - phi) * ri[u];
+                    const float fp = -fmaf(dFi, der_i, fmaf(q[u].w, der_j, dphi)) * ri[u];
+                    const float fdx = fp * dx[u], fdy = fp * dy[u], fdz = fp * dz[u];
+                    kahan_add(fx, fxc, fdx);
+                    kahan_add(fy, fyc, fdy);
+                    kahan_add(fz, fzc, fdz);
+                    kahan_add(ep, epc, phi);
+                    w[0] = fmaf(fdx, dx[u], w[0]);
+                    w[1] = fmaf(fdx, dy[u], w[1]);
+                    w[2] = fmaf(fdx, dz[u], w[2]);
+                    w[3] = fmaf(fdy, dy[u], w[3]);
+                    w[4] = fmaf(fdy, dz[u], w[4]);
+                    w[5] = fmaf(fdz, dz[u], w[5]);
+                }
+            };
+            if (a.cutmask && nn <= 32 * TPA) {
+                // only the entries the density pass found inside the cutoff (the
+                // same positions), in the same order: the skin shell's entries
+                // cost no gather and no geometry here
+                unsigned bits = __ldg(a.cutmask + (size_t)i * TPA + lane);
                 while (bits) {
-                    const int t = __ffs(bits) - 1;
-                    bits &= bits - 1u;
-                    const int e = __ldg(row + lane + t * TPA);
-                    pair(e, __ldg(a.q32 + entry_j(e)), true);
+                    int e[U];
+                    const int cnt = U == 1 ? 1 : __popc(bits);
+                    int t = 0;
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        if (u == 0 || bits) {
+                            t = __ffs(bits) - 1;
+                            bits &= bits - 1u;
+                        }
+                        e[u] = __ldg(row + lane + t * TPA);
+                    }
+                    step(e, cnt, true);
                 }
             } else {
-                while (bits) {
-                    const int t0 = __ffs(bits) - 1;
-                    bits &= bits - 1u;
-                    const bool v1 = bits != 0u;
-                    const int t1 = v1 ? __ffs(bits) - 1 : t0;
-                    if (v1) bits &= bits - 1u;
-                    const int e0 = __ldg(row + lane + t0 * TPA);
-                    const int e1 = v1 ? __ldg(row + lane + t1 * TPA) : e0;
-                    const float4 q0 = __ldg(a.q32 + entry_j(e0));
-                    const float4 q1 = __ldg(a.q32 + entry_j(e1));
-                    pair(e0, q0, true);
-                    if (v1) pair(e1, q1, true);
+                for (int k = lane; k < nn; k += U * TPA) {
+                    int e[U];
+#pragma unroll
+                    for (int u = 0; u < U; u++) e[u] = __ldg(row + (u == 0 || k + u * TPA < nn ? k + u * TPA : k));
+                    step(e, U == 1 ? 1 : (nn - k + TPA - 1) / TPA, false);
                 }
             }
-        } else if (U == 1) {
-            for (int k = lane; k < nn; k += TPA) {
-                const int e = __ldg(row + k);
-                pair(e, __ldg(a.q32 + entry_j(e)), false);
-            }
         } else {
-            // two entries per step, sums in the order of the one-entry loop
-            for (int k = lane; k < nn; k += 2 * TPA) {
-                const bool v1 = k + TPA < nn;
-                const int e0 = __ldg(row + k);
-                const int e1 = v1 ? __ldg(row + k + TPA) : e0;
-                const float4 q0 = __ldg(a.q32 + entry_j(e0));
-                const float4 q1 = __ldg(a.q32 + entry_j(e1));
-                pair(e0, q0, false);
-                if (v1) pair(e1, q1, false);
+            // inside: the entry is known to lie inside the cutoff (a set bit of the
+            // density pass's mask: the same positions and arithmetic give the same
+            // test), so the test is left out
+            auto pair = [&](int e, const float4& q, bool inside) {
+                const int ej = entry_elem(e);
+                const int t = ei * a.ne + ej;
+                float4 o;
+                image_offset(e, o);
+                float dx, dy, dz;
+                cart<ORTHO>(fr, (pi.x - q.x) + o.x, (pi.y - q.y) + o.y, (pi.z - q.z) + o.z, dx, dy, dz);
+                const float rsq = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                if (inside || rsq < (a.cut_uniform ? cut0 : S.cut_sq[t])) {
+                    const float rinv = inv_sqrt(rsq);
+                    const float r = rsq * rinv;
+                    float fr;
+                    const int m = knot32(fmaf(r, K.dri, r * K.dri_lo), a.nr - 2, fr);
+                    const size_t kt = (size_t)t * a.nr + m;
+                    const int ms = m - a.fs_mlo;
+                    const bool in_smem = SM && ms >= 0 && ms < a.fs_w;
+                    float4 r0, r1;
+                    if (in_smem) {
+                        const float4 z = stab[ej * a.fs_w + ms];
+                        const float4 d = stab[(a.ne + ej) * a.fs_w + ms];
+                        r0 = make_float4(d.x, d.y, d.z, z.w);
+                        r1 = make_float4(z.x, z.y, z.z, d.w);
+                    } else {
+                        ldg8(a.ftab + 2 * kt, r0, r1);
+                    }
+                    const float der_i = fmaf(fmaf(r0.z, fr, r0.y), fr, r0.x);
+                    float der_j = der_i;
+                    if (ej != ei) {
+                        float4 r2;
+                        if (in_smem) {
+                            // rho'_{g->ej}: with one density function per source
+                            // element it is the group's own rho'_{g->g} record
+                            const int rj = a.rho_ei ? 2 * a.ne + (ej < ei ? ej : ej - 1) : a.ne + ei;
+                            r2 = stab[rj * a.fs_w + ms];
+                        } else {
+                            r2 = __ldg(a.fjtab + kt);
+                        }
+                        der_j = fmaf(fmaf(r2.z, fr, r2.y), fr, r2.x);
+                    }
+                    const float zpoly = fmaf(fmaf(r1.z, fr, r1.y), fr, r1.x);
+                    const float z = r0.w + fmaf(fr, zpoly, r1.w);
+                    const float zp = fmaf(fmaf(3.0f * r1.z, fr, 2.0f * r1.y), fr, r1.x) * K.dri;
+                    const float phi = z * rinv;
+                    const float dphi = (zp - phi) * rinv;
+                    const float fp = -fmaf(dFi, der_i, fmaf(q.w, der_j, dphi)) * rinv;
+                    const float fdx = fp * dx, fdy = fp * dy, fdz = fp * dz;
+                    kahan_add(fx, fxc, fdx);
+                    kahan_add(fy, fyc, fdy);
+                    kahan_add(fz, fzc, fdz);
+                    kahan_add(ep, epc, phi);
+                    w[0] = fmaf(fdx, dx, w[0]);
+                    w[1] = fmaf(fdx, dy, w[1]);
+                    w[2] = fmaf(fdx, dz, w[2]);
+                    w[3] = fmaf(fdy, dy, w[3]);
+                    w[4] = fmaf(fdy, dz, w[4]);
+                    w[5] = fmaf(fdz, dz, w[5]);
+                }
+            };
+            if (a.cutmask && nn <= 32 * TPA) {
+                // only the entries the density pass found inside the cutoff (the
+                // same positions), in the same order: the skin shell's entries
+                // cost no gather and no geometry here
+                unsigned bits = __ldg(a.cutmask + (size_t)i * TPA + lane);
+                if (U == 1) {
+                    while (bits) {
+                        const int t = __ffs(bits) - 1;
+                        bits &= bits - 1u;
+                        const int e = __ldg(row + lane + t * TPA);
+                        pair(e, __ldg(a.q32 + entry_j(e)), true);
+                    }
+                } else {
+                    while (bits) {
+                        const int t0 = __ffs(bits) - 1;
+                        bits &= bits - 1u;
+                        const bool v1 = bits != 0u;
+                        const int t1 = v1 ? __ffs(bits) - 1 : t0;
+                        if (v1) bits &= bits - 1u;
+                        const int e0 = __ldg(row + lane + t0 * TPA);
+                        const int e1 = v1 ? __ldg(row + lane + t1 * TPA) : e0;
+                        const float4 q0 = __ldg(a.q32 + entry_j(e0));
+                        const float4 q1 = __ldg(a.q32 + entry_j(e1));
+                        pair(e0, q0, true);
+                        if (v1) pair(e1, q1, true);
+                    }
+                }
+            } else if (U == 1) {
+                for (int k = lane; k < nn; k += TPA) {
+                    const int e = __ldg(row + k);
+                    pair(e, __ldg(a.q32 + entry_j(e)), false);
+                }
+            } else {
+                // two entries per step, sums in the order of the one-entry loop
+                for (int k = lane; k < nn; k += 2 * TPA) {
+                    const bool v1 = k + TPA < nn;
+                    const int e0 = __ldg(row + k);
+                    const int e1 = v1 ? __ldg(row + k + TPA) : e0;
+                    const float4 q0 = __ldg(a.q32 + entry_j(e0));
+                    const float4 q1 = __ldg(a.q32 + entry_j(e1));
+                    pair(e0, q0, false);
+                    if (v1) pair(e1, q1, false);
+                }
             }
         }
         kahan_add(es, ec, ep);
@@ -529,7 +672,7 @@ __device__ __forceinline__ void force_atom(const EamArgs& a, const Smem32& S, co
 }
 
 template <int TPA, bool ORTHO, int U>
-__global__ void __launch_bounds__(256, 4) k_force32(EamArgs a) {
+__global__ void __launch_bounds__(256, U == 4 ? 1 : 4) k_force32(EamArgs a) {
     __shared__ Smem32 S;
     S.fill(a);
     const Consts32 K(a);
@@ -1011,6 +1154,10 @@ __global__ void k_cells_done(EamArgs a, const int* __restrict__ cell_chunk, Cell
 // loop step U); TPA and U come from the system (mappg_sys_autotune)
 template <int TPA, bool ORTHO, int U>
 static void density_t(mappg_sys* s, const EamArgs& a) {
+    if (TPA == 8 && s->unroll == 4) {
+        k_density32<8, ORTHO, 4><<<atom_blocks(s, 8), 256, 0, s->stream>>>(a);
+        return;
+    }
     if (s->n <= kDensSmallAtoms) {
         static int grid = 0;
         if (!grid) grid = occupancy_grid(s, k_density32<TPA, ORTHO, U>, 256);
@@ -1038,6 +1185,10 @@ static void force_t(mappg_sys* s, const EamArgs& a) {
         }
         const size_t bytes = sizeof(float4) * (size_t)a.fs_rec * a.fs_w;
         k_force32s<TPA, ORTHO, U><<<s->sm_count, 1024, bytes, s->stream>>>(a);
+        return;
+    }
+    if (TPA == 8 && s->unroll == 4 && !s->unroll_force) {
+        k_force32<8, ORTHO, 4><<<atom_blocks(s, 8), 256, 0, s->stream>>>(a);
         return;
     }
     static int grid = 0;
@@ -1107,7 +1258,7 @@ static void pick_ortho(bool o, F&& fn) {
     do {                                                                                              \
         const bool o = (ORTHO_EXPR);                                                                  \
         auto call = [&](auto T, auto O, auto U) { FN<decltype(T)::value, decltype(O)::value, decltype(U)::value>(s, a); }; \
-        const bool u2 = (UNROLL) == 2;                                                                \
+        const bool u2 = (UNROLL) >= 2;                                                                \
         switch (s->tpa) {                                                                             \
             case 4: u2 ? pick_ortho<4, 2>(o, call) : pick_ortho<4, 1>(o, call); break;                \
             case 16: u2 ? pick_ortho<16, 2>(o, call) : pick_ortho<16, 1>(o, call); break;            \
