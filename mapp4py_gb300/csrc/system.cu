@@ -713,8 +713,10 @@ __global__ void __launch_bounds__(32 * kBuildWarps) k_build_bins(const __grid_co
                         build_scan<UNI>(a, cut, cand, nt, h, self, s_geo, h6, s_row[w], kBuildRow, cin, cout);
                         tot = cin + cout;
                         __syncwarp();
-                        if (tot <= min(kBuildRow, a.maxnbr))
-                            for (int k = lane; k < tot; k += 32) row[k] = s_row[w][k < cin ? k : kBuildRow - tot + k];
+                        // (of a row that does not fit only the inner entries)
+                        if (tot <= kBuildRow)
+                            for (int k = lane; k < min(tot <= a.maxnbr ? tot : cin, a.maxnbr); k += 32)
+                                row[k] = s_row[w][k < cin ? k : kBuildRow - tot + k];
                         __syncwarp();  // s_row is refilled for the warp's next atom
                     }
                     if (tot > kBuildRow) {
@@ -745,8 +747,9 @@ __global__ void __launch_bounds__(32 * kBuildWarps) k_build_bins(const __grid_co
                         }
                     }
                     // a row that does not fit is built again with a larger
-                    // capacity
-                    if (lane == 0) a.nnbr[i] = min(tot, a.maxnbr);
+                    // capacity; until then (the passes of an MD step may
+                    // still walk it) it counts the slots that were written
+                    if (lane == 0) a.nnbr[i] = tot <= a.maxnbr ? tot : min(cin, a.maxnbr);
                     overflow |= tot > a.maxnbr;
                     maxrow = max(maxrow, tot);
                     sumrow += tot;
