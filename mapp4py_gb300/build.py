@@ -46,7 +46,7 @@ def _stale(target, deps):
 def build(verbose=False, force=False, extra=()):
     os.makedirs(OBJ, exist_ok=True)
     srcs = sources()
-    headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".h")]
+    headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
     headers.append(os.path.join(INCLUDE, "mappg.h"))
     cc = nvcc()
     jobs = []

@@ -334,6 +334,16 @@ int mappg_sys_create(const mappg_ff* ff, int natoms, const double* H, const doub
             // 4,000 27.8 / 20.8; beyond the line 8,788 30.1 / 30.7, 32,000
             // 49.0 / 77.7
             if (precision == MAPPG_MIXED && natoms <= 32 * s->sm_count) s->unroll = 4;
+            // a small FP64 system takes as many lanes per atom as one block
+            // of 256 threads per SM has (density + force at 32 / 16 / 8: 500
+            // atoms 30.5 / 36.6 / 44.8 us, 2,048 40.9 / 36.2 / 45.2, 4,000
+            // 58.8 / 48.6 / 46.2); from two such blocks at eight on, four
+            // lanes share a list more evenly (8 / 4: 16,384 atoms 114.7 /
+            // 109.7, 256,000 1,194 / 1,133)
+            if (precision == MAPPG_FP64) {
+                const long long block = 256LL * s->sm_count;
+                s->tpa = 32LL * natoms <= block ? 32 : 16LL * natoms <= block ? 16 : 8LL * natoms <= 2 * block ? 8 : 4;
+            }
             sys_set_box(s, H);
             sys_alloc(s, x);
             sys_alloc_bins(s);

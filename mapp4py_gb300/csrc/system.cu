@@ -484,6 +484,7 @@ struct BuildArgs {
     const int* bin_start;
     int* nbr;
     int* nnbr;
+    int *own_ent, *other_ent, *nown, *nother;  // FP64: the row's entries by owner (null: not kept)
     Geo g;
     float G[3][3];  // frame to Cartesian
     float lo2[kMaxElem * kMaxElem], hi2[kMaxElem * kMaxElem];
@@ -717,7 +718,6 @@ __global__ void __launch_bounds__(32 * kBuildWarps) k_build_bins(const __grid_co
                         if (tot <= kBuildRow)
                             for (int k = lane; k < min(tot <= a.maxnbr ? tot : cin, a.maxnbr); k += 32)
                                 row[k] = s_row[w][k < cin ? k : kBuildRow - tot + k];
-                        __syncwarp();  // s_row is refilled for the warp's next atom
                     }
                     if (tot > kBuildRow) {
                         if (one_tile)
@@ -750,6 +750,31 @@ __global__ void __launch_bounds__(32 * kBuildWarps) k_build_bins(const __grid_co
                     // capacity; until then (the passes of an MD step may
                     // still walk it) it counts the slots that were written
                     if (lane == 0) a.nnbr[i] = tot <= a.maxnbr ? tot : min(cin, a.maxnbr);
+                    if (!BATCH && a.own_ent) {
+                        const bool chip = one_tile && tot <= kBuildRow;
+                        const int len = tot <= a.maxnbr ? tot : 0;
+                        const size_t base = (size_t)i * a.maxnbr;
+                        int no = 0, nx = 0;
+                        for (int k0 = 0; k0 < len; k0 += 32) {
+                            const int k = k0 + lane;
+                            const int e = k >= len ? 0 : chip ? s_row[w][k < cin ? k : kBuildRow - tot + k] : row[k];
+                            const bool own = k < len && pair_owned(i, e);
+                            const unsigned mo = __ballot_sync(0xffffffffu, own);
+                            const unsigned mx = __ballot_sync(0xffffffffu, k < len && !own);
+                            const unsigned below = (1u << lane) - 1u;
+                            if (own)
+                                a.own_ent[base + no + __popc(mo & below)] = e;
+                            else if (k < len)
+                                a.other_ent[base + nx + __popc(mx & below)] = e;
+                            no += __popc(mo);
+                            nx += __popc(mx);
+                        }
+                        if (lane == 0) {
+                            a.nown[i] = no;
+                            a.nother[i] = nx;
+                        }
+                    }
+                    __syncwarp();  // s_row is refilled for the warp's next atom
                     overflow |= tot > a.maxnbr;
                     maxrow = max(maxrow, tot);
                     sumrow += tot;
@@ -884,6 +909,10 @@ void launch_rebuild_chain(mappg_sys* s) {
     a.bin_start = s->bin_start;
     a.nbr = s->nbr;
     a.nnbr = s->nnbr;
+    a.own_ent = s->own_ent;
+    a.other_ent = s->other_ent;
+    a.nown = s->nown;
+    a.nother = s->nother;
     a.g = g;
     for (int p = 0; p < s->ne * s->ne; p++) {
         a.cut_sk_sq[p] = s->cut_sk_sq[p];
@@ -923,6 +952,7 @@ void launch_rebuild_chain(mappg_sys* s) {
             by_uni(std::false_type(), std::true_type());
         else
             by_uni(std::false_type(), std::false_type());
+        if (s->own_ent) launch_link64(s);
     }
     MAPPG_CUDA(cudaGetLastError());
 }
@@ -952,6 +982,14 @@ EamArgs eam_args(mappg_sys* s) {
     a.x = s->x;
     a.p32 = s->p32;
     a.binc = s->binc;
+    a.own_ent = s->own_ent;
+    a.nown = s->nown;
+    a.other_ent = s->other_ent;
+    a.nother = s->nother;
+    a.other_slot = s->other_slot;
+    a.pair_rec = s->pair_rec;
+    a.pair_rho = s->pair_rho;
+    a.pair_mask = s->pair_mask;
     a.rho64 = ff->dev.rho64;
     a.rphi64 = ff->dev.rphi64;
     a.F64 = ff->dev.F64;
@@ -1033,7 +1071,7 @@ void sys_free(mappg_sys* s) {
                     s->rho32, s->binc, s->binid, s->bin_count, s->bin_start, s->bin_tmp, s->bin_pos, s->nbr, s->nnbr,
                     s->rho, s->dF, s->partials, s->sc, s->stage, s->thermo_dev, s->cells_dev, s->cell_of,
                     s->chunk_begin, s->chunk_cell, s->cell_chunk, s->chunk_part, s->chunk_disp, s->cmd,
-                    s->cell_out, s->dof, s->stage2, s->cutmask, s->fs_tab, s->grp_atoms, s->cell_reb};
+                    s->pair_mem, s->cell_out, s->dof, s->stage2, s->cutmask, s->fs_tab, s->grp_atoms, s->cell_reb};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (s->ev_main) cudaEventDestroy(s->ev_main);
@@ -1146,11 +1184,47 @@ void sys_alloc_bins(mappg_sys* s) {
     MAPPG_CUDA(cudaMemsetAsync(s->bin_count, 0, sizeof(int) * s->nbins, s->stream));
 }
 
+// the lists and records of pair64.cu for rows of maxnbr entries, one
+// allocation of 76 bytes an entry.  Where it would take more than a quarter
+// of the card's free memory, or more slots than 32 bits count, the system
+// keeps the full-row passes
+static void alloc_pairs64(mappg_sys* s) {
+    if (s->pair_mem) cudaFree(s->pair_mem);
+    s->pair_mem = nullptr;
+    s->own_ent = nullptr;
+    if (s->precision != MAPPG_FP64 || s->ncell > 1) return;
+    const size_t n = (size_t)s->n, slots = n * s->maxnbr;
+    const size_t bytes[] = {48 * slots, 16 * slots, 4 * slots, 4 * slots, 4 * slots, 256 * n, 4 * n, 4 * n};
+    size_t at[9] = {0};
+    for (int k = 0; k < 8; k++) at[k + 1] = at[k] + (bytes[k] + 255) / 256 * 256;
+    if (slots >= kNoSlot) return;
+    if (at[8] > (size_t)1 << 28) {
+        size_t free_b = 0, total_b = 0;
+        MAPPG_CUDA(cudaMemGetInfo(&free_b, &total_b));
+        if (at[8] > free_b / 4) return;
+    }
+    if (cudaMalloc((void**)&s->pair_mem, at[8]) != cudaSuccess) {
+        cudaGetLastError();
+        s->pair_mem = nullptr;
+        return;
+    }
+    char* p = s->pair_mem;
+    s->pair_rec = (double2*)(p + at[0]);
+    s->pair_rho = (double2*)(p + at[1]);
+    s->own_ent = (int*)(p + at[2]);
+    s->other_ent = (int*)(p + at[3]);
+    s->other_slot = (unsigned*)(p + at[4]);
+    s->pair_mask = (unsigned*)(p + at[5]);
+    s->nown = (int*)(p + at[6]);
+    s->nother = (int*)(p + at[7]);
+}
+
 void sys_alloc_nbr(mappg_sys* s, int maxnbr) {
     if (s->nbr) cudaFree(s->nbr);
     s->nbr = nullptr;
     s->maxnbr = maxnbr;
     dev_alloc((void**)&s->nbr, sizeof(int) * (size_t)s->n * maxnbr);
+    alloc_pairs64(s);
 }
 
 // upload caller-order AoS doubles into a SoA device array

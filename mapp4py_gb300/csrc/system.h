@@ -53,6 +53,22 @@ __host__ __device__ inline int make_entry(int j, int ej, int c) {
     return (int)((unsigned)j << kEntryShift | (unsigned)ej << 6 | k);
 }
 
+// an entry seen from the other atom of its pair: atom i (element ei) reached
+// by the opposite bin step
+__host__ __device__ inline int mirrored_entry(int e, int i, int ei) {
+    const unsigned k = (2u - ((unsigned)e & 3u)) | (2u - (((unsigned)e >> 2) & 3u)) << 2 | (2u - (((unsigned)e >> 4) & 3u)) << 4;
+    return (int)((unsigned)i << kEntryShift | (unsigned)ei << 6 | k);
+}
+// whether atom i owns the pair of its entry e (exactly one of a pair's two
+// entries is owned): by the parity of the two indices, so that every atom
+// owns about half of its pairs; an atom's own images by their bin step
+__host__ __device__ inline bool pair_owned(int i, int e) {
+    const int j = entry_j(e);
+    if (j == i) return (e & 63) > 21;
+    return ((i ^ j) & 1) ? i < j : i > j;
+}
+constexpr unsigned kNoSlot = 0xffffffffu;
+
 struct Box {
     double H[3][3], B[3][3], h6[6], b6[6], vol, depth_inv[3];
 };
@@ -180,6 +196,16 @@ struct EamArgs {
     float* f32;            // SoA 3n (mixed kernels)
     double* partials;
     DevScalars* sc;
+    // FP64, every pair computed once (pair64.cu): per atom the entries it
+    // owns and the others, maxnbr of each, a record per owned entry
+    const int* own_ent;
+    const int* nown;
+    const int* other_ent;
+    const int* nother;
+    const unsigned* other_slot;  // record of another atom's pair (kNoSlot: none)
+    double2* pair_rec;           // 3 double2 per slot
+    double2* pair_rho;
+    unsigned* pair_mask;
     // line searches of mixed-precision minimizers: the density pass also
     // writes the FP64 density here when non-null; the energy-difference pass
     // (k_de32) reads it with the search direction h (float4 per atom,
@@ -278,6 +304,12 @@ struct mappg_sys {
     int maxnbr = 0;
     int* nbr = nullptr;
     int* nnbr = nullptr;
+    // FP64 single cells: pairs by owner (pair64.cu); null where the card has
+    // no room for them (the full-row passes then run)
+    int *own_ent = nullptr, *other_ent = nullptr, *nown = nullptr, *nother = nullptr;
+    unsigned *other_slot = nullptr, *pair_mask = nullptr;
+    double2 *pair_rec = nullptr, *pair_rho = nullptr;
+    char* pair_mem = nullptr;  // the allocation that holds them
     double *rho = nullptr, *dF = nullptr;
     double* partials = nullptr;
     mappg::DevScalars* sc = nullptr;
@@ -365,6 +397,12 @@ void launch_force(mappg_sys* s);           // density+embed, force; totals in sc
 void launch_energy(mappg_sys* s);          // energy only; total in sc->energy
 void launch_density_only(mappg_sys* s);    // the density kernel alone (timing)
 void launch_force_only(mappg_sys* s);      // the force kernel alone (timing; needs dF)
+
+// pair64.cu (FP64 passes of a single cell, every pair computed once)
+void launch_link64(mappg_sys* s);          // rebuild: record slots of the pairs owned by other atoms
+void launch_pair_density64(mappg_sys* s, const EamArgs& a);
+void launch_pair_force64(mappg_sys* s, const EamArgs& a);
+void launch_pair_energy64(mappg_sys* s, const EamArgs& a);
 
 // eam32.cu (mixed kernels)
 void launch_density32(mappg_sys* s, const EamArgs& a);

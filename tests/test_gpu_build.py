@@ -59,3 +59,20 @@ def test_batch_rows_equal_single_cells_at_the_builders_edges(potentials):
         e[:, 0] -= lo
         s = _lib.System(ff, H, x, elem, masses, skin=5.0, precision=_lib.MIXED)
         assert np.array_equal(keys(cnt[lo:hi], e), keys(*s.neighbors()))
+
+
+@pytest.mark.parametrize("cells,skin", [((2, 4, 5), 0.5), ((4, 4, 5), 6.5), ((7, 6, 6), 0.5), ((9, 9, 8), 0.5)])
+def test_fp64_pairs_by_owner_match_the_oracle(potentials, cells, skin):
+    """Forces, energy and virial with every pair computed once: 32, 16 and 8
+    lanes an atom, several images of one neighbour (a side of 7.2 A), lists
+    longer than the lanes' mask (a reach of 12 A: ~300 pairs owned)."""
+    path, _ = potentials[("A", "B")]
+    c = synth.alloy(cells, xB=0.4, sigma=0.08, vac=0.02, seed=6)
+    o = O.System(O.Eam.setfl(path), c.H, c.x, c.elem, c.masses, skin=0.5)
+    pe_o, vir_o = o.force()
+    s = _lib.System(_lib.ForceField.setfl(path), c.H, c.x, c.elem, c.masses, skin=skin)
+    pe, vir = s.force()
+    assert abs(pe - pe_o) <= 1e-12 * abs(pe_o)
+    assert np.max(np.abs(vir - vir_o)) <= 1e-11 * np.max(np.abs(vir_o))
+    assert np.max(np.abs(s.get_f() - o.f)) <= 1e-10 * max(1.0, np.max(np.abs(o.f)))
+    assert abs(s.energy() - pe_o) <= 1e-12 * abs(pe_o)
