@@ -93,7 +93,7 @@ __device__ __forceinline__ void bl_store(const double (&v)[K], const int (&op)[K
             if (lane == 0) redm[w][k] = t;
         }
     }
-    double t = block_sums<K>(u);
+    double t = block_sums<K, true>(u);
     if (threadIdx.x < K) {
         if (op[threadIdx.x]) {
             unsigned long long m = 0;
@@ -123,6 +123,7 @@ __device__ __forceinline__ double bl_cell_total(const BlArgs& a, int c, int k, b
 
 // x0 = x, f0 = f, h = f for the cells in `st`
 __global__ void k_bl_start(BlArgs a, int st) {
+    dep_wait();
     const int n = a.n;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int s = a.cs[a.cell_of[i]].state;
@@ -147,6 +148,7 @@ __global__ void k_bl_start(BlArgs a, int st) {
 // then the partial of the next dot, Vn[slot(i_next)].h (none if Vn null)
 __global__ void __launch_bounds__(256) k_bl_step(BlArgs a, int st, int mode, int i, const double* __restrict__ Vu,
                                                  const double* __restrict__ Vn, int i_next) {
+    dep_wait();
     const int n = a.n;
     const size_t N3 = 3 * (size_t)n;
     for (int ch = blockIdx.x; ch < a.nchunk; ch += gridDim.x) {
@@ -184,6 +186,7 @@ __global__ void __launch_bounds__(256) k_bl_step(BlArgs a, int st, int mode, int
 
 // per-cell dot from the chunk partials; mode 1 also forms alpha_i
 __global__ void k_bl_cells_dot(BlArgs a, int st, int set_alpha, int i) {
+    dep_wait();
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (c >= a.ncell) return;
     const double t = bl_cell_total(a, c, 0, false);
@@ -196,6 +199,7 @@ __global__ void k_bl_cells_dot(BlArgs a, int st, int set_alpha, int i) {
 
 // f.h, h.h, max|h|, max|f| per chunk (cells in `st`, or all with st < 0)
 __global__ void __launch_bounds__(256) k_bl_prep(BlArgs a, int st) {
+    dep_wait();
     const int n = a.n;
     for (int ch = blockIdx.x; ch < a.nchunk; ch += gridDim.x) {
         const bool on = st < 0 || a.cs[a.chunk_cell[ch]].state == st;
@@ -218,6 +222,7 @@ __global__ void __launch_bounds__(256) k_bl_prep(BlArgs a, int st) {
 // after the direction: learned cells with a non-descent direction go to
 // BL_PLAIN (recomputed with gamma*I); plain ones fall back to h = f
 __global__ void k_bl_cells_dir(BlArgs a, int st, int learned) {
+    dep_wait();
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (c >= a.ncell) return;
     double t[4];
@@ -236,6 +241,7 @@ __global__ void k_bl_cells_dir(BlArgs a, int st, int learned) {
 
 // h = f and the history dropped for the cells marked by k_bl_cells_dir
 __global__ void k_bl_reset_dir(BlArgs a) {
+    dep_wait();
     const int n = a.n;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const BlCell& c = a.cs[a.cell_of[i]];
@@ -246,6 +252,7 @@ __global__ void k_bl_reset_dir(BlArgs a) {
 
 // line-search set-up per cell (LineSearchBackTrack::min, ls.h:711-740)
 __global__ void k_bl_cells_ls_init(BlArgs a) {
+    dep_wait();
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (c >= a.ncell) return;
     double t[4];
@@ -289,6 +296,7 @@ __global__ void k_bl_cells_ls_init(BlArgs a) {
 
 // x = x0 + a h for the cells searching (MinMDHandler::F, min_cg.h:260-267)
 __global__ void k_bl_trial(BlArgs a) {
+    dep_wait();
     const int n = a.n;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const BlCell& c = a.cs[a.cell_of[i]];
@@ -304,6 +312,7 @@ __global__ void k_bl_trial(BlArgs a) {
 // energy, x0's energy plus the energy difference of the trial, or plus the
 // difference of two FP32 energies
 __global__ void k_bl_cells_ls(BlArgs a) {
+    dep_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= a.ncell) return;
     BlCell& cs = a.cs[c];
@@ -329,6 +338,7 @@ __global__ void k_bl_cells_ls(BlArgs a) {
 
 // failed searches go back to x0
 __global__ void k_bl_restore(BlArgs a) {
+    dep_wait();
     const int n = a.n;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const BlCell& c = a.cs[a.cell_of[i]];
@@ -340,6 +350,7 @@ __global__ void k_bl_restore(BlArgs a) {
 // after the force pass: tolerances and, for cells going on, the history
 // pair of this step: S[head] = a h, Y[head] = f0 - f, with s.y and y.y
 __global__ void __launch_bounds__(256) k_bl_hist(BlArgs a) {
+    dep_wait();
     const int n = a.n;
     const size_t N3 = 3 * (size_t)n;
     for (int ch = blockIdx.x; ch < a.nchunk; ch += gridDim.x) {
@@ -367,6 +378,7 @@ __global__ void __launch_bounds__(256) k_bl_hist(BlArgs a) {
 }
 
 __global__ void k_bl_cells_step(BlArgs a) {
+    dep_wait();
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (c >= a.ncell) return;
     const double sy = bl_cell_total(a, c, 0, false);
@@ -406,6 +418,7 @@ __global__ void k_bl_cells_step(BlArgs a) {
 
 // start: per-cell energy from the opening force call, max|F|, f_tol check
 __global__ void k_bl_cells_open(BlArgs a) {
+    dep_wait();
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (c >= a.ncell) return;
     const double fm = bl_cell_total(a, c, 3, true);
@@ -432,6 +445,7 @@ __global__ void k_bl_cells_open(BlArgs a) {
 // cells whose mixed-precision search stalled above f_tol go on with FP64
 // forces from where they stopped (history dropped)
 __global__ void k_bl_revive(BlArgs a) {
+    dep_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= a.ncell) return;
     BlCell& cs = a.cs[c];
@@ -450,12 +464,14 @@ __global__ void k_bl_revive(BlArgs a) {
 
 // the chunk kernels' cell mask: cells in state st
 __global__ void k_bl_active(BlArgs a, int st) {
+    dep_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < a.ncell) a.active[c] = a.cs[c].state == st ? 1 : 0;
 }
 
 // per-chunk max |x - x_build| of the searching cells into part[ch][0]
 __global__ void __launch_bounds__(256) k_bl_dx(BlArgs a) {
+    dep_wait();
     const int n = a.n;
     for (int ch = blockIdx.x; ch < a.nchunk; ch += gridDim.x) {
         const bool on = a.cs[a.chunk_cell[ch]].state == BL_LS;
@@ -474,6 +490,7 @@ __global__ void __launch_bounds__(256) k_bl_dx(BlArgs a) {
 // counts the searching cells whose first (largest) trial could take an atom
 // beyond half the skin of the list's build positions
 __global__ void k_bl_cells_bound(BlArgs a) {
+    dep_wait();
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (c >= a.ncell) return;
     const double dx = bl_cell_total(a, c, 0, true);
@@ -489,6 +506,7 @@ __global__ void k_bl_cells_bound(BlArgs a) {
 // search start (the batch rebuilds cells one by one, so a cell's list can be
 // older than its neighbours' in the batch); counts them
 __global__ void k_bl_refresh(BlArgs a) {
+    dep_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= a.ncell) return;
     const BlCell& cs = a.cs[c];
@@ -503,6 +521,7 @@ __global__ void k_bl_refresh(BlArgs a) {
 
 // the search start of the searching cells after a rebuild wrapped x
 __global__ void k_bl_restart(BlArgs a) {
+    dep_wait();
     const int n = a.n;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         if (a.cs[a.cell_of[i]].state != BL_LS) continue;
@@ -514,6 +533,7 @@ __global__ void k_bl_restart(BlArgs a) {
 // the skin or more (a search of FP32 energy differences goes over to energy
 // differences once none does)
 __global__ void k_bl_count_long(BlArgs a) {
+    dep_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= a.ncell) return;
     const BlCell& cs = a.cs[c];
@@ -522,6 +542,7 @@ __global__ void k_bl_count_long(BlArgs a) {
 
 // the searching cells back at x0
 __global__ void k_bl_restore_ls(BlArgs a) {
+    dep_wait();
     const int n = a.n;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         if (a.cs[a.cell_of[i]].state != BL_LS) continue;
@@ -531,21 +552,25 @@ __global__ void k_bl_restore_ls(BlArgs a) {
 
 // per-cell trial steps for the energy-difference pass; FP32 energies of x0
 __global__ void k_bl_alpha(BlArgs a) {
+    dep_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < a.ncell) a.alpha_cell[c] = a.cs[c].state == BL_LS ? a.cs[c].a : 0.0;
 }
 
 __global__ void k_bl_e0_32(BlArgs a) {
+    dep_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < a.ncell && a.cs[c].state == BL_LS) a.cs[c].e0_32 = a.cmd[c].energy;
 }
 
 __global__ void k_lb_h32b(int n, const double* __restrict__ h, float4* __restrict__ h32) {
+    dep_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         h32[i] = make_float4((float)h[i], (float)h[n + i], (float)h[2 * n + i], 0.f);
 }
 
 __global__ void k_bl_count(BlArgs a, int st) {
+    dep_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < a.ncell && a.cs[c].state == st) atomicAdd(a.count, 1);
 }
@@ -587,11 +612,28 @@ void batch_lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_
     memset(&a, 0, sizeof(a));
     a.n = n;
     a.ncell = nc;
-    a.nchunk = s->nchunk;
     a.m = m;
-    a.chunk_begin = s->chunk_begin;
-    a.chunk_cell = s->chunk_cell;
-    a.cell_chunk = s->cell_chunk;
+    // the vector kernels' own chunks, of kChunk atoms whatever the tuner took
+    // for the force passes: the dot products' order, and with it the
+    // relaxation, does not depend on a timing
+    std::vector<int> cb, cc, ccell(nc + 1, 0);
+    for (int c = 0; c < nc; c++) {
+        for (int i = s->cell_begin[c]; i < s->cell_begin[c + 1]; i += kChunk) {
+            cb.push_back(i);
+            cc.push_back(c);
+        }
+        ccell[c + 1] = (int)cb.size();
+    }
+    a.nchunk = (int)cb.size();
+    cb.push_back(n);
+    auto upload = [&](const std::vector<int>& v) {
+        int* p = (int*)dalloc(sizeof(int) * v.size());
+        MAPPG_CUDA(cudaMemcpy(p, v.data(), sizeof(int) * v.size(), cudaMemcpyHostToDevice));
+        return p;
+    };
+    a.chunk_begin = upload(cb);
+    a.chunk_cell = upload(cc);
+    a.cell_chunk = upload(ccell);
     a.cell_of = s->cell_of;
     a.cs = (BlCell*)dalloc(sizeof(BlCell) * nc);
     a.cmd = s->cmd;
@@ -602,7 +644,7 @@ void batch_lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_
     a.h = (double*)dalloc(sizeof(double) * N3);
     a.S = (double*)dalloc(sizeof(double) * N3 * std::max(m, 1));
     a.Y = (double*)dalloc(sizeof(double) * N3 * std::max(m, 1));
-    a.part = (double*)dalloc(sizeof(double) * 4 * s->nchunk);
+    a.part = (double*)dalloc(sizeof(double) * 4 * a.nchunk);
     a.count = (int*)dalloc(sizeof(int));
     a.P = P;
     a.c_ls = c_ls;
@@ -632,12 +674,12 @@ void batch_lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_
     s->keep_rho64 = mixed;
     s->h32 = h32;
     cudaStream_t st = s->stream;
-    const int gc = std::min(s->nchunk, s->sm_count * 8);
+    const int gc = std::min(a.nchunk, s->sm_count * 8);
     const int ga = grid_for(s, n, 256);
     const int gw = (nc * 32 + 255) / 256, g1 = (nc + 255) / 256;
     auto count = [&](int state) {
         MAPPG_CUDA(cudaMemsetAsync(a.count, 0, sizeof(int), st));
-        k_bl_count<<<g1, 256, 0, st>>>(a, state);
+        launch_dep(st, k_bl_count, g1, 256, 0, a, state);
         int h = 0;
         MAPPG_CUDA(cudaMemcpyAsync(&h, a.count, sizeof(int), cudaMemcpyDeviceToHost, st));
         MAPPG_CUDA(cudaStreamSynchronize(st));
@@ -645,16 +687,16 @@ void batch_lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_
     };
     // the recursion for the cells in state `cst`
     auto two_loop = [&](int cst, bool diag) {
-        k_bl_start<<<ga, 256, 0, st>>>(a, cst);
-        if (m > 0) k_bl_step<<<gc, 256, 0, st>>>(a, cst, 0, 0, nullptr, a.S, 0);
+        launch_dep(st, k_bl_start, ga, 256, 0, a, cst);
+        if (m > 0) launch_dep(st, k_bl_step, gc, 256, 0, a, cst, 0, 0, nullptr, a.S, 0);
         for (int i = 0; i < m; i++) {
-            k_bl_cells_dot<<<gw, 256, 0, st>>>(a, cst, 1, i);
-            k_bl_step<<<gc, 256, 0, st>>>(a, cst, 1, i, a.Y, i + 1 < m ? a.S : nullptr, i + 1);
+            launch_dep(st, k_bl_cells_dot, gw, 256, 0, a, cst, 1, i);
+            launch_dep(st, k_bl_step, gc, 256, 0, a, cst, 1, i, a.Y, i + 1 < m ? a.S : nullptr, i + 1);
         }
-        k_bl_step<<<gc, 256, 0, st>>>(a, cst, diag ? 4 : 3, 0, nullptr, m > 0 ? a.Y : nullptr, m - 1);
+        launch_dep(st, k_bl_step, gc, 256, 0, a, cst, diag ? 4 : 3, 0, nullptr, m > 0 ? a.Y : nullptr, m - 1);
         for (int i = m - 1; i >= 0; i--) {
-            k_bl_cells_dot<<<gw, 256, 0, st>>>(a, cst, 0, i);
-            k_bl_step<<<gc, 256, 0, st>>>(a, cst, 2, i, a.S, i > 0 ? a.Y : nullptr, i - 1);
+            launch_dep(st, k_bl_cells_dot, gw, 256, 0, a, cst, 0, i);
+            launch_dep(st, k_bl_step, gc, 256, 0, a, cst, 2, i, a.S, i > 0 ? a.Y : nullptr, i - 1);
         }
         MAPPG_CUDA(cudaGetLastError());
     };
@@ -665,8 +707,8 @@ void batch_lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_
     sync_forces64(s);
     launch_energy64(s);  // FP64 reference energies of the line searches
     MAPPG_CUDA(cudaMemcpyAsync(a.h, a.f, sizeof(double) * N3, cudaMemcpyDeviceToDevice, st));
-    k_bl_prep<<<gc, 256, 0, st>>>(a, -1);
-    k_bl_cells_open<<<gw, 256, 0, st>>>(a);
+    launch_dep(st, k_bl_prep, gc, 256, 0, a, -1);
+    launch_dep(st, k_bl_cells_open, gw, 256, 0, a);
     MAPPG_CUDA(cudaGetLastError());
     struct Promote {
         mappg_sys* s;
@@ -682,7 +724,7 @@ void batch_lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_
         sync_forces64(s);
         launch_energy64(s);
         MAPPG_CUDA(cudaMemsetAsync(a.count, 0, sizeof(int), st));
-        k_bl_revive<<<g1, 256, 0, st>>>(a);
+        launch_dep(st, k_bl_revive, g1, 256, 0, a);
         int nrev = 0;
         MAPPG_CUDA(cudaMemcpyAsync(&nrev, a.count, sizeof(int), cudaMemcpyDeviceToHost, st));
         MAPPG_CUDA(cudaStreamSynchronize(st));
@@ -694,16 +736,16 @@ void batch_lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_
         bit++;
         // direction: learned (or plain) two-loop for the running cells
         two_loop(BL_RUN, P != nullptr);
-        k_bl_prep<<<gc, 256, 0, st>>>(a, BL_RUN);
-        k_bl_cells_dir<<<gw, 256, 0, st>>>(a, BL_RUN, P != nullptr);
+        launch_dep(st, k_bl_prep, gc, 256, 0, a, BL_RUN);
+        launch_dep(st, k_bl_cells_dir, gw, 256, 0, a, BL_RUN, P != nullptr);
         if (P) {
             two_loop(BL_PLAIN, false);
-            k_bl_prep<<<gc, 256, 0, st>>>(a, BL_PLAIN);
-            k_bl_cells_dir<<<gw, 256, 0, st>>>(a, BL_PLAIN, 0);
+            launch_dep(st, k_bl_prep, gc, 256, 0, a, BL_PLAIN);
+            launch_dep(st, k_bl_cells_dir, gw, 256, 0, a, BL_PLAIN, 0);
         }
-        k_bl_reset_dir<<<ga, 256, 0, st>>>(a);
-        k_bl_prep<<<gc, 256, 0, st>>>(a, -1);
-        k_bl_cells_ls_init<<<gw, 256, 0, st>>>(a);
+        launch_dep(st, k_bl_reset_dir, ga, 256, 0, a);
+        launch_dep(st, k_bl_prep, gc, 256, 0, a, -1);
+        launch_dep(st, k_bl_cells_ls_init, gw, 256, 0, a);
         MAPPG_CUDA(cudaGetLastError());
         // line search over all searching cells.  Mixed cells take energy
         // differences on x0's lists when every searching cell's trials stay
@@ -714,8 +756,8 @@ void batch_lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_
         a.emode = BL_E64;
         if (mixed && !s->force64) {
             MAPPG_CUDA(cudaMemsetAsync(a.count, 0, sizeof(int), st));
-            k_bl_dx<<<gc, 256, 0, st>>>(a);
-            k_bl_cells_bound<<<gw, 256, 0, st>>>(a);
+            launch_dep(st, k_bl_dx, gc, 256, 0, a);
+            launch_dep(st, k_bl_cells_bound, gw, 256, 0, a);
             int wide = 0;
             MAPPG_CUDA(cudaMemcpyAsync(&wide, a.count, sizeof(int), cudaMemcpyDeviceToHost, st));
             MAPPG_CUDA(cudaStreamSynchronize(st));
@@ -724,54 +766,54 @@ void batch_lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_
                 // search start (x does not move; the rebuild may wrap it,
                 // so the start is taken again) and test the bound again
                 MAPPG_CUDA(cudaMemsetAsync(a.count, 0, sizeof(int), st));
-                k_bl_refresh<<<g1, 256, 0, st>>>(a);
+                launch_dep(st, k_bl_refresh, g1, 256, 0, a);
                 int nref = 0;
                 MAPPG_CUDA(cudaMemcpyAsync(&nref, a.count, sizeof(int), cudaMemcpyDeviceToHost, st));
                 MAPPG_CUDA(cudaStreamSynchronize(st));
                 if (nref > 0) {
                     bl_rebuild_flagged(s);
-                    k_bl_restart<<<ga, 256, 0, st>>>(a);
+                    launch_dep(st, k_bl_restart, ga, 256, 0, a);
                     MAPPG_CUDA(cudaMemsetAsync(a.count, 0, sizeof(int), st));
-                    k_bl_dx<<<gc, 256, 0, st>>>(a);
-                    k_bl_cells_bound<<<gw, 256, 0, st>>>(a);
+                    launch_dep(st, k_bl_dx, gc, 256, 0, a);
+                    launch_dep(st, k_bl_cells_bound, gw, 256, 0, a);
                     MAPPG_CUDA(cudaMemcpyAsync(&wide, a.count, sizeof(int), cudaMemcpyDeviceToHost, st));
                     MAPPG_CUDA(cudaStreamSynchronize(st));
                 }
             }
             a.emode = wide == 0 ? BL_EDELTA : BL_E32DIFF;
-            k_bl_active<<<gb, 256, 0, st>>>(a, BL_LS);
+            launch_dep(st, k_bl_active, gb, 256, 0, a, BL_LS);
             s->cell_active = a.active;
             if (a.emode == BL_EDELTA) {
-                k_lb_h32b<<<ga, 256, 0, st>>>(n, a.h, h32);
+                launch_dep(st, k_lb_h32b, ga, 256, 0, n, a.h, h32);
             } else {
                 // each searching cell's FP32 energy of x0 is its last force
                 // call's (CellMd::energy): every searching cell took a step
                 // and a force call in the previous iteration (or is at the
                 // opening force call)
-                k_bl_e0_32<<<gb, 256, 0, st>>>(a);
+                launch_dep(st, k_bl_e0_32, gb, 256, 0, a);
             }
             MAPPG_CUDA(cudaGetLastError());
         }
         while (true) {
-            k_bl_trial<<<ga, 256, 0, st>>>(a);
+            launch_dep(st, k_bl_trial, ga, 256, 0, a);
             if (a.emode == BL_EDELTA) {
-                k_bl_active<<<gb, 256, 0, st>>>(a, BL_LS);
-                k_bl_alpha<<<gb, 256, 0, st>>>(a);
+                launch_dep(st, k_bl_active, gb, 256, 0, a, BL_LS);
+                launch_dep(st, k_bl_alpha, gb, 256, 0, a);
                 launch_de32b(s, a.alpha_cell);
             } else {
                 lb_update(s);
                 if (a.emode == BL_E32DIFF) {
-                    k_bl_active<<<gb, 256, 0, st>>>(a, BL_LS);
+                    launch_dep(st, k_bl_active, gb, 256, 0, a, BL_LS);
                     launch_energy32(s, eam_args(s));
                 } else {
-                    k_bl_active<<<gb, 256, 0, st>>>(a, BL_LS);
+                    launch_dep(st, k_bl_active, gb, 256, 0, a, BL_LS);
                     s->cell_active = a.active;
                     launch_energy64(s);
                     s->cell_active = nullptr;
                 }
             }
             MAPPG_CUDA(cudaMemsetAsync(a.count, 0, sizeof(int), st));
-            k_bl_cells_ls<<<g1, 256, 0, st>>>(a);
+            launch_dep(st, k_bl_cells_ls, g1, 256, 0, a);
             int left = 0;
             MAPPG_CUDA(cudaMemcpyAsync(&left, a.count, sizeof(int), cudaMemcpyDeviceToHost, st));
             MAPPG_CUDA(cudaStreamSynchronize(st));
@@ -781,37 +823,37 @@ void batch_lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_
                 // energies would drown in their rounding: back to x0 (and a
                 // list around it) and on with energy differences
                 MAPPG_CUDA(cudaMemsetAsync(a.count, 0, sizeof(int), st));
-                k_bl_count_long<<<gb, 256, 0, st>>>(a);
+                launch_dep(st, k_bl_count_long, gb, 256, 0, a);
                 int longer = 0;
                 MAPPG_CUDA(cudaMemcpyAsync(&longer, a.count, sizeof(int), cudaMemcpyDeviceToHost, st));
                 MAPPG_CUDA(cudaStreamSynchronize(st));
                 if (longer == 0) {
-                    k_bl_restore_ls<<<ga, 256, 0, st>>>(a);
+                    launch_dep(st, k_bl_restore_ls, ga, 256, 0, a);
                     lb_update(s);
                     MAPPG_CUDA(cudaMemsetAsync(a.count, 0, sizeof(int), st));
-                    k_bl_dx<<<gc, 256, 0, st>>>(a);
-                    k_bl_cells_bound<<<gw, 256, 0, st>>>(a);
+                    launch_dep(st, k_bl_dx, gc, 256, 0, a);
+                    launch_dep(st, k_bl_cells_bound, gw, 256, 0, a);
                     int wide = 0;
                     MAPPG_CUDA(cudaMemcpyAsync(&wide, a.count, sizeof(int), cudaMemcpyDeviceToHost, st));
                     MAPPG_CUDA(cudaStreamSynchronize(st));
                     if (wide == 0) {
                         a.emode = BL_EDELTA;
-                        k_lb_h32b<<<ga, 256, 0, st>>>(n, a.h, h32);
+                        launch_dep(st, k_lb_h32b, ga, 256, 0, n, a.h, h32);
                         MAPPG_CUDA(cudaGetLastError());
                     }
                 }
             }
         }
-        k_bl_restore<<<ga, 256, 0, st>>>(a);
+        launch_dep(st, k_bl_restore, ga, 256, 0, a);
         lb_update(s);
         // force pass of the cells that took a step, tolerances and history
-        k_bl_active<<<gb, 256, 0, st>>>(a, BL_ACCEPT);
+        launch_dep(st, k_bl_active, gb, 256, 0, a, BL_ACCEPT);
         s->cell_active = a.active;
         launch_force(s);
         sync_forces64(s);
         s->cell_active = nullptr;
-        k_bl_hist<<<gc, 256, 0, st>>>(a);
-        k_bl_cells_step<<<gw, 256, 0, st>>>(a);
+        launch_dep(st, k_bl_hist, gc, 256, 0, a);
+        launch_dep(st, k_bl_cells_step, gw, 256, 0, a);
         MAPPG_CUDA(cudaGetLastError());
     }
     }

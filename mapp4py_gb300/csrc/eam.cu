@@ -534,6 +534,7 @@ void launch_density_only(mappg_sys* s) {
 // degree of freedom carry no force
 template <class T>
 __global__ void k_dof_mask(int n, const uint8_t* __restrict__ dof, T* __restrict__ f) {
+    dep_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const unsigned d = dof[i];
         if (d == 7u) continue;
@@ -545,9 +546,9 @@ __global__ void k_dof_mask(int n, const uint8_t* __restrict__ dof, T* __restrict
 void launch_dof_mask(mappg_sys* s, bool f32) {
     if (!s->dof) return;
     if (f32)
-        k_dof_mask<float><<<grid_for(s, s->n, 256), 256, 0, s->stream>>>(s->n, s->dof, s->f32);
+        launch_dep(s->stream, k_dof_mask<float>, grid_for(s, s->n, 256), 256, 0, s->n, s->dof, s->f32);
     else
-        k_dof_mask<double><<<grid_for(s, s->n, 256), 256, 0, s->stream>>>(s->n, s->dof, s->f);
+        launch_dep(s->stream, k_dof_mask<double>, grid_for(s, s->n, 256), 256, 0, s->n, s->dof, s->f);
     MAPPG_CUDA(cudaGetLastError());
 }
 

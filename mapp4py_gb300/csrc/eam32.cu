@@ -349,6 +349,7 @@ __device__ __forceinline__ void density_atom(const EamArgs& a, const Smem32& S, 
 
 template <int TPA, bool ORTHO, int U>
 __global__ void __launch_bounds__(256) k_density32(EamArgs a) {
+    dep_wait();
     __shared__ Smem32 S;
     S.fill(a);
     const Consts32 K(a);
@@ -379,6 +380,7 @@ __global__ void __launch_bounds__(256) k_density32(EamArgs a) {
 // than the first copied knot read global memory
 template <int TPA, bool ORTHO, int U>
 __global__ void __launch_bounds__(1024, 1) k_density32s(EamArgs a) {
+    dep_wait();
     extern __shared__ float4 stab[];
     const int W = a.rho_w, ntab = a.rho_ntab;
     for (int k = threadIdx.x; k < ntab * W; k += blockDim.x) {
@@ -413,6 +415,7 @@ __global__ void __launch_bounds__(1024, 1) k_density32s(EamArgs a) {
 // batch: blocks walk chunks; the chunk's embedding energy goes to slot 13
 template <int TPA, bool ORTHO, int U>
 __global__ void __launch_bounds__(256) k_density32b(EamArgs a) {
+    dep_wait();
     __shared__ Smem32 S;
     S.fill(a);
     const Consts32 K(a);
@@ -673,6 +676,7 @@ __device__ __forceinline__ void force_atom(const EamArgs& a, const Smem32& S, co
 
 template <int TPA, bool ORTHO, int U>
 __global__ void __launch_bounds__(256, U == 4 ? 1 : 4) k_force32(EamArgs a) {
+    dep_wait();
     __shared__ Smem32 S;
     S.fill(a);
     const Consts32 K(a);
@@ -707,6 +711,7 @@ __global__ void __launch_bounds__(256, U == 4 ? 1 : 4) k_force32(EamArgs a) {
 // records cost shared-memory reads instead of L1/L2 traffic
 template <int TPA, bool ORTHO, int U>
 __global__ void __launch_bounds__(1024, 1) k_force32s(EamArgs a) {
+    dep_wait();
     extern __shared__ float4 ftab_s[];
     __shared__ Smem32 S;
     S.fill(a);  // ends with __syncthreads
@@ -779,6 +784,7 @@ __global__ void k_fs_fill(EamArgs a, float4* __restrict__ out, int R, int W, int
 // batch: chunk slots 0 pair energy, 1-6 virial
 template <int TPA, bool ORTHO, int U>
 __global__ void __launch_bounds__(256, 4) k_force32b(EamArgs a) {
+    dep_wait();
     __shared__ Smem32 S;
     S.fill(a);
     const Consts32 K(a);
@@ -851,6 +857,7 @@ __device__ __forceinline__ void energy_atom(const EamArgs& a, const Smem32& S, c
 
 template <int TPA, bool ORTHO>
 __global__ void __launch_bounds__(256) k_energy32(EamArgs a) {
+    dep_wait();
     __shared__ Smem32 S;
     S.fill(a);
     const Consts32 K(a);
@@ -878,6 +885,7 @@ __global__ void __launch_bounds__(256) k_energy32(EamArgs a) {
 // batch: the chunk's energy goes to slot 0
 template <int TPA, bool ORTHO>
 __global__ void __launch_bounds__(256) k_energy32b(EamArgs a) {
+    dep_wait();
     __shared__ Smem32 S;
     S.fill(a);
     const Consts32 K(a);
@@ -1049,6 +1057,7 @@ __device__ __forceinline__ void de_atom(const EamArgs& a, const Smem32& S, const
 
 template <int TPA, bool ORTHO>
 __global__ void __launch_bounds__(256) k_de32(EamArgs a) {
+    dep_wait();
     __shared__ Smem32 S;
     S.fill(a);
     const Consts32 K(a);
@@ -1078,6 +1087,7 @@ __global__ void __launch_bounds__(256) k_de32(EamArgs a) {
 // cell_active only)
 template <int TPA, bool ORTHO>
 __global__ void __launch_bounds__(256) k_de32b(EamArgs a) {
+    dep_wait();
     __shared__ Smem32 S;
     S.fill(a);
     const Consts32 K(a);
@@ -1105,6 +1115,7 @@ __global__ void __launch_bounds__(256) k_de32b(EamArgs a) {
 // (kinetic tensor and the closing half of each cell's chain, thermo rows of
 // pe and T per cell)
 __global__ void k_cells_done(EamArgs a, const int* __restrict__ cell_chunk, CellMd* __restrict__ cmd, int what) {
+    dep_wait();
     const int lane = threadIdx.x & 31;
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (c >= a.ncell) return;
@@ -1155,13 +1166,13 @@ __global__ void k_cells_done(EamArgs a, const int* __restrict__ cell_chunk, Cell
 template <int TPA, bool ORTHO, int U>
 static void density_t(mappg_sys* s, const EamArgs& a) {
     if (TPA == 8 && s->unroll == 4) {
-        k_density32<8, ORTHO, 4><<<atom_blocks(s, 8), 256, 0, s->stream>>>(a);
+        launch_dep(s->stream, k_density32<8, ORTHO, 4>, atom_blocks(s, 8), 256, 0, a);
         return;
     }
     if (s->n <= kDensSmallAtoms) {
         static int grid = 0;
         if (!grid) grid = occupancy_grid(s, k_density32<TPA, ORTHO, U>, 256);
-        k_density32<TPA, ORTHO, U><<<std::min(grid, atom_blocks(s, TPA)), 256, 0, s->stream>>>(a);
+        launch_dep(s->stream, k_density32<TPA, ORTHO, U>, std::min(grid, atom_blocks(s, TPA)), 256, 0, a);
         return;
     }
     static bool attr = false;
@@ -1171,7 +1182,7 @@ static void density_t(mappg_sys* s, const EamArgs& a) {
         attr = true;
     }
     const size_t bytes = sizeof(float4) * (size_t)a.rho_ntab * a.rho_w;
-    k_density32s<TPA, ORTHO, U><<<s->sm_count, 1024, bytes, s->stream>>>(a);
+    launch_dep(s->stream, k_density32s<TPA, ORTHO, U>, s->sm_count, 1024, bytes, a);
 }
 
 template <int TPA, bool ORTHO, int U>
@@ -1184,58 +1195,58 @@ static void force_t(mappg_sys* s, const EamArgs& a) {
             attr = true;
         }
         const size_t bytes = sizeof(float4) * (size_t)a.fs_rec * a.fs_w;
-        k_force32s<TPA, ORTHO, U><<<s->sm_count, 1024, bytes, s->stream>>>(a);
+        launch_dep(s->stream, k_force32s<TPA, ORTHO, U>, s->sm_count, 1024, bytes, a);
         return;
     }
     if (TPA == 8 && s->unroll == 4 && !s->unroll_force) {
-        k_force32<8, ORTHO, 4><<<atom_blocks(s, 8), 256, 0, s->stream>>>(a);
+        launch_dep(s->stream, k_force32<8, ORTHO, 4>, atom_blocks(s, 8), 256, 0, a);
         return;
     }
     static int grid = 0;
     if (!grid) grid = occupancy_grid(s, k_force32<TPA, ORTHO, U>, 256);
-    k_force32<TPA, ORTHO, U><<<std::min(grid, atom_blocks(s, TPA)), 256, 0, s->stream>>>(a);
+    launch_dep(s->stream, k_force32<TPA, ORTHO, U>, std::min(grid, atom_blocks(s, TPA)), 256, 0, a);
 }
 
 template <int TPA, bool ORTHO, int U>
 static void energy_t(mappg_sys* s, const EamArgs& a) {
     static int grid = 0;
     if (!grid) grid = occupancy_grid(s, k_energy32<TPA, ORTHO>, 256);
-    k_energy32<TPA, ORTHO><<<std::min(grid, atom_blocks(s, TPA)), 256, 0, s->stream>>>(a);
+    launch_dep(s->stream, k_energy32<TPA, ORTHO>, std::min(grid, atom_blocks(s, TPA)), 256, 0, a);
 }
 
 template <int TPA, bool ORTHO, int U>
 static void de_t(mappg_sys* s, const EamArgs& a) {
     static int grid = 0;
     if (!grid) grid = occupancy_grid(s, k_de32<TPA, ORTHO>, 256);
-    k_de32<TPA, ORTHO><<<std::min(grid, atom_blocks(s, TPA)), 256, 0, s->stream>>>(a);
+    launch_dep(s->stream, k_de32<TPA, ORTHO>, std::min(grid, atom_blocks(s, TPA)), 256, 0, a);
 }
 
 template <int TPA, bool ORTHO, int U>
 static void de_b(mappg_sys* s, const EamArgs& a) {
     static int grid = 0;
     if (!grid) grid = occupancy_grid(s, k_de32b<TPA, ORTHO>, 256);
-    k_de32b<TPA, ORTHO><<<std::min(grid, a.nchunk), 256, 0, s->stream>>>(a);
+    launch_dep(s->stream, k_de32b<TPA, ORTHO>, std::min(grid, a.nchunk), 256, 0, a);
 }
 
 template <int TPA, bool ORTHO, int U>
 static void density_b(mappg_sys* s, const EamArgs& a) {
     static int grid = 0;
     if (!grid) grid = occupancy_grid(s, k_density32b<TPA, ORTHO, U>, 256);
-    k_density32b<TPA, ORTHO, U><<<std::min(grid, a.nchunk), 256, 0, s->stream>>>(a);
+    launch_dep(s->stream, k_density32b<TPA, ORTHO, U>, std::min(grid, a.nchunk), 256, 0, a);
 }
 
 template <int TPA, bool ORTHO, int U>
 static void force_b(mappg_sys* s, const EamArgs& a) {
     static int grid = 0;
     if (!grid) grid = occupancy_grid(s, k_force32b<TPA, ORTHO, U>, 256);
-    k_force32b<TPA, ORTHO, U><<<std::min(grid, a.nchunk), 256, 0, s->stream>>>(a);
+    launch_dep(s->stream, k_force32b<TPA, ORTHO, U>, std::min(grid, a.nchunk), 256, 0, a);
 }
 
 template <int TPA, bool ORTHO, int U>
 static void energy_b(mappg_sys* s, const EamArgs& a) {
     static int grid = 0;
     if (!grid) grid = occupancy_grid(s, k_energy32b<TPA, ORTHO>, 256);
-    k_energy32b<TPA, ORTHO><<<std::min(grid, a.nchunk), 256, 0, s->stream>>>(a);
+    launch_dep(s->stream, k_energy32b<TPA, ORTHO>, std::min(grid, a.nchunk), 256, 0, a);
 }
 
 // a batch takes the orthorhombic kernels only when every cell is orthorhombic
@@ -1275,7 +1286,7 @@ static void pick_ortho(bool o, F&& fn) {
 #define MAPPG_FORCE_U (s->unroll_force ? s->unroll_force : s->unroll)
 
 static void cells_done(mappg_sys* s, const EamArgs& a, int what) {
-    k_cells_done<<<(s->ncell * 32 + 255) / 256, 256, 0, s->stream>>>(a, s->cell_chunk, s->cmd, what);
+    launch_dep(s->stream, k_cells_done, (s->ncell * 32 + 255) / 256, 256, 0, a, s->cell_chunk, s->cmd, what);
     MAPPG_CUDA(cudaGetLastError());
 }
 

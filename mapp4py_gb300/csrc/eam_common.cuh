@@ -18,6 +18,33 @@
 
 namespace mappg {
 
+// Programmatic dependent launch: a kernel launched by launch_dep is brought
+// onto the SMs as the blocks of the kernel before it in the stream leave
+// them, and waits in dep_wait, its first statement, until that kernel has
+// completed and its writes are visible.  What it hides is launch latency: a
+// force call of 500 FP64 atoms 152 -> 138 us, 10 L-BFGS iterations of 4,000
+// 3.55 -> 2.99 ms, 100 MD steps of 4,000 mixed atoms 4.87 -> 4.76.  Letting the
+// next kernel on earlier (griddepcontrol.launch_dependents) was measured and
+// not kept: its blocks crowd the SMs that happen to be free (100 FP64 steps
+// 7.5 -> 8.7 ms at the start of a kernel, 8.2 before its reduction).  A kernel
+// with dep_wait launched in the ordinary way runs as ever.
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+static void launch_dep(cudaStream_t stream, void (*kernel)(P...), int grid, int block, size_t smem, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    MAPPG_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+
 // 32-byte read-only loads (one sector per lane, one instruction): the spline
 // records are 32 bytes and 32-byte aligned, so a lane fetches a whole record
 // with one L1 request instead of two
@@ -129,13 +156,20 @@ __device__ __forceinline__ double (*red_rows())[W] {
 }
 
 // the sum of the block's rows of P values in red_rows, by the first warp:
-// lane k < P returns value k (a dependent FP64 add takes 65 clocks here, so
-// the lanes share the rows and add up pairwise)
-template <int P>
+// lane k < P returns value k.  A dependent FP64 add takes 65 clocks here, so
+// the lanes share the rows and add up pairwise; ORDERED adds the warps' rows
+// one by one (the minimizers' dot products: their order is part of a
+// relaxation's path, which magnifies a last bit)
+template <int P, bool ORDERED>
 __device__ __forceinline__ double rows_sum() {
     double(*red)[red_width(P)] = red_rows<red_width(P)>();
     const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     double t = 0.0;
+    if (ORDERED) {
+        if (lane < P)
+            for (int q = 0; q < nw; q++) t += red[q][lane];
+        return t;
+    }
     for (int q = lane / P; q < nw; q += 32 / P) t += red[q][lane % P];
 #pragma unroll
     for (int o = P; o < 32; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
@@ -144,7 +178,7 @@ __device__ __forceinline__ double rows_sum() {
 
 // block totals of K values of type T, as doubles: value k in lane k of the
 // first warp
-template <int K, class T>
+template <int K, bool ORDERED = false, class T>
 __device__ __forceinline__ double block_sums(const T (&v)[K]) {
     constexpr int P = red_pow2(K);
     static_assert(P <= 16, "a row holds 16 values");
@@ -155,7 +189,7 @@ __device__ __forceinline__ double block_sums(const T (&v)[K]) {
     const T t = warp_reduce(u, RedAdd());
     if (lane % (32 / P) == 0) red_rows<red_width(P)>()[w][lane / (32 / P)] = red_double(t);
     __syncthreads();
-    return w == 0 ? rows_sum<P>() : 0.0;
+    return w == 0 ? rows_sum<P, ORDERED>() : 0.0;
 }
 
 // the first warp, whose lanes stored the block's partials, counts the block
@@ -180,9 +214,9 @@ __device__ __forceinline__ bool last_block(unsigned* counter) {
 // warp sums need no more than FP32) into
 // partials[blockIdx.x*kRedSlots + slot0 + k]; returns true in the block that
 // finished last (its threads then see all partials)
-template <int K, class T>
+template <int K, bool ORDERED = false, class T>
 __device__ bool block_partials(const T (&v)[K], double* partials, int slot0, unsigned* counter) {
-    const double t = block_sums<K>(v);
+    const double t = block_sums<K, ORDERED>(v);
     if (threadIdx.x < K) partials[blockIdx.x * kRedSlots + slot0 + threadIdx.x] = t;
     return last_block(counter);
 }
@@ -212,8 +246,41 @@ __device__ void final_sums(const double* partials, int nblk, double* tot, int nb
     if (lane < P) red_rows<red_width(P)>()[w][lane] = t;
     __syncthreads();
     if (w == 0) {
-        const double r = rows_sum<P>();
+        const double r = rows_sum<P, false>();
         if (lane < K) tot[lane] = r;
+    }
+    __syncthreads();
+}
+
+// the same in an order that does not depend on the block's size (see
+// rows_sum): 32 strided sums of the blocks' rows per slot, then a butterfly
+// over them, a warp per slot
+template <int K>
+__device__ void final_sums_ordered(const double* partials, int nblk, double* tot) {
+    constexpr int P = red_pow2(K);
+    double(*red)[red_width(P)] = red_rows<red_width(P)>();
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int k = threadIdx.x % P;
+    for (int r = threadIdx.x / P; r < 32; r += blockDim.x / P) {
+        double t = 0.0;
+        for (int b0 = r; b0 < nblk; b0 += 8 * 32) {
+            double u[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const int b = b0 + 32 * q;
+                u[q] = k < K && b < nblk ? __ldcg(partials + b * kRedSlots + k) : 0.0;
+            }
+#pragma unroll
+            for (int q = 0; q < 8; q++) t += u[q];
+        }
+        red[r][k] = t;
+    }
+    __syncthreads();
+    for (int c = w; c < K; c += nw) {
+        double t = red[lane][c];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) tot[c] = t;
     }
     __syncthreads();
 }

@@ -51,6 +51,7 @@ constexpr int kLbU = 4;  // components a thread of the vector kernels loads at a
 __global__ void __launch_bounds__(256) k_lb_axpy_dot(int N, double* __restrict__ h, const double* __restrict__ y,
                                                      const double* __restrict__ s, LbScal* L, int mode, int idx,
                                                      int dot_in, int dot_out, double* partials, unsigned* counter) {
+    dep_wait();
     double coef = 0.0;
     if (mode == 1) {
         coef = -L->rho[idx] * L->dot[dot_in];
@@ -93,8 +94,8 @@ __global__ void __launch_bounds__(256) k_lb_axpy_dot(int N, double* __restrict__
     if (!s) return;
     double v[1] = {acc};
     __shared__ double t[1];
-    if (block_partials<1>(v, partials, 0, counter)) {
-        final_sums<1>(partials, gridDim.x, t);
+    if (block_partials<1, true>(v, partials, 0, counter)) {
+        final_sums_ordered<1>(partials, gridDim.x, t);
         if (threadIdx.x == 0) {
             L->dot[dot_out] = t[0];
             *counter = 0;
@@ -108,6 +109,7 @@ __global__ void __launch_bounds__(256) k_lb_axpy_dot(int N, double* __restrict__
 __global__ void __launch_bounds__(256) k_lb_prep(int N, const double* __restrict__ f, const double* __restrict__ h,
                                                  const double* __restrict__ x, const double* __restrict__ xb,
                                                  LbScal* L, double* partials, unsigned* counter) {
+    dep_wait();
     double v[2] = {0.0, 0.0};
     unsigned long long mx[4] = {0, 0, 0, 0};  // bits of the maxima (integer compares; FP64 ones are slow here)
     const int stride = gridDim.x * blockDim.x;
@@ -142,8 +144,8 @@ __global__ void __launch_bounds__(256) k_lb_prep(int N, const double* __restrict
         for (int q = 0; q < nw; q++) r = RedMaxBits()(r, redm[q][threadIdx.x]);
         partials[blockIdx.x * kRedSlots + 2 + threadIdx.x] = __longlong_as_double((long long)r);
     }
-    if (block_partials<2>(v, partials, 0, counter)) {
-        final_sums<2>(partials, gridDim.x, tot);
+    if (block_partials<2, true>(v, partials, 0, counter)) {
+        final_sums_ordered<2>(partials, gridDim.x, tot);
         unsigned long long b[4] = {0, 0, 0, 0};
         for (int bb = threadIdx.x; bb < (int)gridDim.x; bb += blockDim.x)
 #pragma unroll
@@ -174,6 +176,7 @@ __global__ void __launch_bounds__(256) k_lb_prep(int N, const double* __restrict
 // order as the values do, so an integer maximum of the bits is the maximum)
 __global__ void k_lb_dxmax(int N, const double* __restrict__ x, const double* __restrict__ xb,
                            unsigned long long* out) {
+    dep_wait();
     double m = 0.0;
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < N; q += gridDim.x * blockDim.x)
         m = fmax(m, fabs(x[q] - xb[q]));
@@ -184,6 +187,7 @@ __global__ void k_lb_dxmax(int N, const double* __restrict__ x, const double* __
 
 // the search direction as one float4 per atom (Cartesian) for k_de32
 __global__ void k_lb_h32(int n, const double* __restrict__ h, float4* __restrict__ h32) {
+    dep_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         h32[i] = make_float4((float)h[i], (float)h[n + i], (float)h[2 * n + i], 0.f);
 }
@@ -191,6 +195,7 @@ __global__ void k_lb_h32(int n, const double* __restrict__ h, float4* __restrict
 // x = x0 + alpha*h  (MinMDHandler::F, min_cg.h:260-267)
 __global__ void k_lb_trial(int N, double* __restrict__ x, const double* __restrict__ x0, const double* __restrict__ h,
                            double alpha) {
+    dep_wait();
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < N; q += gridDim.x * blockDim.x)
         x[q] = x0[q] + alpha * h[q];
 }
@@ -204,6 +209,7 @@ __global__ void __launch_bounds__(256) k_lb_hist(int N, double* __restrict__ s0,
                                                  const double* __restrict__ h, const double* __restrict__ f0,
                                                  const double* __restrict__ f, const double* __restrict__ P,
                                                  double alpha, LbScal* L, double* partials, unsigned* counter) {
+    dep_wait();
     double v[3] = {0.0, 0.0, 0.0};
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < N; q += gridDim.x * blockDim.x) {
         double sv = alpha * h[q];
@@ -215,8 +221,8 @@ __global__ void __launch_bounds__(256) k_lb_hist(int N, double* __restrict__ s0,
         if (P) v[2] += yv * yv * P[q];
     }
     __shared__ double t[3];
-    if (block_partials<3>(v, partials, 0, counter)) {
-        final_sums<3>(partials, gridDim.x, t);
+    if (block_partials<3, true>(v, partials, 0, counter)) {
+        final_sums_ordered<3>(partials, gridDim.x, t);
         if (threadIdx.x == 0) {
             if (t[0] > 0.0 && t[1] > 0.0) {
                 L->gamma = t[0] / t[1];
@@ -231,6 +237,7 @@ __global__ void __launch_bounds__(256) k_lb_hist(int N, double* __restrict__ s0,
 }
 
 __global__ void k_lb_shift_rho(LbScal* L, int m) {
+    dep_wait();
     for (int i = m - 1; i > 0; i--) L->rho[i] = L->rho[i - 1];
 }
 
@@ -261,10 +268,11 @@ static double lb_energy(mappg_sys* s) {
     return e;
 }
 
-__global__ void k_clear_rebuild(DevScalars* sc) { sc->rebuild = 0; }
+__global__ void k_clear_rebuild(DevScalars* sc) {
+    dep_wait(); sc->rebuild = 0; }
 
 void lb_update(mappg_sys* s) {
-    k_clear_rebuild<<<1, 1, 0, s->stream>>>(s->sc);
+    launch_dep(s->stream, k_clear_rebuild, 1, 1, 0, s->sc);
     launch_skin_test(s);
     launch_rebuild_chain(s);
     // positions moved without a rebuild: refresh the mixed kernels' frame
@@ -320,7 +328,7 @@ struct TrialLine {
         // an E32DIFF search whose trials have become short goes over to
         // energy differences (FP32 differences would drown in rounding)
         if (mode == E32DIFF && 1.7320508075688772 * a * hmax < 0.25 * s->skin) to_delta(a);
-        k_lb_trial<<<grid, 256, 0, s->stream>>>(N, s->x, xs, h, a);
+        launch_dep(s->stream, k_lb_trial, grid, 256, 0, N, s->x, xs, h, a);
         (*n_en)++;
         if (mode == E64) return lb_energy(s);
         double e;
@@ -342,7 +350,7 @@ struct TrialLine {
         MAPPG_CUDA(cudaMemcpyAsync(s->x, xs, sizeof(double) * N, cudaMemcpyDeviceToDevice, s->stream));
         lb_update(s);
         MAPPG_CUDA(cudaMemsetAsync(&L->dxbits, 0, sizeof(unsigned long long), s->stream));
-        k_lb_dxmax<<<grid, 256, 0, s->stream>>>(N, s->x, s->x0, &L->dxbits);
+        launch_dep(s->stream, k_lb_dxmax, grid, 256, 0, N, s->x, s->x0, &L->dxbits);
         unsigned long long bits = 0;
         MAPPG_CUDA(cudaMemcpyAsync(&bits, &L->dxbits, sizeof(bits), cudaMemcpyDeviceToHost, s->stream));
         MAPPG_CUDA(cudaStreamSynchronize(s->stream));
@@ -443,7 +451,7 @@ void lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_tol, c
     int err = nsteps == 0 ? MIN_F_MAX_ITER : LS_S;
     double dxmax = 0.0;
     auto read_prep = [&](double* fh, double* hh, double* hmax, double* fmax_) {
-        k_lb_prep<<<grid, 256, 0, st>>>(N, s->f, h, s->x, s->x0, L, part, counter);
+        launch_dep(st, k_lb_prep, grid, 256, 0, N, s->f, h, s->x, s->x0, L, part, counter);
         MAPPG_CUDA(cudaGetLastError());
         double buf[6];
         MAPPG_CUDA(cudaMemcpyAsync(buf, &L->fh, sizeof(buf), cudaMemcpyDeviceToHost, st));
@@ -465,18 +473,18 @@ void lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_tol, c
     auto two_loop = [&](bool diag) {
         MAPPG_CUDA(cudaMemcpyAsync(h, s->f, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
         // first loop: alpha_i = -rho_i (s_i.h); h += alpha_i y_i
-        if (k > 0) k_lb_axpy_dot<<<grid, 256, 0, st>>>(N, h, nullptr, sv[0], L, 0, 0, 0, 0, part, counter);
+        if (k > 0) launch_dep(st, k_lb_axpy_dot, grid, 256, 0, N, h, nullptr, sv[0], L, 0, 0, 0, 0, part, counter);
         for (int i = 0; i < k; i++) {
             const double* nxt = (i + 1 < k) ? sv[i + 1] : nullptr;
-            k_lb_axpy_dot<<<grid, 256, 0, st>>>(N, h, yv[i], nxt, L, 1, i, i, i + 1, part, counter);
+            launch_dep(st, k_lb_axpy_dot, grid, 256, 0, N, h, yv[i], nxt, L, 1, i, i, i + 1, part, counter);
         }
         // h *= H0, and the first dot of the second loop y_{k-1}.h
-        k_lb_axpy_dot<<<grid, 256, 0, st>>>(N, h, diag ? P : nullptr, k > 0 ? yv[k - 1] : nullptr, L, diag ? 4 : 3,
-                                            0, 0, 64, part, counter);
+        launch_dep(st, k_lb_axpy_dot, grid, 256, 0, N, h, diag ? P : nullptr, k > 0 ? yv[k - 1] : nullptr, L,
+                   diag ? 4 : 3, 0, 0, 64, part, counter);
         for (int i = k - 1; i > -1; i--) {
             const double* nxt = i > 0 ? yv[i - 1] : nullptr;
-            k_lb_axpy_dot<<<grid, 256, 0, st>>>(N, h, sv[i], nxt, L, 2, i, 64 + (k - 1 - i), 64 + (k - i), part,
-                                                counter);
+            launch_dep(st, k_lb_axpy_dot, grid, 256, 0, N, h, sv[i], nxt, L, 2, i, 64 + (k - 1 - i), 64 + (k - i),
+                       part, counter);
         }
         MAPPG_CUDA(cudaGetLastError());
     };
@@ -521,7 +529,7 @@ void lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_tol, c
         if (mixed && !s->force64 && dfa < 0.0 && max_a > 0.0) {
             line.e0 = e_curr;
             line.hmax = hmax;
-            k_lb_h32<<<grid_for(s, s->n, 256), 256, 0, st>>>(s->n, h, s->h32);
+            launch_dep(st, k_lb_h32, grid_for(s, s->n, 256), 256, 0, s->n, h, s->h32);
             MAPPG_CUDA(cudaGetLastError());
             const double a1 = std::min(max_a, 1.0);
             if (1.7320508075688772 * (a1 * hmax + dxmax) < 0.5 * s->skin) {
@@ -585,8 +593,8 @@ void lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_tol, c
             }
             sv[0] = ts;
             yv[0] = ty;
-            k_lb_shift_rho<<<1, 1, 0, st>>>(L, m);
-            k_lb_hist<<<grid, 256, 0, st>>>(N, sv[0], yv[0], h, f0, s->f, P, alpha_m, L, part, counter);
+            launch_dep(st, k_lb_shift_rho, 1, 1, 0, L, m);
+            launch_dep(st, k_lb_hist, grid, 256, 0, N, sv[0], yv[0], h, f0, s->f, P, alpha_m, L, part, counter);
             MAPPG_CUDA(cudaGetLastError());
         } else {
             // gamma = alpha_m (h.f0 - h.f)/(f.f + f0.f0 - 2 f.f0) on the host
@@ -640,14 +648,15 @@ namespace mappg {
 // f.f and f.f0 into L->dot[0], L->dot[1]
 __global__ void __launch_bounds__(256) k_cg_dots(int N, const double* __restrict__ f, const double* __restrict__ f0,
                                                  LbScal* L, double* partials, unsigned* counter) {
+    dep_wait();
     double v[2] = {0.0, 0.0};
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < N; q += gridDim.x * blockDim.x) {
         v[0] += f[q] * f[q];
         v[1] += f[q] * f0[q];
     }
     __shared__ double t[2];
-    if (block_partials<2>(v, partials, 0, counter)) {
-        final_sums<2>(partials, gridDim.x, t);
+    if (block_partials<2, true>(v, partials, 0, counter)) {
+        final_sums_ordered<2>(partials, gridDim.x, t);
         if (threadIdx.x == 0) {
             L->dot[0] = t[0];
             L->dot[1] = t[1];
@@ -657,6 +666,7 @@ __global__ void __launch_bounds__(256) k_cg_dots(int N, const double* __restrict
 }
 
 __global__ void k_cg_dir(int N, double* __restrict__ h, const double* __restrict__ f, double ratio) {
+    dep_wait();
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < N; q += gridDim.x * blockDim.x) h[q] = ratio * h[q] + f[q];
 }
 
@@ -690,7 +700,7 @@ void cg_run(mappg_sys* s, double e_tol, double max_dx, double f_tol, const LsPar
     double* part = s->partials;
     double dxmax = 0.0;
     auto read_prep = [&](double* fh, double* hh, double* hmax, double* fmax_) {
-        k_lb_prep<<<grid, 256, 0, st>>>(N, s->f, h, s->x, s->x0, L, part, counter);
+        launch_dep(st, k_lb_prep, grid, 256, 0, N, s->f, h, s->x, s->x0, L, part, counter);
         MAPPG_CUDA(cudaGetLastError());
         double buf[6];
         MAPPG_CUDA(cudaMemcpyAsync(buf, &L->fh, sizeof(buf), cudaMemcpyDeviceToHost, st));
@@ -782,13 +792,13 @@ void cg_run(mappg_sys* s, double e_tol, double max_dx, double f_tol, const LsPar
         }
         if (istep + 1 == nsteps) err = MIN_F_MAX_ITER;
         if (err) continue;
-        k_cg_dots<<<grid, 256, 0, st>>>(N, s->f, f0, L, part, counter);
+        launch_dep(st, k_cg_dots, grid, 256, 0, N, s->f, f0, L, part, counter);
         MAPPG_CUDA(cudaGetLastError());
         double dd[2];
         MAPPG_CUDA(cudaMemcpyAsync(dd, &L->dot[0], sizeof(dd), cudaMemcpyDeviceToHost, st));
         MAPPG_CUDA(cudaStreamSynchronize(st));
         const double ratio = (dd[0] - dd[1]) / f0_f0;
-        k_cg_dir<<<grid, 256, 0, st>>>(N, h, s->f, ratio);
+        launch_dep(st, k_cg_dir, grid, 256, 0, N, h, s->f, ratio);
         MAPPG_CUDA(cudaGetLastError());
         f0_f0 = dd[0];
     }
@@ -857,7 +867,7 @@ extern "C" int mappg_sys_energy_delta(mappg_sys* s, const double* h, double alph
         MAPPG_CUDA(cudaMalloc(&L, sizeof(LbScal)));
         MAPPG_CUDA(cudaMalloc(&counter, sizeof(unsigned)));
         MAPPG_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned), s->stream));
-        k_lb_prep<<<grid, 256, 0, s->stream>>>(N, hd, hd, s->x, s->x0, L, s->partials, counter);
+        launch_dep(s->stream, k_lb_prep, grid, 256, 0, N, hd, hd, s->x, s->x0, L, s->partials, counter);
         MAPPG_CUDA(cudaGetLastError());
         double dxmax = 0.0;
         MAPPG_CUDA(cudaMemcpyAsync(&dxmax, &L->dxmax, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
@@ -867,7 +877,7 @@ extern "C" int mappg_sys_energy_delta(mappg_sys* s, const double* h, double alph
         s->keep_rho64 = true;
         s->h32 = h32;
         launch_force(s);  // density of x kept in FP64, F'(rho) and forces of x
-        k_lb_h32<<<grid_for(s, n, 256), 256, 0, s->stream>>>(n, hd, h32);
+        launch_dep(s->stream, k_lb_h32, grid_for(s, n, 256), 256, 0, n, hd, h32);
         launch_de32(s, alpha);
         MAPPG_CUDA(cudaMemcpyAsync(de, &s->sc->de, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
         MAPPG_CUDA(cudaStreamSynchronize(s->stream));

@@ -102,6 +102,7 @@ __device__ __forceinline__ NhcParams cell_nhc(const NhcParams& P0, const CellMd*
 // pre_init (md_nvt.cpp:256-340): kinetic tensor and temperature of the
 // incoming velocities
 __global__ void k_mvv_init(MdArgs a) {
+    dep_wait();
     double d[6] = {0, 0, 0, 0, 0, 0};
     const int n = a.n;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -216,6 +217,7 @@ __device__ __forceinline__ bool close_partials(const T (&v)[K], const MdArgs& a,
 // run start: thermo row 0, no pending velocity scale or kick, the first
 // step's opening half
 __global__ void k_run_begin(MdArgs a) {
+    dep_wait();
     DevScalars* sc = a.sc;
     write_thermo_row(a.thermo, sc, 0);
     double eta[kMaxChain];
@@ -232,6 +234,7 @@ __global__ void k_run_begin(MdArgs a) {
 
 // ------------------------------------------------------------------ FP64 path
 __global__ void __launch_bounds__(256) k_kick_drift64(MdArgs a) {
+    dep_wait();
     const int n = a.n;
     const double fac = a.sc->fac_next;
     double dsum[3] = {0, 0, 0};
@@ -262,6 +265,7 @@ __global__ void __launch_bounds__(256) k_kick_drift64(MdArgs a) {
 }
 
 __global__ void __launch_bounds__(256) k_com_skin64(MdArgs a) {
+    dep_wait();
     const int n = a.n;
     const double c0 = a.sc->com[0], c1 = a.sc->com[1], c2 = a.sc->com[2];
     int moved = 0;
@@ -278,6 +282,7 @@ __global__ void __launch_bounds__(256) k_com_skin64(MdArgs a) {
 }
 
 __global__ void __launch_bounds__(256) k_kick2_64(MdArgs a) {
+    dep_wait();
     const int n = a.n;
     __shared__ CloseStep S;
     S.load(a.sc);
@@ -322,6 +327,7 @@ __global__ void __launch_bounds__(256) k_kick2_64(MdArgs a) {
 }
 
 __global__ void k_run_end64(MdArgs a) {
+    dep_wait();
     const int n = a.n;
     const double fac = a.sc->fac_x_d;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * n; i += gridDim.x * blockDim.x)
@@ -331,6 +337,7 @@ __global__ void k_run_end64(MdArgs a) {
 // ------------------------------------------------------------------ mixed path
 template <bool ORTHO>
 __global__ void __launch_bounds__(256) k_integrate32(MdArgs a) {
+    dep_wait();
     const int n = a.n;
     const double A = a.sc->kickA;
     const float B = (float)a.sc->kickB;
@@ -396,6 +403,7 @@ __global__ void __launch_bounds__(256) k_integrate32(MdArgs a) {
 // velocity v + f dt/2m (FP32 terms, FP64 sums), then in the last block the
 // mean displacement of the step and what CloseStep does
 __global__ void __launch_bounds__(256) k_close32(MdArgs a) {
+    dep_wait();
     const int n = a.n;
     __shared__ CloseStep S;
     S.load(a.sc);
@@ -445,6 +453,7 @@ __global__ void __launch_bounds__(256) k_close32(MdArgs a) {
 // the same kinetic tensor per chunk of a batch (slots 7-12), for the
 // per-cell closing half in k_cells_done
 __global__ void __launch_bounds__(256) k_ke32b(MdArgs a) {
+    dep_wait();
     const int n = a.n;
     for (int ch = blockIdx.x; ch < a.nchunk; ch += gridDim.x) {
         const int lo = a.chunk_begin[ch], hi = a.chunk_begin[ch + 1];
@@ -470,6 +479,7 @@ __global__ void __launch_bounds__(256) k_ke32b(MdArgs a) {
 // end of a mixed run: the pending closing kick and scale, v = (v + f dt/2m) fc,
 // and the accumulated mean displacement removed from x
 __global__ void k_run_end32(MdArgs a) {
+    dep_wait();
     const int n = a.n;
     const bool pend = a.sc->pending_kick != 0;
     const double fc = pend ? a.sc->fac_close : a.sc->fac_x_d;
@@ -484,6 +494,7 @@ __global__ void k_run_end32(MdArgs a) {
 }
 
 __global__ void k_clear_drift(DevScalars* sc) {
+    dep_wait();
     sc->drift[0] = sc->drift[1] = sc->drift[2] = 0.0;
     sc->pending_kick = 0;
 }
@@ -506,6 +517,7 @@ __device__ __forceinline__ void cell_sums(const MdArgs& a, const double* part, i
 
 // kinetic tensor of the incoming velocities per chunk (slots 7-12)
 __global__ void __launch_bounds__(256) k_mvv_init_b(MdArgs a) {
+    dep_wait();
     const int n = a.n;
     for (int ch = blockIdx.x; ch < a.nchunk; ch += gridDim.x) {
         const int lo = a.chunk_begin[ch], hi = a.chunk_begin[ch + 1];
@@ -526,6 +538,7 @@ __global__ void __launch_bounds__(256) k_mvv_init_b(MdArgs a) {
 
 // run start per cell: kinetic tensor, T, thermo row 0, no pending scale/kick
 __global__ void k_cells_begin(MdArgs a) {
+    dep_wait();
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (c >= a.ncell) return;
     double t[6];
@@ -545,6 +558,7 @@ __global__ void k_cells_begin(MdArgs a) {
 
 // opening half of every cell's chain and its kick factors (open_ahead)
 __global__ void k_cells_open(MdArgs a) {
+    dep_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c == 0) a.sc->rebuild = 0;
     if (c >= a.ncell) return;
@@ -564,6 +578,7 @@ __global__ void k_cells_open(MdArgs a) {
 // k_integrate32 per chunk: the cell's kick factors and frame, displacement
 // sums per chunk
 __global__ void __launch_bounds__(256) k_integrate32b(MdArgs a) {
+    dep_wait();
     const int n = a.n;
     int moved = 0;
     for (int ch = blockIdx.x; ch < a.nchunk; ch += gridDim.x) {
@@ -623,6 +638,7 @@ __global__ void __launch_bounds__(256) k_integrate32b(MdArgs a) {
 
 // per-cell mean displacement of the step, added to the cell's drift
 __global__ void k_cells_com(MdArgs a) {
+    dep_wait();
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (c >= a.ncell) return;
     double t[3];
@@ -639,6 +655,7 @@ __global__ void k_cells_com(MdArgs a) {
 
 // end of a batch run: pending closing kick and scale, drift removed, per cell
 __global__ void k_run_end32b(MdArgs a) {
+    dep_wait();
     const int n = a.n;
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < 3 * n; q += gridDim.x * blockDim.x) {
         const int i = q % n, k = q / n;
@@ -653,6 +670,7 @@ __global__ void k_run_end32b(MdArgs a) {
 }
 
 __global__ void k_cells_clear(MdArgs a) {
+    dep_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= a.ncell) return;
     CellMd* m = a.cmd + c;
@@ -765,41 +783,41 @@ struct NoHook {
 template <class A = NoHook, class B = NoHook>
 static void launch_step64(mappg_sys* s, const MdArgs& a, A listed = A(), B closing = B()) {
     const MdShape m = md_shape(s, true);
-    k_kick_drift64<<<m.grid, m.block, 0, s->stream>>>(a);
-    k_com_skin64<<<m.grid, m.block, 0, s->stream>>>(a);
+    launch_dep(s->stream, k_kick_drift64, m.grid, m.block, 0, a);
+    launch_dep(s->stream, k_com_skin64, m.grid, m.block, 0, a);
     launch_rebuild_chain(s);
     listed();
     launch_force(s);
     closing();
-    k_kick2_64<<<m.grid, m.block, 0, s->stream>>>(a);
+    launch_dep(s->stream, k_kick2_64, m.grid, m.block, 0, a);
 }
 
 template <class A = NoHook, class B = NoHook>
 static void launch_step32(mappg_sys* s, const MdArgs& a, A listed = A(), B closing = B()) {
     const MdShape m = md_shape(s, true), c = md_shape(s, false);
     if (a.fr.ortho)
-        k_integrate32<true><<<m.grid, m.block, 0, s->stream>>>(a);
+        launch_dep(s->stream, k_integrate32<true>, m.grid, m.block, 0, a);
     else
-        k_integrate32<false><<<m.grid, m.block, 0, s->stream>>>(a);
+        launch_dep(s->stream, k_integrate32<false>, m.grid, m.block, 0, a);
     launch_rebuild_chain(s);
     listed();
     EamArgs e = eam_args(s);
     launch_density32(s, e);
     launch_force32(s, e);
     closing();
-    k_close32<<<c.grid, c.block, 0, s->stream>>>(a);
+    launch_dep(s->stream, k_close32, c.grid, c.block, 0, a);
 }
 
 static void launch_step32b(mappg_sys* s, const MdArgs& a) {
     const int nc = s->ncell;
-    k_cells_open<<<(nc + 255) / 256, 256, 0, s->stream>>>(a);
-    k_integrate32b<<<std::min(s->nchunk, s->sm_count * 8), 256, 0, s->stream>>>(a);
-    k_cells_com<<<(nc * 32 + 255) / 256, 256, 0, s->stream>>>(a);
+    launch_dep(s->stream, k_cells_open, (nc + 255) / 256, 256, 0, a);
+    launch_dep(s->stream, k_integrate32b, std::min(s->nchunk, s->sm_count * 8), 256, 0, a);
+    launch_dep(s->stream, k_cells_com, (nc * 32 + 255) / 256, 256, 0, a);
     launch_rebuild_chain(s);
     EamArgs e = eam_args(s);
     launch_density32(s, e);
     launch_force32(s, e);
-    k_ke32b<<<std::min(s->nchunk, s->sm_count * 8), 256, 0, s->stream>>>(a);
+    launch_dep(s->stream, k_ke32b, std::min(s->nchunk, s->sm_count * 8), 256, 0, a);
     e.thermo = a.thermo;
     e.nsteps = a.nsteps;
     e.nhc = a.nhc;
@@ -903,8 +921,8 @@ void nvt_begin(mappg_sys* s, double T, double dt, double kB, double t_relax, int
         MAPPG_CUDA(cudaStreamSynchronize(s->stream));
         sys_build(s);
         launch_force(s);
-        k_mvv_init_b<<<std::min(s->nchunk, s->sm_count * 8), 256, 0, s->stream>>>(a);
-        k_cells_begin<<<(s->ncell * 32 + 255) / 256, 256, 0, s->stream>>>(a);
+        launch_dep(s->stream, k_mvv_init_b, std::min(s->nchunk, s->sm_count * 8), 256, 0, a);
+        launch_dep(s->stream, k_cells_begin, (s->ncell * 32 + 255) / 256, 256, 0, a);
         MAPPG_CUDA(cudaGetLastError());
         auto capture = [&](long long k, cudaGraph_t* gr, cudaGraphExec_t* ex) {
             MAPPG_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
@@ -928,7 +946,7 @@ void nvt_begin(mappg_sys* s, double T, double dt, double kB, double t_relax, int
     if (eta)
         for (int k = 0; k < L; k++) eta_h[k] = eta[k];
     MAPPG_CUDA(cudaMemcpyAsync(s->sc->eta, eta_h, sizeof(double) * kMaxChain, cudaMemcpyHostToDevice, s->stream));
-    k_clear_drift<<<1, 1, 0, s->stream>>>(s->sc);
+    launch_dep(s->stream, k_clear_drift, 1, 1, 0, s->sc);
     // MDNVT::run builds the list at its start.  A list built for this box
     // whose atoms all stayed within half the skin of their positions at that
     // build still holds every pair within the cutoff, so the skin test
@@ -944,8 +962,8 @@ void nvt_begin(mappg_sys* s, double T, double dt, double kB, double t_relax, int
     // the list and the opening force do not read velocities: an upload of
     // them on the side stream (nvt_run_host) overlaps them and is joined here
     sys_join_side(s);
-    k_mvv_init<<<md_shape(s, true).grid, md_shape(s, true).block, 0, s->stream>>>(a);
-    k_run_begin<<<1, 1, 0, s->stream>>>(a);
+    launch_dep(s->stream, k_mvv_init, md_shape(s, true).grid, md_shape(s, true).block, 0, a);
+    launch_dep(s->stream, k_run_begin, 1, 1, 0, a);
     if (s->precision == MAPPG_MIXED) s->drift_rows = a.drift_rows = md_shape(s, true).grid;
     MAPPG_CUDA(cudaGetLastError());
     if (nsteps < kGraphMinSteps) return;  // nvt_steps launches the kernels itself
@@ -991,8 +1009,8 @@ void nvt_end(mappg_sys* s, double* eta, double* thermo) {
     sys_join_side(s);  // a side-stream read of the positions (nvt_run_xout) comes first
     int g = grid_for(s, 3LL * s->n, 256);
     if (s->ncell > 1) {
-        k_run_end32b<<<g, 256, 0, s->stream>>>(r->a);
-        k_cells_clear<<<(s->ncell + 255) / 256, 256, 0, s->stream>>>(r->a);
+        launch_dep(s->stream, k_run_end32b, g, 256, 0, r->a);
+        launch_dep(s->stream, k_cells_clear, (s->ncell + 255) / 256, 256, 0, r->a);
         MAPPG_CUDA(cudaGetLastError());
         DevScalars h;
         std::vector<CellMd> cm(s->ncell);
@@ -1011,10 +1029,10 @@ void nvt_end(mappg_sys* s, double* eta, double* thermo) {
         return;
     }
     if (s->precision == MAPPG_MIXED) {
-        k_run_end32<<<g, 256, 0, s->stream>>>(r->a);
-        k_clear_drift<<<1, 1, 0, s->stream>>>(s->sc);
+        launch_dep(s->stream, k_run_end32, g, 256, 0, r->a);
+        launch_dep(s->stream, k_clear_drift, 1, 1, 0, s->sc);
     } else {
-        k_run_end64<<<g, 256, 0, s->stream>>>(r->a);
+        launch_dep(s->stream, k_run_end64, g, 256, 0, r->a);
     }
     MAPPG_CUDA(cudaGetLastError());
     DevScalars h;

@@ -14,7 +14,8 @@
 // ~35 FP64 operations an entry instead of ~80, and ~1.2 KB written and ~3.5 KB
 // read per atom, which the memory has room for.  An other pair's record lies
 // with its owner; the builder's k_link64 finds the slot once per list.
-// Sums have a fixed order (own pairs, then others, lane-strided), no atomics.
+// Sums have a fixed order (lane-strided over one list, then the other), no
+// atomics.
 // Density + force at 4,000 atoms 71.5 -> 46.8 us, 256,000 2,610 -> 1,092
 // (k_pair64 727 of it at first, 87 % of the FP64 pipe: what bounds it).
 #include <math.h>
@@ -77,6 +78,7 @@ __device__ __forceinline__ double rsqrt_halley(double x) {
 // ENERGY: the densities and the pair energy only (line-search trials)
 template <int TPA, bool ENERGY>
 __global__ void __launch_bounds__(256) k_pair64(const __grid_constant__ EamArgs a) {
+    dep_wait();
     __shared__ Smem64 S;
     S.fill(a);
     const int lane = threadIdx.x % TPA;
@@ -138,6 +140,7 @@ __global__ void __launch_bounds__(256) k_pair64(const __grid_constant__ EamArgs 
 // ENERGY: the densities stay here, and the last block adds up the energy
 template <int TPA, bool ENERGY>
 __global__ void __launch_bounds__(256) k_rho64(const __grid_constant__ EamArgs a, int rows_pair) {
+    dep_wait();
     const int lane = threadIdx.x % TPA;
     const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / TPA;
     const int stride = (gridDim.x * blockDim.x) / TPA;
@@ -201,6 +204,7 @@ __global__ void __launch_bounds__(256) k_rho64(const __grid_constant__ EamArgs a
 
 template <int TPA>
 __global__ void __launch_bounds__(256) k_gather64(const __grid_constant__ EamArgs a, int rows_pair, int rows_rho) {
+    dep_wait();
     const int lane = threadIdx.x % TPA;
     const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / TPA;
     const int stride = (gridDim.x * blockDim.x) / TPA;
@@ -240,11 +244,6 @@ __global__ void __launch_bounds__(256) k_gather64(const __grid_constant__ EamArg
                 fy = fma(f, r2.x, fy);
                 fz = fma(f, r2.y, fz);
             };
-            if (no <= 32 * TPA)
-                for (unsigned b = mask.x; b; b &= b - 1u) own(lane + (__ffs(b) - 1) * TPA);
-            else
-                for (int q = lane; q < no; q += TPA)
-                    if (!is_outside(a.pair_rho[row + q].x)) own(q);
             if (nr <= 32 * TPA) {
                 for (unsigned b = mask.y; b; b &= b - 1u) other(lane + (__ffs(b) - 1) * TPA);
             } else {
@@ -253,6 +252,11 @@ __global__ void __launch_bounds__(256) k_gather64(const __grid_constant__ EamArg
                     if (slot != kNoSlot && !is_outside(a.pair_rho[slot].x)) other(q);
                 }
             }
+            if (no <= 32 * TPA)
+                for (unsigned b = mask.x; b; b &= b - 1u) own(lane + (__ffs(b) - 1) * TPA);
+            else
+                for (int q = lane; q < no; q += TPA)
+                    if (!is_outside(a.pair_rho[row + q].x)) own(q);
         }
 #pragma unroll
         for (int o = TPA / 2; o > 0; o >>= 1) {
@@ -293,6 +297,7 @@ __global__ void __launch_bounds__(256) k_link64(int n, int cap, int parts, const
                                                 const int* __restrict__ nown, const int* __restrict__ other_ent,
                                                 const int* __restrict__ nother, const uint8_t* __restrict__ elem,
                                                 unsigned* __restrict__ other_slot, const DevScalars* sc) {
+    dep_wait();
     if (!sc->rebuild) return;
     const int lane = threadIdx.x & 31, g = lane >> 3, l = lane & 7;
     const int nw = (gridDim.x * blockDim.x) >> 5;
@@ -335,26 +340,26 @@ __global__ void __launch_bounds__(256) k_link64(int n, int cap, int parts, const
 
 void launch_link64(mappg_sys* s) {
     const int parts = s->n < 64 * s->sm_count ? 4 : 1;  // fill the warps that the SMs hold
-    k_link64<<<grid_for(s, 32LL * s->n * parts, 256), 256, 0, s->stream>>>(
-        s->n, s->maxnbr, parts, s->own_ent, s->nown, s->other_ent, s->nother, s->elem, s->other_slot, s->sc);
+    launch_dep(s->stream, k_link64, grid_for(s, 32LL * s->n * parts, 256), 256, 0, s->n, s->maxnbr, parts, s->own_ent,
+               s->nown, s->other_ent, s->nother, s->elem, s->other_slot, s->sc);
     MAPPG_CUDA(cudaGetLastError());
 }
 
 template <int TPA>
 static void pair_density(mappg_sys* s, const EamArgs& a, int grid) {
-    k_pair64<TPA, false><<<grid, 256, 0, s->stream>>>(a);
-    k_rho64<TPA, false><<<grid, 256, 0, s->stream>>>(a, grid);
+    launch_dep(s->stream, k_pair64<TPA, false>, grid, 256, 0, a);
+    launch_dep(s->stream, k_rho64<TPA, false>, grid, 256, 0, a, grid);
 }
 
 template <int TPA>
 static void pair_energy(mappg_sys* s, const EamArgs& a, int grid) {
-    k_pair64<TPA, true><<<grid, 256, 0, s->stream>>>(a);
-    k_rho64<TPA, true><<<grid, 256, 0, s->stream>>>(a, grid);
+    launch_dep(s->stream, k_pair64<TPA, true>, grid, 256, 0, a);
+    launch_dep(s->stream, k_rho64<TPA, true>, grid, 256, 0, a, grid);
 }
 
 template <int TPA>
 static void pair_force(mappg_sys* s, const EamArgs& a, int grid) {
-    k_gather64<TPA><<<grid, 256, 0, s->stream>>>(a, grid, grid);
+    launch_dep(s->stream, k_gather64<TPA>, grid, 256, 0, a, grid, grid);
 }
 
 #define MAPPG_PAIR64(FN)                                                  \

@@ -268,6 +268,7 @@ __global__ void k_wrap_bin(int n, double* __restrict__ x, double* __restrict__ s
                            int* __restrict__ binc, int* __restrict__ binid, int* __restrict__ bin_count,
                            float4* __restrict__ p32, float4* __restrict__ p0, const double* __restrict__ partials,
                            int drift_rows, DevScalars* sc) {
+    dep_wait();
     if (!sc->rebuild) return;
     int bad = 0;
     double drift[3];
@@ -309,6 +310,7 @@ __global__ void k_wrap_bin_b(int n, double* __restrict__ x, double* __restrict__
                              const CellMd* __restrict__ cmd, int* __restrict__ binc, int* __restrict__ binid,
                              int* __restrict__ bin_count, const uint8_t* __restrict__ cell_reb,
                              float4* __restrict__ p32, float4* __restrict__ p0, DevScalars* sc) {
+    dep_wait();
     if (!sc->rebuild) return;
     int bad = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -354,6 +356,7 @@ __device__ __forceinline__ void rebuild_reset(DevScalars* sc) {
 // rebuild step 2: exclusive scan of bin counts (one block), counts zeroed
 __global__ void k_scan_bins(int nbins, int* __restrict__ bin_count, int* __restrict__ bin_start,
                             double* __restrict__ partials, int drift_rows, DevScalars* sc) {
+    dep_wait();
     if (!sc->rebuild) return;
     // the running step's displacement sums went into x with the drift
     for (int q = threadIdx.x; q < 3 * drift_rows; q += blockDim.x) partials[(q / 3) * kRedSlots + 8 + q % 3] = 0.0;
@@ -388,6 +391,7 @@ __global__ void k_scan_bins(int nbins, int* __restrict__ bin_count, int* __restr
 __global__ void k_scan_bins_b(int ncell, int n, int nbins, const CellGeo* __restrict__ cells,
                               const uint8_t* __restrict__ cell_reb, int* __restrict__ bin_count,
                               int* __restrict__ bin_start, CellMd* __restrict__ cmd, DevScalars* sc) {
+    dep_wait();
     if (!sc->rebuild) return;
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
@@ -424,6 +428,7 @@ __global__ void k_scan_bins_b(int ncell, int n, int nbins, const CellGeo* __rest
 __global__ void k_scatter_bins(int n, const int* __restrict__ binid, const int* __restrict__ bin_start,
                                int* __restrict__ bin_count, int* __restrict__ bin_tmp, const int* __restrict__ cell_of,
                                const uint8_t* __restrict__ cell_reb, DevScalars* sc) {
+    dep_wait();
     if (!sc->rebuild) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         if (cell_reb && !cell_reb[cell_of[i]]) continue;
@@ -441,6 +446,7 @@ __global__ void k_sort_bins(int nbins, const int* __restrict__ bin_start, const 
                             const float4* __restrict__ p32, const uint8_t* __restrict__ elem,
                             float4* __restrict__ bin_pos, int* __restrict__ bin_count, const int* __restrict__ cell_of,
                             const uint8_t* __restrict__ cell_reb, DevScalars* sc) {
+    dep_wait();
     if (!sc->rebuild) return;
     int lane = threadIdx.x & 31;
     int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -465,6 +471,7 @@ __global__ void k_sort_bins(int nbins, const int* __restrict__ bin_start, const 
 // frame positions of atoms that moved without a rebuild
 __global__ void k_shadow(int n, const double* __restrict__ x, const int* __restrict__ binc, float4* __restrict__ p32,
                          Geo g) {
+    dep_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         p32[i] = frame_pos(g.bs, x[i], x[n + i], x[2 * n + i], binc[i]);
 }
@@ -472,6 +479,7 @@ __global__ void k_shadow(int n, const double* __restrict__ x, const int* __restr
 __global__ void k_shadow_b(int n, const double* __restrict__ x, const int* __restrict__ binc,
                            const CellGeo* __restrict__ cells, const int* __restrict__ cell_of,
                            float4* __restrict__ p32) {
+    dep_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         p32[i] = frame_pos(cells[cell_of[i]].bs, x[i], x[n + i], x[2 * n + i], binc[i]);
 }
@@ -481,12 +489,13 @@ struct BuildArgs {
     const double* x;
     const double* s;
     const float4* bin_pos;
+    const float4* p32;
     const int* bin_start;
     int* nbr;
     int* nnbr;
     int *own_ent, *other_ent, *nown, *nother;  // FP64: the row's entries by owner (null: not kept)
     Geo g;
-    float G[3][3];  // frame to Cartesian
+    Frame fr;       // frame to Cartesian
     float lo2[kMaxElem * kMaxElem], hi2[kMaxElem * kMaxElem];
     float in2[kMaxElem * kMaxElem];  // pair cutoff squared: entries below it lead their row
     double cut_sk_sq[kMaxElem * kMaxElem];
@@ -516,6 +525,35 @@ __device__ __noinline__ bool exact_keep(const BuildArgs& a, const double* h6, co
     return rsq < a.cut_sk_sq[pe];
 }
 
+// the distance of an entry as the frame positions give it, in the operations
+// that say which entries lead a row: the staged Cartesian positions differ
+// from it by rounding, and a pair on the other side of the cutoff would
+// change the order of the row's sums
+template <bool ORTHO>
+__device__ __noinline__ float frame_r2(const BuildArgs& a, const CellGeo* cg, int i, int ent) {
+    const float4 pi = a.p32[i], pj = a.p32[entry_j(ent)];
+    const float u = pi.x - (pj.x + kBinW * (float)entry_step(ent, 0));
+    const float v = pi.y - (pj.y + kBinW * (float)entry_step(ent, 1));
+    const float w = pi.z - (pj.z + kBinW * (float)entry_step(ent, 2));
+    const float(*G)[3] = cg ? cg->G : a.fr.G;
+    const float(*L)[3] = cg ? cg->Glo : a.fr.Glo;
+    float x, y, z;
+    if (ORTHO) {
+        x = u * G[0][0];
+        y = v * G[1][1];
+        z = w * G[2][2];
+    } else if (cg ? cg->ortho : a.fr.ortho) {
+        x = fmaf(u, G[0][0], u * L[0][0]);
+        y = fmaf(v, G[1][1], v * L[1][1]);
+        z = fmaf(w, G[2][2], w * L[2][2]);
+    } else {
+        x = fmaf(u, G[0][0], fmaf(v, G[1][0], fmaf(w, G[2][0], u * L[0][0] + v * L[1][0] + w * L[2][0])));
+        y = fmaf(v, G[1][1], fmaf(w, G[2][1], v * L[1][1] + w * L[2][1]));
+        z = fmaf(w, G[2][2], w * L[2][2]);
+    }
+    return fmaf(x, x, fmaf(y, y, z * z));
+}
+
 constexpr int kBuildWarps = 4;    // warps of a builder block
 constexpr int kBuildTile = 768;   // candidates staged at a time (12 KB)
 constexpr int kBuildHome = 32;    // atoms of the bin worked on at a time
@@ -535,10 +573,10 @@ struct BuildCut {
 // against atom h: its inner entries go to dst[0], dst[1], ..., its shell
 // entries to dst[cap - 1], dst[cap - 2], ...; entries that would leave the
 // row or meet are dropped (the caller sees it from the counts)
-template <bool UNI>
+template <bool ORTHO, bool UNI>
 __device__ __forceinline__ void build_scan(const BuildArgs& a, const BuildCut<UNI>& cut, const float4* cand, int nt,
-                                           const float4& h, int self, const int* geo, const double* h6, int* dst,
-                                           int cap, int& cin, int& cout) {
+                                           const float4& h, int self, const int* geo, const double* h6,
+                                           const CellGeo* cg, int* dst, int cap, int& cin, int& cout) {
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     const int pe0 = entry_elem(self) * a.ne;
@@ -560,8 +598,18 @@ __device__ __forceinline__ void build_scan(const BuildArgs& a, const BuildCut<UN
                 keep = exact_keep(a, h6, geo, entry_j(self), ent, pe0 + entry_elem(ent));
             m = __ballot_sync(0xffffffffu, keep);
         }
-        const bool inner = r2 < cut.in(pe);
-        const unsigned mi = __ballot_sync(0xffffffffu, inner) & m, mo = m & ~mi;
+        const float in2 = cut.in(pe);
+        unsigned mi = __ballot_sync(0xffffffffu, r2 < in2 * 0.99999f);
+        const unsigned mn = __ballot_sync(0xffffffffu, r2 < in2 * 1.00001f);
+        if ((mn ^ mi) & m) {
+            // pairs within the rounding of the pair cutoff
+            bool lead = (mi >> lane) & 1u;
+            if (((mn ^ mi) & m) >> lane & 1u) lead = frame_r2<ORTHO>(a, cg, entry_j(self), ent) < in2;
+            mi = __ballot_sync(0xffffffffu, lead);
+        }
+        mi &= m;
+        const unsigned mo = m & ~mi;
+        const bool inner = (mi >> lane) & 1u;
         const int at = __popc((inner ? mi : mo) & below);
         const int pos = inner ? cin + at : cap - 1 - cout - at;
         if (((m >> lane) & 1u) && (unsigned)pos < (unsigned)cap) dst[pos] = ent;
@@ -600,6 +648,7 @@ __device__ __forceinline__ void build_scan(const BuildArgs& a, const BuildCut<UN
 template <bool BATCH, bool ORTHO, bool UNI>
 __global__ void __launch_bounds__(32 * kBuildWarps) k_build_bins(const __grid_constant__ BuildArgs a, int nbins,
                                                                  DevScalars* sc) {
+    dep_wait();
     if (!sc->rebuild) return;
     __shared__ float4 cand[kBuildTile], home[kBuildHome];
     __shared__ int s_pre[33], s_lo[32], s_cin[kBuildHome], s_cout[kBuildHome], s_geo[6];
@@ -624,7 +673,7 @@ __global__ void __launch_bounds__(32 * kBuildWarps) k_build_bins(const __grid_co
         const CellGeo* cg = BATCH ? a.cells + cell : nullptr;
         const int* nb = BATCH ? cg->nb : a.g.nb;
         const double* h6 = BATCH ? cg->h6 : a.g.h6;
-        const float(*G)[3] = BATCH ? cg->G : a.G;
+        const float(*G)[3] = BATCH ? cg->G : a.fr.G;
         const int bin_base = BATCH ? cg->bin_base : 0;
         const int bl = b - bin_base;
         const int b0 = bl % nb[0], b1 = (bl / nb[0]) % nb[1], b2 = bl / (nb[0] * nb[1]);
@@ -711,7 +760,7 @@ __global__ void __launch_bounds__(32 * kBuildWarps) k_build_bins(const __grid_co
                     int* row = a.nbr + (size_t)i * a.maxnbr;
                     int cin = 0, cout = 0, tot = kBuildRow + 1;
                     if (one_tile) {
-                        build_scan<UNI>(a, cut, cand, nt, h, self, s_geo, h6, s_row[w], kBuildRow, cin, cout);
+                        build_scan<ORTHO, UNI>(a, cut, cand, nt, h, self, s_geo, h6, cg, s_row[w], kBuildRow, cin, cout);
                         tot = cin + cout;
                         __syncwarp();
                         // (of a row that does not fit only the inner entries)
@@ -724,7 +773,7 @@ __global__ void __launch_bounds__(32 * kBuildWarps) k_build_bins(const __grid_co
                             cin = cout = 0;
                         else
                             cin = s_cin[q], cout = s_cout[q];
-                        build_scan<UNI>(a, cut, cand, nt, h, self, s_geo, h6, row, a.maxnbr, cin, cout);
+                        build_scan<ORTHO, UNI>(a, cut, cand, nt, h, self, s_geo, h6, cg, row, a.maxnbr, cin, cout);
                         tot = cin + cout;
                         if (!last) {
                             if (lane == 0) {
@@ -791,6 +840,7 @@ __global__ void __launch_bounds__(32 * kBuildWarps) k_build_bins(const __grid_co
 
 // batch: the rebuilt cells' flags
 __global__ void k_rebuild_done_b(DevScalars* sc, uint8_t* cell_reb, int ncell) {
+    dep_wait();
     if (!sc->rebuild) return;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell; c += gridDim.x * blockDim.x) cell_reb[c] = 0;
 }
@@ -799,6 +849,7 @@ __global__ void k_rebuild_done_b(DevScalars* sc, uint8_t* cell_reb, int ncell) {
 // |x - x0|^2 > skin^2/4, RSQ order, FP64
 __global__ void k_skin(int n, const double* __restrict__ x, const double* __restrict__ x0, double skin_sq,
                        DevScalars* sc) {
+    dep_wait();
     int moved = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double d0 = dsub(x0[i], x[i]), d1 = dsub(x0[n + i], x[n + i]), d2 = dsub(x0[2 * n + i], x[2 * n + i]);
@@ -811,6 +862,7 @@ __global__ void k_skin(int n, const double* __restrict__ x, const double* __rest
 // batch: the same test, flagging the cells whose atoms moved
 __global__ void k_skin_b(int n, const double* __restrict__ x, const double* __restrict__ x0, double skin_sq,
                          const int* __restrict__ cell_of, uint8_t* __restrict__ cell_reb, DevScalars* sc) {
+    dep_wait();
     int moved = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double d0 = dsub(x0[i], x[i]), d1 = dsub(x0[n + i], x[n + i]), d2 = dsub(x0[2 * n + i], x[2 * n + i]);
@@ -824,12 +876,14 @@ __global__ void k_skin_b(int n, const double* __restrict__ x, const double* __re
 }
 
 __global__ void k_set_rebuild(DevScalars* sc, int v) {
+    dep_wait();
     sc->rebuild = v;
 }
 
 // caller order (AoS) <-> bin-sorted order (SoA)
 __global__ void k_gather_aos(int n, const int* __restrict__ id, const double* __restrict__ src,
                              double* __restrict__ dst) {
+    dep_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         int u = id[i];
         dst[i] = src[3 * (size_t)u];
@@ -840,6 +894,7 @@ __global__ void k_gather_aos(int n, const int* __restrict__ id, const double* __
 
 __global__ void k_scatter_aos(int n, const int* __restrict__ id, const double* __restrict__ src,
                               double* __restrict__ dst) {
+    dep_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         int u = id[i];
         dst[3 * (size_t)u] = src[i];
@@ -849,19 +904,20 @@ __global__ void k_scatter_aos(int n, const int* __restrict__ id, const double* _
 }
 
 __global__ void k_f32_to_f64(int n3, const float* __restrict__ a, double* __restrict__ b) {
+    dep_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += gridDim.x * blockDim.x) b[i] = (double)a[i];
 }
 
 // ------------------------------------------------------------------ launchers
 void sync_forces64(mappg_sys* s) {
     if (!s->f_is_f32) return;
-    k_f32_to_f64<<<grid_for(s, 3LL * s->n, 256), 256, 0, s->stream>>>(3 * s->n, s->f32, s->f);
+    launch_dep(s->stream, k_f32_to_f64, grid_for(s, 3LL * s->n, 256), 256, 0, 3 * s->n, s->f32, s->f);
     MAPPG_CUDA(cudaGetLastError());
     s->f_is_f32 = false;
 }
 
 void request_rebuild(mappg_sys* s) {
-    k_set_rebuild<<<1, 1, 0, s->stream>>>(s->sc, 1);
+    launch_dep(s->stream, k_set_rebuild, 1, 1, 0, s->sc, 1);
     MAPPG_CUDA(cudaGetLastError());
     if (s->cell_reb) MAPPG_CUDA(cudaMemsetAsync(s->cell_reb, 1, s->ncell, s->stream));
 }
@@ -869,9 +925,9 @@ void request_rebuild(mappg_sys* s) {
 void launch_shadow(mappg_sys* s) {
     const int gb = grid_for(s, s->n, 256);
     if (s->ncell > 1)
-        k_shadow_b<<<gb, 256, 0, s->stream>>>(s->n, s->x, s->binc, s->cells_dev, s->cell_of, s->p32);
+        launch_dep(s->stream, k_shadow_b, gb, 256, 0, s->n, s->x, s->binc, s->cells_dev, s->cell_of, s->p32);
     else
-        k_shadow<<<gb, 256, 0, s->stream>>>(s->n, s->x, s->binc, s->p32, make_geo(s));
+        launch_dep(s->stream, k_shadow, gb, 256, 0, s->n, s->x, s->binc, s->p32, make_geo(s));
     MAPPG_CUDA(cudaGetLastError());
 }
 
@@ -884,21 +940,20 @@ void launch_rebuild_chain(mappg_sys* s) {
     // all of its atoms
     const uint8_t* reb = batch ? s->cell_reb : nullptr;
     if (batch) {
-        k_wrap_bin_b<<<gb, B, 0, s->stream>>>(s->n, s->x, s->s, s->x0, s->cells_dev, s->cell_of, s->cmd, s->binc,
-                                              s->binid, s->bin_count, s->cell_reb, s->p32, s->p0, s->sc);
-        k_scan_bins_b<<<(s->ncell * 32 + B - 1) / B, B, 0, s->stream>>>(s->ncell, s->n, s->nbins, s->cells_dev,
-                                                                         s->cell_reb, s->bin_count, s->bin_start,
-                                                                         s->cmd, s->sc);
+        launch_dep(s->stream, k_wrap_bin_b, gb, B, 0, s->n, s->x, s->s, s->x0, s->cells_dev, s->cell_of, s->cmd,
+                   s->binc, s->binid, s->bin_count, s->cell_reb, s->p32, s->p0, s->sc);
+        launch_dep(s->stream, k_scan_bins_b, (s->ncell * 32 + B - 1) / B, B, 0, s->ncell, s->n, s->nbins,
+                   s->cells_dev, s->cell_reb, s->bin_count, s->bin_start, s->cmd, s->sc);
     } else {
-        k_wrap_bin<<<gb, B, 0, s->stream>>>(s->n, s->x, s->s, s->x0, g, s->binc, s->binid, s->bin_count, s->p32, s->p0,
-                                            s->partials, s->drift_rows, s->sc);
-        k_scan_bins<<<1, 1024, 0, s->stream>>>(s->nbins, s->bin_count, s->bin_start, s->partials, s->drift_rows,
-                                               s->sc);
+        launch_dep(s->stream, k_wrap_bin, gb, B, 0, s->n, s->x, s->s, s->x0, g, s->binc, s->binid, s->bin_count,
+                   s->p32, s->p0, s->partials, s->drift_rows, s->sc);
+        launch_dep(s->stream, k_scan_bins, 1, 1024, 0, s->nbins, s->bin_count, s->bin_start, s->partials,
+                   s->drift_rows, s->sc);
     }
-    k_scatter_bins<<<gb, B, 0, s->stream>>>(s->n, s->binid, s->bin_start, s->bin_count, s->bin_tmp, s->cell_of, reb,
-                                            s->sc);
-    k_sort_bins<<<grid_for(s, (long long)s->nbins * 32, B), B, 0, s->stream>>>(
-        s->nbins, s->bin_start, s->bin_tmp, s->p32, s->elem, s->bin_pos, s->bin_count, s->cell_of, reb, s->sc);
+    launch_dep(s->stream, k_scatter_bins, gb, B, 0, s->n, s->binid, s->bin_start, s->bin_count, s->bin_tmp,
+               s->cell_of, reb, s->sc);
+    launch_dep(s->stream, k_sort_bins, grid_for(s, (long long)s->nbins * 32, B), B, 0, s->nbins, s->bin_start,
+               s->bin_tmp, s->p32, s->elem, s->bin_pos, s->bin_count, s->cell_of, reb, s->sc);
     BuildArgs a;
     a.n = s->n;
     a.maxnbr = s->maxnbr;
@@ -906,6 +961,7 @@ void launch_rebuild_chain(mappg_sys* s) {
     a.x = s->x;
     a.s = s->s;
     a.bin_pos = s->bin_pos;
+    a.p32 = s->p32;
     a.bin_start = s->bin_start;
     a.nbr = s->nbr;
     a.nnbr = s->nnbr;
@@ -920,7 +976,7 @@ void launch_rebuild_chain(mappg_sys* s) {
         a.hi2[p] = (float)(s->cut_sk_sq[p] + s->band);
         a.in2[p] = (float)s->cut_sq[p];
     }
-    memcpy(a.G, s->frame.G, sizeof(a.G));
+    a.fr = s->frame;
     a.cells = s->cells_dev;
     a.cell_of = s->cell_of;
     a.cell_reb = reb;
@@ -933,7 +989,7 @@ void launch_rebuild_chain(mappg_sys* s) {
             MAPPG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kBuildWarps, 0));
             per_sm = std::max(per_sm, 1);
         }
-        kern<<<std::min(s->nbins, per_sm * s->sm_count), 32 * kBuildWarps, 0, s->stream>>>(a, s->nbins, s->sc);
+        launch_dep(s->stream, kern, std::min(s->nbins, per_sm * s->sm_count), 32 * kBuildWarps, 0, a, s->nbins, s->sc);
     };
     auto by_uni = [&](auto BT, auto OT) {
         if (uni)
@@ -946,7 +1002,7 @@ void launch_rebuild_chain(mappg_sys* s) {
             by_uni(std::true_type(), std::true_type());
         else
             by_uni(std::true_type(), std::false_type());
-        k_rebuild_done_b<<<(s->ncell + 255) / 256, 256, 0, s->stream>>>(s->sc, s->cell_reb, s->ncell);
+        launch_dep(s->stream, k_rebuild_done_b, (s->ncell + 255) / 256, 256, 0, s->sc, s->cell_reb, s->ncell);
     } else {
         if (s->frame.ortho)
             by_uni(std::false_type(), std::true_type());
@@ -960,10 +1016,10 @@ void launch_rebuild_chain(mappg_sys* s) {
 void launch_skin_test(mappg_sys* s) {
     double skin_sq = 0.25 * s->skin * s->skin;
     if (s->cell_reb)
-        k_skin_b<<<grid_for(s, s->n, 256), 256, 0, s->stream>>>(s->n, s->x, s->x0, skin_sq, s->cell_of, s->cell_reb,
-                                                                s->sc);
+        launch_dep(s->stream, k_skin_b, grid_for(s, s->n, 256), 256, 0, s->n, s->x, s->x0, skin_sq, s->cell_of,
+                   s->cell_reb, s->sc);
     else
-        k_skin<<<grid_for(s, s->n, 256), 256, 0, s->stream>>>(s->n, s->x, s->x0, skin_sq, s->sc);
+        launch_dep(s->stream, k_skin, grid_for(s, s->n, 256), 256, 0, s->n, s->x, s->x0, skin_sq, s->sc);
     MAPPG_CUDA(cudaGetLastError());
 }
 
@@ -1230,7 +1286,7 @@ void sys_alloc_nbr(mappg_sys* s, int maxnbr) {
 // upload caller-order AoS doubles into a SoA device array
 void sys_upload(mappg_sys* s, const double* host, double* dev) {
     MAPPG_CUDA(cudaMemcpyAsync(s->stage, host, sizeof(double) * 3 * (size_t)s->n, cudaMemcpyHostToDevice, s->stream));
-    k_gather_aos<<<grid_for(s, s->n, 256), 256, 0, s->stream>>>(s->n, s->id, s->stage, dev);
+    launch_dep(s->stream, k_gather_aos, grid_for(s, s->n, 256), 256, 0, s->n, s->id, s->stage, dev);
     MAPPG_CUDA(cudaGetLastError());
 }
 
@@ -1246,7 +1302,7 @@ void sys_upload_side(mappg_sys* s, const double* host, double* dev) {
     MAPPG_CUDA(cudaEventRecord(s->ev_main, s->stream));
     MAPPG_CUDA(cudaStreamWaitEvent(s->side, s->ev_main, 0));
     MAPPG_CUDA(cudaMemcpyAsync(s->stage2, host, sizeof(double) * 3 * (size_t)s->n, cudaMemcpyHostToDevice, s->side));
-    k_gather_aos<<<grid_for(s, s->n, 256), 256, 0, s->side>>>(s->n, s->id, s->stage2, dev);
+    launch_dep(s->side, k_gather_aos, grid_for(s, s->n, 256), 256, 0, s->n, s->id, s->stage2, dev);
     MAPPG_CUDA(cudaGetLastError());
     MAPPG_CUDA(cudaEventRecord(s->ev_side, s->side));
     s->v_pending = true;
@@ -1262,13 +1318,13 @@ void sys_join_side(mappg_sys* s) {
 // queue a caller-order download without waiting for it (the stage array is
 // reused in stream order by the next one)
 void sys_download_async(mappg_sys* s, const double* dev, double* host) {
-    k_scatter_aos<<<grid_for(s, s->n, 256), 256, 0, s->stream>>>(s->n, s->id, dev, s->stage);
+    launch_dep(s->stream, k_scatter_aos, grid_for(s, s->n, 256), 256, 0, s->n, s->id, dev, s->stage);
     MAPPG_CUDA(cudaGetLastError());
     MAPPG_CUDA(cudaMemcpyAsync(host, s->stage, sizeof(double) * 3 * (size_t)s->n, cudaMemcpyDeviceToHost, s->stream));
 }
 
 void sys_download(mappg_sys* s, const double* dev, double* host) {
-    k_scatter_aos<<<grid_for(s, s->n, 256), 256, 0, s->stream>>>(s->n, s->id, dev, s->stage);
+    launch_dep(s->stream, k_scatter_aos, grid_for(s, s->n, 256), 256, 0, s->n, s->id, dev, s->stage);
     MAPPG_CUDA(cudaGetLastError());
     MAPPG_CUDA(cudaMemcpyAsync(host, s->stage, sizeof(double) * 3 * (size_t)s->n, cudaMemcpyDeviceToHost, s->stream));
     MAPPG_CUDA(cudaStreamSynchronize(s->stream));
@@ -1285,7 +1341,7 @@ void sys_build(mappg_sys* s) {
         MAPPG_CUDA(cudaStreamSynchronize(s->stream));
         if (h.bad) throw Error{MAPPG_ERR_NAN, "non-finite or far out-of-cell position"};
         if (!h.overflow) {
-            k_set_rebuild<<<1, 1, 0, s->stream>>>(s->sc, 0);
+            launch_dep(s->stream, k_set_rebuild, 1, 1, 0, s->sc, 0);
             s->built = true;
             s->list_box = true;
             return;
