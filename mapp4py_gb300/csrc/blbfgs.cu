@@ -595,19 +595,6 @@ void batch_lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_
     if (nsteps < 0) throw Error{MAPPG_ERR_ARG, "nsteps must be >= 0"};
     const int n = s->n, nc = s->ncell;
     const size_t N3 = 3 * (size_t)n;
-    std::vector<void*> owned;
-    auto dalloc = [&](size_t bytes) {
-        void* p = nullptr;
-        MAPPG_CUDA(cudaMalloc(&p, bytes > 0 ? bytes : 16));
-        owned.push_back(p);
-        return p;
-    };
-    struct Guard {
-        std::vector<void*>& o;
-        ~Guard() {
-            for (void* p : o) cudaFree(p);
-        }
-    } guard{owned};
     BlArgs a;
     memset(&a, 0, sizeof(a));
     a.n = n;
@@ -626,26 +613,33 @@ void batch_lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_
     }
     a.nchunk = (int)cb.size();
     cb.push_back(n);
+    const bool mixed = s->precision == MAPPG_MIXED;
+    const size_t hist = N3 * std::max(m, 1);
+    Work work(s);
+    work.reserve(Work::room<int>(cb.size()) + Work::room<int>(cc.size()) + Work::room<int>(ccell.size()) +
+                 Work::room<BlCell>(nc) + 3 * Work::room<double>(N3) + 2 * Work::room<double>(hist) +
+                 Work::room<double>(4 * (size_t)a.nchunk) + Work::room<int>(1) + Work::room<uint8_t>(nc) +
+                 Work::room<double>(nc) + (mixed ? Work::room<float4>(n) : 0));
     auto upload = [&](const std::vector<int>& v) {
-        int* p = (int*)dalloc(sizeof(int) * v.size());
-        MAPPG_CUDA(cudaMemcpy(p, v.data(), sizeof(int) * v.size(), cudaMemcpyHostToDevice));
+        int* p = work.take<int>(v.size());
+        MAPPG_CUDA(cudaMemcpyAsync(p, v.data(), sizeof(int) * v.size(), cudaMemcpyHostToDevice, s->stream));
         return p;
     };
     a.chunk_begin = upload(cb);
     a.chunk_cell = upload(cc);
     a.cell_chunk = upload(ccell);
     a.cell_of = s->cell_of;
-    a.cs = (BlCell*)dalloc(sizeof(BlCell) * nc);
+    a.cs = work.take<BlCell>(nc);
     a.cmd = s->cmd;
     a.x = s->x;
     a.f = s->f;
-    a.x0 = (double*)dalloc(sizeof(double) * N3);
-    a.f0 = (double*)dalloc(sizeof(double) * N3);
-    a.h = (double*)dalloc(sizeof(double) * N3);
-    a.S = (double*)dalloc(sizeof(double) * N3 * std::max(m, 1));
-    a.Y = (double*)dalloc(sizeof(double) * N3 * std::max(m, 1));
-    a.part = (double*)dalloc(sizeof(double) * 4 * a.nchunk);
-    a.count = (int*)dalloc(sizeof(int));
+    a.x0 = work.take<double>(N3);
+    a.f0 = work.take<double>(N3);
+    a.h = work.take<double>(N3);
+    a.S = work.take<double>(hist);
+    a.Y = work.take<double>(hist);
+    a.part = work.take<double>(4 * (size_t)a.nchunk);
+    a.count = work.take<int>(1);
     a.P = P;
     a.c_ls = c_ls;
     a.rho_ls = rho_ls;
@@ -656,12 +650,11 @@ void batch_lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_
     a.nsteps = nsteps;
     a.xb = s->x0;
     a.skin_half = 0.5 * s->skin;
-    a.active = (uint8_t*)dalloc(nc);
-    a.alpha_cell = (double*)dalloc(sizeof(double) * nc);
+    a.active = work.take<uint8_t>(nc);
+    a.alpha_cell = work.take<double>(nc);
     a.cell_reb = s->cell_reb;
     a.sc = s->sc;
-    const bool mixed = s->precision == MAPPG_MIXED;
-    float4* h32 = mixed ? (float4*)dalloc(sizeof(float4) * (size_t)n) : nullptr;
+    float4* h32 = mixed ? work.take<float4>(n) : nullptr;
     // the masks and the kept density belong to this run only
     struct Masks {
         mappg_sys* s;

@@ -241,56 +241,83 @@ __global__ void k_lb_shift_rho(LbScal* L, int m) {
     for (int i = m - 1; i > 0; i--) L->rho[i] = L->rho[i - 1];
 }
 
-struct LbState {
-    mappg_sys* s;
-    int N, grid;
-    double *f0, *h, *xs;  // xs: the minimizer's x0
-    std::vector<double*> sv, yv;
-    LbScal* L;
-    unsigned* counter;
-};
+// x0 = x, f0 = f, h = f: the start of an iteration
+__global__ void k_lb_start(int N, const double* __restrict__ x, const double* __restrict__ f, double* __restrict__ xs,
+                           double* __restrict__ f0, double* __restrict__ h) {
+    dep_wait();
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < N; q += gridDim.x * blockDim.x) {
+        const double fq = f[q];
+        xs[q] = x[q];
+        f0[q] = fq;
+        if (h) h[q] = fq;
+    }
+}
 
 void launch_energy64(mappg_sys* s);  // eam.cu
 void launch_de32(mappg_sys* s, double alpha);  // eam32.cu
 
-static double lb_energy(mappg_sys* s) {
-    // skin test and (gated) rebuild, then the energy kernel; mixed systems
-    // compare FP64 line-search energies, so FP32 rounding of the pair terms
-    // does not decide the Armijo test near convergence
-    lb_update(s);
-    if (s->precision == MAPPG_MIXED)
-        launch_energy64(s);
-    else
-        launch_energy(s);
-    double e;
-    MAPPG_CUDA(cudaMemcpyAsync(&e, &s->sc->energy, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
+// what the host reads of a pass: the device scalars with the capacity flag
+// of the list check before it, and the vector kernels' results
+struct LbRead {
+    DevScalars sc;
+    double prep[6];  // f.h, h.h, max|h|, max|f|, tau, max|x - x_build|
+};
+static_assert(sizeof(LbRead) <= 4096, "the landing place holds 4 KB");
+
+static LbRead* lb_read(mappg_sys* s, const LbScal* L) {
+    LbRead* r = (LbRead*)sys_landing(s);
+    MAPPG_CUDA(cudaMemcpyAsync(&r->sc, s->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, s->stream));
+    if (L) MAPPG_CUDA(cudaMemcpyAsync(r->prep, &L->fh, sizeof(r->prep), cudaMemcpyDeviceToHost, s->stream));
     MAPPG_CUDA(cudaStreamSynchronize(s->stream));
-    return e;
+    return r;
 }
 
 __global__ void k_clear_rebuild(DevScalars* sc) {
-    dep_wait(); sc->rebuild = 0; }
+    dep_wait();
+    sc->rebuild = 0;
+}
 
-void lb_update(mappg_sys* s) {
+// skin test and (gated) rebuild; the caller reads sc->overflow with what it
+// runs next: a relaxation can crowd atoms beyond the rows' capacity, and a
+// rebuild that ran out of room is redone with wider rows (sys_build)
+static void lb_update_launch(mappg_sys* s) {
     launch_dep(s->stream, k_clear_rebuild, 1, 1, 0, s->sc);
     launch_skin_test(s);
     launch_rebuild_chain(s);
     // positions moved without a rebuild: refresh the mixed kernels' frame
     if (s->precision == MAPPG_MIXED) launch_shadow(s);
     MAPPG_CUDA(cudaGetLastError());
-    // a relaxation can crowd atoms beyond the rows' capacity: a rebuild that
-    // ran out of room is redone with wider rows
-    int ov = 0;
-    MAPPG_CUDA(cudaMemcpyAsync(&ov, &s->sc->overflow, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
-    MAPPG_CUDA(cudaStreamSynchronize(s->stream));
-    if (ov) sys_build(s);
+}
+
+void lb_update(mappg_sys* s) {
+    lb_update_launch(s);
+    if (lb_read(s, nullptr)->sc.overflow) sys_build(s);
+}
+
+// list check, then the energy by `launch`, one read for both
+template <class F>
+static double lb_checked_energy(mappg_sys* s, F launch) {
+    lb_update_launch(s);
+    launch(s);
+    const LbRead* r = lb_read(s, nullptr);
+    if (r->sc.overflow) {
+        sys_build(s);
+        launch(s);
+        r = lb_read(s, nullptr);
+    }
+    return r->sc.energy;
+}
+
+static double lb_energy(mappg_sys* s) {
+    // mixed systems compare FP64 line-search energies, so FP32 rounding of
+    // the pair terms does not decide the Armijo test near convergence
+    return lb_checked_energy(s, s->precision == MAPPG_MIXED ? launch_energy64 : launch_energy);
 }
 
 static void lb_force(mappg_sys* s, double* pe) {
     launch_force(s);
     sync_forces64(s);
-    MAPPG_CUDA(cudaMemcpyAsync(pe, &s->sc->energy, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
-    MAPPG_CUDA(cudaStreamSynchronize(s->stream));
+    *pe = lb_read(s, nullptr)->sc.energy;
 }
 
 // The caller's function after an iteration's force call, where the
@@ -331,12 +358,9 @@ struct TrialLine {
         launch_dep(s->stream, k_lb_trial, grid, 256, 0, N, s->x, xs, h, a);
         (*n_en)++;
         if (mode == E64) return lb_energy(s);
-        double e;
         if (mode == DELTA) {
             launch_de32(s, a);
-            MAPPG_CUDA(cudaMemcpyAsync(&e, &s->sc->de, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
-            MAPPG_CUDA(cudaStreamSynchronize(s->stream));
-            return e0 + e;
+            return e0 + lb_read(s, nullptr)->sc.de;
         }
         return e0 + (energy32(s) - e0_32);
     }
@@ -359,14 +383,7 @@ struct TrialLine {
         if (1.7320508075688772 * (a * hmax + dx) < 0.5 * s->skin) mode = DELTA;
     }
     // skin test, gated rebuild, then the FP32 energy
-    static double energy32(mappg_sys* s) {
-        lb_update(s);
-        launch_energy(s);
-        double e;
-        MAPPG_CUDA(cudaMemcpyAsync(&e, &s->sc->energy, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
-        MAPPG_CUDA(cudaStreamSynchronize(s->stream));
-        return e;
-    }
+    static double energy32(mappg_sys* s) { return lb_checked_energy(s, launch_energy); }
 };
 
 // grid of the FP64 vector kernels with grid-wide sums: two blocks per SM, so
@@ -387,29 +404,20 @@ void lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_tol, c
     if (nsteps < 0) throw Error{MAPPG_ERR_ARG, "nsteps must be >= 0"};
     const int N = 3 * s->n;
     const int grid = lb_grid(s, N);
-    std::vector<void*> owned;
-    auto dalloc = [&](size_t bytes) {
-        void* p = nullptr;
-        MAPPG_CUDA(cudaMalloc(&p, bytes));
-        owned.push_back(p);
-        return p;
-    };
-    struct Guard {
-        std::vector<void*>& o;
-        ~Guard() {
-            for (void* p : o) cudaFree(p);
-        }
-    } guard{owned};
-    double* f0 = (double*)dalloc(sizeof(double) * N);
-    double* h = (double*)dalloc(sizeof(double) * N);
-    double* xs = (double*)dalloc(sizeof(double) * N);
+    const bool mixed = s->precision == MAPPG_MIXED;
+    Work work(s);
+    work.reserve((3 + 2 * (size_t)m) * Work::room<double>(N) + Work::room<LbScal>(1) + Work::room<unsigned>(4) +
+                 (mixed ? Work::room<float4>(s->n) : 0));
+    double* f0 = work.take<double>(N);
+    double* h = work.take<double>(N);
+    double* xs = work.take<double>(N);
     std::vector<double*> sv(m), yv(m);
     for (int i = 0; i < m; i++) {
-        sv[i] = (double*)dalloc(sizeof(double) * N);
-        yv[i] = (double*)dalloc(sizeof(double) * N);
+        sv[i] = work.take<double>(N);
+        yv[i] = work.take<double>(N);
     }
-    LbScal* L = (LbScal*)dalloc(sizeof(LbScal));
-    unsigned* counter = (unsigned*)dalloc(sizeof(unsigned) * 4);
+    LbScal* L = work.take<LbScal>(1);
+    unsigned* counter = work.take<unsigned>(4);
     MAPPG_CUDA(cudaMemsetAsync(L, 0, sizeof(LbScal), s->stream));
     MAPPG_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned) * 4, s->stream));
     const double one = 1.0;  // gamma starts at 1 (min_l-bfgs.h:140), as does tau
@@ -426,7 +434,6 @@ void lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_tol, c
     // mixed systems: line-search trials inside the skin take energy
     // differences (TrialLine delta mode), which need x0's FP64 density and
     // the direction as float4
-    const bool mixed = s->precision == MAPPG_MIXED;
     struct KeepRho {
         mappg_sys* s;
         ~KeepRho() {
@@ -436,7 +443,7 @@ void lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_tol, c
     } keep_rho{s};
     if (mixed) {
         s->keep_rho64 = true;
-        s->h32 = (float4*)dalloc(sizeof(float4) * (size_t)s->n);
+        s->h32 = work.take<float4>(s->n);
     }
 
     // NewDynamicMD::init then the opening force call
@@ -452,15 +459,13 @@ void lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_tol, c
     double dxmax = 0.0;
     auto read_prep = [&](double* fh, double* hh, double* hmax, double* fmax_) {
         launch_dep(st, k_lb_prep, grid, 256, 0, N, s->f, h, s->x, s->x0, L, part, counter);
-        MAPPG_CUDA(cudaGetLastError());
-        double buf[6];
-        MAPPG_CUDA(cudaMemcpyAsync(buf, &L->fh, sizeof(buf), cudaMemcpyDeviceToHost, st));
-        MAPPG_CUDA(cudaStreamSynchronize(st));
-        *fh = buf[0];
-        *hh = buf[1];
-        *hmax = buf[2];
-        *fmax_ = buf[3];
-        dxmax = buf[5];
+        const LbRead* r = lb_read(s, L);
+        *fh = r->prep[0];
+        *hh = r->prep[1];
+        *hmax = r->prep[2];
+        *fmax_ = r->prep[3];
+        dxmax = r->prep[5];
+        return r;
     };
     double fh, hh, hmax, fmaxv;
     if (err == LS_S && f_tol > 0.0) {
@@ -471,7 +476,6 @@ void lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_tol, c
     // the two-loop recursion (min_l-bfgs.h:148-170) with the initial inverse
     // Hessian gamma*I, or diag(P) when a learned preconditioner is given
     auto two_loop = [&](bool diag) {
-        MAPPG_CUDA(cudaMemcpyAsync(h, s->f, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
         // first loop: alpha_i = -rho_i (s_i.h); h += alpha_i y_i
         if (k > 0) launch_dep(st, k_lb_axpy_dot, grid, 256, 0, N, h, nullptr, sv[0], L, 0, 0, 0, 0, part, counter);
         for (int i = 0; i < k; i++) {
@@ -493,14 +497,14 @@ void lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_tol, c
     int istep = 0;
     for (; err == LS_S; istep++) {
         if (P && s->precond_every > 0 && istep > 0 && istep % s->precond_every == 0) s->precond_refresh();
-        MAPPG_CUDA(cudaMemcpyAsync(xs, s->x, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
-        MAPPG_CUDA(cudaMemcpyAsync(f0, s->f, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
+        launch_dep(st, k_lb_start, grid_for(s, N, 256), 256, 0, N, s->x, s->f, xs, f0, h);
         two_loop(P != nullptr);
         e_prev = e_curr;
         read_prep(&fh, &hh, &hmax, &fmaxv);
         if (P && fh < 0.0) {
             // a non-descent preconditioned direction: plain L-BFGS instead
             if (n_fallback) (*n_fallback)++;
+            MAPPG_CUDA(cudaMemcpyAsync(h, s->f, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
             two_loop(false);
             read_prep(&fh, &hh, &hmax, &fmaxv);
         }
@@ -550,11 +554,11 @@ void lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_tol, c
         else
             lerr = search.min(dfa, max_a, e_curr, alpha_m, 0);
         err = lerr;
-        if (line.mode == TrialLine::DELTA) {
-            // the accepted (or restored) positions: skin test, and the FP32
-            // frame positions the force call reads
-            lb_update(s);
-        }
+        // after a DELTA search: the accepted (or restored) positions' skin
+        // test, and the FP32 frame positions the force call reads
+        const bool moved = line.mode == TrialLine::DELTA;
+        if (moved) lb_update_launch(s);
+        if (moved && err != LS_S && lb_read(s, nullptr)->sc.overflow) sys_build(s);
         if (ls_failed(err) && s->precision == MAPPG_MIXED && !s->force64 && f_tol > 0.0) {
             s->force64 = true;
             lb_force(s, &pe_force);
@@ -572,15 +576,27 @@ void lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_tol, c
             continue;
         }
         // handler.force_calc(): forces and atoms->pe; e_curr stays the line
-        // search's energy, as in min_l-bfgs.h:181-188
-        lb_force(s, &pe_force);
+        // search's energy, as in min_l-bfgs.h:181-188.  max|F| and the energy
+        // come back in one read, with the capacity flag of the list check
+        // (max|F| after the caller's function where there is one: it may
+        // change the system)
+        auto force = [&] {
+            launch_force(s);
+            sync_forces64(s);
+            if (f_tol > 0.0 && !s->hook) return (const LbRead*)read_prep(&fh, &hh, &hmax, &fmaxv);
+            return (const LbRead*)lb_read(s, nullptr);
+        };
+        const LbRead* r = force();
+        if (moved && r->sc.overflow) {
+            sys_build(s);
+            r = force();
+        }
+        pe_force = r->sc.energy;
         n_fc++;
         iteration_hook(s, istep);
         if (e_prev - e_curr < e_tol) err = MIN_S_TOLERANCE;
-        if (f_tol > 0.0) {
-            read_prep(&fh, &hh, &hmax, &fmaxv);
-            if (fmaxv < f_tol) err = MIN_S_FTOL;
-        }
+        if (f_tol > 0.0 && s->hook) read_prep(&fh, &hh, &hmax, &fmaxv);
+        if (f_tol > 0.0 && fmaxv < f_tol) err = MIN_S_FTOL;
         if (istep + 1 == nsteps) err = MIN_F_MAX_ITER;
         if (err) continue;
         if (m) {
@@ -676,24 +692,13 @@ void cg_run(mappg_sys* s, double e_tol, double max_dx, double f_tol, const LsPar
     if (nsteps < 0) throw Error{MAPPG_ERR_ARG, "nsteps must be >= 0"};
     const int N = 3 * s->n;
     const int grid = lb_grid(s, N);
-    std::vector<void*> owned;
-    auto dalloc = [&](size_t bytes) {
-        void* p = nullptr;
-        MAPPG_CUDA(cudaMalloc(&p, bytes));
-        owned.push_back(p);
-        return p;
-    };
-    struct Guard {
-        std::vector<void*>& o;
-        ~Guard() {
-            for (void* p : o) cudaFree(p);
-        }
-    } guard{owned};
-    double* f0 = (double*)dalloc(sizeof(double) * N);
-    double* h = (double*)dalloc(sizeof(double) * N);
-    double* xs = (double*)dalloc(sizeof(double) * N);
-    LbScal* L = (LbScal*)dalloc(sizeof(LbScal));
-    unsigned* counter = (unsigned*)dalloc(sizeof(unsigned) * 4);
+    Work work(s);
+    work.reserve(3 * Work::room<double>(N) + Work::room<LbScal>(1) + Work::room<unsigned>(4));
+    double* f0 = work.take<double>(N);
+    double* h = work.take<double>(N);
+    double* xs = work.take<double>(N);
+    LbScal* L = work.take<LbScal>(1);
+    unsigned* counter = work.take<unsigned>(4);
     cudaStream_t st = s->stream;
     MAPPG_CUDA(cudaMemsetAsync(L, 0, sizeof(LbScal), st));
     MAPPG_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned) * 4, st));
@@ -701,15 +706,12 @@ void cg_run(mappg_sys* s, double e_tol, double max_dx, double f_tol, const LsPar
     double dxmax = 0.0;
     auto read_prep = [&](double* fh, double* hh, double* hmax, double* fmax_) {
         launch_dep(st, k_lb_prep, grid, 256, 0, N, s->f, h, s->x, s->x0, L, part, counter);
-        MAPPG_CUDA(cudaGetLastError());
-        double buf[6];
-        MAPPG_CUDA(cudaMemcpyAsync(buf, &L->fh, sizeof(buf), cudaMemcpyDeviceToHost, st));
-        MAPPG_CUDA(cudaStreamSynchronize(st));
-        *fh = buf[0];
-        *hh = buf[1];
-        *hmax = buf[2];
-        *fmax_ = buf[3];
-        dxmax = buf[5];
+        const LbRead* r = lb_read(s, L);
+        *fh = r->prep[0];
+        *hh = r->prep[1];
+        *hmax = r->prep[2];
+        *fmax_ = r->prep[3];
+        dxmax = r->prep[5];
     };
     sys_build(s);
     long long n_en = 0, n_fc = 1;
@@ -735,8 +737,7 @@ void cg_run(mappg_sys* s, double e_tol, double max_dx, double f_tol, const LsPar
             err = LS_F_GRAD0;
             continue;
         }
-        MAPPG_CUDA(cudaMemcpyAsync(xs, s->x, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
-        MAPPG_CUDA(cudaMemcpyAsync(f0, s->f, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
+        launch_dep(st, k_lb_start, grid_for(s, N, 256), 256, 0, N, s->x, s->f, xs, f0, nullptr);
         e_prev = e_curr;
         read_prep(&fh, &hh, &hmax, &fmaxv);
         if (fh < 0.0) {

@@ -375,9 +375,46 @@ struct mappg_sys {
     double* stage2 = nullptr;
     cudaEvent_t ev_main = nullptr, ev_side = nullptr;
     bool v_pending = false;  // s->v is being written on `side` until ev_side
+    // the minimizers' vectors (one allocation, kept between runs up to a
+    // bound) and their pinned landing place for scalars
+    char* work = nullptr;
+    size_t work_bytes = 0;
+    bool work_busy = false;
+    void* landing = nullptr;
 };
 
 namespace mappg {
+
+// A run's device arrays, cut from the system's workspace; a run started
+// inside another one's hook gets an allocation of its own.  The caller adds
+// its arrays up (room), reserves, then takes them.
+class Work {
+   public:
+    explicit Work(mappg_sys* s) : s_(s) {}
+    ~Work();
+    Work(const Work&) = delete;
+    Work& operator=(const Work&) = delete;
+    void reserve(size_t bytes);
+    template <class T>
+    T* take(size_t count) {
+        char* p = base_ + at_;
+        at_ += room<T>(count);
+        return (T*)p;
+    }
+    template <class T>
+    static size_t room(size_t count) {
+        return (sizeof(T) * (count ? count : 1) + 255) / 256 * 256;
+    }
+
+   private:
+    void drop();
+    mappg_sys* s_;
+    char* base_ = nullptr;
+    size_t at_ = 0;
+    bool shared_ = false;
+};
+// pinned host memory for scalars read back (4 KB)
+void* sys_landing(mappg_sys* s);
 
 // system.cu
 void sys_set_box(mappg_sys* s, const double* H);
