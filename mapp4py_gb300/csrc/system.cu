@@ -497,6 +497,7 @@ struct BuildArgs {
     Geo g;
     Frame fr;       // frame to Cartesian
     float lo2[kMaxElem * kMaxElem], hi2[kMaxElem * kMaxElem];
+    float hi2max;                    // the largest of hi2
     float in2[kMaxElem * kMaxElem];  // pair cutoff squared: entries below it lead their row
     double cut_sk_sq[kMaxElem * kMaxElem];
     const CellGeo* cells;  // batch: per-cell geometry, indexed by cell_of
@@ -558,6 +559,8 @@ constexpr int kBuildWarps = 4;    // warps of a builder block
 constexpr int kBuildTile = 768;   // candidates staged at a time (12 KB)
 constexpr int kBuildHome = 32;    // atoms of the bin worked on at a time
 constexpr int kBuildRow = 256;    // longest row put together on chip
+constexpr int kBuildAtoms = 4;    // atoms of a warp that test a candidate together
+constexpr int kBuildHits = 160;   // candidates within reach noted per atom
 
 // list thresholds of a pair: kept below lo2, decided in FP64 up to hi2, leading its row below in2
 template <bool UNI>
@@ -569,20 +572,57 @@ struct BuildCut {
     __device__ __forceinline__ float in(int e) const { return UNI ? in2 : tab[2 * kMaxElem * kMaxElem + e]; }
 };
 
-// the staged candidates (nt of them, the rest of the last 32 far away)
-// against atom h: its inner entries go to dst[0], dst[1], ..., its shell
-// entries to dst[cap - 1], dst[cap - 2], ...; entries that would leave the
-// row or meet are dropped (the caller sees it from the counts)
-template <bool ORTHO, bool UNI>
-__device__ __forceinline__ void build_scan(const BuildArgs& a, const BuildCut<UNI>& cut, const float4* cand, int nt,
-                                           const float4& h, int self, const int* geo, const double* h6,
-                                           const CellGeo* cg, int* dst, int cap, int& cin, int& cout) {
+// the candidates within reach2 (squared) of each of the A atoms h[0..A-1], by
+// their place in cand and in its order, into hits[u]; nh[u] of them (those
+// beyond kBuildHits are not noted)
+template <int A>
+__device__ __forceinline__ void build_hits(const float4* cand, int nt, const float4* home, int q0, int ng, float reach2,
+                                           uint16_t (*hits)[kBuildHits], int* nh) {
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
-    const int pe0 = entry_elem(self) * a.ne;
+    float hx[A], hy[A], hz[A];
+    int c[A];
+#pragma unroll
+    for (int u = 0; u < A; u++) {
+        const float4 h = home[min(q0 + u * kBuildWarps, ng - 1)];
+        hx[u] = h.x;
+        hy[u] = h.y;
+        hz[u] = h.z;
+        c[u] = 0;
+    }
 #pragma unroll 2
     for (int k0 = 0; k0 < nt; k0 += 32) {
         const float4 p = cand[k0 + lane];
+#pragma unroll
+        for (int u = 0; u < A; u++) {
+            const float dx = hx[u] - p.x, dy = hy[u] - p.y, dz = hz[u] - p.z;
+            const bool in = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= reach2;
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            const int at = c[u] + __popc(m & below);
+            if (in && at < kBuildHits) hits[u][at] = (uint16_t)(k0 + lane);
+            c[u] += __popc(m);
+        }
+    }
+    if (lane == 0)
+#pragma unroll
+        for (int u = 0; u < A; u++) nh[u] = c[u];
+}
+
+// the staged candidates (nt of them, the rest of the last 32 far away), or
+// with hits the nt of them that it names, against atom h: its inner entries
+// go to dst[0], dst[1], ..., its shell entries to dst[cap - 1], dst[cap - 2],
+// ...; entries that would leave the row or meet are dropped (the caller sees
+// it from the counts)
+template <bool ORTHO, bool UNI>
+__device__ __forceinline__ void build_scan(const BuildArgs& a, const BuildCut<UNI>& cut, const float4* cand, int nt,
+                                           const uint16_t* hits, const float4& h, int self, const int* geo,
+                                           const double* h6, const CellGeo* cg, int* dst, int cap, int& cin,
+                                           int& cout) {
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const int pe0 = entry_elem(self) * a.ne;
+    for (int k0 = 0; k0 < nt; k0 += 32) {
+        const float4 p = !hits ? cand[k0 + lane] : k0 + lane < nt ? cand[hits[k0 + lane]] : make_float4(1e18f, 0.f, 0.f, 0.f);
         const int ent = __float_as_int(p.w);
         const float dx = h.x - p.x, dy = h.y - p.y, dz = h.z - p.z;
         const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
@@ -621,28 +661,34 @@ __device__ __forceinline__ void build_scan(const BuildArgs& a, const BuildCut<UN
 // rebuild step 5: one block per bin.  The candidates of the bin's 27-bin
 // stencil are staged in shared memory as Cartesian positions beside the bin
 // (bin_pos: one coalesced load a candidate), and the block's warps take the
-// bin's atoms in turn, 32 candidates against one atom at a time.  A row
+// bin's atoms in turn.  A warp first tests the candidates against up to four
+// atoms at once, 32 at a time, and notes those within reach (one candidate in
+// six); then it goes through what it noted, atom by atom, in the same order,
+// with the tests that decide what is kept and where.  A row
 // holds first its atom's neighbours inside the pair cutoff at build time, in
 // (bin step, bin order) order, bin steps c = (d0+1) + 3(d1+1) + 9(d2+1), then
 // those of the skin shell in the reverse of that order: it is put together
 // in shared memory, inner entries from the front and shell entries from the
-// end, and written out in one piece.  Rows longer than kBuildRow, and those
-// of bins whose candidates need several tiles, are put together in place.
-// With the inner entries in front, the lanes of an atom (slots lane,
-// lane + TPA, ...) get equal shares of the pairs inside the cutoff, and the
-// density pass's lanes reach the shell together.  A batch finds the bin's
-// cell through its first atom (the bins of a cell hold only that cell's
-// atoms).
+// end, and written out in one piece.  Rows longer than kBuildRow, atoms with
+// more than kBuildHits candidates in reach, and bins whose candidates need
+// several tiles go through the candidates directly; the latter's rows are put
+// together in place.  With the inner entries in front, the lanes of an atom
+// (slots lane, lane + TPA, ...) get equal shares of the pairs inside the
+// cutoff, and the density pass's lanes reach the shell together.  A batch
+// finds the bin's cell through its first atom (the bins of a cell hold only
+// that cell's atoms).
 //
-// Bound by instruction issue.  The atom's two counters are uniform in its
-// warp, so 32 tests are the distance, three ballots and a store, and a step
-// without any neighbour (a quarter of them) ends at the first ballot.  With
-// the warp walking candidates in the outer loop (one warp per bin, as this
-// kernel was built before) the counters went through shuffles, an iteration
-// waited ~800 clocks on its chain, and the bins of a 500-atom cell had 27
-// warps in all.
-// Whole rebuild (all its kernels) before and now: 4,000 atoms 129 -> 45 us,
-// 32,000 164 -> 68, 256,000 509 -> 318, 500,000 905 -> 599.
+// Bound by instruction issue (69 % of the slots at 500,000 atoms, 774 warp
+// instructions an atom).  The atom's counters are uniform in its warp.  With
+// every step of 32 candidates taking the full set of tests the pass had 1,000
+// instructions an atom; the noting step has 14 for one atom, and a candidate
+// read from shared memory serves four.  Four warps a block: eight are faster
+// below 10,000 atoms (25 instead of 29 us at 4,000) and slower above (598
+// instead of 545 at 500,000).
+// Whole rebuild (all its kernels) as this kernel was first built (one warp
+// per bin, candidates in the outer loop), with a block a bin and direct
+// tests, and now: 4,000 atoms 129, 35 and 29 us; 32,000 164, 60 and 49;
+// 256,000 509, 339 and 286; 500,000 905, 650 and 545.
 // ORTHO: every cell orthorhombic (one product per axis to Cartesian).
 // UNI: every pair type has the same list cutoff (thresholds in registers).
 template <bool BATCH, bool ORTHO, bool UNI>
@@ -652,7 +698,8 @@ __global__ void __launch_bounds__(32 * kBuildWarps) k_build_bins(const __grid_co
     if (!sc->rebuild) return;
     __shared__ float4 cand[kBuildTile], home[kBuildHome];
     __shared__ int s_pre[33], s_lo[32], s_cin[kBuildHome], s_cout[kBuildHome], s_geo[6];
-    __shared__ int s_row[kBuildWarps][kBuildRow];
+    __shared__ int s_row[kBuildWarps][kBuildRow], s_nh[kBuildWarps][kBuildAtoms];
+    __shared__ uint16_t s_hits[kBuildWarps][kBuildAtoms][kBuildHits];
     __shared__ float s_cut[UNI ? 1 : 3 * kMaxElem * kMaxElem];
     if (!UNI)
         for (int t = threadIdx.x; t < a.ne * a.ne; t += 32 * kBuildWarps) {
@@ -753,27 +800,41 @@ __global__ void __launch_bounds__(32 * kBuildWarps) k_build_bins(const __grid_co
                         cand[k] = p;
                     }
                 __syncthreads();
-                for (int q = w; q < ng; q += kBuildWarps) {
+                for (int q = w, u = 0; q < ng; q += kBuildWarps, u = (u + 1) % kBuildAtoms) {
+                    if (one_tile && u == 0) {
+                        const int more = (ng - 1 - q) / kBuildWarps;  // atoms of the warp after this one
+                        if (more >= 2)
+                            build_hits<4>(cand, nt, home, q, ng, a.hi2max, s_hits[w], s_nh[w]);
+                        else if (more)
+                            build_hits<2>(cand, nt, home, q, ng, a.hi2max, s_hits[w], s_nh[w]);
+                        else
+                            build_hits<1>(cand, nt, home, q, ng, a.hi2max, s_hits[w], s_nh[w]);
+                        __syncwarp();
+                    }
                     const float4 h = home[q];
                     const int self = __float_as_int(h.w) | make_entry(0, 0, 13);  // the atom itself, unshifted
                     const int i = entry_j(self);
                     int* row = a.nbr + (size_t)i * a.maxnbr;
-                    int cin = 0, cout = 0, tot = kBuildRow + 1;
-                    if (one_tile) {
-                        build_scan<ORTHO, UNI>(a, cut, cand, nt, h, self, s_geo, h6, cg, s_row[w], kBuildRow, cin, cout);
+                    int cin = 0, cout = 0, tot = 0;
+                    bool chip = false;  // the row is in s_row
+                    if (one_tile && s_nh[w][u] <= kBuildHits) {
+                        build_scan<ORTHO, UNI>(a, cut, cand, s_nh[w][u], s_hits[w][u], h, self, s_geo, h6, cg, s_row[w],
+                                               kBuildRow, cin, cout);
                         tot = cin + cout;
+                        chip = tot <= kBuildRow;
                         __syncwarp();
                         // (of a row that does not fit only the inner entries)
-                        if (tot <= kBuildRow)
+                        if (chip)
                             for (int k = lane; k < min(tot <= a.maxnbr ? tot : cin, a.maxnbr); k += 32)
                                 row[k] = s_row[w][k < cin ? k : kBuildRow - tot + k];
                     }
-                    if (tot > kBuildRow) {
+                    if (!chip) {
                         if (one_tile)
                             cin = cout = 0;
                         else
                             cin = s_cin[q], cout = s_cout[q];
-                        build_scan<ORTHO, UNI>(a, cut, cand, nt, h, self, s_geo, h6, cg, row, a.maxnbr, cin, cout);
+                        build_scan<ORTHO, UNI>(a, cut, cand, nt, nullptr, h, self, s_geo, h6, cg, row, a.maxnbr, cin,
+                                               cout);
                         tot = cin + cout;
                         if (!last) {
                             if (lane == 0) {
@@ -800,7 +861,6 @@ __global__ void __launch_bounds__(32 * kBuildWarps) k_build_bins(const __grid_co
                     // still walk it) it counts the slots that were written
                     if (lane == 0) a.nnbr[i] = tot <= a.maxnbr ? tot : min(cin, a.maxnbr);
                     if (!BATCH && a.own_ent) {
-                        const bool chip = one_tile && tot <= kBuildRow;
                         const int len = tot <= a.maxnbr ? tot : 0;
                         const size_t base = (size_t)i * a.maxnbr;
                         int no = 0, nx = 0;
@@ -975,6 +1035,7 @@ void launch_rebuild_chain(mappg_sys* s) {
         a.lo2[p] = (float)(s->cut_sk_sq[p] - s->band);
         a.hi2[p] = (float)(s->cut_sk_sq[p] + s->band);
         a.in2[p] = (float)s->cut_sq[p];
+        a.hi2max = std::max(p ? a.hi2max : 0.f, a.hi2[p]);
     }
     a.fr = s->frame;
     a.cells = s->cells_dev;

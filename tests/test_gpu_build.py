@@ -76,3 +76,19 @@ def test_fp64_pairs_by_owner_match_the_oracle(potentials, cells, skin):
     assert np.max(np.abs(vir - vir_o)) <= 1e-11 * np.max(np.abs(vir_o))
     assert np.max(np.abs(s.get_f() - o.f)) <= 1e-10 * max(1.0, np.max(np.abs(o.f)))
     assert abs(s.energy() - pe_o) <= 1e-12 * abs(pe_o)
+
+
+@pytest.mark.parametrize("precision", [_lib.FP64, _lib.MIXED])
+@pytest.mark.parametrize("n", [5, 13, 32, 33, 160, 161, 200, 257])
+def test_neighbor_sets_of_one_crowded_bin(potentials, n, precision):
+    """Every remainder of the atoms a warp tests together, and rows around the
+    number of candidates it notes and around the row it puts together on chip."""
+    path, _ = potentials[("A", "B")]
+    rng = np.random.default_rng(n)
+    x = 20.0 + rng.uniform(-1.4, 1.4, (n, 3))
+    H, elem, masses = np.diag([43.0, 41.0, 40.0]), (rng.random(n) < 0.5).astype(np.uint8), [synth.MASS, synth.MASS]
+    o = O.System(O.Eam.setfl(path), H, x, elem, masses, skin=0.5, pair_wise=False)
+    o.init_dynamic()
+    s = _lib.System(_lib.ForceField.setfl(path), H, x, elem, masses, skin=0.5, precision=precision)
+    s.build()
+    assert np.array_equal(keys(*s.neighbors()), keys(*o.neighbors()))
