@@ -30,19 +30,29 @@ namespace mappg {
 // with dep_wait launched in the ordinary way runs as ever.
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// cluster: blocks of the grid's thread-block clusters
 template <class... P, class... A>
-static void launch_dep(cudaStream_t stream, void (*kernel)(P...), int grid, int block, size_t smem, A&&... args) {
+static void launch_dep_cluster(cudaStream_t stream, void (*kernel)(P...), int cluster, int grid, int block, size_t smem,
+                               A&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     MAPPG_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+
+template <class... P, class... A>
+static void launch_dep(cudaStream_t stream, void (*kernel)(P...), int grid, int block, size_t smem, A&&... args) {
+    launch_dep_cluster(stream, kernel, 1, grid, block, smem, std::forward<A>(args)...);
 }
 
 // 32-byte read-only loads (one sector per lane, one instruction): the spline

@@ -92,3 +92,24 @@ def test_neighbor_sets_of_one_crowded_bin(potentials, n, precision):
     s = _lib.System(_lib.ForceField.setfl(path), H, x, elem, masses, skin=0.5, precision=precision)
     s.build()
     assert np.array_equal(keys(*s.neighbors()), keys(*o.neighbors()))
+
+
+@pytest.mark.parametrize("n,bins", [(1, (4, 4, 4)), (33, (4, 5, 6)), (1025, (16, 16, 8)), (8191, (12, 13, 13)),
+                                    (8192, (16, 16, 8)), (8193, (16, 16, 8)), (700, (13, 13, 13))])
+def test_neighbor_sets_where_binning_changes_kernels(potentials, n, bins):
+    """Around the largest system that one cluster of blocks bins, by atoms and
+    by bins, and a second build from moved positions."""
+    path, rc = potentials[("A", "B")]
+    rng = np.random.default_rng(n)
+    ff = _lib.ForceField.setfl(path)
+    H = np.diag([b * 6.2 for b in bins])
+    H[1, 0] = 1.3
+    x, elem, masses = rng.random((n, 3)) @ H, (rng.random(n) < 0.5).astype(np.uint8), [synth.MASS, synth.MASS]
+    s = _lib.System(ff, H, x, elem, masses, skin=0.5, precision=_lib.MIXED)
+    for _ in range(2):
+        s.set_x(x)
+        s.build()
+        o = O.System(O.Eam.setfl(path), H, x, elem, masses, skin=0.5, pair_wise=False)
+        o.init_dynamic()
+        assert np.array_equal(keys(*s.neighbors()), keys(*o.neighbors()))
+        x = rng.random((n, 3)) @ H
