@@ -305,6 +305,25 @@ __device__ inline void drift_now(const DevScalars* sc, const double* partials, i
     for (int c = 0; c < 3; c++) d[c] = sc->drift[c] + (rows ? tot[c] * n_inv : 0.0);
 }
 
+// energy and virial of a force call from its passes' rows, by the whole block:
+// out[0] the energy, out[1..6] the virial (shared memory, set by the first
+// warp, which may read them after __syncwarp)
+__device__ inline void pass_totals(const double* partials, const PassRows& r, double* out) {
+    __shared__ double tot[8];
+    const int k = threadIdx.x % 8;
+    final_sums<8>(partials, k == 0 ? r.pair : k == 7 ? r.rho : r.force, tot);
+    if (threadIdx.x < 7) out[threadIdx.x] = r.scale * tot[threadIdx.x] + (threadIdx.x == 0 ? tot[7] : 0.0);
+    if (threadIdx.x < 32) __syncwarp();
+}
+
+// the last block of a force pass (all threads): energy and virial of the call
+__device__ inline void store_totals(const double* partials, const PassRows& r, DevScalars* sc, unsigned* counter) {
+    __shared__ double out[7];
+    pass_totals(partials, r, out);
+    if (threadIdx.x < 7) (threadIdx.x ? sc->virial[threadIdx.x - 1] : sc->energy) = out[threadIdx.x];
+    if (threadIdx.x == 0) *counter = 0;
+}
+
 // block sums of K values (as block_partials) into out[0..K-1], one batch chunk
 template <int K, class T>
 __device__ __forceinline__ void chunk_store(const T (&v)[K], double* out) {

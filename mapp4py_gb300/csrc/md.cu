@@ -68,6 +68,8 @@ struct MdArgs {
     float m32[kMaxElem];   // masses as floats (the kinetic tensors' FP32 products)
     double dt, dt2, n_inv, skin_sq;
     int drift_rows;        // mixed: blocks of k_integrate32
+    const double* pass_part;  // the force call's partial sums, where its totals
+    PassRows pass;            // are left to the closing kernel (else pass.force = 0)
     float dt32, skin_sq32;
     double bs[6];          // x -> scaled frame
     Frame fr;
@@ -168,6 +170,13 @@ struct CloseStep {
             }
         }
         return nhc_any(a.nhc, eta, T_r);
+    }
+    // whole last block: the energy and virial of the step's force call, where
+    // its passes left them as partial sums
+    __device__ __forceinline__ void totals(const MdArgs& a) {
+        if (!a.pass.force) return;
+        pass_totals(a.pass_part, a.pass, ev);
+        if (threadIdx.x < 7) (threadIdx.x ? a.sc->virial[threadIdx.x - 1] : a.sc->energy) = ev[threadIdx.x];
     }
     // first warp of the block; returns the closing factor
     __device__ __forceinline__ double close(const MdArgs& a, const double* mvv) {
@@ -314,6 +323,7 @@ __global__ void __launch_bounds__(256) k_kick2_64(MdArgs a) {
     }
     __shared__ double t[6];
     if (close_partials<6>(d, a, &a.sc->counter[5], S)) {
+        S.totals(a);
         final_sums<6>(a.partials, gridDim.x, t);
         if (threadIdx.x < 32) {
             const double fac = S.close(a, t);
@@ -433,6 +443,7 @@ __global__ void __launch_bounds__(256) k_close32(MdArgs a) {
     if (close_partials<6>(d, a, &a.sc->counter[5], S)) {
         // the kinetic tensor in t[0..5], k_integrate32's displacement sums
         // in t[8..10]
+        S.totals(a);
         final_sums<11>(a.partials, gridDim.x, t, a.drift_rows);
         for (int q = threadIdx.x; q < 3 * a.drift_rows; q += blockDim.x) a.partials[(q / 3) * kRedSlots + 8 + q % 3] = 0.0;
         if (threadIdx.x < 32) {
@@ -690,6 +701,7 @@ static MdArgs md_args(mappg_sys* s, double T, double dt, double kB, double t_rel
     MdArgs a;
     memset(&a, 0, sizeof(a));
     a.n = s->n;
+    a.pass_part = s->partials + kRedSlots * kMaxBlocks;
     a.x = s->x;
     a.v = s->v;
     a.f = s->f;
@@ -787,9 +799,18 @@ static void launch_step64(mappg_sys* s, const MdArgs& a, A listed = A(), B closi
     launch_dep(s->stream, k_com_skin64, m.grid, m.block, 0, a);
     launch_rebuild_chain(s);
     listed();
-    launch_force(s);
+    MdArgs b = a;
+    {
+        struct Defer {
+            mappg_sys* s;
+            ~Defer() { s->defer_totals = false; }
+        } defer{s};
+        s->defer_totals = s->own_ent != nullptr;
+        launch_force(s);
+        if (s->defer_totals) b.pass = s->pass_rows;
+    }
     closing();
-    launch_dep(s->stream, k_kick2_64, m.grid, m.block, 0, a);
+    launch_dep(s->stream, k_kick2_64, m.grid, m.block, 0, b);
 }
 
 template <class A = NoHook, class B = NoHook>
@@ -802,10 +823,13 @@ static void launch_step32(mappg_sys* s, const MdArgs& a, A listed = A(), B closi
     launch_rebuild_chain(s);
     listed();
     EamArgs e = eam_args(s);
+    e.defer = 1;
     launch_density32(s, e);
     launch_force32(s, e);
+    MdArgs b = a;
+    b.pass = s->pass_rows;
     closing();
-    launch_dep(s->stream, k_close32, c.grid, c.block, 0, a);
+    launch_dep(s->stream, k_close32, c.grid, c.block, 0, b);
 }
 
 static void launch_step32b(mappg_sys* s, const MdArgs& a) {

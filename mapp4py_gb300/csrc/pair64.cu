@@ -270,21 +270,15 @@ __global__ void __launch_bounds__(256) k_gather64(const __grid_constant__ EamArg
             a.f[2 * a.n + i] = fz;
         }
     }
-    // virial in slots 1-6; the last block adds those up with the pair energy
-    // (slot 0, k_pair64's blocks) and the embedding energy (slot 7, k_rho64's)
+    // virial in slots 1-6; the last block, or the kernel that closes an MD
+    // step, adds those up with the pair energy (slot 0, k_pair64's blocks) and
+    // the embedding energy (slot 7, k_rho64's)
     const double v[8] = {0.0, w[0], w[1], w[2], w[3], w[4], w[5], 0.0};
     const double t = block_sums<8>(v);
     if (threadIdx.x >= 1 && threadIdx.x < 7) a.partials[blockIdx.x * kRedSlots + threadIdx.x] = t;
-    __shared__ double tot[8];
-    if (last_block(&a.sc->counter[0])) {
-        const int k = threadIdx.x % 8;
-        final_sums<8>(a.partials, k == 0 ? rows_pair : k == 7 ? rows_rho : (int)gridDim.x, tot);
-        if (threadIdx.x == 0) {
-            a.sc->energy = tot[0] + tot[7];
-            for (int c = 0; c < 6; c++) a.sc->virial[c] = tot[c + 1];
-            a.sc->counter[0] = 0;
-        }
-    }
+    if (a.defer) return;
+    if (last_block(&a.sc->counter[0]))
+        store_totals(a.partials, PassRows{rows_pair, (int)gridDim.x, rows_rho, 1.0}, a.sc, &a.sc->counter[0]);
 }
 
 // the record slot of each pair that another atom owns, by the mirrored entry
@@ -359,6 +353,7 @@ static void pair_energy(mappg_sys* s, const EamArgs& a, int grid) {
 
 template <int TPA>
 static void pair_force(mappg_sys* s, const EamArgs& a, int grid) {
+    s->pass_rows = PassRows{grid, grid, grid, 1.0};
     launch_dep(s->stream, k_gather64<TPA>, grid, 256, 0, a, grid, grid);
 }
 

@@ -1317,7 +1317,9 @@ EamArgs eam_args(mappg_sys* s) {
     a.rho32out = s->rho32;
     a.f = s->f;
     a.f32 = s->f32;
-    a.partials = s->partials;
+    a.partials = s->partials + kRedSlots * kMaxBlocks;
+    a.rows_rho = s->pass_rows.rho;
+    a.defer = s->defer_totals;
     a.sc = s->sc;
     a.ncell = s->ncell;
     a.nchunk = s->nchunk;
@@ -1429,7 +1431,7 @@ void sys_alloc(mappg_sys* s, const double* x_host) {
     dev_alloc((void**)&s->nnbr, sizeof(int) * n);
     dev_alloc((void**)&s->rho, sizeof(double) * n);
     dev_alloc((void**)&s->dF, sizeof(double) * n);
-    dev_alloc((void**)&s->partials, sizeof(double) * kRedSlots * kMaxBlocks);
+    dev_alloc((void**)&s->partials, sizeof(double) * kRedSlots * kMaxBlocks * 2);
     dev_alloc((void**)&s->sc, sizeof(DevScalars));
     MAPPG_CUDA(cudaMemsetAsync(s->sc, 0, sizeof(DevScalars), s->stream));
     MAPPG_CUDA(cudaMemsetAsync(s->v, 0, nd, s->stream));

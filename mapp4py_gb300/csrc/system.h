@@ -162,6 +162,13 @@ constexpr int kDensSmallAtoms = 300000;
 // kept out of its dynamic table budget
 constexpr size_t kForceSmemReserve = 4 * 1024;
 
+// rows of a force call's partial sums (EamArgs::partials): the pair energy in
+// slot 0, the virial in slots 1-6, the embedding energy in slot 7
+struct PassRows {
+    int pair, force, rho;
+    double scale;  // of the pair sums: the mixed pass meets each pair twice
+};
+
 struct EamArgs {
     int n, maxnbr, ne, nr, nrho;
     const int* nbr;
@@ -195,6 +202,8 @@ struct EamArgs {
     double* f;             // SoA 3n (FP64 kernels)
     float* f32;            // SoA 3n (mixed kernels)
     double* partials;
+    int rows_rho;  // mixed: blocks of the density pass before the force pass
+    int defer;     // the force pass leaves its totals to the kernel that closes the MD step
     DevScalars* sc;
     // FP64, every pair computed once (pair64.cu): per atom the entries it
     // owns and the others, maxnbr of each, a record per owned entry
@@ -311,7 +320,9 @@ struct mappg_sys {
     double2 *pair_rec = nullptr, *pair_rho = nullptr;
     char* pair_mem = nullptr;  // the allocation that holds them
     double *rho = nullptr, *dF = nullptr;
-    double* partials = nullptr;
+    double* partials = nullptr;  // block sums: the vector and MD kernels', then the force passes'
+    bool defer_totals = false;   // see EamArgs::defer
+    mappg::PassRows pass_rows = {0, 0, 0, 1.0};  // of the last passes
     mappg::DevScalars* sc = nullptr;
     double* stage = nullptr;      // device staging, 3n doubles (caller order)
     double* thermo_dev = nullptr; // per-step thermo rows of an NVT run

@@ -30,3 +30,20 @@ def test_chain_follows_oracle(potentials, precision, L, niters, relax):
     assert np.max(np.abs(th[:, 1] - th_o[:, 1])) <= rel * np.max(np.abs(th_o[:, 1]))
     if precision == _lib.FP64:  # a stiff chain takes a temperature's FP32 rounding far beyond it
         assert np.max(np.abs(eta - eta_o)) <= rel * np.max(np.abs(eta_o))
+
+
+@pytest.mark.parametrize("cells", [(3, 3, 3), (5, 4, 6), (11, 11, 11), (16, 17, 16)])
+@pytest.mark.parametrize("precision", [_lib.FP64, _lib.MIXED])
+def test_energy_and_virial_of_the_last_step(potentials, precision, cells):
+    """An MD step's energy and virial (added up where the step closes) against
+    a force call at the positions that the step reached."""
+    path, _ = potentials[("A", "B")]
+    c = synth.alloy(cells, xB=0.5, sigma=0.05, T=600.0, seed=9)
+    s = _lib.System(_lib.ForceField.setfl(path), c.H, c.x, c.elem, c.masses, precision=precision)
+    s.set_v(c.v)
+    th, _ = s.nvt_run(700.0, synth.FS, synth.KB, 7, thermo=True)
+    pe, vir = s.force()
+    # sums in another order; mixed: positions rounded to FP32 in another frame
+    rel, relv = (1e-13, 1e-12) if precision == _lib.FP64 else (1e-7, 1e-5)
+    assert abs(th[-1, 0] - pe) <= rel * abs(pe)
+    assert np.max(np.abs(th[-1, 8:] - vir)) <= relv * np.sqrt(s.n) * np.max(np.abs(vir))
