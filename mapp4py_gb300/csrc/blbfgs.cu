@@ -40,7 +40,6 @@ enum BlErr { BL_S = 0, BL_DOWNHILL = 1, BL_GRAD0 = 2, BL_MIN_ALPHA = 3, BL_ETOL 
 
 struct BlCell {
     double gamma, tau, rho[kBlMaxHist], alpha[kBlMaxHist];
-    double dot;
     double fh, hh, hmax, fmax;
     double e_curr, e_prev, e0, a, dfa, pe;
     double dxmax;  // max |x - x_build| component over the cell's atoms
@@ -63,6 +62,7 @@ struct BlArgs {
     const double* P;
     double *S, *Y;   // [m][3n]
     double* part;    // [nchunk][4]
+    double *dot_in, *dot_out;  // [nchunk]: the recursion's dot products, of the step before and for the next
     int* count;      // cells still searching
     double c_ls, rho_ls, min_alpha, max_dx, e_tol, f_tol;
     int nsteps;
@@ -121,80 +121,82 @@ __device__ __forceinline__ double bl_cell_total(const BlArgs& a, int c, int k, b
     return t;
 }
 
-// x0 = x, f0 = f, h = f for the cells in `st`
-__global__ void k_bl_start(BlArgs a, int st) {
-    dep_wait();
-    const int n = a.n;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int s = a.cs[a.cell_of[i]].state;
-        if (s != st) continue;
-        for (int q = 0; q < 3; q++) {
-            const size_t j = (size_t)q * n + i;
-            if (st == BL_RUN) {
-                a.x0[j] = a.x[j];
-                a.f0[j] = a.f[j];
-            }
-            a.h[j] = a.f[j];
-        }
-    }
-}
+// One step of the recursion for the cells in `st`, chunk by chunk:
+//   kStart: h = f (and x0 = x, f0 = f in a search's first direction)
+//   kFirst: alpha_i = -rho_i (S_i.h), h += alpha_i Y_i
+//   kLast:  kFirst, then the initial inverse Hessian: h *= gamma, or h *= tau P
+//           (the learned diagonal, scaled by (s.y)/(y.P.y) of the newest pair)
+//   kSecond: h += (-alpha_i - rho_i (Y_i.h)) S_i
+// then the chunk's part of the next step's dot product, Vn[slot(i_next)].h
+// (none with Vn null), into dot_out.  The dot product of this step is the sum
+// of dot_in over the cell's chunks, which every warp forms for itself while
+// its loads are on their way: the chunks of a cell are few, and a kernel
+// between the steps for it cost more than the sum.  Bound by the history,
+// which the steps of a batch read from DRAM (330,000 atoms, m = 10: 160 MB).
+// 44 launches a direction before (9.5 us a step, 3.4 a sum), 21 now.
+enum BlMode { kStart, kFirst, kLast, kSecond };
 
-// one step of the recursion for the cells in `st`, chunk by chunk:
-//   mode 0: dot = V[slot(i)].h only
-//   mode 1: h += alpha_i Y[slot(i)] with alpha_i = -rho dot (first loop)
-//   mode 2: h += (-alpha_i - rho dot) S[slot(i)]      (second loop)
-//   mode 3: h *= gamma, mode 4: h *= tau P (the learned diagonal, scaled
-//   by (s.y)/(y.P.y) of the newest pair)
-// then the partial of the next dot, Vn[slot(i_next)].h (none if Vn null)
-__global__ void __launch_bounds__(256) k_bl_step(BlArgs a, int st, int mode, int i, const double* __restrict__ Vu,
+template <int MODE>
+__global__ void __launch_bounds__(256) k_bl_step(BlArgs a, int st, int i, bool diag, const double* __restrict__ Vu,
                                                  const double* __restrict__ Vn, int i_next) {
     dep_wait();
-    const int n = a.n;
+    const int n = a.n, lane = threadIdx.x & 31;
     const size_t N3 = 3 * (size_t)n;
     for (int ch = blockIdx.x; ch < a.nchunk; ch += gridDim.x) {
-        const BlCell& c = a.cs[a.chunk_cell[ch]];
-        const bool on = c.state == st;
-        if (!on) continue;  // uniform per block: the chunk's partial is not read
-        double coef = 0.0;
-        int su = 0, sn = 0;
-        if (on) {
-            if (mode == 1 && i < c.k) coef = c.alpha[i];
-            if (mode == 2 && i < c.k) coef = -c.alpha[i] - c.rho[slot_of(c, i, a.m)] * c.dot;
-            if (mode == 3) coef = c.gamma;
-            su = slot_of(c, i, a.m);
-            sn = slot_of(c, i_next, a.m);
-        }
-        double acc = 0.0;
-        const bool dot_on = on && Vn && i_next >= 0 && i_next < c.k;
-        for (int ii = a.chunk_begin[ch] + threadIdx.x; ii < a.chunk_begin[ch + 1]; ii += blockDim.x) {
-            if (!on) break;
+        const int cell = a.chunk_cell[ch];
+        BlCell& c = a.cs[cell];
+        if (c.state != st) continue;  // uniform per block: the chunk's partial is not read
+        const int ii = a.chunk_begin[ch] + threadIdx.x, end = a.chunk_begin[ch + 1];  // an atom a thread
+        const int su = slot_of(c, i, a.m), sn = slot_of(c, i_next, a.m);
+        const bool use = MODE != kStart && i < c.k;
+        const bool dot_on = Vn && i_next >= 0 && i_next < c.k;
+        double hv[3] = {0.0, 0.0, 0.0}, u[3] = {0.0, 0.0, 0.0}, w[3] = {0.0, 0.0, 0.0};
+        if (ii < end) {
+#pragma unroll
             for (int q = 0; q < 3; q++) {
                 const size_t j = (size_t)q * n + ii;
-                double hv = a.h[j];
-                if ((mode == 1 || mode == 2) && coef != 0.0) hv += coef * Vu[(size_t)su * N3 + j];
-                if (mode == 3) hv *= coef;
-                if (mode == 4) hv *= c.tau * a.P[j];
-                if (mode) a.h[j] = hv;
-                if (dot_on) acc += Vn[(size_t)sn * N3 + j] * hv;
+                hv[q] = MODE == kStart ? a.f[j] : a.h[j];
+                if (use) u[q] = Vu[(size_t)su * N3 + j];
+                if (dot_on) w[q] = Vn[(size_t)sn * N3 + j];
+            }
+        }
+        double coef = 0.0;
+        if (use) {
+            double t = 0.0;
+            for (int k = a.cell_chunk[cell] + lane; k < a.cell_chunk[cell + 1]; k += 32) t = t + a.dot_in[k];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) t = t + __shfl_xor_sync(0xffffffffu, t, o);
+            if (MODE == kSecond) {
+                coef = -c.alpha[i] - c.rho[su] * t;
+            } else {
+                coef = -c.rho[su] * t;
+                if (ch == a.cell_chunk[cell] && threadIdx.x == 0) c.alpha[i] = coef;
+            }
+        }
+        double acc = 0.0;
+        if (ii < end) {
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                const size_t j = (size_t)q * n + ii;
+                if (MODE == kStart && st == BL_RUN) {
+                    a.x0[j] = a.x[j];
+                    a.f0[j] = hv[q];
+                }
+                if (coef != 0.0) hv[q] += coef * u[q];
+                if (MODE == kLast) {
+                    if (diag)
+                        hv[q] *= c.tau * a.P[j];
+                    else
+                        hv[q] *= c.gamma;
+                }
+                a.h[j] = hv[q];
+                if (dot_on) acc += w[q] * hv[q];
             }
         }
         const double v[1] = {acc};
         const int op[1] = {0};
-        bl_store<1>(v, op, a.part + (size_t)ch * 4);
+        bl_store<1>(v, op, a.dot_out + ch);
     }
-}
-
-// per-cell dot from the chunk partials; mode 1 also forms alpha_i
-__global__ void k_bl_cells_dot(BlArgs a, int st, int set_alpha, int i) {
-    dep_wait();
-    const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (c >= a.ncell) return;
-    const double t = bl_cell_total(a, c, 0, false);
-    if ((threadIdx.x & 31) != 0) return;
-    BlCell& cs = a.cs[c];
-    if (cs.state != st) return;
-    cs.dot = t;
-    if (set_alpha) cs.alpha[i] = i < cs.k ? -cs.rho[slot_of(cs, i, a.m)] * t : 0.0;
 }
 
 // f.h, h.h, max|h|, max|f| per chunk (cells in `st`, or all with st < 0)
@@ -618,7 +620,7 @@ void batch_lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_
     Work work(s);
     work.reserve(Work::room<int>(cb.size()) + Work::room<int>(cc.size()) + Work::room<int>(ccell.size()) +
                  Work::room<BlCell>(nc) + 3 * Work::room<double>(N3) + 2 * Work::room<double>(hist) +
-                 Work::room<double>(4 * (size_t)a.nchunk) + Work::room<int>(1) + Work::room<uint8_t>(nc) +
+                 Work::room<double>(4 * (size_t)a.nchunk) + 2 * Work::room<double>(a.nchunk) + Work::room<int>(1) + Work::room<uint8_t>(nc) +
                  Work::room<double>(nc) + (mixed ? Work::room<float4>(n) : 0));
     auto upload = [&](const std::vector<int>& v) {
         int* p = work.take<int>(v.size());
@@ -639,6 +641,8 @@ void batch_lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_
     a.S = work.take<double>(hist);
     a.Y = work.take<double>(hist);
     a.part = work.take<double>(4 * (size_t)a.nchunk);
+    a.dot_in = work.take<double>(a.nchunk);
+    a.dot_out = work.take<double>(a.nchunk);
     a.count = work.take<int>(1);
     a.P = P;
     a.c_ls = c_ls;
@@ -680,17 +684,14 @@ void batch_lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_
     };
     // the recursion for the cells in state `cst`
     auto two_loop = [&](int cst, bool diag) {
-        launch_dep(st, k_bl_start, ga, 256, 0, a, cst);
-        if (m > 0) launch_dep(st, k_bl_step, gc, 256, 0, a, cst, 0, 0, nullptr, a.S, 0);
-        for (int i = 0; i < m; i++) {
-            launch_dep(st, k_bl_cells_dot, gw, 256, 0, a, cst, 1, i);
-            launch_dep(st, k_bl_step, gc, 256, 0, a, cst, 1, i, a.Y, i + 1 < m ? a.S : nullptr, i + 1);
-        }
-        launch_dep(st, k_bl_step, gc, 256, 0, a, cst, diag ? 4 : 3, 0, nullptr, m > 0 ? a.Y : nullptr, m - 1);
-        for (int i = m - 1; i >= 0; i--) {
-            launch_dep(st, k_bl_cells_dot, gw, 256, 0, a, cst, 0, i);
-            launch_dep(st, k_bl_step, gc, 256, 0, a, cst, 2, i, a.S, i > 0 ? a.Y : nullptr, i - 1);
-        }
+        auto step = [&](auto kern, int i, const double* Vu, const double* Vn, int i_next) {
+            launch_dep(st, kern, a.nchunk, 256, 0, a, cst, i, diag, Vu, Vn, i_next);
+            std::swap(a.dot_in, a.dot_out);
+        };
+        step(k_bl_step<kStart>, 0, nullptr, a.S, 0);
+        for (int i = 0; i + 1 < m; i++) step(k_bl_step<kFirst>, i, a.Y, a.S, i + 1);
+        step(k_bl_step<kLast>, m - 1, a.Y, a.Y, m - 1);
+        for (int i = m - 1; i >= 0; i--) step(k_bl_step<kSecond>, i, a.S, i > 0 ? a.Y : nullptr, i - 1);
         MAPPG_CUDA(cudaGetLastError());
     };
 
