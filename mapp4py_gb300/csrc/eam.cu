@@ -1,5 +1,9 @@
-// FP64 EAM kernels over the full neighbour list (the plain path), and the
-// launch dispatch for both precisions (the mixed kernels are in eam32.cu).
+// FP64 EAM kernels over the full neighbour list, and the launch dispatch for
+// both precisions (the mixed kernels are in eam32.cu).  FP64 single cells take
+// the passes of pair64.cu, which compute a pair once; those here serve
+// batches, mixed systems where they want FP64 (line-search energies, forces
+// near convergence), caller-provided scratch, and systems whose pair records
+// do not fit in memory.
 //
 // The reference (ForceFieldEAM::__force_calc, ff_eam.cpp:65-240) walks a half
 // list twice and scatters to both atoms of a pair.  Here every atom owns a
@@ -34,8 +38,8 @@ namespace mappg {
 __device__ __forceinline__ double spl_val(const Dbl4& c, double p) { return ((c.w * p + c.z) * p + c.y) * p + c.x; }
 __device__ __forceinline__ double spl_der(const Dbl4& c, double p) { return (3.0 * c.w * p + 2.0 * c.z) * p + c.y; }
 
-// batch: atom i's position and image flags from its cell's bins; image
-// shifts n*H from the cell's box
+// a batch's atoms of any cell: atom i's position and image flags from its
+// cell's bins; image shifts n*H from the cell's box
 struct PosCell {
     double x, y, z;
     int lo[3], hi[3];
@@ -60,13 +64,17 @@ struct PosCell {
         const int n0 = (d0 < 0 && lo[0]) ? -1 : ((d0 > 0 && hi[0]) ? 1 : 0);
         const int n1 = (d1 < 0 && lo[1]) ? -1 : ((d1 > 0 && hi[1]) ? 1 : 0);
         const int n2 = (d2 < 0 && lo[2]) ? -1 : ((d2 > 0 && hi[2]) ? 1 : 0);
-        // rows of H: (h0,0,0), (h1,h3,0), (h2,h4,h5)
-        const double s0 = n0 * h6[0] + n1 * h6[1] + n2 * h6[2];
-        const double s1 = n1 * h6[3] + n2 * h6[4];
-        const double s2 = n2 * h6[5];
-        dx = x - (__ldg(a.x + j) + s0);
-        dy = y - (__ldg(a.x + a.n + j) + s1);
-        dz = z - (__ldg(a.x + 2 * a.n + j) + s2);
+        double xj = __ldg(a.x + j), yj = __ldg(a.x + a.n + j), zj = __ldg(a.x + 2 * a.n + j);
+        // most pairs reach no image: a dozen FP64 operations and conversions less
+        if ((n0 | n1 | n2) != 0) {
+            // rows of H: (h0,0,0), (h1,h3,0), (h2,h4,h5)
+            xj += n0 * h6[0] + n1 * h6[1] + n2 * h6[2];
+            yj += n1 * h6[3] + n2 * h6[4];
+            zj += n2 * h6[5];
+        }
+        dx = x - xj;
+        dy = y - yj;
+        dz = z - zj;
     }
 };
 
@@ -91,9 +99,9 @@ __device__ __forceinline__ double density64_lane(const EamArgs& a, const Smem64&
         double dx, dy, dz;
         P.delta(a, S.sh, e, dx, dy, dz);
         double rsq = dx * dx + dy * dy + dz * dz;
-        if (rsq < S.cut_sq[ei * a.ne + ej]) {
+        if (below(rsq, S.cut_sq[ei * a.ne + ej])) {
             double p;
-            int m = knot64(sqrt(rsq), a, p);
+            const int m = knot64_fast(rsq > 0.0 ? rsq * recip_root(rsq) : 0.0, a.dr_inv, a.nr - 2, p);
             acc += spl_val(ldg4(a.rho64 + (size_t)(ej * a.ne + ei * a.rho_ei) * a.nr + m), p);
         }
     }
@@ -114,21 +122,21 @@ __device__ __forceinline__ void force64_lane(const EamArgs& a, const Smem64& S, 
         double dx, dy, dz;
         P.delta(a, S.sh, e, dx, dy, dz);
         double rsq = dx * dx + dy * dy + dz * dz;
-        if (rsq < S.cut_sq[ei * a.ne + ej]) {
+        if (below(rsq, S.cut_sq[ei * a.ne + ej])) {
             const int j = entry_j(e);
-            // 1/r from the FP64 reciprocal square root and r = rsq/r: one
-            // root instead of a root and a division, within an ulp or two of
-            // sqrt and 1/sqrt (GB300's FP64 pipe bounds this kernel)
-            const double rinv = rsqrt(rsq);
+            // 1/r from the reciprocal square root and r = rsq/r: one root
+            // instead of a root and a division, within an ulp or two of sqrt
+            // and 1/sqrt (GB300's FP64 pipe bounds this kernel)
+            const double rinv = recip_root(rsq);
             const double r = rsq * rinv;
             double p;
-            const int m = knot64(r, a, p);
+            const int m = knot64_fast(r, dri, a.nr - 2, p);
             const double der_i = spl_der(ldg4(a.rho64 + (size_t)(ej * a.ne + ei * a.rho_ei) * a.nr + m), p) * dri;
             double der_j = der_i;
             if (ej != ei) der_j = spl_der(ldg4(a.rho64 + (size_t)(ei * a.ne + ej * a.rho_ei) * a.nr + m), p) * dri;
-            const Dbl4 cz = ldg4(a.rphi64 + (size_t)(ei * a.ne + ej) * a.nr + m);
-            const double z = spl_val(cz, p);
-            const double zp = spl_der(cz, p) * dri;
+            double z, dz_;
+            spl_both(ldg4(a.rphi64 + (size_t)(ei * a.ne + ej) * a.nr + m), p, z, dz_);
+            const double zp = dz_ * dri;
             const double phi = z * rinv;
             const double dphi = (zp - phi) * rinv;
             const double fp = -(dphi + dFi * der_i + __ldg(a.dF + j) * der_j) * rinv;
@@ -145,6 +153,30 @@ __device__ __forceinline__ void force64_lane(const EamArgs& a, const Smem64& S, 
             w[5] += fdz * dz;
         }
     }
+}
+
+// one lane's share of atom i's density (returned) and pair energy
+template <int TPA, class POS>
+__device__ __forceinline__ double energy64_lane(const EamArgs& a, const Smem64& S, const POS& P, int ei, int i,
+                                                int lane, double& ep) {
+    double acc = 0.0;
+    const int nn = __ldg(a.nnbr + i);
+    const int* row = a.nbr + (size_t)i * a.maxnbr;
+    for (int k = lane; k < nn; k += TPA) {
+        const int e = __ldg(row + k);
+        const int ej = entry_elem(e);
+        double dx, dy, dz;
+        P.delta(a, S.sh, e, dx, dy, dz);
+        const double rsq = dx * dx + dy * dy + dz * dz;
+        if (below(rsq, S.cut_sq[ei * a.ne + ej])) {
+            const double rinv = recip_root(rsq);  // as in force64_lane
+            double p;
+            const int m = knot64_fast(rsq * rinv, a.dr_inv, a.nr - 2, p);
+            acc += spl_val(ldg4(a.rho64 + (size_t)(ej * a.ne + ei * a.rho_ei) * a.nr + m), p);
+            ep += spl_val(ldg4(a.rphi64 + (size_t)(ei * a.ne + ej) * a.nr + m), p) * rinv;
+        }
+    }
+    return acc;
 }
 
 template <int TPA>
@@ -190,13 +222,15 @@ __global__ void __launch_bounds__(256) k_density64(EamArgs a) {
 
 // batch: FP64 density per chunk, embedding energy into chunk slot 13
 template <int TPA>
-__global__ void __launch_bounds__(256) k_density64b(EamArgs a, const int* __restrict__ cell_of) {
+__global__ void __launch_bounds__(256) k_density64b(EamArgs a) {
     __shared__ Smem64 S;
     S.fill(a);
     const int lane = threadIdx.x % TPA;
     const int apb = blockDim.x / TPA;
     for (int ch = blockIdx.x; ch < a.nchunk; ch += gridDim.x) {
         if (a.cell_active && !a.cell_active[a.chunk_cell[ch]]) continue;
+        const CellGeo& g = a.cells[a.chunk_cell[ch]];
+        S.fill_cell(g);
         const int lo = a.chunk_begin[ch], hi = a.chunk_begin[ch + 1];
         double eacc = 0.0;
         for (int i0 = lo; i0 < hi; i0 += apb) {
@@ -205,8 +239,8 @@ __global__ void __launch_bounds__(256) k_density64b(EamArgs a, const int* __rest
             double acc = 0.0;
             int ei = 0;
             if (active) {
-                PosCell P;
-                P.load(a, cell_of, i);
+                Pos64 P;
+                P.load(a, i, g.nb);
                 ei = a.elem[i];
                 acc = density64_lane<TPA>(a, S, P, ei, i, lane);
             }
@@ -273,13 +307,15 @@ __global__ void __launch_bounds__(256) k_force64(EamArgs a) {
 
 // batch: FP64 forces per chunk, pair energy and virial into slots 0-6
 template <int TPA>
-__global__ void __launch_bounds__(256) k_force64b(EamArgs a, const int* __restrict__ cell_of) {
+__global__ void __launch_bounds__(256) k_force64b(EamArgs a) {
     __shared__ Smem64 S;
     S.fill(a);
     const int lane = threadIdx.x % TPA;
     const int apb = blockDim.x / TPA;
     for (int ch = blockIdx.x; ch < a.nchunk; ch += gridDim.x) {
         if (a.cell_active && !a.cell_active[a.chunk_cell[ch]]) continue;
+        const CellGeo& g = a.cells[a.chunk_cell[ch]];
+        S.fill_cell(g);
         const int lo = a.chunk_begin[ch], hi = a.chunk_begin[ch + 1];
         double ep = 0;
         double w[6] = {0, 0, 0, 0, 0, 0};
@@ -288,8 +324,8 @@ __global__ void __launch_bounds__(256) k_force64b(EamArgs a, const int* __restri
             const bool active = i < hi;
             double fx = 0, fy = 0, fz = 0;
             if (active) {
-                PosCell P;
-                P.load(a, cell_of, i);
+                Pos64 P;
+                P.load(a, i, g.nb);
                 const int ei = a.elem[i];
                 force64_lane<TPA>(a, S, P, ei, __ldg(a.dF + i), i, lane, fx, fy, fz, ep, w);
             }
@@ -407,22 +443,7 @@ __global__ void __launch_bounds__(256) k_energy64(EamArgs a) {
             Pos64 P;
             P.load(a, i);
             ei = a.elem[i];
-            const int nn = __ldg(a.nnbr + i);
-            const int* row = a.nbr + (size_t)i * a.maxnbr;
-            for (int k = lane; k < nn; k += TPA) {
-                const int e = __ldg(row + k);
-                const int ej = entry_elem(e);
-                double dx, dy, dz;
-                P.delta(a, S.sh, e, dx, dy, dz);
-                double rsq = dx * dx + dy * dy + dz * dz;
-                if (rsq < S.cut_sq[ei * a.ne + ej]) {
-                    const double rinv = rsqrt(rsq);  // as in force64_lane
-                    double p;
-                    const int m = knot64(rsq * rinv, a, p);
-                    acc += spl_val(ldg4(a.rho64 + (size_t)(ej * a.ne + ei * a.rho_ei) * a.nr + m), p);
-                    ep += spl_val(ldg4(a.rphi64 + (size_t)(ei * a.ne + ej) * a.nr + m), p) * rinv;
-                }
-            }
+            acc = energy64_lane<TPA>(a, S, P, ei, i, lane, ep);
         }
 #pragma unroll
         for (int o = TPA / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o, TPA);
@@ -446,13 +467,15 @@ __global__ void __launch_bounds__(256) k_energy64(EamArgs a) {
 // batch: FP64 energy of every cell (the line-search energies of mixed
 // batches), chunk sums into slot 0 of the chunk partials
 template <int TPA>
-__global__ void __launch_bounds__(256) k_energy64b(EamArgs a, const int* __restrict__ cell_of) {
+__global__ void __launch_bounds__(256) k_energy64b(EamArgs a) {
     __shared__ Smem64 S;
     S.fill(a);
     const int lane = threadIdx.x % TPA;
     const int apb = blockDim.x / TPA;
     for (int ch = blockIdx.x; ch < a.nchunk; ch += gridDim.x) {
         if (a.cell_active && !a.cell_active[a.chunk_cell[ch]]) continue;
+        const CellGeo& g = a.cells[a.chunk_cell[ch]];
+        S.fill_cell(g);
         const int lo = a.chunk_begin[ch], hi = a.chunk_begin[ch + 1];
         double ep = 0.0, eacc = 0.0;
         for (int i0 = lo; i0 < hi; i0 += apb) {
@@ -461,25 +484,10 @@ __global__ void __launch_bounds__(256) k_energy64b(EamArgs a, const int* __restr
             double acc = 0.0;
             int ei = 0;
             if (active) {
-                PosCell P;
-                P.load(a, cell_of, i);
+                Pos64 P;
+                P.load(a, i, g.nb);
                 ei = a.elem[i];
-                const int nn = __ldg(a.nnbr + i);
-                const int* row = a.nbr + (size_t)i * a.maxnbr;
-                for (int k = lane; k < nn; k += TPA) {
-                    const int e = __ldg(row + k);
-                    const int ej = entry_elem(e);
-                    double dx, dy, dz;
-                    P.delta(a, nullptr, e, dx, dy, dz);
-                    const double rsq = dx * dx + dy * dy + dz * dz;
-                    if (rsq < S.cut_sq[ei * a.ne + ej]) {
-                        const double rinv = rsqrt(rsq);  // as in force64_lane
-                        double p;
-                        const int m = knot64(rsq * rinv, a, p);
-                        acc += spl_val(ldg4(a.rho64 + (size_t)(ej * a.ne + ei * a.rho_ei) * a.nr + m), p);
-                        ep += spl_val(ldg4(a.rphi64 + (size_t)(ei * a.ne + ej) * a.nr + m), p) * rinv;
-                    }
-                }
+                acc = energy64_lane<TPA>(a, S, P, ei, i, lane, ep);
             }
 #pragma unroll
             for (int o = TPA / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o, TPA);
@@ -512,7 +520,12 @@ void launch_cells_done(mappg_sys* s, const EamArgs& a, int what);  // eam32.cu
 // FP64 batch passes take a block per chunk: a chunk is 50-100 us of FP64
 // work, so the hardware's own assignment of blocks to free SMs beats a fixed
 // share of the chunks per block (10 relaxation steps of 64 cells with 128-atom
-// chunks: 48.5 -> 47.9 ms)
+// chunks: 48.5 -> 47.9 ms).  They are bound by the FP64 pipe: the image shifts
+// of a cell are a table in shared memory (most warps of a batch hold a pair
+// that reaches an image, and forming its shift took 12 operations and
+// conversions), 1/r starts from an FP32 root, the knot is cut out of the
+// mantissa.  330,000 atoms: energy 1.74 -> 1.28 ms, density 1.61 -> 1.17,
+// forces 2.68 -> 2.23; energy of a single cell of 253,000 1.04 -> 0.85.
 
 void launch_density_only(mappg_sys* s) {
     EamArgs a = eam_args(s);
@@ -521,7 +534,7 @@ void launch_density_only(mappg_sys* s) {
         return;
     }
     if (s->ncell > 1) {
-        k_density64b<8><<<s->nchunk, 256, 0, s->stream>>>(a, s->cell_of);
+        k_density64b<8><<<s->nchunk, 256, 0, s->stream>>>(a);
     } else if (s->own_ent) {
         launch_pair_density64(s, a);
     } else {
@@ -561,7 +574,7 @@ void launch_force_only(mappg_sys* s) {
         return;
     }
     if (s->ncell > 1) {
-        k_force64b<8><<<s->nchunk, 256, 0, s->stream>>>(a, s->cell_of);
+        k_force64b<8><<<s->nchunk, 256, 0, s->stream>>>(a);
         MAPPG_CUDA(cudaGetLastError());
         launch_cells_done(s, a, 0);
     } else if (s->own_ent) {
@@ -617,7 +630,7 @@ void preload_force64() {
 void launch_energy64(mappg_sys* s) {
     EamArgs a = eam_args(s);
     if (s->ncell > 1) {
-        k_energy64b<8><<<s->nchunk, 256, 0, s->stream>>>(a, s->cell_of);
+        k_energy64b<8><<<s->nchunk, 256, 0, s->stream>>>(a);
         MAPPG_CUDA(cudaGetLastError());
         launch_cells_done(s, a, 1);
         return;

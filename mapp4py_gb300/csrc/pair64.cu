@@ -35,46 +35,6 @@ __device__ __forceinline__ bool is_outside(double v) {
 
 __device__ __forceinline__ double spl_val(const Dbl4& c, double p) { return fma(fma(fma(c.w, p, c.z), p, c.y), p, c.x); }
 
-// cubic value and derivative (per knot) by Horner's scheme and its synthetic
-// division
-__device__ __forceinline__ void spl_both(const Dbl4& c, double p, double& v, double& d) {
-    const double b2 = fma(c.w, p, c.z), b1 = fma(b2, p, c.y);
-    v = fma(b1, p, c.x);
-    d = fma(fma(c.w, p, b2), p, b1);
-}
-
-// m = min(floor(q), nr-2), p = min(q - m, 1) of q = r/dr: the integer part of
-// a double below 2^20 is the top of its mantissa, cut out and shifted down by
-// integer instructions (an FP64 conversion each way holds the FP64 pipe)
-__device__ __forceinline__ int knot64_fast(double r, double dr_inv, int mmax, double& p) {
-    const double q = r * dr_inv;
-    const int hi = __double2hiint(q), ex = (hi >> 20) - 1023;  // q >= 0
-    if (ex >= 20) {  // beyond any table
-        p = 1.0;
-        return mmax;
-    }
-    const int keep = ex < 0 ? 0 : hi & ~(0xfffff >> ex);
-    int m = ex < 0 ? 0 : ((hi & 0xfffff) | 0x100000) >> (20 - ex);
-    p = q - __hiloint2double(keep, 0);
-    if (m > mmax) {
-        m = mmax;
-        p = 1.0;
-    }
-    return m;
-}
-
-// 1/sqrt(x): the FP32 reciprocal root of x as a start (its bits converted by
-// integer instructions: an FP64 conversion holds the FP64 pipe like an
-// addition), then one step of Halley's method, y + y e (1/2 + 3/8 e) with
-// e = 1 - x y^2 (|e| < 2^-21, so the next term is below 2^-64)
-__device__ __forceinline__ double rsqrt_halley(double x) {
-    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-    const unsigned f = __float_as_uint(rsqrtf(__uint_as_float(((hi - 0x38000000u) << 3) | (lo >> 29))));
-    const double y = __hiloint2double((int)((f >> 3) + 0x38000000u), (int)(f << 29));
-    const double e = fma(-(x * y), y, 1.0);
-    return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
 // ENERGY: the densities and the pair energy only (line-search trials)
 template <int TPA, bool ENERGY>
 __global__ void __launch_bounds__(256) k_pair64(const __grid_constant__ EamArgs a) {
@@ -99,11 +59,8 @@ __global__ void __launch_bounds__(256) k_pair64(const __grid_constant__ EamArgs 
             P.delta(a, S.sh, e, dx, dy, dz);
             const double rsq = dx * dx + dy * dy + dz * dz;
             double2 rho = {__longlong_as_double((long long)kOutside), 0.0};
-            // the comparison of two non-negative doubles by their bits, and a
-            // root that FP32 can start (else the library's)
-            const unsigned long long bits = (unsigned long long)__double_as_longlong(rsq);
-            if (bits < (unsigned long long)__double_as_longlong(S.cut_sq[ei * a.ne + ej])) {
-                const double rinv = bits - 0x3a00000000000000ull < 0x0a00000000000000ull ? rsqrt_halley(rsq) : rsqrt(rsq);
+            if (below(rsq, S.cut_sq[ei * a.ne + ej])) {
+                const double rinv = recip_root(rsq);
                 double p;
                 const int m = knot64_fast(rsq * rinv, dri, a.nr - 2, p);
                 if (ENERGY) {

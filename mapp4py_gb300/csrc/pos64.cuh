@@ -10,7 +10,9 @@ namespace mappg {
 struct Pos64 {
     double x, y, z;
     int lo[3], hi[3];
-    __device__ __forceinline__ void load(const EamArgs& a, int i) {
+    __device__ __forceinline__ void load(const EamArgs& a, int i) { load(a, i, a.nb); }
+    // nb: the bins of the atom's cell
+    __device__ __forceinline__ void load(const EamArgs& a, int i, const int* nb) {
         x = a.x[i];
         y = a.x[a.n + i];
         z = a.x[2 * a.n + i];
@@ -19,7 +21,7 @@ struct Pos64 {
 #pragma unroll
         for (int d = 0; d < 3; d++) {
             lo[d] = b[d] == 0;
-            hi[d] = b[d] == a.nb[d] - 1;
+            hi[d] = b[d] == nb[d] - 1;
         }
     }
     // dx = x_i - (x_j + n*H)
@@ -44,9 +46,71 @@ struct Pos64 {
     }
 };
 
+// cubic value and derivative (per knot) by Horner's scheme and its synthetic
+// division
+__device__ __forceinline__ void spl_both(const Dbl4& c, double p, double& v, double& d) {
+    const double b2 = fma(c.w, p, c.z), b1 = fma(b2, p, c.y);
+    v = fma(b1, p, c.x);
+    d = fma(fma(c.w, p, b2), p, b1);
+}
+
+// m = min(floor(q), nr-2), p = min(q - m, 1) of q = r/dr: the integer part of
+// a double below 2^20 is the top of its mantissa, cut out and shifted down by
+// integer instructions (an FP64 conversion each way holds the FP64 pipe)
+__device__ __forceinline__ int knot64_fast(double r, double dr_inv, int mmax, double& p) {
+    const double q = r * dr_inv;
+    const int hi = __double2hiint(q), ex = (hi >> 20) - 1023;  // q >= 0
+    if (ex >= 20) {  // beyond any table
+        p = 1.0;
+        return mmax;
+    }
+    const int keep = ex < 0 ? 0 : hi & ~(0xfffff >> ex);
+    int m = ex < 0 ? 0 : ((hi & 0xfffff) | 0x100000) >> (20 - ex);
+    p = q - __hiloint2double(keep, 0);
+    if (m > mmax) {
+        m = mmax;
+        p = 1.0;
+    }
+    return m;
+}
+
+// 1/sqrt(x): the FP32 reciprocal root of x as a start (its bits converted by
+// integer instructions: an FP64 conversion holds the FP64 pipe like an
+// addition), then one step of Halley's method, y + y e (1/2 + 3/8 e) with
+// e = 1 - x y^2 (|e| < 2^-21, so the next term is below 2^-64)
+__device__ __forceinline__ double rsqrt_halley(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const unsigned f = __float_as_uint(rsqrtf(__uint_as_float(((hi - 0x38000000u) << 3) | (lo >> 29))));
+    const double y = __hiloint2double((int)((f >> 3) + 0x38000000u), (int)(f << 29));
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// the same where FP32 can start it, else the library's
+__device__ __forceinline__ double recip_root(double x) {
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
+    return bits - 0x3a00000000000000ull < 0x0a00000000000000ull ? rsqrt_halley(x) : rsqrt(x);
+}
+
+// x < y of two non-negative doubles by their bits (NaN is not below)
+__device__ __forceinline__ bool below(double x, double y) {
+    return (unsigned long long)__double_as_longlong(x) < (unsigned long long)__double_as_longlong(y);
+}
+
 struct Smem64 {
     double sh[27][3];
     double cut_sq[kMaxElem * kMaxElem];
+    // batch: the shifts n*H of one cell (called by the whole block, after fill)
+    __device__ void fill_cell(const CellGeo& g) {
+        const double* h = g.h6;  // rows of H: (h0,0,0), (h1,h3,0), (h2,h4,h5)
+        for (int t = threadIdx.x; t < 27; t += blockDim.x) {
+            const int n0 = t % 3 - 1, n1 = (t / 3) % 3 - 1, n2 = t / 9 - 1;
+            sh[t][0] = n0 * h[0] + n1 * h[1] + n2 * h[2];
+            sh[t][1] = n1 * h[3] + n2 * h[4];
+            sh[t][2] = n2 * h[5];
+        }
+        __syncthreads();
+    }
     __device__ void fill(const EamArgs& a) {
         for (int t = threadIdx.x; t < 27; t += blockDim.x) {
             sh[t][0] = a.shift[t][0];
