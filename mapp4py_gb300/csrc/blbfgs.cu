@@ -121,6 +121,37 @@ __device__ __forceinline__ double bl_cell_total(const BlArgs& a, int c, int k, b
     return t;
 }
 
+// the sum of 256 threads' values in the first warp (every lane): the tree of
+// bl_store's sum, by one warp instead of all (17 FP64 additions of a warp
+// instead of 48: the FP64 pipe takes 16 clocks for one)
+__device__ __forceinline__ double bl_tree_sum(const double* v) {
+    const int lane = threadIdx.x & 31;
+    // level 1 of the eight rows of 32: rows lane/16 + 2k, column lane % 16
+    double a[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const double* r = v + ((lane >> 4) + 2 * k) * 32 + (lane & 15);
+        a[k] = r[0] + r[16];
+    }
+    // levels 2 and 3 halve the values a lane holds
+#pragma unroll
+    for (int h = 2, o = 8; h > 0; h >>= 1, o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int k = 0; k < h; k++) {
+            const double give = up ? a[k] : a[k + h], keep = up ? a[k + h] : a[k];
+            a[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    a[0] += __shfl_xor_sync(0xffffffffu, a[0], 2);
+    a[0] += __shfl_xor_sync(0xffffffffu, a[0], 1);
+    // the rows' sums one by one
+    double t = 0.0;
+#pragma unroll
+    for (int q = 0; q < 8; q++) t += __shfl_sync(0xffffffffu, a[0], (q & 1) * 16 + (q >> 2) * 8 + ((q >> 1) & 1) * 4);
+    return t;
+}
+
 // One step of the recursion for the cells in `st`, chunk by chunk:
 //   kStart: h = f (and x0 = x, f0 = f in a search's first direction)
 //   kFirst: alpha_i = -rho_i (S_i.h), h += alpha_i Y_i
@@ -129,17 +160,19 @@ __device__ __forceinline__ double bl_cell_total(const BlArgs& a, int c, int k, b
 //   kSecond: h += (-alpha_i - rho_i (Y_i.h)) S_i
 // then the chunk's part of the next step's dot product, Vn[slot(i_next)].h
 // (none with Vn null), into dot_out.  The dot product of this step is the sum
-// of dot_in over the cell's chunks, which every warp forms for itself while
-// its loads are on their way: the chunks of a cell are few, and a kernel
-// between the steps for it cost more than the sum.  Bound by the history,
-// which the steps of a batch read from DRAM (330,000 atoms, m = 10: 160 MB).
-// 44 launches a direction before (9.5 us a step, 3.4 a sum), 21 now.
+// of dot_in over the cell's chunks, which the first warp forms while the
+// block's loads are on their way: the chunks of a cell are few, and a kernel
+// between the steps for it cost more than the sum.  Bound by the FP64 pipe
+// (two operations a component and the sums) and by the history, which the
+// steps of a batch read from DRAM (330,000 atoms, m = 10: 160 MB).  44
+// launches a direction before (9.5 us a step, 3.4 a sum), 21 now.
 enum BlMode { kStart, kFirst, kLast, kSecond };
 
 template <int MODE>
 __global__ void __launch_bounds__(256) k_bl_step(BlArgs a, int st, int i, bool diag, const double* __restrict__ Vu,
                                                  const double* __restrict__ Vn, int i_next) {
     dep_wait();
+    __shared__ double s_coef, s_acc[256];
     const int n = a.n, lane = threadIdx.x & 31;
     const size_t N3 = 3 * (size_t)n;
     for (int ch = blockIdx.x; ch < a.nchunk; ch += gridDim.x) {
@@ -162,16 +195,21 @@ __global__ void __launch_bounds__(256) k_bl_step(BlArgs a, int st, int i, bool d
         }
         double coef = 0.0;
         if (use) {
-            double t = 0.0;
-            for (int k = a.cell_chunk[cell] + lane; k < a.cell_chunk[cell + 1]; k += 32) t = t + a.dot_in[k];
+            if (threadIdx.x < 32) {
+                double t = 0.0;
+                for (int k = a.cell_chunk[cell] + lane; k < a.cell_chunk[cell + 1]; k += 32) t = t + a.dot_in[k];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) t = t + __shfl_xor_sync(0xffffffffu, t, o);
-            if (MODE == kSecond) {
-                coef = -c.alpha[i] - c.rho[su] * t;
-            } else {
-                coef = -c.rho[su] * t;
-                if (ch == a.cell_chunk[cell] && threadIdx.x == 0) c.alpha[i] = coef;
+                for (int o = 16; o > 0; o >>= 1) t = t + __shfl_xor_sync(0xffffffffu, t, o);
+                if (MODE == kSecond) {
+                    coef = -c.alpha[i] - c.rho[su] * t;
+                } else {
+                    coef = -c.rho[su] * t;
+                    if (ch == a.cell_chunk[cell] && lane == 0) c.alpha[i] = coef;
+                }
+                if (lane == 0) s_coef = coef;
             }
+            __syncthreads();
+            coef = s_coef;
         }
         double acc = 0.0;
         if (ii < end) {
@@ -193,9 +231,15 @@ __global__ void __launch_bounds__(256) k_bl_step(BlArgs a, int st, int i, bool d
                 if (dot_on) acc += w[q] * hv[q];
             }
         }
-        const double v[1] = {acc};
-        const int op[1] = {0};
-        bl_store<1>(v, op, a.dot_out + ch);
+        if (dot_on) {
+            s_acc[threadIdx.x] = acc;
+            __syncthreads();
+            if (threadIdx.x < 32) {
+                const double t = bl_tree_sum(s_acc);
+                if (lane == 0) a.dot_out[ch] = t;
+            }
+        }
+        if (ch + gridDim.x < a.nchunk) __syncthreads();  // s_coef and s_acc are used again
     }
 }
 
