@@ -38,54 +38,6 @@ namespace mappg {
 __device__ __forceinline__ double spl_val(const Dbl4& c, double p) { return ((c.w * p + c.z) * p + c.y) * p + c.x; }
 __device__ __forceinline__ double spl_der(const Dbl4& c, double p) { return (3.0 * c.w * p + 2.0 * c.z) * p + c.y; }
 
-// a batch's atoms of any cell: atom i's position and image flags from its
-// cell's bins; image shifts n*H from the cell's box
-struct PosCell {
-    double x, y, z;
-    int lo[3], hi[3];
-    double h6[6];
-    __device__ __forceinline__ void load(const EamArgs& a, const int* cell_of, int i) {
-        const CellGeo& g = a.cells[cell_of[i]];
-        x = a.x[i];
-        y = a.x[a.n + i];
-        z = a.x[2 * a.n + i];
-        const int bc = a.binc[i];
-        const int b[3] = {bc & 1023, (bc >> 10) & 1023, (bc >> 20) & 1023};
-        for (int d = 0; d < 3; d++) {
-            lo[d] = b[d] == 0;
-            hi[d] = b[d] == g.nb[d] - 1;
-        }
-        for (int k = 0; k < 6; k++) h6[k] = g.h6[k];
-    }
-    __device__ __forceinline__ void delta(const EamArgs& a, const double (*)[3], int e, double& dx, double& dy,
-                                          double& dz) const {
-        const int j = entry_j(e);
-        const int d0 = entry_step(e, 0), d1 = entry_step(e, 1), d2 = entry_step(e, 2);
-        const int n0 = (d0 < 0 && lo[0]) ? -1 : ((d0 > 0 && hi[0]) ? 1 : 0);
-        const int n1 = (d1 < 0 && lo[1]) ? -1 : ((d1 > 0 && hi[1]) ? 1 : 0);
-        const int n2 = (d2 < 0 && lo[2]) ? -1 : ((d2 > 0 && hi[2]) ? 1 : 0);
-        double xj = __ldg(a.x + j), yj = __ldg(a.x + a.n + j), zj = __ldg(a.x + 2 * a.n + j);
-        // most pairs reach no image: a dozen FP64 operations and conversions less
-        if ((n0 | n1 | n2) != 0) {
-            // rows of H: (h0,0,0), (h1,h3,0), (h2,h4,h5)
-            xj += n0 * h6[0] + n1 * h6[1] + n2 * h6[2];
-            yj += n1 * h6[3] + n2 * h6[4];
-            zj += n2 * h6[5];
-        }
-        dx = x - xj;
-        dy = y - yj;
-        dz = z - zj;
-    }
-};
-
-__device__ __forceinline__ int knot64(double r, const EamArgs& a, double& p) {
-    p = r * a.dr_inv;
-    int m = min((int)p, a.nr - 2);
-    p -= (double)m;
-    p = fmin(p, 1.0);
-    return m;
-}
-
 // one lane's share of atom i's density (FP64)
 template <int TPA, class POS>
 __device__ __forceinline__ double density64_lane(const EamArgs& a, const Smem64& S, const POS& P, int ei, int i,
@@ -354,18 +306,26 @@ __global__ void __launch_bounds__(256) k_force64b(EamArgs a) {
 constexpr int kDescR = 16;
 constexpr float kDescRc = 5.5f, kDescW = 0.3f;
 
+// a batch: a block per chunk, whose cell's shifts are in shared memory
 template <int TPA, bool BATCH>
-__global__ void __launch_bounds__(256) k_descriptors(EamArgs a, const int* __restrict__ cell_of,
-                                                     float* __restrict__ out) {
+__global__ void __launch_bounds__(256) k_descriptors(EamArgs a, float* __restrict__ out) {
     __shared__ Smem64 S;
     S.fill(a);
     const int lane = threadIdx.x % TPA;
-    const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / TPA;
-    const int stride = (gridDim.x * blockDim.x) / TPA;
+    int gid = (blockIdx.x * blockDim.x + threadIdx.x) / TPA, stride = (gridDim.x * blockDim.x) / TPA, end = a.n;
+    const int* nb = a.nb;
+    if (BATCH) {
+        const CellGeo& cell = a.cells[a.chunk_cell[blockIdx.x]];
+        S.fill_cell(cell);
+        nb = cell.nb;
+        gid = a.chunk_begin[blockIdx.x] + (int)threadIdx.x / TPA;
+        stride = blockDim.x / TPA;
+        end = a.chunk_begin[blockIdx.x + 1];
+    }
     const float inv2w2 = 1.f / (2.f * kDescW * kDescW);
     for (int base = 0;; base += stride) {
         const int i = gid + base;
-        const bool active = i < a.n;
+        const bool active = i < end;
         if (!__any_sync(0xffffffffu, active)) break;
         float g[2 * kDescR];
 #pragma unroll
@@ -373,11 +333,7 @@ __global__ void __launch_bounds__(256) k_descriptors(EamArgs a, const int* __res
         double rho = 0.0;
         if (active) {
             Pos64 P;
-            PosCell PC;
-            if (BATCH)
-                PC.load(a, cell_of, i);
-            else
-                P.load(a, i);
+            P.load(a, i, nb);
             const int ei = a.elem[i];
             const int nn = __ldg(a.nnbr + i);
             const int* row = a.nbr + (size_t)i * a.maxnbr;
@@ -385,17 +341,15 @@ __global__ void __launch_bounds__(256) k_descriptors(EamArgs a, const int* __res
                 const int e = __ldg(row + k);
                 const int ej = entry_elem(e);
                 double dx, dy, dz;
-                if (BATCH)
-                    PC.delta(a, nullptr, e, dx, dy, dz);
-                else
-                    P.delta(a, S.sh, e, dx, dy, dz);
+                P.delta(a, S.sh, e, dx, dy, dz);
                 const double rsq = dx * dx + dy * dy + dz * dz;
-                if (rsq < S.cut_sq[ei * a.ne + ej]) {
+                const double rd = rsq > 0.0 ? rsq * recip_root(rsq) : 0.0;
+                if (below(rsq, S.cut_sq[ei * a.ne + ej])) {
                     double p;
-                    const int m = knot64(sqrt(rsq), a, p);
+                    const int m = knot64_fast(rd, a.dr_inv, a.nr - 2, p);
                     rho += spl_val(ldg4(a.rho64 + (size_t)(ej * a.ne + ei * a.rho_ei) * a.nr + m), p);
                 }
-                const float r = (float)sqrt(rsq);
+                const float r = (float)rd;
                 if (r < kDescRc && ej < 2) {
                     const float fc = 0.5f * (1.f + cosf(3.14159265f * r / kDescRc));
 #pragma unroll
@@ -596,9 +550,9 @@ void launch_force(mappg_sys* s) {
 void launch_descriptors(mappg_sys* s, float* out) {
     EamArgs a = eam_args(s);
     if (s->ncell > 1)
-        k_descriptors<8, true><<<grid64<8>(s), 256, 0, s->stream>>>(a, s->cell_of, out);
+        k_descriptors<8, true><<<s->nchunk, 256, 0, s->stream>>>(a, out);
     else
-        k_descriptors<8, false><<<grid64<8>(s), 256, 0, s->stream>>>(a, nullptr, out);
+        k_descriptors<8, false><<<grid64<8>(s), 256, 0, s->stream>>>(a, out);
     MAPPG_CUDA(cudaGetLastError());
 }
 
