@@ -42,52 +42,67 @@ struct LbScal {
 
 constexpr int kLbU = 4;  // components a thread of the vector kernels loads at a time
 
-// h <- h + coef*y, then dot = s.h (s may be null: no dot).  coef is read
-// from the device: mode 0: coef = 0 (plain dot); mode 1: alpha_i =
-// -rho_i*dot_in, stored; mode 2: beta = -alpha_i - rho_i*dot_in; mode 3:
-// coef applies as a scale: h <- gamma*h; mode 4: h <- tau*P*h elementwise
-// with P (passed as y) the learned diagonal initial inverse Hessian and tau
-// its scale from the newest pair
-__global__ void __launch_bounds__(256) k_lb_axpy_dot(int N, double* __restrict__ h, const double* __restrict__ y,
-                                                     const double* __restrict__ s, LbScal* L, int mode, int idx,
-                                                     int dot_in, int dot_out, double* partials, unsigned* counter) {
+// One step of the two-loop recursion, by MODE, then dot = s.h for the next
+// one (s null: none).  Coefficients are read from the device:
+//   kLbStart   h = f, and the iteration's start x0 = x, f0 = f
+//   kLbFirst   alpha_i = -rho_i*dot_in, stored; h += alpha_i*y
+//   kLbLast    kLbFirst, then the initial inverse Hessian (kLbH0)
+//   kLbH0      h *= gamma; with P, the learned diagonal, h *= tau*P
+//              elementwise (tau: its scale from the newest pair)
+//   kLbSecond  h += (-alpha_i - rho_i*dot_in)*y
+// A step is launch, the vectors' traffic and the last block's sum; the start
+// and the scaling had launches of their own before (9.5 us each for 759,000
+// components).
+enum LbMode { kLbStart, kLbFirst, kLbLast, kLbH0, kLbSecond };
+struct LbVec {
+    int N;
+    const double *x, *f;
+    double *xs, *f0, *h;
+    const double* P;
+};
+template <int MODE>
+__global__ void __launch_bounds__(256) k_lb_step(LbVec a, const double* __restrict__ y, const double* __restrict__ s,
+                                                 LbScal* L, int idx, int dot_in, int dot_out, double* partials,
+                                                 unsigned* counter) {
     dep_wait();
+    const int N = a.N;
     double coef = 0.0;
-    if (mode == 1) {
+    if (MODE == kLbFirst || MODE == kLbLast) {
         coef = -L->rho[idx] * L->dot[dot_in];
         if (blockIdx.x == 0 && threadIdx.x == 0) L->alpha[idx] = coef;
-    } else if (mode == 2) {
+    } else if (MODE == kLbSecond) {
         coef = -L->alpha[idx] - L->rho[idx] * L->dot[dot_in];
-    } else if (mode == 3) {
-        coef = L->gamma;
     }
-    const double tau = mode == 4 ? L->tau : 0.0;
+    constexpr bool AXPY = MODE == kLbFirst || MODE == kLbLast || MODE == kLbSecond;
+    constexpr bool H0 = MODE == kLbLast || MODE == kLbH0;
+    const double gamma = H0 ? L->gamma : 0.0, tau = H0 ? L->tau : 0.0;
     double acc = 0.0;
     // kLbU components in flight per thread: their loads are issued together
     // (a thread has ~10 components in all, so the pass is load latency);
     // the products are added in component order
     const int stride = gridDim.x * blockDim.x;
     for (int q0 = blockIdx.x * blockDim.x + threadIdx.x; q0 < N; q0 += kLbU * stride) {
-        double hv[kLbU], yv[kLbU], sv[kLbU];
+        double hv[kLbU], yv[kLbU], sv[kLbU], xv[kLbU];
 #pragma unroll
         for (int u = 0; u < kLbU; u++) {
             const int q = q0 + u * stride;
             const bool in = q < N;
-            hv[u] = in ? h[q] : 0.0;
-            yv[u] = in && y ? y[q] : 0.0;
+            hv[u] = in ? (MODE == kLbStart ? a.f[q] : a.h[q]) : 0.0;
+            yv[u] = in && AXPY ? y[q] : 0.0;
             sv[u] = in && s ? s[q] : 0.0;
+            xv[u] = !in ? 0.0 : MODE == kLbStart ? a.x[q] : H0 && a.P ? a.P[q] : 0.0;
         }
 #pragma unroll
         for (int u = 0; u < kLbU; u++) {
             const int q = q0 + u * stride;
             if (q >= N) break;
-            if (mode == 1 || mode == 2)
-                hv[u] = hv[u] + coef * yv[u];
-            else if (mode == 3)
-                hv[u] = hv[u] * coef;
-            else if (mode == 4)
-                hv[u] = hv[u] * (tau * yv[u]);
-            if (mode) h[q] = hv[u];
+            if (MODE == kLbStart) {
+                a.xs[q] = xv[u];
+                a.f0[q] = hv[u];
+            }
+            if (AXPY) hv[u] = hv[u] + coef * yv[u];
+            if (H0) hv[u] = a.P ? hv[u] * (tau * xv[u]) : hv[u] * gamma;
+            a.h[q] = hv[u];
             if (s) acc += sv[u] * hv[u];
         }
     }
@@ -172,6 +187,32 @@ __global__ void __launch_bounds__(256) k_lb_prep(int N, const double* __restrict
     }
 }
 
+// max|f| alone, into L->fmax (set to zero before): what the tolerance after
+// a force call needs of k_lb_prep (21 us for 759,000 components, 5 this way)
+__global__ void __launch_bounds__(256) k_lb_fmax(int N, const double* __restrict__ f, LbScal* L) {
+    dep_wait();
+    unsigned long long m = 0;
+    const int stride = gridDim.x * blockDim.x;
+    for (int q0 = blockIdx.x * blockDim.x + threadIdx.x; q0 < N; q0 += kLbU * stride) {
+        double fv[kLbU];
+#pragma unroll
+        for (int u = 0; u < kLbU; u++) fv[u] = q0 + u * stride < N ? f[q0 + u * stride] : 0.0;
+#pragma unroll
+        for (int u = 0; u < kLbU; u++) m = RedMaxBits()(m, bits_of_abs(fv[u]));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = RedMaxBits()(m, __shfl_xor_sync(0xffffffffu, m, o));
+    __shared__ unsigned long long red[8];
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x < 8) {
+        m = red[threadIdx.x];
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) m = RedMaxBits()(m, __shfl_xor_sync(0xffu, m, o));
+        if (threadIdx.x == 0) atomicMax((unsigned long long*)&L->fmax, m);
+    }
+}
+
 // max |x - xb| over components into *out (the bits of a non-negative double
 // order as the values do, so an integer maximum of the bits is the maximum)
 __global__ void k_lb_dxmax(int N, const double* __restrict__ x, const double* __restrict__ xb,
@@ -241,15 +282,13 @@ __global__ void k_lb_shift_rho(LbScal* L, int m) {
     for (int i = m - 1; i > 0; i--) L->rho[i] = L->rho[i - 1];
 }
 
-// x0 = x, f0 = f, h = f: the start of an iteration
+// x0 = x, f0 = f: the start of an iteration of the conjugate gradients
 __global__ void k_lb_start(int N, const double* __restrict__ x, const double* __restrict__ f, double* __restrict__ xs,
-                           double* __restrict__ f0, double* __restrict__ h) {
+                           double* __restrict__ f0) {
     dep_wait();
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < N; q += gridDim.x * blockDim.x) {
-        const double fq = f[q];
         xs[q] = x[q];
-        f0[q] = fq;
-        if (h) h[q] = fq;
+        f0[q] = f[q];
     }
 }
 
@@ -468,6 +507,13 @@ void lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_tol, c
         return r;
     };
     double fh, hh, hmax, fmaxv;
+    auto read_fmax = [&]() -> const LbRead* {
+        MAPPG_CUDA(cudaMemsetAsync(&L->fmax, 0, sizeof(double), st));
+        launch_dep(st, k_lb_fmax, grid, 256, 0, N, s->f, L);
+        const LbRead* r = lb_read(s, L);
+        fmaxv = r->prep[3];
+        return r;
+    };
     if (err == LS_S && f_tol > 0.0) {
         MAPPG_CUDA(cudaMemcpyAsync(h, s->f, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
         read_prep(&fh, &hh, &hmax, &fmaxv);
@@ -476,20 +522,20 @@ void lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_tol, c
     // the two-loop recursion (min_l-bfgs.h:148-170) with the initial inverse
     // Hessian gamma*I, or diag(P) when a learned preconditioner is given
     auto two_loop = [&](bool diag) {
-        // first loop: alpha_i = -rho_i (s_i.h); h += alpha_i y_i
-        if (k > 0) launch_dep(st, k_lb_axpy_dot, grid, 256, 0, N, h, nullptr, sv[0], L, 0, 0, 0, 0, part, counter);
-        for (int i = 0; i < k; i++) {
-            const double* nxt = (i + 1 < k) ? sv[i + 1] : nullptr;
-            launch_dep(st, k_lb_axpy_dot, grid, 256, 0, N, h, yv[i], nxt, L, 1, i, i, i + 1, part, counter);
-        }
-        // h *= H0, and the first dot of the second loop y_{k-1}.h
-        launch_dep(st, k_lb_axpy_dot, grid, 256, 0, N, h, diag ? P : nullptr, k > 0 ? yv[k - 1] : nullptr, L,
-                   diag ? 4 : 3, 0, 0, 64, part, counter);
-        for (int i = k - 1; i > -1; i--) {
-            const double* nxt = i > 0 ? yv[i - 1] : nullptr;
-            launch_dep(st, k_lb_axpy_dot, grid, 256, 0, N, h, sv[i], nxt, L, 2, i, 64 + (k - 1 - i), 64 + (k - i),
-                       part, counter);
-        }
+        const LbVec V = {N, s->x, s->f, xs, f0, h, diag ? P : nullptr};
+        auto step = [&](auto kern, const double* y, const double* next, int i, int in, int out) {
+            launch_dep(st, kern, grid, 256, 0, V, y, next, L, i, in, out, part, counter);
+        };
+        step(k_lb_step<kLbStart>, nullptr, k > 0 ? sv[0] : nullptr, 0, 0, 0);
+        // first loop: alpha_i = -rho_i (s_i.h); h += alpha_i y_i; its last
+        // step applies H0 and takes the second loop's first dot, y_{k-1}.h
+        for (int i = 0; i + 1 < k; i++) step(k_lb_step<kLbFirst>, yv[i], sv[i + 1], i, i, i + 1);
+        if (k > 0)
+            step(k_lb_step<kLbLast>, yv[k - 1], yv[k - 1], k - 1, k - 1, 64);
+        else
+            step(k_lb_step<kLbH0>, nullptr, nullptr, 0, 0, 64);
+        for (int i = k - 1; i > -1; i--)
+            step(k_lb_step<kLbSecond>, sv[i], i > 0 ? yv[i - 1] : nullptr, i, 64 + (k - 1 - i), 64 + (k - i));
         MAPPG_CUDA(cudaGetLastError());
     };
     TrialLine line{s, N, grid, xs, h, &n_en, L};
@@ -497,14 +543,12 @@ void lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_tol, c
     int istep = 0;
     for (; err == LS_S; istep++) {
         if (P && s->precond_every > 0 && istep > 0 && istep % s->precond_every == 0) s->precond_refresh();
-        launch_dep(st, k_lb_start, grid_for(s, N, 256), 256, 0, N, s->x, s->f, xs, f0, h);
         two_loop(P != nullptr);
         e_prev = e_curr;
         read_prep(&fh, &hh, &hmax, &fmaxv);
         if (P && fh < 0.0) {
             // a non-descent preconditioned direction: plain L-BFGS instead
             if (n_fallback) (*n_fallback)++;
-            MAPPG_CUDA(cudaMemcpyAsync(h, s->f, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));
             two_loop(false);
             read_prep(&fh, &hh, &hmax, &fmaxv);
         }
@@ -583,8 +627,7 @@ void lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_tol, c
         auto force = [&] {
             launch_force(s);
             sync_forces64(s);
-            if (f_tol > 0.0 && !s->hook) return (const LbRead*)read_prep(&fh, &hh, &hmax, &fmaxv);
-            return (const LbRead*)lb_read(s, nullptr);
+            return f_tol > 0.0 && !s->hook ? read_fmax() : lb_read(s, nullptr);
         };
         const LbRead* r = force();
         if (moved && r->sc.overflow) {
@@ -595,7 +638,7 @@ void lbfgs_run(mappg_sys* s, int m, double e_tol, double max_dx, double f_tol, c
         n_fc++;
         iteration_hook(s, istep);
         if (e_prev - e_curr < e_tol) err = MIN_S_TOLERANCE;
-        if (f_tol > 0.0 && s->hook) read_prep(&fh, &hh, &hmax, &fmaxv);
+        if (f_tol > 0.0 && s->hook) read_fmax();
         if (f_tol > 0.0 && fmaxv < f_tol) err = MIN_S_FTOL;
         if (istep + 1 == nsteps) err = MIN_F_MAX_ITER;
         if (err) continue;
@@ -737,7 +780,7 @@ void cg_run(mappg_sys* s, double e_tol, double max_dx, double f_tol, const LsPar
             err = LS_F_GRAD0;
             continue;
         }
-        launch_dep(st, k_lb_start, grid_for(s, N, 256), 256, 0, N, s->x, s->f, xs, f0, nullptr);
+        launch_dep(st, k_lb_start, grid_for(s, N, 256), 256, 0, N, s->x, s->f, xs, f0);
         e_prev = e_curr;
         read_prep(&fh, &hh, &hmax, &fmaxv);
         if (fh < 0.0) {
