@@ -248,19 +248,26 @@ __global__ void __launch_bounds__(256) k_kick_drift64(MdArgs a) {
     const double fac = a.sc->fac_next;
     double dsum[3] = {0, 0, 0};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        // all loads before the first store, which they could not pass
         const int e = a.elem[i];
         const unsigned b = a.dof ? a.dof[i] : 7u;
+        double vv[3], ff[3], xx[3];
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-            double vv = a.v[c * n + i], ff = a.f[c * n + i], xx = a.x[c * n + i];
+            vv[c] = a.v[c * n + i];
+            ff[c] = a.f[c * n + i];
+            xx[c] = a.x[c * n + i];
+        }
+        const double dtm = a.dtm[e];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
             // a frozen component keeps its velocity and still drifts
             // (update_x_d__x_w_dof, md_nvt.cpp:144-180)
-            if ((b >> c) & 1u) vv = __dadd_rn(__dmul_rn(vv, fac), __dmul_rn(ff, a.dtm[e]));
-            double dx = __dmul_rn(vv, a.dt);
+            if ((b >> c) & 1u) vv[c] = __dadd_rn(__dmul_rn(vv[c], fac), __dmul_rn(ff[c], dtm));
+            double dx = __dmul_rn(vv[c], a.dt);
             dsum[c] = __dadd_rn(dsum[c], dx);
-            xx = __dadd_rn(xx, dx);
-            a.v[c * n + i] = vv;
-            a.x[c * n + i] = xx;
+            a.v[c * n + i] = vv[c];
+            a.x[c * n + i] = __dadd_rn(xx[c], dx);
         }
     }
     __shared__ double t[3];
@@ -279,11 +286,12 @@ __global__ void __launch_bounds__(256) k_com_skin64(MdArgs a) {
     const double c0 = a.sc->com[0], c1 = a.sc->com[1], c2 = a.sc->com[2];
     int moved = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const double b0 = a.x0[i], b1 = a.x0[n + i], b2 = a.x0[2 * n + i];  // before the stores
         double x0 = __dsub_rn(a.x[i], c0), x1 = __dsub_rn(a.x[n + i], c1), x2 = __dsub_rn(a.x[2 * n + i], c2);
         a.x[i] = x0;
         a.x[n + i] = x1;
         a.x[2 * n + i] = x2;
-        double d0 = __dsub_rn(a.x0[i], x0), d1 = __dsub_rn(a.x0[n + i], x1), d2 = __dsub_rn(a.x0[2 * n + i], x2);
+        double d0 = __dsub_rn(b0, x0), d1 = __dsub_rn(b1, x1), d2 = __dsub_rn(b2, x2);
         double r = __dadd_rn(__dmul_rn(d0, d0), __dadd_rn(__dmul_rn(d1, d1), __dmul_rn(d2, d2)));
         moved |= r > a.skin_sq;
     }
@@ -300,16 +308,20 @@ __global__ void __launch_bounds__(256) k_kick2_64(MdArgs a) {
         const int e = a.elem[i];
         const double m = a.masses[e];
         const unsigned b = a.dof ? a.dof[i] : 7u;
-        double vv[3];
+        const double dtm = a.dtm[e];
+        double vv[3], ff[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {  // before the stores
+            vv[c] = a.v[c * n + i];
+            ff[c] = a.f[c * n + i];
+        }
 #pragma unroll
         for (int c = 0; c < 3; c++) {
             // update_x_d_w_dof (md_nvt.cpp:184-215): frozen components are
             // neither kicked nor counted in the kinetic tensor
             if ((b >> c) & 1u) {
-                double v0 = a.v[c * n + i], ff = a.f[c * n + i];
-                v0 = __dadd_rn(v0, __dmul_rn(ff, a.dtm[e]));
-                a.v[c * n + i] = v0;
-                vv[c] = v0;
+                vv[c] = __dadd_rn(vv[c], __dmul_rn(ff[c], dtm));
+                a.v[c * n + i] = vv[c];
             } else {
                 vv[c] = 0.0;
             }
@@ -354,28 +366,33 @@ __global__ void __launch_bounds__(256) k_integrate32(MdArgs a) {
     float dsum0 = 0.f, dsum1 = 0.f, dsum2 = 0.f;
     int moved = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int e = a.elem[i];
-        const float kf = a.dtm32[e] * B;
+        // all loads before the first store, which they could not pass
+        const int e = a.elem[i], bc = a.binc[i];
         const unsigned b = a.dof ? a.dof[i] : 7u;
-        double xv[3];
-        float vf[3];
+        const float4 q = a.p0[i];
+        double xv[3], vv[3];
+        float vf[3], ff[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            vv[c] = a.v[c * n + i];
+            xv[c] = a.x[c * n + i];
+            ff[c] = a.f32[c * n + i];
+        }
+        const float kf = a.dtm32[e] * B;
 #pragma unroll
         for (int c = 0; c < 3; c++) {
             // a frozen component (atoms.x_dof) keeps its velocity and drifts
-            double v = a.v[c * n + i];
-            if ((b >> c) & 1u) v = fma(v, A, (double)(a.f32[c * n + i] * kf));
-            double x = fma(v, a.dt, a.x[c * n + i]);
-            a.v[c * n + i] = v;
-            a.x[c * n + i] = x;
-            xv[c] = x;
-            vf[c] = (float)v;
+            if ((b >> c) & 1u) vv[c] = fma(vv[c], A, (double)(ff[c] * kf));
+            xv[c] = fma(vv[c], a.dt, xv[c]);
+            a.v[c * n + i] = vv[c];
+            a.x[c * n + i] = xv[c];
+            vf[c] = (float)vv[c];
             a.v32[c * n + i] = vf[c];
         }
         dsum0 = fmaf(vf[0], a.dt32, dsum0);
         dsum1 = fmaf(vf[1], a.dt32, dsum1);
         dsum2 = fmaf(vf[2], a.dt32, dsum2);
         // frame position and the skin test against the position at the build
-        const int bc = a.binc[i];
         // the scaled frame; for an orthorhombic box one product per axis
         const double u0 = ORTHO ? a.bs[0] * xv[0] : a.bs[0] * xv[0] + (a.bs[1] * xv[1] + a.bs[2] * xv[2]);
         const double u1 = ORTHO ? a.bs[3] * xv[1] : a.bs[3] * xv[1] + a.bs[4] * xv[2];
@@ -386,7 +403,6 @@ __global__ void __launch_bounds__(256) k_integrate32(MdArgs a) {
         p.z = (float)(u2 - (double)(8 * ((bc >> 20) & 1023)));
         p.w = 0.f;
         a.p32[i] = p;
-        const float4 q = a.p0[i];
         const float da = p.x - q.x, db = p.y - q.y, dc = p.z - q.z;
         float cx, cy, cz;
         if (ORTHO) {
@@ -599,41 +615,49 @@ __global__ void __launch_bounds__(256) k_integrate32b(MdArgs a) {
         const CellGeo& g = a.cells[c];
         const double A = a.cmd[c].kickA;
         const float B = (float)a.cmd[c].kickB;
+        // the cell's frame, read before the loop's stores
+        const bool orth = g.ortho != 0;  // uniform over the chunk
+        const double bs[6] = {g.bs[0], g.bs[1], g.bs[2], g.bs[3], g.bs[4], g.bs[5]};
+        const float G0 = g.G[0][0], G1 = g.G[1][0], G2 = g.G[2][0], G3 = g.G[1][1], G4 = g.G[2][1], G5 = g.G[2][2];
         float dsum0 = 0.f, dsum1 = 0.f, dsum2 = 0.f;
         for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-            const int e = a.elem[i];
-            const float kf = a.dtm32[e] * B;
-            double xv[3];
-            float vf[3];
+            // all loads before the first store, which they could not pass
+            const int e = a.elem[i], bc = a.binc[i];
+            const float4 p0 = a.p0[i];
+            double xv[3], vv[3];
+            float vf[3], ff[3];
 #pragma unroll
             for (int q = 0; q < 3; q++) {
-                double v = fma(a.v[q * n + i], A, (double)(a.f32[q * n + i] * kf));
-                double x = fma(v, a.dt, a.x[q * n + i]);
-                a.v[q * n + i] = v;
-                a.x[q * n + i] = x;
-                xv[q] = x;
-                vf[q] = (float)v;
+                vv[q] = a.v[q * n + i];
+                xv[q] = a.x[q * n + i];
+                ff[q] = a.f32[q * n + i];
+            }
+            const float kf = a.dtm32[e] * B;
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                vv[q] = fma(vv[q], A, (double)(ff[q] * kf));
+                xv[q] = fma(vv[q], a.dt, xv[q]);
+                a.v[q * n + i] = vv[q];
+                a.x[q * n + i] = xv[q];
+                vf[q] = (float)vv[q];
                 a.v32[q * n + i] = vf[q];
             }
             dsum0 = fmaf(vf[0], a.dt32, dsum0);
             dsum1 = fmaf(vf[1], a.dt32, dsum1);
             dsum2 = fmaf(vf[2], a.dt32, dsum2);
-            const int bc = a.binc[i];
-            const bool orth = g.ortho != 0;  // uniform over the chunk
-            const double u0 = orth ? g.bs[0] * xv[0] : g.bs[0] * xv[0] + (g.bs[1] * xv[1] + g.bs[2] * xv[2]);
-            const double u1 = orth ? g.bs[3] * xv[1] : g.bs[3] * xv[1] + g.bs[4] * xv[2];
-            const double u2 = g.bs[5] * xv[2];
+            const double u0 = orth ? bs[0] * xv[0] : bs[0] * xv[0] + (bs[1] * xv[1] + bs[2] * xv[2]);
+            const double u1 = orth ? bs[3] * xv[1] : bs[3] * xv[1] + bs[4] * xv[2];
+            const double u2 = bs[5] * xv[2];
             float4 p;
             p.x = (float)(u0 - (double)(8 * (bc & 1023)));
             p.y = (float)(u1 - (double)(8 * ((bc >> 10) & 1023)));
             p.z = (float)(u2 - (double)(8 * ((bc >> 20) & 1023)));
             p.w = 0.f;
             a.p32[i] = p;
-            const float4 q = a.p0[i];
-            const float da = p.x - q.x, db = p.y - q.y, dc = p.z - q.z;
-            const float cx = da * g.G[0][0] + db * g.G[1][0] + dc * g.G[2][0];
-            const float cy = db * g.G[1][1] + dc * g.G[2][1];
-            const float cz = dc * g.G[2][2];
+            const float da = p.x - p0.x, db = p.y - p0.y, dc = p.z - p0.z;
+            const float cx = da * G0 + db * G1 + dc * G2;
+            const float cy = db * G3 + dc * G4;
+            const float cz = dc * G5;
             moved_ch |= fmaf(cx, cx, fmaf(cy, cy, cz * cz)) > a.skin_sq32;
         }
         // the chunk's cell is rebuilt at the next list check
