@@ -1100,33 +1100,49 @@ __global__ void __launch_bounds__(256) k_de32b(EamArgs a) {
 // virial), 1 after an energy pass, 2 after a force pass with the MD tail
 // (kinetic tensor and the closing half of each cell's chain, thermo rows of
 // pe and T per cell)
-__global__ void k_cells_done(EamArgs a, const int* __restrict__ cell_chunk, CellMd* __restrict__ cmd, int what) {
+template <int WHAT>
+__global__ void __launch_bounds__(256) k_cells_done(EamArgs a, const int* __restrict__ cell_chunk,
+                                                    CellMd* __restrict__ cmd) {
     dep_wait();
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (c >= a.ncell) return;
     const int lo = cell_chunk[c], hi = cell_chunk[c + 1];
-    double t[14];
-#pragma unroll 1
-    for (int k = 0; k < 14; k++) {
+    // all values of a chunk at once, and one reduction for them: the tree of
+    // a butterfly per value (14 of those, each behind its own loads, took
+    // most of 20 us)
+    __shared__ double s_t[8][16];
+    double* t = s_t[w];
+    if (WHAT == 1) {
         double v = 0.0;
-        const bool need = what == 1 ? k == 0 : (what == 0 ? (k <= 6 || k == 13) : true);
-        if (need)
-            for (int ch = lo + lane; ch < hi; ch += 32) v += a.chunk_part[(size_t)ch * kChunkSlots + k];
+        for (int ch = lo + lane; ch < hi; ch += 32) v += a.chunk_part[(size_t)ch * kChunkSlots];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        t[k] = v;
+        if (lane == 0) t[0] = v;
+    } else {
+        double u[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) u[k] = 0.0;
+        for (int ch = lo + lane; ch < hi; ch += 32) {
+            const double* row = a.chunk_part + (size_t)ch * kChunkSlots;
+#pragma unroll
+            for (int k = 0; k < 14; k++)
+                if (WHAT == 2 || k <= 6 || k == 13) u[k] += row[k];
+        }
+        const double r = warp_reduce(u, RedAdd());
+        if (lane % 2 == 0) t[lane / 2] = r;
     }
+    __syncwarp();
     if (lane != 0) return;
     CellMd* m = cmd + c;
-    if (what == 1) {
+    if (WHAT == 1) {
         m->energy = t[0];
         return;
     }
     m->e_embed = t[13];
     m->energy = t[0] + t[13];
     for (int k = 0; k < 6; k++) m->virial[k] = t[1 + k];
-    if (what == 2) {
+    if (WHAT == 2) {
         NhcParams P = a.nhc;
         P.T = m->T;
         P.T_inv = 1.0 / m->T;
@@ -1282,7 +1298,13 @@ static void pick_ortho(bool o, F&& fn) {
 #define MAPPG_FORCE_U (s->unroll_force ? s->unroll_force : s->unroll)
 
 static void cells_done(mappg_sys* s, const EamArgs& a, int what) {
-    launch_dep(s->stream, k_cells_done, (s->ncell * 32 + 255) / 256, 256, 0, a, s->cell_chunk, s->cmd, what);
+    const int grid = (s->ncell * 32 + 255) / 256;
+    if (what == 0)
+        launch_dep(s->stream, k_cells_done<0>, grid, 256, 0, a, s->cell_chunk, s->cmd);
+    else if (what == 1)
+        launch_dep(s->stream, k_cells_done<1>, grid, 256, 0, a, s->cell_chunk, s->cmd);
+    else
+        launch_dep(s->stream, k_cells_done<2>, grid, 256, 0, a, s->cell_chunk, s->cmd);
     MAPPG_CUDA(cudaGetLastError());
 }
 
@@ -1323,7 +1345,7 @@ int force_smem_max_kb(const mappg_sys* s) {
 void launch_force32(mappg_sys* s, const EamArgs& a) {
     if (s->ncell > 1) {
         MAPPG_DISPATCH32U(force_b, all_ortho(s), MAPPG_FORCE_U);
-        cells_done(s, a, 0);
+        if (!a.defer) cells_done(s, a, 0);  // (an MD step's closing call takes these sums with its own)
     } else {
         MAPPG_DISPATCH32U(force_t, a.fr.ortho != 0, MAPPG_FORCE_U);
     }

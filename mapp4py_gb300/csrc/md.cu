@@ -863,6 +863,7 @@ static void launch_step32b(mappg_sys* s, const MdArgs& a) {
     launch_dep(s->stream, k_cells_com, (nc * 32 + 255) / 256, 256, 0, a);
     launch_rebuild_chain(s);
     EamArgs e = eam_args(s);
+    e.defer = 1;
     launch_density32(s, e);
     launch_force32(s, e);
     launch_dep(s->stream, k_ke32b, std::min(s->nchunk, s->sm_count * 8), 256, 0, a);
