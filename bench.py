@@ -29,8 +29,10 @@ METRIC = "EAM MD atom-steps/s"
 N_CELLS = (80, 80, 80)
 T_K = 600.0
 REF_BUDGET_S = 60  # CPU seconds of the reference arm's timed sample
-# kernels in one step's CUDA graph: FP64 step_open, kick_drift, com_skin, 7 rebuild-chain, density,
-# force, kick2; mixed step_open32, integrate32, 7 rebuild-chain, density32, force32, close32
+# kernels in one step's CUDA graph: FP64 kick_drift, com_skin, 6 rebuild-chain (link64 with them),
+# pair64, rho64, gather64, kick2; mixed integrate32, 5 rebuild-chain, density32, force32, close32.
+# Systems of up to 8,192 atoms have 3 fewer (bin_small for wrap, scan, scatter, sort): not the
+# workloads counted here.
 KERNELS_PER_STEP = {"fp64": 12, "mixed": 9}
 # how the sums of the pair terms are carried (the line's dtype in words)
 ACCUMULATION = {

@@ -14,7 +14,8 @@
 //   force       one force pass; per-cell max|F|, tolerances, history update
 // History slots form a ring per cell: the i-th newest pair (s, y) of cell c
 // is slot (head_c - i) mod m.  Per-cell sums come from per-chunk partials
-// (chunks never cross cells) added by one warp per cell in a fixed order.
+// (chunks never cross cells) added by one warp per cell in a fixed order; the
+// recursion's by the first warp of each chunk that needs them.
 #include <math.h>
 #include <string.h>
 

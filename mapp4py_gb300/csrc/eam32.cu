@@ -1096,7 +1096,7 @@ __global__ void __launch_bounds__(256) k_de32b(EamArgs a) {
 }
 
 // per-cell totals of a batch from the chunk slots, one warp per cell in a
-// fixed order: what = 0 after a force pass (energy = pair + embedding,
+// fixed order: WHAT = 0 after a force pass (energy = pair + embedding,
 // virial), 1 after an energy pass, 2 after a force pass with the MD tail
 // (kinetic tensor and the closing half of each cell's chain, thermo rows of
 // pe and T per cell)

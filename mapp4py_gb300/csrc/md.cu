@@ -12,9 +12,10 @@
 //   k_com_skin64     x -= mean displacement; skin test (DynamicMD::decide,
 //                    dynamic_md.cpp:90-105) opens the rebuild gate
 //   rebuild chain    (system.cu) only when the gate is open
-//   density, force   (eam.cu)
+//   density, force   (pair64.cu, or eam.cu over full rows)
 //   k_kick2_64       v += f*dt2/m, kinetic tensor (update_x_d,
-//                    md_nvt.cpp:106-128), closing thermostat half, thermo
+//                    md_nvt.cpp:106-128), the force call's energy and virial
+//                    from its partial sums, closing thermostat half, thermo
 //                    row, and the next step's opening half
 //
 // Mixed path (FP64 state, fewer FP64 instructions; GB300 runs FP64 at a
@@ -29,7 +30,8 @@
 //                    at the end of the run (a uniform shift leaves forces and
 //                    energies unchanged)
 //   rebuild chain, k_density32, k_force32
-//   k_close32        kinetic tensor of v + f dt/2m, closing half, thermo row,
+//   k_close32        kinetic tensor of v + f dt/2m, the force call's energy and
+//                    virial from its partial sums, closing half, thermo row,
 //                    the next step's opening half
 // Velocity scaling stays lazy as in the reference: the chain's factor is
 // folded into the next kick and applied at the end of the run

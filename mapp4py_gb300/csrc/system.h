@@ -81,7 +81,7 @@ struct DevScalars {
     int pending_kick;  // mixed MD: v still lacks the closing half kick
     unsigned counter[8];  // last-block-done counters, one per reduction site
     double energy;     // last force/energy call
-    double e_embed;    // embedding energy of the last mixed density pass
+    double e_embed;    // embedding energy of the last FP64 density pass over full rows
     double de;         // last energy difference of a line-search trial (k_de32)
     double virial[6];  // F_H voigt
     double com[3];     // mean displacement of the step
