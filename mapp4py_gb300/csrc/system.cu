@@ -693,6 +693,7 @@ __device__ __noinline__ float frame_r2(const BuildArgs& a, const CellGeo* cg, in
 }
 
 constexpr int kBuildWarps = 4;    // warps of a builder block
+constexpr int kBuildWide = 8;     // the same for systems of few bins
 constexpr int kBuildTile = 768;   // candidates staged at a time (12 KB)
 constexpr int kBuildHome = 32;    // atoms of the bin worked on at a time
 constexpr int kBuildRow = 256;    // longest row put together on chip
@@ -709,10 +710,10 @@ struct BuildCut {
     __device__ __forceinline__ float in(int e) const { return UNI ? in2 : tab[2 * kMaxElem * kMaxElem + e]; }
 };
 
-// the candidates within reach2 (squared) of each of the A atoms h[0..A-1], by
+// the candidates within reach2 (squared) of each of the A atoms q0, q0 + W, ... of home, by
 // their place in cand and in its order, into hits[u]; nh[u] of them (those
 // beyond kBuildHits are not noted)
-template <int A>
+template <int A, int W>
 __device__ __forceinline__ void build_hits(const float4* cand, int nt, const float4* home, int q0, int ng, float reach2,
                                            uint16_t (*hits)[kBuildHits], int* nh) {
     const int lane = threadIdx.x & 31;
@@ -721,7 +722,7 @@ __device__ __forceinline__ void build_hits(const float4* cand, int nt, const flo
     int c[A];
 #pragma unroll
     for (int u = 0; u < A; u++) {
-        const float4 h = home[min(q0 + u * kBuildWarps, ng - 1)];
+        const float4 h = home[min(q0 + u * W, ng - 1)];
         hx[u] = h.x;
         hy[u] = h.y;
         hz[u] = h.z;
@@ -819,27 +820,28 @@ __device__ __forceinline__ void build_scan(const BuildArgs& a, const BuildCut<UN
 // instructions an atom).  The atom's counters are uniform in its warp.  With
 // every step of 32 candidates taking the full set of tests the pass had 1,000
 // instructions an atom; the noting step has 14 for one atom, and a candidate
-// read from shared memory serves four.  Four warps a block: eight are faster
-// below 10,000 atoms (25 instead of 29 us at 4,000) and slower above (598
-// instead of 545 at 500,000).
+// read from shared memory serves four.  Four warps a block; eight where the
+// bins are few (the whole rebuild 21.9 instead of 29.6 us at 4,000 atoms, 16.5
+// instead of 21.5 at 500, 34 instead of 47 at 8,788; at 500,000 598 instead of
+// 545).
 // Whole rebuild (all its kernels) as this kernel was first built (one warp
 // per bin, candidates in the outer loop), with a block a bin and direct
-// tests, and now: 4,000 atoms 129, 35 and 29 us; 32,000 164, 60 and 49;
+// tests, and now: 4,000 atoms 129, 35 and 22 us; 32,000 164, 60 and 49;
 // 256,000 509, 339 and 286; 500,000 905, 650 and 545.
 // ORTHO: every cell orthorhombic (one product per axis to Cartesian).
 // UNI: every pair type has the same list cutoff (thresholds in registers).
-template <bool BATCH, bool ORTHO, bool UNI>
-__global__ void __launch_bounds__(32 * kBuildWarps) k_build_bins(const __grid_constant__ BuildArgs a, int nbins,
+template <bool BATCH, bool ORTHO, bool UNI, int W>
+__global__ void __launch_bounds__(32 * W) k_build_bins(const __grid_constant__ BuildArgs a, int nbins,
                                                                  DevScalars* sc) {
     dep_wait();
     if (!sc->rebuild) return;
     __shared__ float4 cand[kBuildTile], home[kBuildHome];
     __shared__ int s_pre[33], s_lo[32], s_cin[kBuildHome], s_cout[kBuildHome], s_geo[6];
-    __shared__ int s_row[kBuildWarps][kBuildRow], s_nh[kBuildWarps][kBuildAtoms];
-    __shared__ uint16_t s_hits[kBuildWarps][kBuildAtoms][kBuildHits];
+    __shared__ int s_row[W][kBuildRow], s_nh[W][kBuildAtoms];
+    __shared__ uint16_t s_hits[W][kBuildAtoms][kBuildHits];
     __shared__ float s_cut[UNI ? 1 : 3 * kMaxElem * kMaxElem];
     if (!UNI)
-        for (int t = threadIdx.x; t < a.ne * a.ne; t += 32 * kBuildWarps) {
+        for (int t = threadIdx.x; t < a.ne * a.ne; t += 32 * W) {
             s_cut[t] = a.lo2[t];
             s_cut[kMaxElem * kMaxElem + t] = a.hi2[t];
             s_cut[2 * kMaxElem * kMaxElem + t] = a.in2[t];
@@ -919,7 +921,7 @@ __global__ void __launch_bounds__(32 * kBuildWarps) k_build_bins(const __grid_co
                 const bool last = t0 + kBuildTile >= total;
                 if (t0) __syncthreads();  // the previous tile is no longer read
                 if (!one_tile || g0 == 0)
-                    for (int k = threadIdx.x; k < ((nt + 31) & ~31); k += 32 * kBuildWarps) {
+                    for (int k = threadIdx.x; k < ((nt + 31) & ~31); k += 32 * W) {
                         float4 p = make_float4(1e18f, 0.f, 0.f, 0.f);
                         if (k < nt) {
                             const int t = t0 + k;
@@ -937,15 +939,15 @@ __global__ void __launch_bounds__(32 * kBuildWarps) k_build_bins(const __grid_co
                         cand[k] = p;
                     }
                 __syncthreads();
-                for (int q = w, u = 0; q < ng; q += kBuildWarps, u = (u + 1) % kBuildAtoms) {
+                for (int q = w, u = 0; q < ng; q += W, u = (u + 1) % kBuildAtoms) {
                     if (one_tile && u == 0) {
-                        const int more = (ng - 1 - q) / kBuildWarps;  // atoms of the warp after this one
+                        const int more = (ng - 1 - q) / W;  // atoms of the warp after this one
                         if (more >= 2)
-                            build_hits<4>(cand, nt, home, q, ng, a.hi2max, s_hits[w], s_nh[w]);
+                            build_hits<4, W>(cand, nt, home, q, ng, a.hi2max, s_hits[w], s_nh[w]);
                         else if (more)
-                            build_hits<2>(cand, nt, home, q, ng, a.hi2max, s_hits[w], s_nh[w]);
+                            build_hits<2, W>(cand, nt, home, q, ng, a.hi2max, s_hits[w], s_nh[w]);
                         else
-                            build_hits<1>(cand, nt, home, q, ng, a.hi2max, s_hits[w], s_nh[w]);
+                            build_hits<1, W>(cand, nt, home, q, ng, a.hi2max, s_hits[w], s_nh[w]);
                         __syncwarp();
                     }
                     const float4 h = home[q];
@@ -1206,14 +1208,23 @@ void launch_rebuild_chain(mappg_sys* s) {
     a.cell_reb = reb;
     bool uni = true;
     for (int p = 1; p < s->ne * s->ne; p++) uni = uni && a.lo2[p] == a.lo2[0] && a.hi2[p] == a.hi2[0];
-    auto launch = [&](auto BT, auto OT, auto UT) {
-        constexpr auto kern = k_build_bins<decltype(BT)::value, decltype(OT)::value, decltype(UT)::value>;
+    auto launch_w = [&](auto BT, auto OT, auto UT, auto WT) {
+        constexpr int W = decltype(WT)::value;
+        constexpr auto kern = k_build_bins<decltype(BT)::value, decltype(OT)::value, decltype(UT)::value, W>;
         static int per_sm = 0;
         if (!per_sm) {
-            MAPPG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kBuildWarps, 0));
+            MAPPG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * W, 0));
             per_sm = std::max(per_sm, 1);
         }
-        launch_dep(s->stream, kern, std::min(s->nbins, per_sm * s->sm_count), 32 * kBuildWarps, 0, a, s->nbins, s->sc);
+        launch_dep(s->stream, kern, std::min(s->nbins, per_sm * s->sm_count), 32 * W, 0, a, s->nbins, s->sc);
+    };
+    // few bins: every block is on the chip at once and a bin's atoms in turn
+    // are what the pass waits for, so eight warps share them
+    auto launch = [&](auto BT, auto OT, auto UT) {
+        if (!decltype(BT)::value && s->nbins <= 3 * s->sm_count)
+            launch_w(std::false_type(), OT, UT, std::integral_constant<int, kBuildWide>());
+        else
+            launch_w(BT, OT, UT, std::integral_constant<int, kBuildWarps>());
     };
     auto by_uni = [&](auto BT, auto OT) {
         if (uni)

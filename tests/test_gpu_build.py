@@ -113,3 +113,18 @@ def test_neighbor_sets_where_binning_changes_kernels(potentials, n, bins):
         o.init_dynamic()
         assert np.array_equal(keys(*s.neighbors()), keys(*o.neighbors()))
         x = rng.random((n, 3)) @ H
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 161, 300, 900])
+def test_neighbor_sets_of_a_crowded_bin_among_many(potentials, n):
+    """The same edges where the bins are many and a block has fewer warps:
+    900 atoms in one bin need several tiles of candidates."""
+    path, _ = potentials[("A", "B")]
+    rng = np.random.default_rng(n)
+    x = np.concatenate([20.0 + rng.uniform(-1.4, 1.4, (n, 3)), rng.random((300, 3)) * 50.0])
+    H, elem = np.diag([50.0, 50.5, 51.0]), (rng.random(n + 300) < 0.5).astype(np.uint8)
+    o = O.System(O.Eam.setfl(path), H, x, elem, [synth.MASS, synth.MASS], skin=0.5, pair_wise=False)
+    o.init_dynamic()
+    s = _lib.System(_lib.ForceField.setfl(path), H, x, elem, [synth.MASS, synth.MASS], skin=0.5, precision=_lib.MIXED)
+    s.build()
+    assert np.array_equal(keys(*s.neighbors()), keys(*o.neighbors()))
