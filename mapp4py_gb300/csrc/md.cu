@@ -225,10 +225,13 @@ __device__ __forceinline__ bool close_partials(const T (&v)[K], const MdArgs& a,
     return last_block(counter);
 }
 
-// run start: thermo row 0, no pending velocity scale or kick, the first
-// step's opening half
+// run start (one block): no displacement sums yet (a list build before the
+// first step reads them), thermo row 0, no pending velocity scale or kick, the
+// first step's opening half
 __global__ void k_run_begin(MdArgs a) {
     dep_wait();
+    for (int q = threadIdx.x; q < 3 * a.drift_rows; q += blockDim.x) a.partials[(q / 3) * kRedSlots + 8 + q % 3] = 0.0;
+    if (threadIdx.x != 0) return;
     DevScalars* sc = a.sc;
     write_thermo_row(a.thermo, sc, 0);
     double eta[kMaxChain];
@@ -1014,8 +1017,8 @@ void nvt_begin(mappg_sys* s, double T, double dt, double kB, double t_relax, int
     // them on the side stream (nvt_run_host) overlaps them and is joined here
     sys_join_side(s);
     launch_dep(s->stream, k_mvv_init, md_shape(s, true).grid, md_shape(s, true).block, 0, a);
-    launch_dep(s->stream, k_run_begin, 1, 1, 0, a);
     if (s->precision == MAPPG_MIXED) s->drift_rows = a.drift_rows = md_shape(s, true).grid;
+    launch_dep(s->stream, k_run_begin, 1, 256, 0, a);
     MAPPG_CUDA(cudaGetLastError());
     if (nsteps < kGraphMinSteps) return;  // nvt_steps launches the kernels itself
     MAPPG_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
