@@ -264,24 +264,27 @@ int mappg_nvt_snapshot(mappg_sys* sys, double* x, double* x_d);
 int mappg_sys_stream(mappg_sys* sys, void** stream);
 int mappg_sys_sync(mappg_sys* sys);
 
-/* Choose the lanes per atom (4, 8 or 16; 256/lanes atoms per block) and the
- * neighbour entries per loop step (1 or 2, mixed kernels) of the density and
- * force kernels by timing them on this system's atoms and neighbour list;
+/* Choose the lanes per atom (4, 8, 16 or 32; 256/lanes atoms per block) and
+ * the neighbour entries per loop step (1 or 2, mixed kernels) of the density
+ * and force kernels by timing them on this system's atoms and neighbour list;
  * the two passes share the lanes per atom and each takes its own entries per
- * step; the choice is kept for the system.  tpa, unroll (may be NULL)
- * receive it (unroll: the density pass's), ms (7 doubles, may be NULL) the
- * density+force time of each candidate
+ * step; the fastest is kept for the system.  tpa, unroll (may be NULL)
+ * receive the best of these candidates (unroll: the density pass's), ms (7
+ * doubles, may be NULL) the density+force time of each
  * (4,1) (8,1) (16,1) (4,2) (8,2) (16,2) (32,1); FP64 systems try the
  * one-entry forms only (the others stay 0).  Single mixed cells also time
  * each candidate with both force-record sources (mappg_sys_force_tables);
- * ms then holds the faster.  No counterpart in the reference. */
+ * ms then holds the faster.  A single mixed cell of at most 32 atoms per SM
+ * starts with a form of 8 lanes and 4 entries, times it beside the candidates
+ * and keeps it where it is the fastest: mappg_sys_tuning has what is in use.
+ * No counterpart in the reference. */
 int mappg_sys_autotune(mappg_sys* sys, int* tpa, int* unroll, double* ms);
 
-/* The kernel shape in use (set by mappg_sys_autotune / mappg_batch_autotune):
- * out[0] lanes per atom, out[1] entries per loop step of the density pass,
- * out[2] of the force pass, out[3] the force pass's shared-memory budget in
- * KB (mappg_sys_force_tables), out[4] atoms per chunk of a batch (0 for one
- * cell).  No counterpart in the reference. */
+/* The kernel shape in use (as created, or kept by mappg_sys_autotune /
+ * mappg_batch_autotune): out[0] lanes per atom, out[1] entries per loop step
+ * of the density pass (1, 2 or 4), out[2] of the force pass, out[3] the force
+ * pass's shared-memory budget in KB (mappg_sys_force_tables), out[4] atoms per
+ * chunk of a batch (0 for one cell).  No counterpart in the reference. */
 int mappg_sys_tuning(mappg_sys* sys, int* out);
 
 /* The mixed force pass's record source: mode 0 reads the force records

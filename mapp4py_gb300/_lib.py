@@ -444,7 +444,9 @@ class System:
         check(load().mappg_sys_sync(self.h))
 
     def autotune(self):
-        """(lanes per atom, entries per step, {(lanes, entries): ms})"""
+        """(lanes per atom, entries per step, {(lanes, entries): ms}) of the
+        best candidate; a small mixed cell may keep four entries per step,
+        which tuning() tells."""
         tpa, unroll = C.c_int(), C.c_int()
         ms = np.zeros(7)
         check(load().mappg_sys_autotune(self.h, C.byref(tpa), C.byref(unroll), dptr(ms)))

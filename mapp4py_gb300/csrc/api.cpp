@@ -52,6 +52,17 @@ void box_min_run(mappg_sys* s, int method, int m, double e_tol, double max_dx, c
 void launch_density_only(mappg_sys* s);
 void launch_force_only(mappg_sys* s);
 
+// a small mixed cell walks four neighbour entries per step, from its creation
+// and as a candidate of its tuning: its lanes wait for memory, not for each
+// other, and one block of 256 threads per SM (32 atoms) leaves the registers
+// for it.  Density + force with one / four: 500 atoms 25.7 / 20.6 us, 4,000
+// 27.8 / 20.8; beyond the line 8,788 30.1 / 30.7, 32,000 49.0 / 77.7.  (Back to
+// back, against the best of the tuner's other candidates, 16 or 32 lanes: 500
+// atoms 14.7 / 11.7, 2,304 15.9 / 14.8, 4,000 16.2 / 16.7, 4,840 16.8 / 17.8;
+// more lanes change the order of an atom's sums.)
+static bool four_entries(const mappg_sys* s) {
+    return s->precision == MAPPG_MIXED && s->ncell == 1 && s->n <= 32 * s->sm_count;
+}
 
 void upload_tables(mappg_ff* ff) {
     HostTables& t = ff->host;
@@ -327,13 +338,7 @@ int mappg_sys_create(const mappg_ff* ff, int natoms, const double* H, const doub
             MAPPG_CUDA(cudaGetDeviceProperties(&p, s->device));
             s->sm_count = p.multiProcessorCount;
             s->smem_optin = (int)p.sharedMemPerBlockOptin;
-            // a small mixed system walks four entries per step until it is
-            // tuned: its lanes wait for memory, not for each other, and one
-            // block of 256 threads per SM (32 atoms) leaves the registers for
-            // it.  Density + force with one / four: 500 atoms 25.7 / 20.6 us,
-            // 4,000 27.8 / 20.8; beyond the line 8,788 30.1 / 30.7, 32,000
-            // 49.0 / 77.7
-            if (precision == MAPPG_MIXED && natoms <= 32 * s->sm_count) s->unroll = 4;
+            if (four_entries(s)) s->unroll = 4;
             // a small FP64 system takes as many lanes per atom as one block
             // of 256 threads per SM has (density + force at 32 / 16 / 8: 500
             // atoms 30.5 / 36.6 / 44.8 us, 2,048 40.9 / 36.2 / 45.2, 4,000
@@ -547,13 +552,16 @@ int mappg_sys_stats(mappg_sys* s, long long* out6) {
 // lanes per atom (atoms per block) and neighbour entries per loop step of
 // the density and force kernels: both passes on the system's own atoms and
 // neighbour list, timed with CUDA events for each candidate; the fastest is
-// kept for the system's later launches
+// kept for the system's later launches.  The four-entry form of a small mixed
+// cell (the one it starts with) is timed beside the candidates that ms_out
+// reports
 int mappg_sys_autotune(mappg_sys* s, int* tpa_out, int* unroll_out, double* ms_out) {
     return guard([&] {
         if (!s) throw Error{MAPPG_ERR_ARG, "null handle"};
         if (s->run) throw Error{MAPPG_ERR_ARG, "an NVT run is in progress"};
         if (!s->built) sys_build(s);
-        const int cand[7][2] = {{4, 1}, {8, 1}, {16, 1}, {4, 2}, {8, 2}, {16, 2}, {32, 1}};
+        constexpr int kCand = 8, kListed = 7;
+        const int cand[kCand][2] = {{4, 1}, {8, 1}, {16, 1}, {4, 2}, {8, 2}, {16, 2}, {32, 1}, {8, 4}};
         // the FP64 kernels have no unrolled form; 32 lanes per atom spread a
         // small system's FP64 work over more of the SMs
         const bool mixed = s->precision == MAPPG_MIXED;
@@ -572,8 +580,8 @@ int mappg_sys_autotune(mappg_sys* s, int* tpa_out, int* unroll_out, double* ms_o
                 if (kb <= mx && kb > modes[nmodes - 1]) modes[nmodes++] = kb;
         }
         const int tpa0 = s->tpa, u0 = s->unroll, uf0 = s->unroll_force, sm0 = s->force_smem;
-        double td[7], tf[7];
-        int tf_mode[7];
+        double td[kCand], tf[kCand];
+        int tf_mode[kCand];
         auto time_ms = [&](auto&& launch) {
             launch();  // warm-up (and first-use set-up)
             MAPPG_CUDA(cudaEventRecord(e0, s->stream));
@@ -585,16 +593,18 @@ int mappg_sys_autotune(mappg_sys* s, int* tpa_out, int* unroll_out, double* ms_o
             return ms / 3.0;
         };
         try {
-            for (int c = 0; c < 7; c++) {
+            for (int c = 0; c < kCand; c++) {
                 td[c] = tf[c] = 0.0;
                 tf_mode[c] = 0;
                 if (!mixed && cand[c][1] != 1) continue;
+                if (c >= kListed && !four_entries(s)) continue;
                 s->tpa = cand[c][0];
                 s->unroll = cand[c][1];
                 s->unroll_force = 0;
                 td[c] = time_ms([&] { launch_density_only(s); });
                 tf[c] = 1e30;
-                for (int mi = 0; mi < nmodes; mi++) {
+                // (the four-entry force pass reads its records through L1)
+                for (int mi = 0; mi < (c < kListed ? nmodes : 1); mi++) {
                     s->force_smem = modes[mi];
                     const double t = time_ms([&] { launch_force_only(s); });
                     if (t < tf[c]) {
@@ -602,7 +612,7 @@ int mappg_sys_autotune(mappg_sys* s, int* tpa_out, int* unroll_out, double* ms_o
                         tf_mode[c] = modes[mi];
                     }
                 }
-                if (ms_out) ms_out[c] = td[c] + tf[c];
+                if (ms_out && c < kListed) ms_out[c] = td[c] + tf[c];
             }
         } catch (...) {
             cudaEventDestroy(e0);
@@ -616,28 +626,29 @@ int mappg_sys_autotune(mappg_sys* s, int* tpa_out, int* unroll_out, double* ms_o
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         // per lanes per atom: the best density unroll plus the best force
-        // unroll and record source
-        double best = 1e30;
-        int best_tpa = tpa0, best_u = u0, best_uf = 0, best_sm = sm0;
-        for (int c = 0; c < 7; c++) {
-            if (td[c] <= 0.0) continue;
-            for (int c2 = 0; c2 < 7; c2++) {
-                if (tf[c2] <= 0.0 || cand[c2][0] != cand[c][0]) continue;
-                if (td[c] + tf[c2] < best) {
-                    best = td[c] + tf[c2];
-                    best_tpa = cand[c][0];
-                    best_u = cand[c][1];
-                    best_uf = cand[c2][1];
-                    best_sm = tf_mode[c2];
+        // unroll and record source, of the first `count` candidates
+        struct Pick {
+            double ms;
+            int tpa, u, uf, sm;
+        };
+        auto pick = [&](int count) {
+            Pick k{1e30, tpa0, u0, 0, sm0};
+            for (int c = 0; c < count; c++) {
+                if (td[c] <= 0.0) continue;
+                for (int c2 = 0; c2 < count; c2++) {
+                    if (tf[c2] <= 0.0 || cand[c2][0] != cand[c][0]) continue;
+                    if (td[c] + tf[c2] < k.ms) k = {td[c] + tf[c2], cand[c][0], cand[c][1], cand[c2][1], tf_mode[c2]};
                 }
             }
-        }
-        s->tpa = best_tpa;
-        s->unroll = best_u;
-        s->unroll_force = best_uf == best_u ? 0 : best_uf;
-        s->force_smem = best_sm;
-        if (tpa_out) *tpa_out = best_tpa;
-        if (unroll_out) *unroll_out = best_u;
+            return k;
+        };
+        const Pick best = pick(kCand), listed = pick(kListed);
+        s->tpa = best.tpa;
+        s->unroll = best.u;
+        s->unroll_force = best.uf == best.u ? 0 : best.uf;
+        s->force_smem = best.sm;
+        if (tpa_out) *tpa_out = listed.tpa;
+        if (unroll_out) *unroll_out = listed.u;
     });
 }
 

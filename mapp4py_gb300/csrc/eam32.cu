@@ -1208,7 +1208,7 @@ static void force_t(mappg_sys* s, const EamArgs& args) {
         launch_dep(s->stream, k_force32s<TPA, ORTHO, U>, s->sm_count, 1024, bytes, a);
         return;
     }
-    if (TPA == 8 && s->unroll == 4 && !s->unroll_force) {
+    if (TPA == 8 && (s->unroll_force ? s->unroll_force : s->unroll) == 4) {
         rows.pair = rows.force = atom_blocks(s, 8);
         launch_dep(s->stream, k_force32<8, ORTHO, 4>, rows.force, 256, 0, a);
         return;
