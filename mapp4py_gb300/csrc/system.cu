@@ -579,30 +579,28 @@ __global__ void __launch_bounds__(kSmallBlock) k_bin_small(const __grid_constant
 }
 
 // a cluster of that many blocks is beyond the portable eight: asked for, and
-// the device asked whether it can run one
+// the current device asked whether it can run one (both hold for one device,
+// so every system asks for its own)
 static bool small_cluster_ok() {
-    static const bool ok = [] {
-        if (cudaFuncSetAttribute(k_bin_small, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(kSmallCluster);
-        cfg.blockDim = dim3(kSmallBlock);
-        cudaLaunchAttribute at;
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = kSmallCluster;
-        at.val.clusterDim.y = at.val.clusterDim.z = 1;
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
-        int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, k_bin_small, &cfg) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        return clusters > 0;
-    }();
-    return ok;
+    if (cudaFuncSetAttribute(k_bin_small, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kSmallCluster);
+    cfg.blockDim = dim3(kSmallBlock);
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = kSmallCluster;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, k_bin_small, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return clusters > 0;
 }
 
 // frame positions of atoms that moved without a rebuild
@@ -1163,7 +1161,7 @@ void launch_rebuild_chain(mappg_sys* s) {
         w.elem = s->elem;
         w.partials = s->partials;
         w.drift_rows = s->drift_rows;
-        small = s->n <= kSmallAtoms && s->nbins <= kSmallBins && small_cluster_ok();
+        small = s->bin_cluster && s->nbins <= kSmallBins;
         if (small)
             launch_dep_cluster(s->stream, k_bin_small, kSmallCluster, kSmallCluster, kSmallBlock, 0, w, s->sc);
         else
@@ -1391,6 +1389,7 @@ static unsigned long long morton3(unsigned a, unsigned b, unsigned c) {
 void sys_alloc(mappg_sys* s, const double* x_host) {
     const int n = s->n;
     MAPPG_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
+    s->bin_cluster = s->ncell == 1 && n <= kSmallAtoms && small_cluster_ok();
     // fixed atom order: Morton order of the initial bins, then caller index
     // (a batch: cell by cell, Morton order within each cell)
     std::vector<unsigned long long> key(n);
