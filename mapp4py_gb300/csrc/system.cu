@@ -694,9 +694,8 @@ constexpr int kBuildWarps = 4;    // warps of a builder block
 constexpr int kBuildWide = 8;     // the same for systems of few bins
 constexpr int kBuildTile = 768;   // candidates staged at a time (12 KB)
 constexpr int kBuildHome = 32;    // atoms of the bin worked on at a time
-constexpr int kBuildRow = 256;    // longest row put together on chip
 constexpr int kBuildAtoms = 4;    // atoms of a warp that test a candidate together
-constexpr int kBuildHits = 160;   // candidates within reach noted per atom
+constexpr int kBuildHits = 160;   // candidates within reach noted per atom, and so the longest row put together on chip
 
 // list thresholds of a pair: kept below lo2, decided in FP64 up to hi2, leading its row below in2
 template <bool UNI>
@@ -805,10 +804,10 @@ __device__ __forceinline__ void build_scan(const BuildArgs& a, const BuildCut<UN
 // (bin step, bin order) order, bin steps c = (d0+1) + 3(d1+1) + 9(d2+1), then
 // those of the skin shell in the reverse of that order: it is put together
 // in shared memory, inner entries from the front and shell entries from the
-// end, and written out in one piece.  Rows longer than kBuildRow, atoms with
-// more than kBuildHits candidates in reach, and bins whose candidates need
-// several tiles go through the candidates directly; the latter's rows are put
-// together in place.  With the inner entries in front, the lanes of an atom
+// end, and written out in one piece.  Atoms with more than kBuildHits candidates
+// in reach, and those of bins whose candidates need several tiles, go through
+// the candidates directly; their rows are put together in place.  With the
+// inner entries in front, the lanes of an atom
 // (slots lane, lane + TPA, ...) get equal shares of the pairs inside the
 // cutoff, and the density pass's lanes reach the shell together.  A batch
 // finds the bin's cell through its first atom (the bins of a cell hold only
@@ -835,7 +834,7 @@ __global__ void __launch_bounds__(32 * W) k_build_bins(const __grid_constant__ B
     if (!sc->rebuild) return;
     __shared__ float4 cand[kBuildTile], home[kBuildHome];
     __shared__ int s_pre[33], s_lo[32], s_cin[kBuildHome], s_cout[kBuildHome], s_geo[6];
-    __shared__ int s_row[W][kBuildRow], s_nh[W][kBuildAtoms];
+    __shared__ int s_row[W][kBuildHits], s_nh[W][kBuildAtoms];
     __shared__ uint16_t s_hits[W][kBuildAtoms][kBuildHits];
     __shared__ float s_cut[UNI ? 1 : 3 * kMaxElem * kMaxElem];
     if (!UNI)
@@ -953,19 +952,16 @@ __global__ void __launch_bounds__(32 * W) k_build_bins(const __grid_constant__ B
                     const int i = entry_j(self);
                     int* row = a.nbr + (size_t)i * a.maxnbr;
                     int cin = 0, cout = 0, tot = 0;
-                    bool chip = false;  // the row is in s_row
-                    if (one_tile && s_nh[w][u] <= kBuildHits) {
+                    const bool chip = one_tile && s_nh[w][u] <= kBuildHits;  // the row is in s_row
+                    if (chip) {
                         build_scan<ORTHO, UNI>(a, cut, cand, s_nh[w][u], s_hits[w][u], h, self, s_geo, h6, cg, s_row[w],
-                                               kBuildRow, cin, cout);
+                                               kBuildHits, cin, cout);
                         tot = cin + cout;
-                        chip = tot <= kBuildRow;
                         __syncwarp();
                         // (of a row that does not fit only the inner entries)
-                        if (chip)
-                            for (int k = lane; k < min(tot <= a.maxnbr ? tot : cin, a.maxnbr); k += 32)
-                                row[k] = s_row[w][k < cin ? k : kBuildRow - tot + k];
-                    }
-                    if (!chip) {
+                        for (int k = lane; k < min(tot <= a.maxnbr ? tot : cin, a.maxnbr); k += 32)
+                            row[k] = s_row[w][k < cin ? k : kBuildHits - tot + k];
+                    } else {
                         if (one_tile)
                             cin = cout = 0;
                         else
@@ -1003,7 +999,7 @@ __global__ void __launch_bounds__(32 * W) k_build_bins(const __grid_constant__ B
                         int no = 0, nx = 0;
                         for (int k0 = 0; k0 < len; k0 += 32) {
                             const int k = k0 + lane;
-                            const int e = k >= len ? 0 : chip ? s_row[w][k < cin ? k : kBuildRow - tot + k] : row[k];
+                            const int e = k >= len ? 0 : chip ? s_row[w][k < cin ? k : kBuildHits - tot + k] : row[k];
                             const bool own = k < len && pair_owned(i, e);
                             const unsigned mo = __ballot_sync(0xffffffffu, own);
                             const unsigned mx = __ballot_sync(0xffffffffu, k < len && !own);
