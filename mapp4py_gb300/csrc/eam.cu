@@ -53,7 +53,7 @@ __device__ __forceinline__ double density64_lane(const EamArgs& a, const Smem64&
         double rsq = dx * dx + dy * dy + dz * dz;
         if (below(rsq, S.cut_sq[ei * a.ne + ej])) {
             double p;
-            const int m = knot64_fast(rsq > 0.0 ? rsq * recip_root(rsq) : 0.0, a.dr_inv, a.nr - 2, p);
+            const int m = knot64_fast(root_from(rsq, recip_root(rsq)), a.dr_inv, a.nr - 2, p);
             acc += spl_val(ldg4(a.rho64 + (size_t)(ej * a.ne + ei * a.rho_ei) * a.nr + m), p);
         }
     }
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(256) k_descriptors(EamArgs a, float* __restric
                 double dx, dy, dz;
                 P.delta(a, S.sh, e, dx, dy, dz);
                 const double rsq = dx * dx + dy * dy + dz * dz;
-                const double rd = rsq > 0.0 ? rsq * recip_root(rsq) : 0.0;
+                const double rd = root_from(rsq, recip_root(rsq));
                 if (below(rsq, S.cut_sq[ei * a.ne + ej])) {
                     double p;
                     const int m = knot64_fast(rd, a.dr_inv, a.nr - 2, p);

@@ -62,7 +62,8 @@ __global__ void __launch_bounds__(256) k_pair64(const __grid_constant__ EamArgs 
             if (below(rsq, S.cut_sq[ei * a.ne + ej])) {
                 const double rinv = recip_root(rsq);
                 double p;
-                const int m = knot64_fast(rsq * rinv, dri, a.nr - 2, p);
+                // (a trial's energy takes r = rsq/r, as those over full rows)
+                const int m = knot64_fast(ENERGY ? rsq * rinv : root_from(rsq, rinv), dri, a.nr - 2, p);
                 if (ENERGY) {
                     rho.x = spl_val(ldg4(a.rho64 + (size_t)(ej * a.ne + ei * a.rho_ei) * a.nr + m), p);
                     rho.y = ej == ei ? rho.x : spl_val(ldg4(a.rho64 + (size_t)(ei * a.ne + ej * a.rho_ei) * a.nr + m), p);
