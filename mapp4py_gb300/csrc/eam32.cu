@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(256) k_density32(EamArgs a) {
         density_atom<TPA, ORTHO, U>(a, S, K, a.fr, i, lane, active, es, ec);
     }
     // the force pass adds the blocks' embedding energies up
-    const Pair32 v[1] = {{es, -ec}};
+    const Sum32 v[1] = {{es, -ec}};
     const double t = block_sums<1>(v);
     if (threadIdx.x == 0) a.partials[blockIdx.x * kRedSlots + 7] = t;
 }
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(1024, 1) k_density32s(EamArgs a) {
         density_atom<TPA, ORTHO, U, Frame, true>(a, S, K, a.fr, i, lane, active, es, ec, stab);
     }
     // the force pass adds the blocks' embedding energies up
-    const Pair32 v[1] = {{es, -ec}};
+    const Sum32 v[1] = {{es, -ec}};
     const double t = block_sums<1>(v);
     if (threadIdx.x == 0) a.partials[blockIdx.x * kRedSlots + 7] = t;
 }
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(256) k_density32b(EamArgs a) {
             const int i = i0 + (int)threadIdx.x / TPA;
             density_atom<TPA, ORTHO, U>(a, S, K, fr, i, lane, i < hi, es, ec);
         }
-        const Pair32 v[1] = {{es, -ec}};
+        const Sum32 v[1] = {{es, -ec}};
         chunk_store<1>(v, a.chunk_part + (size_t)ch * kChunkSlots + 13);
     }
 }
@@ -670,7 +670,7 @@ __device__ __forceinline__ void force_atom(const EamArgs& a, const Smem32& S, co
 // for a fence, a count and the partial sums to come back: with the two of the
 // force call taken together there, 100 MD steps of 4,000 atoms 4.48 -> 4.15 ms
 // (FP64 7.32 -> 7.16), 32,000 8.04 -> 7.73, 50 of 256,000 13.6 -> 13.2
-__device__ __forceinline__ void force_totals32(const Pair32 (&v)[7], const EamArgs& a) {
+__device__ __forceinline__ void force_totals32(const Sum32 (&v)[7], const EamArgs& a) {
     const double t = block_sums<7>(v);
     if (threadIdx.x < 7) a.partials[blockIdx.x * kRedSlots + threadIdx.x] = t;
     if (a.defer) return;
@@ -695,7 +695,7 @@ __global__ void __launch_bounds__(256, U == 4 ? 1 : 4) k_force32(EamArgs a) {
         if (!__any_sync(0xffffffffu, active)) break;
         force_atom<TPA, ORTHO, U>(a, S, K, a.fr, i, lane, active, es, ec, w);
     }
-    const Pair32 v[7] = {{es, -ec}, {w[0], 0.f}, {w[1], 0.f}, {w[2], 0.f}, {w[3], 0.f}, {w[4], 0.f}, {w[5], 0.f}};
+    const Sum32 v[7] = {{es, -ec}, {w[0]}, {w[1]}, {w[2]}, {w[3]}, {w[4]}, {w[5]}};
     force_totals32(v, a);
 }
 
@@ -735,7 +735,7 @@ __global__ void __launch_bounds__(1024, 1) k_force32s(EamArgs a) {
             force_atom<TPA, ORTHO, U, Frame, true>(a, S, K, a.fr, i, lane, active, es, ec, w, ftab_s);
         }
     }
-    const Pair32 v[7] = {{es, -ec}, {w[0], 0.f}, {w[1], 0.f}, {w[2], 0.f}, {w[3], 0.f}, {w[4], 0.f}, {w[5], 0.f}};
+    const Sum32 v[7] = {{es, -ec}, {w[0]}, {w[1]}, {w[2]}, {w[3]}, {w[4]}, {w[5]}};
     force_totals32(v, a);
 }
 
@@ -787,8 +787,8 @@ __global__ void __launch_bounds__(256, 4) k_force32b(EamArgs a) {
             force_atom<TPA, ORTHO, U>(a, S, K, fr, i, lane, i < hi, es, ec, w);
         }
         // halves, as each pair stands in both rows (exact)
-        const Pair32 v[7] = {{0.5f * es, -0.5f * ec}, {0.5f * w[0], 0.f}, {0.5f * w[1], 0.f}, {0.5f * w[2], 0.f},
-                             {0.5f * w[3], 0.f},      {0.5f * w[4], 0.f}, {0.5f * w[5], 0.f}};
+        const Sum32 v[7] = {{0.5f * es, -0.5f * ec}, {0.5f * w[0]}, {0.5f * w[1]}, {0.5f * w[2]},
+                            {0.5f * w[3]}, {0.5f * w[4]}, {0.5f * w[5]}};
         chunk_store<7>(v, a.chunk_part + (size_t)ch * kChunkSlots);
     }
 }
@@ -857,7 +857,7 @@ __global__ void __launch_bounds__(256) k_energy32(EamArgs a) {
         if (!__any_sync(0xffffffffu, active)) break;
         energy_atom<TPA, ORTHO>(a, S, K, a.fr, i, lane, active, es, ec);
     }
-    const Pair32 v[1] = {{es, -ec}};
+    const Sum32 v[1] = {{es, -ec}};
     __shared__ double tot[1];
     if (block_partials<1>(v, a.partials, 0, &a.sc->counter[2])) {
         final_sums<1>(a.partials, gridDim.x, tot);
@@ -886,7 +886,7 @@ __global__ void __launch_bounds__(256) k_energy32b(EamArgs a) {
             const int i = i0 + (int)threadIdx.x / TPA;
             energy_atom<TPA, ORTHO>(a, S, K, fr, i, lane, i < hi, es, ec);
         }
-        const Pair32 v[1] = {{es, -ec}};
+        const Sum32 v[1] = {{es, -ec}};
         chunk_store<1>(v, a.chunk_part + (size_t)ch * kChunkSlots);
     }
 }
@@ -1058,7 +1058,7 @@ __global__ void __launch_bounds__(256) k_de32(EamArgs a) {
         if (!__any_sync(0xffffffffu, active)) break;
         de_atom<TPA, ORTHO>(a, S, K, a.fr, i, lane, active, alpha, es, ec);
     }
-    const Pair32 v[1] = {{es, -ec}};
+    const Sum32 v[1] = {{es, -ec}};
     __shared__ double tot[1];
     if (block_partials<1>(v, a.partials, 0, &a.sc->counter[6])) {
         final_sums<1>(a.partials, gridDim.x, tot);
@@ -1090,7 +1090,7 @@ __global__ void __launch_bounds__(256) k_de32b(EamArgs a) {
             const int i = i0 + (int)threadIdx.x / TPA;
             de_atom<TPA, ORTHO>(a, S, K, fr, i, lane, i < hi, alpha, es, ec);
         }
-        const Pair32 v[1] = {{es, -ec}};
+        const Sum32 v[1] = {{es, -ec}};
         chunk_store<1>(v, a.chunk_part + (size_t)ch * kChunkSlots);
     }
 }

@@ -8,7 +8,7 @@
 // SM held it for ~9 us, as long as the force pass itself on 4,000 atoms.
 // So K values are summed together (warp_sums: the lanes halve the values
 // among themselves, 9 adds instead of 40 for eight values), sums of
-// compensated FP32 pairs stay pairs of FP32 across the warp (Pair32), and
+// compensated FP32 pairs stay in FP32 across the warp (Sum32), and
 // all threads of the last block, not one warp, add up the blocks' partials.
 // Density + force on 256 mixed atoms, where nothing else counts: 49.8 us
 // before, 19.5 us after; 4,000 atoms at eight lanes: 53.3 -> 29.8.
@@ -77,40 +77,47 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
     e = (a - (s - bb)) + (b - bb);
 }
 
-// a sum held as two floats, value s + e: adding two of them keeps the
-// rounding error of every addition in e, so a warp's total of FP32 terms
-// carries what an FP64 sum of them would (to ~2^-47 of its size) in FP32
-// instructions only
-struct Pair32 {
-    float s, e;
+// a sum of FP32 terms held as three floats, value s + e + g: the rounding
+// errors of the additions in s go into e, exactly, and those in e into g, so
+// only g is rounded, about 2^-72 of the terms' size.  The warp's total then
+// carries more than an FP64 sum of the terms would, in FP32 instructions only:
+// 21 an addition, a third of the time of one FP64 addition.  (With two floats,
+// good to 2^-47, runs of 4,000 to 256,000 atoms were 0.4 to 0.9 % faster;
+// converting in the block's first warp alone, not in each warp, made them 1.5
+// % slower.)
+struct Sum32 {
+    float s, e, g;
 };
 
 __device__ __forceinline__ double red_add(double a, double b) { return a + b; }
 __device__ __forceinline__ float red_add(float a, float b) { return a + b; }
-__device__ __forceinline__ Pair32 red_add(Pair32 a, Pair32 b) {
-    Pair32 r;
-    float t;
+__device__ __forceinline__ Sum32 red_add(Sum32 a, Sum32 b) {
+    Sum32 r;
+    float t, u, v, w;
     two_sum(a.s, b.s, r.s, t);
-    r.e = (a.e + b.e) + t;
+    two_sum(a.e, b.e, u, v);
+    two_sum(u, t, r.e, w);
+    r.g = (a.g + b.g) + (v + w);
     return r;
 }
 template <class T>
 __device__ __forceinline__ T red_xor(T v, int o) {
     return __shfl_xor_sync(0xffffffffu, v, o);
 }
-__device__ __forceinline__ Pair32 red_xor(Pair32 v, int o) {
-    return {__shfl_xor_sync(0xffffffffu, v.s, o), __shfl_xor_sync(0xffffffffu, v.e, o)};
+__device__ __forceinline__ Sum32 red_xor(Sum32 v, int o) {
+    return {__shfl_xor_sync(0xffffffffu, v.s, o), __shfl_xor_sync(0xffffffffu, v.e, o),
+            __shfl_xor_sync(0xffffffffu, v.g, o)};
 }
 __device__ __forceinline__ double red_double(double v) { return v; }
 __device__ __forceinline__ double red_double(float v) { return (double)v; }
-__device__ __forceinline__ double red_double(Pair32 v) { return (double)v.s + (double)v.e; }
+__device__ __forceinline__ double red_double(Sum32 v) { return (double)v.s + ((double)v.e + (double)v.g); }
 template <class T>
 __device__ __forceinline__ T red_zero() {
     return T(0);
 }
 template <>
-__device__ __forceinline__ Pair32 red_zero<Pair32>() {
-    return {0.f, 0.f};
+__device__ __forceinline__ Sum32 red_zero<Sum32>() {
+    return {0.f, 0.f, 0.f};
 }
 
 struct RedAdd {
@@ -219,7 +226,7 @@ __device__ __forceinline__ bool last_block(unsigned* counter) {
     return last;
 }
 
-// block-wide sums of K values (double, float, or Pair32: FP32 pairs within a
+// block-wide sums of K values (double, float, or Sum32: three floats within a
 // warp, FP64 across warps and blocks; float values are for quantities whose
 // warp sums need no more than FP32) into
 // partials[blockIdx.x*kRedSlots + slot0 + k]; returns true in the block that
