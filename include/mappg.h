@@ -297,6 +297,22 @@ int mappg_sys_tuning(mappg_sys* sys, int* out);
  * forces are the same in every mode.  No counterpart in the reference. */
 int mappg_sys_force_tables(mappg_sys* sys, int mode, int* active);
 
+/* The FP64 passes of a single cell.  mode 1 computes every pair once and
+ * keeps a record of it between the passes: 76 bytes of device memory per slot
+ * of the neighbour list (slots: atoms x capacity, mappg_sys_stats; 19 times
+ * the list itself), 25 GB for 2,048,000 atoms of 160 slots; fails where that
+ * cannot be allocated.  mode 0 keeps none and walks the full rows (about 2.4
+ * times the time of a pass; the same results to the rounding of another
+ * summation order).  mode -1 only queries.  *active (may be NULL) receives
+ * the mode in use.  A system that was never told takes mode 1 unless it would
+ * need more than 256 MB and more than a quarter of the card's memory or half
+ * of what is free there; whether the last applies can depend on other work on
+ * the card, so a caller who needs the same last bits on every run chooses.
+ * The choice holds for the system's life, the neighbour list is built again
+ * by the next call.  Refused during a begun run.  No counterpart in the
+ * reference. */
+int mappg_sys_pair_records(mappg_sys* sys, int mode, int* active);
+
 /* A batch of cells (mappg_batch_create): the atoms per chunk (128, 256 or
  * 512: the atoms a block of the batch kernels works through before it takes
  * another chunk) together with mappg_sys_autotune's lanes per atom and

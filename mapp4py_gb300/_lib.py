@@ -95,6 +95,7 @@ SIGNATURES = {
                                   C.c_double, C.c_int, _D]),
     "mappg_sys_autotune": (C.c_int, [_VP, _I, _I, _D]),
     "mappg_sys_force_tables": (C.c_int, [_VP, C.c_int, _I]),
+    "mappg_sys_pair_records": (C.c_int, [_VP, C.c_int, _I]),
     "mappg_sys_tuning": (C.c_int, [_VP, _I]),
     "mappg_lbfgs_run_diag": (C.c_int, [_VP, _D, C.c_int, C.c_double, C.c_double, C.c_double, C.c_double,
                                        C.c_double, C.c_double, C.c_int, _D]),
@@ -469,6 +470,14 @@ class System:
         in use."""
         act = C.c_int()
         check(load().mappg_sys_force_tables(self.h, -1 if mode is None else int(mode), C.byref(act)))
+        return act.value
+
+    def pair_records(self, mode=None):
+        """FP64 single cells: 1 computes every pair once and keeps a record of
+        it (76 bytes per list slot), 0 walks the full rows; None only
+        queries.  Returns the mode in use."""
+        act = C.c_int()
+        check(load().mappg_sys_pair_records(self.h, -1 if mode is None else int(mode), C.byref(act)))
         return act.value
 
     def enqueue(self, what):

@@ -29,6 +29,7 @@ void sys_download_async(mappg_sys* s, const double* dev, double* host);
 void nvt_run_xout(mappg_sys* s, double T, double dt, double kB, double t_relax, int L, int niters, int nsteps,
                   double* eta, double* thermo, double* x_out);
 void sys_build(mappg_sys* s);
+void sys_choose_pairs(mappg_sys* s, int choice);
 void sys_neighbors(mappg_sys* s, int* counts, int* entries, long long* total);
 void nvt_run(mappg_sys* s, double T, double dt, double kB, double t_relax, int L, int niters, int nsteps, double* eta,
              double* thermo, const double* Tcell);
@@ -675,6 +676,18 @@ int mappg_sys_force_tables(mappg_sys* s, int mode, int* active) {
             s->force_smem = 0;
         }
         if (active) *active = s->force_smem;
+    });
+}
+
+int mappg_sys_pair_records(mappg_sys* s, int mode, int* active) {
+    return guard([&] {
+        if (!s) throw Error{MAPPG_ERR_ARG, "null handle"};
+        if (mode < -1 || mode > 1) throw Error{MAPPG_ERR_ARG, "mode must be -1, 0 or 1"};
+        if (mode == 1 && (s->precision != MAPPG_FP64 || s->ncell > 1))
+            throw Error{MAPPG_ERR_UNSUPP, "pair records need a single FP64 cell"};
+        if (mode >= 0 && s->run) throw Error{MAPPG_ERR_ARG, "an NVT run is in progress"};
+        if (mode >= 0 && mode != s->pairs_choice) sys_choose_pairs(s, mode);
+        if (active) *active = s->own_ent ? 1 : 0;
     });
 }
 

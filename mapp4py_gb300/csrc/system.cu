@@ -1475,27 +1475,34 @@ void sys_alloc_bins(mappg_sys* s) {
 }
 
 // the lists and records of pair64.cu for rows of maxnbr entries, one
-// allocation of 76 bytes an entry.  Where it would take more than a quarter
-// of the card's free memory, or more slots than 32 bits count, the system
-// keeps the full-row passes
+// allocation of 76 bytes an entry.  Unless the caller has chosen
+// (sys_choose_pairs), a system keeps the full-row passes where it would take
+// more than a quarter of the card's memory, or more than half of what is free
+// (other work on the card then decides which passes run, so only where it
+// would be crowded out), or more slots than 32 bits count
 static void alloc_pairs64(mappg_sys* s) {
     if (s->pair_mem) cudaFree(s->pair_mem);
     s->pair_mem = nullptr;
     s->own_ent = nullptr;
-    if (s->precision != MAPPG_FP64 || s->ncell > 1) return;
+    if (s->precision != MAPPG_FP64 || s->ncell > 1 || s->pairs_choice == 0) return;
+    const bool asked = s->pairs_choice == 1;
     const size_t n = (size_t)s->n, slots = n * s->maxnbr;
     const size_t bytes[] = {48 * slots, 16 * slots, 4 * slots, 4 * slots, 4 * slots, 256 * n, 4 * n, 4 * n};
     size_t at[9] = {0};
     for (int k = 0; k < 8; k++) at[k + 1] = at[k] + (bytes[k] + 255) / 256 * 256;
-    if (slots >= kNoSlot) return;
-    if (at[8] > (size_t)1 << 28) {
+    if (slots >= kNoSlot) {
+        if (asked) throw Error{MAPPG_ERR_UNSUPP, "the list has more slots than pair records can count"};
+        return;
+    }
+    if (!asked && at[8] > (size_t)1 << 28) {
         size_t free_b = 0, total_b = 0;
         MAPPG_CUDA(cudaMemGetInfo(&free_b, &total_b));
-        if (at[8] > free_b / 4) return;
+        if (at[8] > total_b / 4 || at[8] > free_b / 2) return;
     }
     if (cudaMalloc((void**)&s->pair_mem, at[8]) != cudaSuccess) {
         cudaGetLastError();
         s->pair_mem = nullptr;
+        if (asked) throw Error{MAPPG_ERR_CUDA, "no device memory for the pair records"};
         return;
     }
     char* p = s->pair_mem;
@@ -1507,6 +1514,21 @@ static void alloc_pairs64(mappg_sys* s) {
     s->pair_mask = (unsigned*)(p + at[5]);
     s->nown = (int*)(p + at[6]);
     s->nother = (int*)(p + at[7]);
+}
+
+// pair records kept (1) or not (0) from here on; the list is built again by
+// the next call that needs one
+void sys_choose_pairs(mappg_sys* s, int choice) {
+    const int before = s->pairs_choice;
+    s->built = s->list_box = false;
+    s->pairs_choice = choice;
+    try {
+        alloc_pairs64(s);
+    } catch (...) {
+        s->pairs_choice = before;
+        alloc_pairs64(s);
+        throw;
+    }
 }
 
 void sys_alloc_nbr(mappg_sys* s, int maxnbr) {

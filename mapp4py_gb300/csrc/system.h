@@ -315,7 +315,8 @@ struct mappg_sys {
     int* nbr = nullptr;
     int* nnbr = nullptr;
     // FP64 single cells: pairs by owner (pair64.cu); null where the card has
-    // no room for them (the full-row passes then run)
+    // no room for them or the caller wants none (the full-row passes then run)
+    int pairs_choice = -1;  // 0 no, 1 yes, -1 by their size
     int *own_ent = nullptr, *other_ent = nullptr, *nown = nullptr, *nother = nullptr;
     unsigned *other_slot = nullptr, *pair_mask = nullptr;
     double2 *pair_rec = nullptr, *pair_rho = nullptr;
