@@ -887,22 +887,57 @@ struct NvtRun {
     cudaGraphExec_t exec_many = nullptr;
     cudaGraph_t graph_many = nullptr;
     long long many = 0;
+    int alloc_gen = 0;  // of the device arrays that the graphs hold (mappg_sys::alloc_gen)
     int L = 3;
     long long planned = 0;
     long long done = 0;
     bool thermo = false;
 };
 
-static void run_clear(mappg_sys* s) {
-    NvtRun* r = (NvtRun*)s->run;
-    if (!r) return;
+static void run_drop_graphs(NvtRun* r) {
     if (r->exec) cudaGraphExecDestroy(r->exec);
     if (r->graph) cudaGraphDestroy(r->graph);
     if (r->exec_many) cudaGraphExecDestroy(r->exec_many);
     if (r->graph_many) cudaGraphDestroy(r->graph_many);
+    r->exec = r->exec_many = nullptr;
+    r->graph = r->graph_many = nullptr;
+}
+
+static void run_clear(mappg_sys* s) {
+    NvtRun* r = (NvtRun*)s->run;
+    if (!r) return;
+    run_drop_graphs(r);
     delete r;
     s->run = nullptr;
     s->drift_rows = 0;
+}
+
+// the run's step graphs, over the device arrays as they are now
+static void run_capture(mappg_sys* s, NvtRun* r) {
+    run_drop_graphs(r);
+    auto capture = [&](long long k, cudaGraph_t* gr, cudaGraphExec_t* ex) {
+        MAPPG_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+        try {
+            for (long long q = 0; q < k; q++) {
+                if (s->ncell > 1)
+                    launch_step32b(s, r->a);
+                else if (s->precision == MAPPG_MIXED)
+                    launch_step32(s, r->a);
+                else
+                    launch_step64(s, r->a);
+            }
+        } catch (...) {
+            cudaGraph_t g2 = nullptr;
+            cudaStreamEndCapture(s->stream, &g2);
+            if (g2) cudaGraphDestroy(g2);
+            throw;
+        }
+        MAPPG_CUDA(cudaStreamEndCapture(s->stream, gr));
+        MAPPG_CUDA(cudaGraphInstantiate(ex, *gr, 0));
+    };
+    capture(1, &r->graph, &r->exec);
+    if (r->many) capture(r->many, &r->graph_many, &r->exec_many);
+    r->alloc_gen = s->alloc_gen;
 }
 
 void nvt_free(mappg_sys* s) { run_clear(s); }
@@ -978,22 +1013,9 @@ void nvt_begin(mappg_sys* s, double T, double dt, double kB, double t_relax, int
         launch_dep(s->stream, k_mvv_init_b, std::min(s->nchunk, s->sm_count * 8), 256, 0, a);
         launch_dep(s->stream, k_cells_begin, (s->ncell * 32 + 255) / 256, 256, 0, a);
         MAPPG_CUDA(cudaGetLastError());
-        auto capture = [&](long long k, cudaGraph_t* gr, cudaGraphExec_t* ex) {
-            MAPPG_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-            try {
-                for (long long q = 0; q < k; q++) launch_step32b(s, a);
-            } catch (...) {
-                cudaGraph_t g2 = nullptr;
-                cudaStreamEndCapture(s->stream, &g2);
-                if (g2) cudaGraphDestroy(g2);
-                throw;
-            }
-            MAPPG_CUDA(cudaStreamEndCapture(s->stream, gr));
-            MAPPG_CUDA(cudaGraphInstantiate(ex, *gr, 0));
-        };
-        capture(1, &r->graph, &r->exec);
         r->many = std::min(nsteps, kBatchGraphSteps);
-        if (r->many >= kGraphMinSteps) capture(r->many, &r->graph_many, &r->exec_many);
+        if (r->many < kGraphMinSteps) r->many = 0;
+        run_capture(s, r);
         return;
     }
     double eta_h[kMaxChain] = {0};
@@ -1021,20 +1043,7 @@ void nvt_begin(mappg_sys* s, double T, double dt, double kB, double t_relax, int
     launch_dep(s->stream, k_run_begin, 1, 256, 0, a);
     MAPPG_CUDA(cudaGetLastError());
     if (nsteps < kGraphMinSteps) return;  // nvt_steps launches the kernels itself
-    MAPPG_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-    try {
-        if (s->precision == MAPPG_MIXED)
-            launch_step32(s, a);
-        else
-            launch_step64(s, a);
-    } catch (...) {
-        cudaGraph_t g2 = nullptr;
-        cudaStreamEndCapture(s->stream, &g2);
-        if (g2) cudaGraphDestroy(g2);
-        throw;
-    }
-    MAPPG_CUDA(cudaStreamEndCapture(s->stream, &r->graph));
-    MAPPG_CUDA(cudaGraphInstantiate(&r->exec, r->graph, 0));
+    run_capture(s, r);
 }
 
 // enqueue steps (no host synchronisation)
@@ -1042,6 +1051,8 @@ void nvt_steps(mappg_sys* s, long long nsteps) {
     NvtRun* r = (NvtRun*)s->run;
     if (!r) throw Error{MAPPG_ERR_ARG, "no NVT run has begun on this system"};
     if (r->done + nsteps > r->planned) throw Error{MAPPG_ERR_ARG, "more steps than the run was begun with"};
+    // a list build of the caller's between the steps may have moved the rows
+    if (r->exec && r->alloc_gen != s->alloc_gen) run_capture(s, r);
     long long st = 0;
     if (r->exec_many)
         for (; nsteps - st >= r->many; st += r->many) MAPPG_CUDA(cudaGraphLaunch(r->exec_many, s->stream));

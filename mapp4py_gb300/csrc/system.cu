@@ -1465,6 +1465,7 @@ void sys_alloc(mappg_sys* s, const double* x_host) {
 }
 
 void sys_alloc_bins(mappg_sys* s) {
+    s->alloc_gen++;
     if (s->bin_count) cudaFree(s->bin_count);
     if (s->bin_start) cudaFree(s->bin_start);
     s->bin_count = nullptr;
@@ -1532,6 +1533,7 @@ void sys_choose_pairs(mappg_sys* s, int choice) {
 }
 
 void sys_alloc_nbr(mappg_sys* s, int maxnbr) {
+    s->alloc_gen++;
     if (s->nbr) cudaFree(s->nbr);
     s->nbr = nullptr;
     s->maxnbr = maxnbr;

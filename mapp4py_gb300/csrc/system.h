@@ -311,6 +311,7 @@ struct mappg_sys {
     int* bin_tmp = nullptr;      // atoms by bin, any order
     bool bin_cluster = false;    // a small cell whose device can run k_bin_small's cluster
     float4* bin_pos = nullptr;   // by bin in index order: frame position, w = the entry bits of atom and element
+    int alloc_gen = 0;  // counts the allocations of rows and bins, whose addresses step graphs hold
     int maxnbr = 0;
     int* nbr = nullptr;
     int* nnbr = nullptr;

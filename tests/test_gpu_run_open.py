@@ -69,3 +69,36 @@ def test_relaxation_after_an_unfinished_run(potentials, spoiled_memory):
     d = out[1][1] - out[0][1]
     d -= np.round(d @ np.linalg.inv(c.H)) @ c.H
     assert np.max(np.abs(d)) <= 1e-5
+
+
+@pytest.mark.parametrize("precision", [_lib.FP64, _lib.MIXED])
+def test_rows_that_grow_before_the_first_step(potentials, precision):
+    """The rows of a thin gas are short.  A begun run whose atoms are put
+    close together has its rows moved by the build that follows: its step
+    graph is taken again.  The steps are those of a run begun there (FP64 to
+    the trajectory's 1e-10; mixed bits differ in nothing but the frame)."""
+    path, _ = potentials[("A", "B")]
+    c = synth.alloy((5, 5, 5), xB=0.4, sigma=0.05, T=300.0, seed=5)
+    H = np.diag([90.0] * 3)
+    rng = np.random.default_rng(2)
+    thin = rng.random((c.natoms, 3)) @ H
+    close = c.x + 30.0
+    ff = _lib.ForceField.setfl(path)
+    out = []
+    for moved in (False, True):
+        s = _lib.System(ff, H, thin if moved else close, c.elem, c.masses, precision=precision)
+        s.set_v(c.v)
+        if not moved:
+            s.build()
+        cap = s.stats()["capacity"]
+        s.nvt_begin(300.0, synth.FS, synth.KB, 20)
+        if moved:
+            s.set_x(close)
+            s.force()
+            assert s.stats()["capacity"] > cap
+        s.nvt_steps(20)
+        s.nvt_end()
+        out.append((s.get_x(), s.get_v()))
+    tol = 1e-10 if precision == _lib.FP64 else 1e-6
+    for a, b in zip(*out):
+        assert np.max(np.abs(a - b)) <= tol * max(1.0, np.max(np.abs(a)))
