@@ -699,6 +699,7 @@ int mappg_batch_autotune(mappg_sys* s, int* tpa_out, int* unroll_out, int* chunk
     return guard([&] {
         if (!s) throw Error{MAPPG_ERR_ARG, "null handle"};
         if (s->ncell <= 1) throw Error{MAPPG_ERR_ARG, "mappg_batch_autotune takes a batch of cells"};
+        if (s->run) throw Error{MAPPG_ERR_ARG, "an NVT run is in progress"};  // before its chunks are taken away
         const int chunks[3] = {128, 256, 512};
         double best = 1e30;
         int bt = s->tpa, bu = s->unroll, bf = s->unroll_force, bc = s->chunk_atoms;

@@ -102,3 +102,24 @@ def test_rows_that_grow_before_the_first_step(potentials, precision):
     tol = 1e-10 if precision == _lib.FP64 else 1e-6
     for a, b in zip(*out):
         assert np.max(np.abs(a - b)) <= tol * max(1.0, np.max(np.abs(a)))
+
+
+def test_tuning_a_batch_is_refused_in_a_run(potentials):
+    """... and leaves the chunks that the run's graphs walk."""
+    path, _ = potentials[("A", "B")]
+    cs = [synth.alloy(k, xB=0.4, sigma=0.05, T=300.0, seed=3) for k in ((4, 4, 4), (5, 4, 4), (6, 5, 5))]
+    ff = _lib.ForceField.setfl(path)
+    x = []
+    for disturbed in (False, True):
+        b = _lib.Batch(ff, [(c.H, c.x, c.elem) for c in cs], cs[0].masses)
+        b.set_v(np.concatenate([c.v for c in cs]))
+        b.nvt_begin([300.0, 400.0, 500.0], synth.FS, synth.KB, 12)
+        chunk = b.tuning()["atoms_per_chunk"]
+        if disturbed:
+            with pytest.raises(_lib.MappgError):
+                b.autotune()
+        assert b.tuning()["atoms_per_chunk"] == chunk
+        b.nvt_steps(12)
+        b.nvt_end()
+        x.append(b.get_x())
+    assert np.array_equal(x[0], x[1])
