@@ -275,12 +275,13 @@ __device__ __forceinline__ void density_atom(const EamArgs& a, const Smem32& S, 
         // inside the cutoff
         unsigned bits = 0u;
         if constexpr (U == 4) {
+            static_assert(!SM, "small systems read the records through L1");
             // a small system, where a lane's waits are the time: the row
             // slots, positions and records of four entries are each loaded
             // together; the additions keep the order of the one-entry loop
             int t = 0;
             for (int k = lane; k < nn; k += U * TPA, t += U) {
-                int e[U], m[U];
+                int e[U];
                 float4 q[U], c[U];
                 float p[U];
                 bool in[U];
@@ -299,12 +300,8 @@ __device__ __forceinline__ void density_atom(const EamArgs& a, const Smem32& S, 
                     in[u] = rsq < (a.cut_uniform ? cut0 : S.cut_sq[ei * a.ne + ej]) && (u == 0 || k + u * TPA < nn);
                     if (in[u]) {
                         const float r = rsq * inv_sqrt(rsq);
-                        m[u] = knot32(fmaf(r, K.dri, r * K.dri_lo), a.nr - 2, p[u]);
-                        const int ms = m[u] - a.rho_mlo;
-                        if (SM && ms >= 0)
-                            c[u] = stab[(a.rho_ei ? ej * a.ne + ei : ej) * a.rho_w + ms];
-                        else
-                            c[u] = __ldg(a.rho32 + (size_t)(ej * a.ne + ei * a.rho_ei) * a.nr + m[u]);
+                        const int m = knot32(fmaf(r, K.dri, r * K.dri_lo), a.nr - 2, p[u]);
+                        c[u] = __ldg(a.rho32 + (size_t)(ej * a.ne + ei * a.rho_ei) * a.nr + m);
                     }
                 }
 #pragma unroll
@@ -444,6 +441,7 @@ __device__ __forceinline__ void force_atom(const EamArgs& a, const Smem32& S, co
         const int* row = a.nbr + (size_t)i * a.maxnbr;
         const float cut0 = S.cut_sq[0];
         if constexpr (U == 4) {
+            static_assert(!SM, "small systems read the records through L1");
             // one step's entries e[0..cnt-1]: positions and records loaded
             // together, forces added in order.  inside: the entries are known to
             // lie inside the cutoff (set bits of the density pass's mask: the
@@ -470,26 +468,8 @@ __device__ __forceinline__ void force_atom(const EamArgs& a, const Smem32& S, co
                         const float r = rsq * ri[u];
                         const int m = knot32(fmaf(r, K.dri, r * K.dri_lo), a.nr - 2, p[u]);
                         const size_t kt = (size_t)t * a.nr + m;
-                        const int ms = m - a.fs_mlo;
-                        const bool in_smem = SM && ms >= 0 && ms < a.fs_w;
-                        if (in_smem) {
-                            const float4 z = stab[ej * a.fs_w + ms];
-                            const float4 d = stab[(a.ne + ej) * a.fs_w + ms];
-                            r0[u] = make_float4(d.x, d.y, d.z, z.w);
-                            r1[u] = make_float4(z.x, z.y, z.z, d.w);
-                        } else {
-                            ldg8(a.ftab + 2 * kt, r0[u], r1[u]);
-                        }
-                        if (ej != ei) {
-                            if (in_smem) {
-                                // rho'_{g->ej}: with one density function per source
-                                // element it is the group's own rho'_{g->g} record
-                                const int rj = a.rho_ei ? 2 * a.ne + (ej < ei ? ej : ej - 1) : a.ne + ei;
-                                r2[u] = stab[rj * a.fs_w + ms];
-                            } else {
-                                r2[u] = __ldg(a.fjtab + kt);
-                            }
-                        }
+                        ldg8(a.ftab + 2 * kt, r0[u], r1[u]);
+                        if (ej != ei) r2[u] = __ldg(a.fjtab + kt);
                     }
                 }
 #pragma unroll
@@ -524,7 +504,7 @@ __device__ __forceinline__ void force_atom(const EamArgs& a, const Smem32& S, co
                 unsigned bits = __ldg(a.cutmask + (size_t)i * TPA + lane);
                 while (bits) {
                     int e[U];
-                    const int cnt = U == 1 ? 1 : __popc(bits);
+                    const int cnt = __popc(bits);
                     int t = 0;
 #pragma unroll
                     for (int u = 0; u < U; u++) {
@@ -541,7 +521,7 @@ __device__ __forceinline__ void force_atom(const EamArgs& a, const Smem32& S, co
                     int e[U];
 #pragma unroll
                     for (int u = 0; u < U; u++) e[u] = __ldg(row + (u == 0 || k + u * TPA < nn ? k + u * TPA : k));
-                    step(e, U == 1 ? 1 : (nn - k + TPA - 1) / TPA, false);
+                    step(e, (nn - k + TPA - 1) / TPA, false);
                 }
             }
         } else {
