@@ -77,12 +77,15 @@ __device__ __forceinline__ int knot64_fast(double r, double dr_inv, int mmax, do
 // 1/sqrt(x): the FP32 reciprocal root of x as a start (its bits converted by
 // integer instructions: an FP64 conversion holds the FP64 pipe like an
 // addition), then one step of Halley's method, y + y e (1/2 + 3/8 e) with
-// e = 1 - x y^2 (|e| < 2^-21, so the next term is below 2^-64)
+// e = 1 - x y^2 (|e| < 2^-21, so the next term is below 2^-64).  y^2 of an FP32
+// y has 48 bits, so e is as good as exact and the last rounding is the only
+// error: measured 0.5000 ulp at most over 78 million x in 1..41, CUDA's rsqrt
+// 0.5075 (with e from the rounded x y it was 0.996)
 __device__ __forceinline__ double rsqrt_halley(double x) {
     const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
     const unsigned f = __float_as_uint(rsqrtf(__uint_as_float(((hi - 0x38000000u) << 3) | (lo >> 29))));
     const double y = __hiloint2double((int)((f >> 3) + 0x38000000u), (int)(f << 29));
-    const double e = fma(-(x * y), y, 1.0);
+    const double e = fma(-x, y * y, 1.0);
     return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
