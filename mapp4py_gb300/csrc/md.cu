@@ -588,7 +588,8 @@ __global__ void k_cells_begin(MdArgs a) {
     }
 }
 
-// opening half of every cell's chain and its kick factors (open_ahead)
+// opening half of every cell's chain and its kick factors (k_run_begin and
+// CloseStep::open of one cell)
 __global__ void k_cells_open(MdArgs a) {
     dep_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
