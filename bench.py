@@ -37,8 +37,9 @@ KERNELS_PER_STEP = {"fp64": 12, "mixed": 9}
 # how the sums of the pair terms are carried (the line's dtype in words)
 ACCUMULATION = {
     "mixed": "FP32 pair terms; per-atom density, force and pair energy in compensated FP32 (Kahan) "
-             "within a lane, exact FP32 two-sums across an atom's lanes, FP64 per atom and across "
-             "blocks; virial in plain FP32 per thread (a few hundred terms), FP64 across threads",
+             "within a lane, exact FP32 two-sums across an atom's lanes; virial in plain FP32 per "
+             "thread (a few hundred terms); totals in three floats across a warp (2^-72), FP64 "
+             "across warps and blocks",
     "fp64": "FP64 throughout",
 }
 

@@ -301,9 +301,9 @@ int mappg_sys_force_tables(mappg_sys* sys, int mode, int* active);
  * keeps a record of it between the passes: 76 bytes of device memory per slot
  * of the neighbour list (slots: atoms x capacity, mappg_sys_stats; 19 times
  * the list itself), 25 GB for 2,048,000 atoms of 160 slots; fails where that
- * cannot be allocated.  mode 0 keeps none and walks the full rows (about 2.4
- * times the time of a pass; the same results to the rounding of another
- * summation order).  mode -1 only queries.  *active (may be NULL) receives
+ * cannot be allocated.  mode 0 keeps none and walks the full rows (1.4 to
+ * 2 times the time of density and force; the same results to the rounding of
+ * another summation order).  mode -1 only queries.  *active (may be NULL) receives
  * the mode in use.  A system that was never told takes mode 1 unless it would
  * need more than 256 MB and more than a quarter of the card's memory or half
  * of what is free there; whether the last applies can depend on other work on

@@ -56,11 +56,11 @@ void launch_force_only(mappg_sys* s);
 // a small mixed cell walks four neighbour entries per step, from its creation
 // and as a candidate of its tuning: its lanes wait for memory, not for each
 // other, and one block of 256 threads per SM (32 atoms) leaves the registers
-// for it.  Density + force with one / four: 500 atoms 25.7 / 20.6 us, 4,000
-// 27.8 / 20.8; beyond the line 8,788 30.1 / 30.7, 32,000 49.0 / 77.7.  (Back to
-// back, against the best of the tuner's other candidates, 16 or 32 lanes: 500
-// atoms 14.7 / 11.7, 2,304 15.9 / 14.8, 4,000 16.2 / 16.7, 4,840 16.8 / 17.8;
-// more lanes change the order of an atom's sums.)
+// for it.  Density + force as the tuner times them, eight lanes with one / four:
+// 500 atoms 20.3 / 16.8 us, 4,000 22.0 / 18.5; beyond the line 8,788 24.8 / 26.9,
+// 32,000 43.7 / 67.7.  Of its other candidates 16 or 32 lanes are the best: 500
+// atoms 14.7, 4,000 19.5; they change the order of an atom's sums, so a cell
+// takes them only where it is tuned.
 static bool four_entries(const mappg_sys* s) {
     return s->precision == MAPPG_MIXED && s->ncell == 1 && s->n <= 32 * s->sm_count;
 }
@@ -342,10 +342,10 @@ int mappg_sys_create(const mappg_ff* ff, int natoms, const double* H, const doub
             if (four_entries(s)) s->unroll = 4;
             // a small FP64 system takes as many lanes per atom as one block
             // of 256 threads per SM has (density + force at 32 / 16 / 8: 500
-            // atoms 30.5 / 36.6 / 44.8 us, 2,048 40.9 / 36.2 / 45.2, 4,000
-            // 58.8 / 48.6 / 46.2); from two such blocks at eight on, four
-            // lanes share a list more evenly (8 / 4: 16,384 atoms 114.7 /
-            // 109.7, 256,000 1,194 / 1,133)
+            // atoms 26.0 / 30.6 / 40.0 us, 2,048 35.2 / 30.8 / 42.1, 4,000
+            // 54.9 / 43.1 / 42.4); from two such blocks at eight on, four
+            // lanes share a list more evenly (8 / 4: 16,384 atoms 107.6 /
+            // 100.8, 256,000 1,181 / 1,140)
             if (precision == MAPPG_FP64) {
                 const long long block = 256LL * s->sm_count;
                 s->tpa = 32LL * natoms <= block ? 32 : 16LL * natoms <= block ? 16 : 8LL * natoms <= 2 * block ? 8 : 4;

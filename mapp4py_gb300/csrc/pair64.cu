@@ -11,13 +11,15 @@
 //               f = (A + F'_owner B + F'_other C) dx is the force on the owner
 //   k_rho64     rho_i over own and other pairs (one addition each), F, F'
 //   k_gather64  f_i over own and other pairs; the virial over own ones
-// ~35 FP64 operations an entry instead of ~80, and ~1.2 KB written and ~3.5 KB
+// ~37 FP64 operations an entry instead of ~80, and ~1.9 KB written and ~3.7 KB
 // read per atom, which the memory has room for.  An other pair's record lies
 // with its owner; the builder's k_link64 finds the slot once per list.
 // Sums have a fixed order (lane-strided over one list, then the other), no
 // atomics.
-// Density + force at 4,000 atoms 71.5 -> 46.8 us, 256,000 2,610 -> 1,092
-// (k_pair64 727 of it at first, 87 % of the FP64 pipe: what bounds it).
+// Density + force against the full rows: 4,000 atoms 63.2 -> 41.1 us, 16,384
+// 186 -> 100, 256,000 2,255 -> 1,137.  The FP64 pipe bounds them still: of it
+// k_pair64 takes 89 %, k_gather64 89 and k_rho64 80, of DRAM 11, 24 and 36
+// (442,368 atoms).
 #include <math.h>
 
 #include <algorithm>

@@ -813,7 +813,7 @@ __device__ __forceinline__ void build_scan(const BuildArgs& a, const BuildCut<UN
 // finds the bin's cell through its first atom (the bins of a cell hold only
 // that cell's atoms).
 //
-// Bound by instruction issue (69 % of the slots at 500,000 atoms, 774 warp
+// Bound by instruction issue (72 % of the slots at 500,000 atoms, 778 warp
 // instructions an atom).  The atom's counters are uniform in its warp.  With
 // every step of 32 candidates taking the full set of tests the pass had 1,000
 // instructions an atom; the noting step has 14 for one atom, and a candidate
